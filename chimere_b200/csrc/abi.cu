@@ -619,53 +619,59 @@ int chimere_b200_mma_i8_probe(int n_mma, int n_cols, int n_acc, int32_t* d_statu
     return launch_mma_i8_probe(n_mma, n_cols, n_acc, d_status, stream);
 }
 
-// ---------------------------------------------------------------- prefill path ----
+// ---------------------------------------------------------------- grouped GEMM path ----
 namespace {
-constexpr int kGemmMin = 8;           // pairs an expert needs to go to the GEMM (a partly filled tile costs the read-back
-                                      // warps only its own columns; eight tokens on the GEMV kernels cost eight passes of dp4a)
-constexpr size_t kMmaTile = 4096 + 512;
+// Token tiles of a batch: at most P / 128 full ones and one partial one per expert with pairs, and the shared expert's.
 int n_tiles_max_for(const chimere_moe_layer* w, int T) {
     const int P = T * w->top_k;
-    int big = P / kGemmMin; if (big > w->E) big = w->E;
-    return P / 128 + big + (w->F_s > 0 ? (T + 127) / 128 : 0) + 1;
+    return P / 128 + (w->E < P ? w->E : P) + (w->F_s > 0 ? (T + 127) / 128 : 0);
 }
-struct PrefillPlan { size_t gu, down, sh_gu, sh_down, total; int64_t sgu, sdown; int rows_per_tile; };
-PrefillPlan prefill_plan(const chimere_moe_layer* w) {
-    PrefillPlan P{};
-    const bool dual = w->act == CHIMERE_ACT_SWIGLU;
-    P.rows_per_tile = dual ? 64 : 128;
-    const size_t nbH = w->H / 32;
-    P.sgu = (int64_t)((w->F + P.rows_per_tile - 1) / P.rows_per_tile) * nbH * kMmaTile;   // a last, partly filled row tile is zero-padded
-    P.sdown = (int64_t)(w->H / 128) * (w->F / 32) * kMmaTile;
-    size_t o = 0;
-    P.gu = o; o += up256((size_t)P.sgu * w->E);
-    P.down = o; o += up256((size_t)P.sdown * w->E);
-    if (w->F_s > 0) {
-        P.sh_gu = o; o += up256((size_t)((w->F_s + P.rows_per_tile - 1) / P.rows_per_tile) * nbH * kMmaTile);
-        P.sh_down = o; o += up256((size_t)(w->H / 128) * (w->F_s / 32) * kMmaTile);
-    }
-    P.total = o;
-    return P;
+// ... and their columns / 16: a tile of n pairs is at most max(16, 2 n) columns wide.
+int64_t n_col16_max_for(const chimere_moe_layer* w, int T) {
+    const int64_t P = (int64_t)T * w->top_k, E = w->E < P ? w->E : P;
+    const int64_t sh = w->F_s > 0 ? T : 0;
+    return (2 * (P + sh) + 15) / 16 + E + 1;
 }
 int prefill_dims_ok(const chimere_moe_layer* w) {
-    // gated experts: 64 gate rows and their 64 up rows share a tile; ungated ones may end in a partly filled tile
     const int rpt = w->act == CHIMERE_ACT_SWIGLU ? 64 : 32;
     if (w->H % 128 || w->F % rpt || w->F_s % rpt) return 0;
     return 1;
 }
-struct PrefillArena { size_t tiles, bx, b2, total; int64_t bx_stride, b2_stride; int n_tiles_max; };
+struct PrefillArena { size_t tiles, bx, b2, total; int64_t bx_col16, b2_col16; };
 PrefillArena prefill_arena(const chimere_moe_layer* w, int T) {
     PrefillArena A{};
-    A.n_tiles_max = n_tiles_max_for(w, T);
     const int Fmax = w->F > w->F_s ? w->F : w->F_s;
-    A.bx_stride = (int64_t)(w->H / 32) * kMmaTile;
-    A.b2_stride = (int64_t)(Fmax / 32) * kMmaTile;
+    A.bx_col16 = (int64_t)(w->H / 32) * 576;   // 16 columns: 36 bytes per column and block
+    A.b2_col16 = (int64_t)(Fmax / 32) * 576;
+    const int64_t cols = n_col16_max_for(w, T);
     size_t o = 0;
-    A.tiles = o; o += up256((size_t)(8 + 4 * A.n_tiles_max) * 4);
-    A.bx = o; o += up256((size_t)A.n_tiles_max * A.bx_stride);
-    A.b2 = o; o += up256((size_t)A.n_tiles_max * A.b2_stride);
+    A.tiles = o; o += up256((size_t)(8 + 4 * n_tiles_max_for(w, T)) * 4);
+    A.bx = o; o += up256((size_t)(cols * A.bx_col16));
+    A.b2 = o; o += up256((size_t)(cols * A.b2_col16));
     A.total = o;
     return A;
+}
+}  // namespace
+
+// The GEMM reads 4-bit weights in the tiled32 form; only Q8_0 matrices get a copy in the MMA's own order (mma128 tiles; gate
+// and up rows interleaved per 64, so that one output tile holds both).
+namespace {
+struct PrefillPlan { size_t gu, down, sh_gu, sh_down, total; int64_t sgu, sdown, s_sh_gu, s_sh_down; };
+PrefillPlan prefill_plan(const chimere_moe_layer* w) {
+    PrefillPlan P{};
+    const int rpt = w->act == CHIMERE_ACT_SWIGLU ? 64 : 128;
+    auto tiles = [](int rows, int per, int cols) { return (int64_t)((rows + per - 1) / per) * (cols / 32) * (4096 + 512); };
+    P.sgu = w->type_up == CHIMERE_TYPE_Q8_0 ? tiles(w->F, rpt, w->H) : 0;
+    P.sdown = w->type_down == CHIMERE_TYPE_Q8_0 ? tiles(w->H, 128, w->F) : 0;
+    P.s_sh_gu = w->F_s > 0 && w->type_sh_up == CHIMERE_TYPE_Q8_0 ? tiles(w->F_s, rpt, w->H) : 0;
+    P.s_sh_down = w->F_s > 0 && w->type_sh_down == CHIMERE_TYPE_Q8_0 ? tiles(w->H, 128, w->F_s) : 0;
+    size_t o = 256;   // (never empty: the size doubles as the check of the dimensions)
+    P.gu = o; o += up256((size_t)P.sgu * w->E);
+    P.down = o; o += up256((size_t)P.sdown * w->E);
+    P.sh_gu = o; o += up256((size_t)P.s_sh_gu);
+    P.sh_down = o; o += up256((size_t)P.s_sh_down);
+    P.total = o;
+    return P;
 }
 }  // namespace
 
@@ -688,21 +694,24 @@ int chimere_b200_moe_pack_prefill(const chimere_moe_layer* raw, void* d_arena, s
     if (bytes < P.total) return -4;
     const bool dual = raw->act == CHIMERE_ACT_SWIGLU;
     uint8_t* base = (uint8_t*)d_arena;
+    std::memset(out, 0, sizeof(*out));
+    out->rows_per_gu_tile = dual ? 64 : 128;
     cudaError_t e = cudaSuccess;
-    if (raw->F % P.rows_per_tile || raw->F_s % P.rows_per_tile) e = cudaMemsetAsync(base, 0, P.total, stream);   // zero rows and scales behind the last real row
-    if (dual && e == cudaSuccess) e = launch_pack_mma128_ggml(raw->type_gate, raw->gate_exps, base + P.gu, raw->E, raw->F, raw->H, 1, raw->stride_gate, P.sgu, stream);
-    if (e == cudaSuccess) e = launch_pack_mma128_ggml(raw->type_up, raw->up_exps, base + P.gu, raw->E, raw->F, raw->H, dual ? 2 : 0, raw->stride_up, P.sgu, stream);
-    if (e == cudaSuccess) e = launch_pack_mma128_ggml(raw->type_down, raw->down_exps, base + P.down, raw->E, raw->H, raw->F, 0, raw->stride_down, P.sdown, stream);
-    if (raw->F_s > 0) {
-        if (dual && e == cudaSuccess) e = launch_pack_mma128_ggml(raw->type_sh_gate, raw->sh_gate, base + P.sh_gu, 1, raw->F_s, raw->H, 1, 0, 0, stream);
-        if (e == cudaSuccess) e = launch_pack_mma128_ggml(raw->type_sh_up, raw->sh_up, base + P.sh_gu, 1, raw->F_s, raw->H, dual ? 2 : 0, 0, 0, stream);
-        if (e == cudaSuccess) e = launch_pack_mma128_ggml(raw->type_sh_down, raw->sh_down, base + P.sh_down, 1, raw->H, raw->F_s, 0, 0, 0, stream);
+    if (!dual && P.sgu + P.s_sh_gu > 0 && (raw->F % 128 || raw->F_s % 128)) e = cudaMemsetAsync(base, 0, P.total, stream);   // zero rows and scales behind the last real row
+    auto gate_up = [&](const void* gate, const void* up, size_t at, int n, int rows, int64_t sg, int64_t su, int64_t so) {
+        if (dual && e == cudaSuccess) e = launch_pack_mma128_q8_0(gate, base + at, n, rows, raw->H, 1, sg, so, stream);
+        if (e == cudaSuccess) e = launch_pack_mma128_q8_0(up, base + at, n, rows, raw->H, dual ? 2 : 0, su, so, stream);
+    };
+    if (P.sgu) { gate_up(raw->gate_exps, raw->up_exps, P.gu, raw->E, raw->F, raw->stride_gate, raw->stride_up, P.sgu); out->gu_exps = base + P.gu; out->stride_gu = P.sgu; }
+    if (P.sdown) {
+        if (e == cudaSuccess) e = launch_pack_mma128_q8_0(raw->down_exps, base + P.down, raw->E, raw->H, raw->F, 0, raw->stride_down, P.sdown, stream);
+        out->down_exps = base + P.down; out->stride_down = P.sdown;
     }
-    out->gu_exps = base + P.gu; out->stride_gu = P.sgu;
-    out->down_exps = base + P.down; out->stride_down = P.sdown;
-    out->sh_gu = raw->F_s > 0 ? base + P.sh_gu : nullptr;
-    out->sh_down = raw->F_s > 0 ? base + P.sh_down : nullptr;
-    out->rows_per_gu_tile = P.rows_per_tile; out->reserved = 0;
+    if (P.s_sh_gu) { gate_up(raw->sh_gate, raw->sh_up, P.sh_gu, 1, raw->F_s, 0, 0, 0); out->sh_gu = base + P.sh_gu; }
+    if (P.s_sh_down) {
+        if (e == cudaSuccess) e = launch_pack_mma128_q8_0(raw->sh_down, base + P.sh_down, 1, raw->H, raw->F_s, 0, 0, 0, stream);
+        out->sh_down = base + P.sh_down;
+    }
     return cuda_rc(e);
 }
 
@@ -735,73 +744,68 @@ static int kshared_chain(const chimere_moe_layer* w, int T, float* d_y, chimere_
     return cuda_rc(e);
 }
 
-// The expert products of a prefill-size batch whose routing (ws->offsets, ws->perm) and Q8_1 planes (ws->x_q, ws->x_d) are
-// in place: token tiles for the experts with at least kGemmMin pairs (and the shared expert, if any) on the grouped GEMM,
-// the rest on the GEMV kernels; per-pair rows land in ws->pair_out.
-static int prefill_gemms(const chimere_moe_layer* w, const chimere_moe_prefill_weights* pw, int T, chimere_moe_workspace* ws, uint8_t* base,
-                         const PrefillArena& A, int32_t* tiles, int n_tiles_max, cudaStream_t stream);
-static int prefill_experts(const chimere_moe_layer* w, const chimere_moe_prefill_weights* pw, int T, chimere_moe_workspace* ws,
-                           cudaStream_t stream, const void* d_packed = nullptr, int row_bytes = 0) {
-    if (!pw || !ws->prefill_arena) return -1;
+// One launch's view of the layer: where the matrices are and how they are cut into 128-row output tiles.
+static PrefillGemmMats gemm_mats(const chimere_moe_layer* w, const chimere_moe_prefill_weights* pw, bool shared, bool down) {
+    PrefillGemmMats m{};
+    const bool dual = !down && w->act == CHIMERE_ACT_SWIGLU;
+    const int width = shared ? w->F_s : w->F;
+    const void* gate = shared ? w->sh_gate : w->gate_exps;
+    const void* up = shared ? w->sh_up : w->up_exps;
+    const void* dn = shared ? w->sh_down : w->down_exps;
+    m.type = shared ? (down ? w->type_sh_down : w->type_sh_up) : (down ? w->type_down : w->type_up);
+    m.ncols = down ? width : w->H;
+    m.rows32 = (down ? w->H : width) / 32;
+    m.row_tiles = dual ? (m.rows32 + 1) / 2 : (m.rows32 + 3) / 4;
+    m.tile_bytes = m.ncols > 0 ? tiled_matrix_bytes(m.type, 32, m.ncols) : 0;
+    m.w0 = (const uint8_t*)(down ? dn : dual ? gate : up);
+    m.w1 = dual ? (const uint8_t*)up : nullptr;
+    if (m.type == CHIMERE_TYPE_Q8_0) {   // the copy in operand order
+        m.type = kTypeOperand;
+        m.w0 = (const uint8_t*)(pw ? (shared ? (down ? pw->sh_down : pw->sh_gu) : (down ? pw->down_exps : pw->gu_exps)) : nullptr);
+        m.stride0 = pw && !shared ? (down ? pw->stride_down : pw->stride_gu) : 0;
+        m.w1 = nullptr;
+        return m;
+    }
+    if (!shared) { m.stride0 = down ? w->stride_down : dual ? w->stride_gate : w->stride_up; m.stride1 = dual ? w->stride_up : 0; }
+    return m;
+}
+
+// The expert products of a batch whose routing (ws->offsets, ws->perm) and Q8_1 planes (ws->x_q, ws->x_d, or the packed rows
+// of an exchange) are in place: token tiles of every expert with pairs (and of the shared expert; E = 0: of it alone), the
+// gate/up GEMM with the activation and the Q8_1 step, the down GEMM; per-pair rows land in ws->pair_out.
+static int gemm_experts(const chimere_moe_layer* w, const chimere_moe_prefill_weights* pw, int E, int T, chimere_moe_workspace* ws, cudaStream_t stream,
+                        const void* d_packed = nullptr, int row_bytes = 0) {
+    if (!ws->prefill_arena) return -1;
     if (w->layout != CHIMERE_LAYOUT_TILED32 || !prefill_dims_ok(w)) return -2;
     const PrefillArena A = prefill_arena(w, ws->max_T);
     if (ws->prefill_bytes < A.total || ((uintptr_t)ws->prefill_arena & 255)) return -4;
     uint8_t* base = (uint8_t*)ws->prefill_arena;
     int32_t* tiles = (int32_t*)(base + A.tiles);
     const Layout L = make_layout(w, ws->max_T);
-    const int n_tiles_max = n_tiles_max_for(w, T);
-    cudaError_t e = launch_build_tiles(ws->offsets, ws->perm, tiles, ws->group_list, w->E, T, w->top_k, w->F_s > 0, kGemmMin, stream);
+    const int n_tiles_max = E > 0 ? n_tiles_max_for(w, T) : (T + 127) / 128;
+    cudaError_t e = launch_build_tiles(ws->offsets, tiles, E, T, w->F_s > 0, stream);
     if (e != cudaSuccess) return cuda_rc(e);
     // the rows' Q8_1 planes: the workspace's, or (expert-parallel owner) the received packed rows in place
     const int8_t* xq = d_packed ? (const int8_t*)d_packed : ws->x_q;
     const float* xd = d_packed ? (const float*)((const uint8_t*)d_packed + w->H) : ws->x_d;
-    const int64_t xq_stride = d_packed ? row_bytes : w->H;
-    const int xd_stride = d_packed ? row_bytes / 4 : L.x_d_stride;
-    e = launch_gather_tiles(tiles, ws->perm, xq, xq_stride, xd, xd_stride, base + A.bx, A.bx_stride, w->H, w->top_k, n_tiles_max, stream);
+    e = launch_gather_tiles(tiles, ws->perm, xq, d_packed ? row_bytes : w->H, xd, d_packed ? row_bytes / 4 : L.x_d_stride, base + A.bx, A.bx_col16,
+                            w->H, w->top_k, n_tiles_max, stream);
     if (e != cudaSuccess) return cuda_rc(e);
-    // the small experts: GEMV kernels on the rewritten work list, per-pair rows only
-    // (the shared expert is not on this list: the kernels are sized for the routed matrices alone)
-    // every expert on this list has fewer than kGemmMin <= kMaxGroupTokens pairs, i.e. one entry; the grid is sized for that,
-    // not for the worst case of the all-GEMV path
-    static_assert(kGemmMin <= kMaxGroupTokens, "a small expert must fit one work entry");
-    const int max_entries = w->E < T * w->top_k ? w->E : T * w->top_k;
-    GemvParams gu = gate_up_params(w, T, ws, L);
-    gu.nrows_shared = 0; gu.ncols_shared = 0; gu.sh_a = nullptr; gu.sh_b = nullptr;
-    if (d_packed) { gu.in_soa_q = xq; gu.in_soa_q_stride = xq_stride; gu.in_soa_d = xd; gu.in_soa_d_stride = xd_stride; }
-    e = launch_gate_up_tiled(gu, max_entries, stream);
-    if (e != cudaSuccess) return cuda_rc(e);
-    GemvParams dn = down_params(w, nullptr, T, ws, L);
-    dn.no_combine = 1;
-    dn.nrows_shared = 0; dn.ncols_shared = 0; dn.sh_a = nullptr; dn.sh_b = nullptr;
-    e = launch_down_tiled(dn, max_entries, stream);
-    if (e != cudaSuccess) return cuda_rc(e);
-    // the large experts and the shared expert: grouped GEMMs
-    return prefill_gemms(w, pw, T, ws, base, A, tiles, n_tiles_max, stream);
-}
-
-// The two grouped GEMM launches over the token tiles in `tiles` (gate/up with the fused activation and Q8_1 step, then down).
-static int prefill_gemms(const chimere_moe_layer* w, const chimere_moe_prefill_weights* pw, int T, chimere_moe_workspace* ws, uint8_t* base,
-                         const PrefillArena& A, int32_t* tiles, int n_tiles_max, cudaStream_t stream) {
-    cudaError_t e;
     PrefillGemmParams g{};
     g.tiles = tiles; g.perm = ws->perm; g.status = ws->status;
-    g.act = w->act; g.T = T; g.top_k = w->top_k; g.H = w->H;
-    g.a_exps = (const uint8_t*)pw->gu_exps; g.stride_a = pw->stride_gu; g.sh_a = (const uint8_t*)pw->sh_gu;
-    g.b_tiles = base + A.bx; g.b_tile_stride = A.bx_stride;
-    g.out_tiles = base + A.b2; g.out_tile_stride = A.b2_stride;
-    g.row_tiles_routed = (w->F + pw->rows_per_gu_tile - 1) / pw->rows_per_gu_tile;
-    g.row_tiles_shared = (w->F_s + pw->rows_per_gu_tile - 1) / pw->rows_per_gu_tile;
-    g.nblk_routed = w->F / 32; g.nblk_shared = w->F_s / 32;
-    g.row_tiles_max = g.row_tiles_routed > g.row_tiles_shared ? g.row_tiles_routed : g.row_tiles_shared;
-    g.ncols_in = w->H; g.ncols_in_shared = w->H;
-    e = launch_prefill_gemm(g, false, n_tiles_max, stream);
-    if (e != cudaSuccess) return cuda_rc(e);
-    g.a_exps = (const uint8_t*)pw->down_exps; g.stride_a = pw->stride_down; g.sh_a = (const uint8_t*)pw->sh_down;
-    g.b_tiles = base + A.b2; g.b_tile_stride = A.b2_stride;
-    g.out_tiles = nullptr; g.pair_out = ws->pair_out;
-    g.row_tiles_routed = g.row_tiles_shared = g.row_tiles_max = w->H / 128;
-    g.ncols_in = w->F; g.ncols_in_shared = w->F_s;
-    return cuda_rc(launch_prefill_gemm(g, true, n_tiles_max, stream));
+    g.T = T; g.top_k = w->top_k; g.H = w->H;
+    for (int down = 0; down < 2 && e == cudaSuccess; ++down) {
+        g.dual = !down && w->act == CHIMERE_ACT_SWIGLU;
+        g.m[0] = gemm_mats(w, pw, false, down != 0);
+        g.m[1] = gemm_mats(w, pw, true, down != 0);
+        if ((E > 0 && !g.m[0].w0) || (w->F_s > 0 && !g.m[1].w0)) return -1;
+        g.row_tiles_max = g.m[0].row_tiles > g.m[1].row_tiles ? g.m[0].row_tiles : g.m[1].row_tiles;
+        g.b_tiles = base + (down ? A.b2 : A.bx); g.b_col16_bytes = down ? A.b2_col16 : A.bx_col16;
+        g.out_tiles = base + A.b2; g.out_col16_bytes = A.b2_col16;
+        g.pair_out = ws->pair_out;
+        e = launch_prefill_gemm(g, down != 0, n_tiles_max, stream);
+    }
+    return cuda_rc(e);
 }
 
 int chimere_b200_moe_forward_prefill(const chimere_moe_layer* w, const chimere_moe_prefill_weights* pw, const float* d_x, float* d_y,
@@ -814,10 +818,10 @@ int chimere_b200_moe_forward_prefill(const chimere_moe_layer* w, const chimere_m
     const chimere_moe_layer* wr = &wr_;
     if (wr->layout != CHIMERE_LAYOUT_TILED32 || !prefill_dims_ok(wr)) return -2;
     RouteParams rp = route_params(wr, d_x, T, ws, ks);
-    rp.list_mode = 2;   // no work entries from the router: the tile builder writes the list of the small experts
+    rp.list_mode = 2;   // no work entries: the tile builder makes its own list
     cudaError_t e = launch_route(rp, stream);
     if (e != cudaSuccess) return cuda_rc(e);
-    rc = prefill_experts(wr, pw, T, ws, stream);
+    rc = gemm_experts(wr, pw, wr->E, T, ws, stream);
     if (rc) return rc;
     // routing-weighted sum of every token's pair rows in slot order + the sigmoid-gated shared expert
     const float* shared_rows = wr->F_s > 0 ? ws->pair_out + (size_t)T * wr->top_k * wr->H : nullptr;
@@ -839,7 +843,8 @@ int chimere_b200_moe_experts_prefill(const chimere_moe_layer* w_local, const chi
     p.list_mode = 2;
     cudaError_t e = launch_permute(p, stream);
     if (e != cudaSuccess) return cuda_rc(e);
-    return prefill_experts(w_local, pw_local, n_rows, ws, stream);
+    if (!pw_local) return -1;
+    return gemm_experts(w_local, pw_local, w_local->E, n_rows, ws, stream);
 }
 
 // Expert-parallel home rank, prefill-size: the shared expert of this rank's T tokens on the grouped GEMM (token tiles of
@@ -849,20 +854,8 @@ int chimere_b200_moe_shared_expert_prefill(const chimere_moe_layer* w, const chi
     int rc = check_call(w, ws, ws, T, ws);
     if (rc) return rc;
     if (w->F_s <= 0) return 0;
-    if (!pw || !pw->sh_gu || !pw->sh_down || !ws->prefill_arena) return -1;
-    if (w->layout != CHIMERE_LAYOUT_TILED32 || !prefill_dims_ok(w)) return -2;
-    const PrefillArena A = prefill_arena(w, ws->max_T);
-    if (ws->prefill_bytes < A.total || ((uintptr_t)ws->prefill_arena & 255)) return -4;
-    uint8_t* base = (uint8_t*)ws->prefill_arena;
-    int32_t* tiles = (int32_t*)(base + A.tiles);
-    const Layout L = make_layout(w, ws->max_T);
-    const int n_tiles = (T + 127) / 128;
-    // no routed expert gets a tile (E = 0): the list holds the shared expert's token tiles alone
-    cudaError_t e = launch_build_tiles(ws->offsets, ws->perm, tiles, ws->group_list, 0, T, w->top_k, 1, kGemmMin, stream);
-    if (e != cudaSuccess) return cuda_rc(e);
-    e = launch_gather_tiles(tiles, ws->perm, ws->x_q, w->H, ws->x_d, L.x_d_stride, base + A.bx, A.bx_stride, w->H, w->top_k, n_tiles, stream);
-    if (e != cudaSuccess) return cuda_rc(e);
-    return prefill_gemms(w, pw, T, ws, base, A, tiles, n_tiles, stream);
+    if (!pw || !ws->prefill_arena) return -1;
+    return gemm_experts(w, pw, 0, T, ws, stream);   // (no routed expert gets a tile)
 }
 
 // ... with the rows where an exchange left them: packed rows [H int8][d_stride f32][int32 local expert id] (see ep_pack).
@@ -882,7 +875,8 @@ int chimere_b200_moe_experts_packed_prefill(const chimere_moe_layer* w_local, co
     p.idx_stride = row_bytes / 4;
     cudaError_t e = launch_permute(p, stream);
     if (e != cudaSuccess) return cuda_rc(e);
-    return prefill_experts(w_local, pw_local, n_rows, ws, stream, d_rows, row_bytes);
+    if (!pw_local) return -1;
+    return gemm_experts(w_local, pw_local, w_local->E, n_rows, ws, stream, d_rows, row_bytes);
 }
 
 int chimere_b200_moe_ep_pack_sorted(const chimere_moe_layer* w, int T, chimere_moe_workspace* ws, void* d_send, int32_t* d_slot,

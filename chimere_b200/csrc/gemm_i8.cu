@@ -1,5 +1,5 @@
-// gemm_i8.cu -- block-scaled int8 GEMM on the 5th-generation tensor cores (tcgen05, sm_100a), the
-// prefill-size counterpart of the GEMV kernels.
+// gemm_i8.cu -- grouped block-scaled int8 GEMM on the 5th-generation tensor cores (tcgen05, sm_100a): the products of
+// every batch whose experts hold more than a token or two.
 //
 // Math per output element:   D[row][tok] = sum over 32-wide blocks b of
 //                            sa[row][b] * sb[tok][b] * (sum_i A[row][32b+i] * B[tok][32b+i])
@@ -8,43 +8,61 @@
 // kept as an exact int32 per block and scaled in fp32 -- the integer results are bit-identical to the
 // GEMV path; only the order of the fp32 operations differs.
 //
-// Operands come in the "mma128" layout made for the MMA: per (128-row tile, block b) 4096 bytes of int8
-// in the canonical K-major no-swizzle core-matrix order [k half (2)][row group (16)][row (8)][16 bytes]
-// followed by 128 f32 scales.  A plain bulk copy of a (tile, block range) lands MMA-ready in shared
-// memory: shared-memory descriptor with leading (K) byte offset 2048 and stride (row group) byte offset 128.
+// 4-bit weights are read in the tiled32 form the GEMV kernels use (tiled.cuh), so there is one copy of them: they travel
+// packed, and two expander warps turn them into int8 on the way (16 * code for Q4_0, 8 * (2 * code + 1) for IQ3_S, the
+// factor taken out of the scale).  Q8_0 weights come from a copy in the MMA's own order (mma128 tiles), because their
+// tiled32 pieces would have to be copied 512 bytes at a time and a copy costs the issuing warp about 50 cycles.  Token tiles hold up to 128 pairs of one expert in the operand order (gather_tiles_kernel); a tile is
+// 16, 32, 64 or 128 columns wide, whatever its pairs need.
 //
-// CTA = 18 warps, persistent (one CTA per SM), output tiles handed out by an atomic counter:
-//   warp 0  takes the next tile index, publishes it to the other warps through a small ring in shared memory, and
-//           feeds the operand ring with cp.async.bulk;
-//   warp 1  owns TMEM (512 columns = four 128x128 int32 accumulators, used as two pairs) and issues one
-//           tcgen05.mma kind::i8 (M 128, N = the tile's token count rounded up to 16, K 32) per block, never
-//           accumulating across blocks;
-//   warps 2..17 read each block's accumulator back (tcgen05.ld, four warps per TMEM lane quarter, each a quarter of
-//           the tile's token columns), convert, scale and add into fp32 registers (thread = output row), then store
-//           the tile.  The loads of one piece are in flight while the previous piece is processed, and a pair of
-//           accumulators is handed back to the MMA warp as soon as its values are in registers.
-// The read-back is what bounds the kernel: per (row, token, block) one integer add and two fused multiply-adds
-// against 32 tensor-pipe multiply-adds, i.e. about four times the MMA's own time on the CUDA cores.
+// CTA = 24 warps, persistent (one CTA per SM), output tiles (128 weight rows x one token tile) from an atomic counter:
+//   warp 0      takes the next tile, publishes it through a small ring, and feeds the operand rings with cp.async.bulk
+//               (ring 1: packed weights and scales, token block; ring 2: the MMA's A operand);
+//   warp 1      owns TMEM (512 columns) and issues the MMAs, one block = one int32 accumulator, several blocks per slot;
+//   warps 2..3  expand packed weights and their scales;
+//   warps 4..7  take a finished tile's sums from the exchange buffer and store it (activation and Q8_1 step, or pair rows);
+//   warps 8..23 read the accumulators back (four warps per TMEM lane quarter), scale and add into fp32 registers
+//               (thread = weight row), and leave a tile's sums in the exchange buffer.
+// What bounds it.  Wide tiles: the read-back -- every value of every block passes through two fp32 multiply-adds on the
+// CUDA cores against 32 on the tensor pipe.  The int32 -> float conversion costs nothing: each accumulator starts from
+// +524288 (a constant MMA, (-128) * (-128) * 32, in front of the real one; |dot| <= 32 * 127 * 128 < 524288), so its bits are
+// a positive denormal float, value * 2^-149, and the first multiply-add takes the offset and the power of two out again
+// exactly (probe: 715 cycles per 128 x 128 x 32 block with an integer add per value, 597 with the constant MMA).  The
+// three-operand f32x2 multiply-adds themselves take 3.2 cycles per warp (two operand pairs of the three fresh: register ports),
+// i.e. 410 of those cycles.  Narrow tiles: the weight bytes, and what a stage costs its warps however few columns it has
+// (an MMA takes 46 cycles at least, a commit another hundred; the read-back's shares are dealt stage by stage).
 // All waits are bounded; a wait that runs out raises a status bit, nothing blocks for good, and the CTA still
 // frees its TMEM.
 #include "common.cuh"
 #include "kernels.h"
+#include "tiled.cuh"
 
 namespace chimere {
 
-constexpr int kG_TileBytes = 4096 + 512;     // one (128 x 32) int8 block + 128 f32 scales
-constexpr int kG_BlocksPerStage = 4;
-constexpr int kG_Stages = 4;
-constexpr int kG_StageBytes = 2 * kG_BlocksPerStage * kG_TileBytes;   // A blocks then B blocks
-constexpr int kG_EpiWarps = 16;                // four per TMEM lane quarter: each takes a quarter of the tile's token columns
-constexpr int kG_EpiCols = 128 / (kG_EpiWarps / 4);   // columns per read-back warp in a full tile
-constexpr int kG_Threads = 32 * (2 + kG_EpiWarps);
-constexpr int kG_TmemCols = 512;
-constexpr int kG_Sched = 4;                    // tile indices in flight between the scheduler and the other warps
+constexpr int kG_MmaTile = 4096 + 512;       // operand of one block: 128 rows x 32 int8 in the MMA's order, then 128 f32 scales
+constexpr int kG_StageUnits = 4;             // 32-wide blocks per ring stage
+constexpr int kG_RawBytes = 9216;            // packed weights of a stage: 4 row tiles x 4 units x 576 (Q4_0, the largest)
+constexpr int kG_ASlot = kG_StageUnits * kG_MmaTile, kG_ASlots = 3;   // ring 2: the A operand
+constexpr int kG_RingSlotWide = kG_RawBytes + kG_StageUnits * 128 * 36, kG_RingSlotsWide = 3;
+constexpr int kG_RingSlotSlim = kG_RawBytes + kG_StageUnits * 32 * 36, kG_RingSlotsSlim = 6;   // tiles of up to 32 columns
+constexpr int kG_RingBytes = kG_RingSlotWide * kG_RingSlotsWide;
+static_assert(kG_RingSlotSlim * kG_RingSlotsSlim <= kG_RingBytes, "both ring geometries share one area");
+static_assert(kG_RingSlotsWide == kG_ASlots && kG_RingSlotsSlim == 2 * kG_ASlots, "an A slot's last user is found from the ring-1 slot of that stage");
+constexpr int kG_ConstBytes = 4096;          // operand of the constant MMA
+constexpr int kG_XchFloats = 128 * 128;      // exchange buffer [K share][column][128 rows]: 1 x 128, 2 x 64 or 4 x 32 columns
+constexpr int kG_ExpWarps = 2, kG_EpiWarps = 4, kG_RbWarps = 16;
+constexpr int kG_FirstEpi = 4, kG_FirstRb = 8;
+constexpr int kG_Threads = 32 * (kG_FirstRb + kG_RbWarps);
+// Registers: the launch gives every thread 80; the read-back warps take 96 (512 x 96) and leave 48 to the others (256 x 48).
+// (With 80 the read-back spills inside its loop: 1150 cycles per block instead of 700.)
+constexpr int kG_RegsRb = 96, kG_RegsAux = 48;
+static_assert(kG_RbWarps * kG_RegsRb + kG_FirstRb * kG_RegsAux == (kG_RbWarps + kG_FirstRb) * 80, "register shares add up to the launch's total");
+constexpr int kG_TmemCols = 512, kG_TmemSlots = 8;
+constexpr int kG_Sched = 4;                  // tile indices in flight between the scheduler and the other warps
+constexpr size_t kG_Smem = 1024 + kG_ConstBytes + (size_t)kG_RingBytes + kG_ASlots * kG_ASlot + kG_XchFloats * 4;
 
-__device__ __forceinline__ uint64_t smem_desc_kmajor(uint32_t saddr) {
-    // start address (>>4) | leading byte offset 2048 (>>4) << 16 | stride byte offset 128 (>>4) << 32 | version 1 << 46
-    return (uint64_t)((saddr & 0x3FFFFu) >> 4) | ((uint64_t)(2048u >> 4) << 16) | ((uint64_t)(128u >> 4) << 32) | (1ull << 46);
+__device__ __forceinline__ uint64_t smem_desc_kmajor(uint32_t saddr, uint32_t lbo) {
+    // start address (>>4) | leading (K) byte offset (>>4) << 16 | stride (8-row group) byte offset 128 (>>4) << 32 | version 1 << 46
+    return (uint64_t)((saddr & 0x3FFFFu) >> 4) | ((uint64_t)(lbo >> 4) << 16) | ((uint64_t)(128u >> 4) << 32) | (1ull << 46);
 }
 // D format S32 (2 << 4), A and B signed int8 (1 << 7, 1 << 10), both K-major, N (>> 3 at bit 17), M = 128 (>> 4 at bit 24)
 __device__ __forceinline__ uint32_t instr_desc_i8(int n) { return (2u << 4) | (1u << 7) | (1u << 10) | (((uint32_t)n >> 3) << 17) | ((128u >> 4) << 24); }
@@ -54,11 +72,11 @@ __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::
 __device__ __forceinline__ void tc_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
-__device__ __forceinline__ void tc_mma_i8(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc) {
+__device__ __forceinline__ void tc_mma_i8(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
         "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
         "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}"
-        ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(0u), "r"(0u), "r"(0u), "r"(0u), "r"(0u) : "memory");
+        ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(0u), "r"(0u), "r"(0u), "r"(0u) : "memory");
 }
 // TMEM -> registers, thread = lane (row), N consecutive 32-bit columns; no wait: tc_wait_ld() before the values are used
 template <int N> __device__ __forceinline__ void tc_ld_nowait(uint32_t taddr, int (&v)[N]);
@@ -79,195 +97,385 @@ template <> __device__ __forceinline__ void tc_ld_nowait<16>(uint32_t taddr, int
           "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
         : "r"(taddr) : "memory");
 }
-template <> __device__ __forceinline__ void tc_ld_nowait<8>(uint32_t taddr, int (&v)[8]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
-        : "r"(taddr) : "memory");
-}
 __device__ __forceinline__ void tc_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-// int32 -> f32 without the conversion unit: |v| <= 32 * 127 * 128 < 2^22, so v + 0x4B400000 read as a float is
-// 12582912 + v exactly.  The subtraction of 12582912 is folded into the first scaling step (see block_piece).
-constexpr uint32_t kMagicBits = 0x4B400000u;
-constexpr float kMagic = 12582912.0f;
+// two 64-bit words (four floats) from a 32-bit shared address, the same for every lane
+__device__ __forceinline__ void lds_2x64(uint32_t a, uint64_t& x, uint64_t& y) { asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(x), "=l"(y) : "r"(a)); }
+__device__ __forceinline__ float lds_f32(uint32_t a) { float v; asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a)); return v; }
+__device__ __forceinline__ void sts128(uint32_t a, uint4 v) { asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory"); }
+__device__ __forceinline__ void sts_f32(uint32_t a, float v) { asm volatile("st.shared.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory"); }
+
+// The powers of two of the read-back: an accumulator's float reading is (dot + 2^19) * 2^-149.  The first multiply-add takes
+// scale * 2^100 and the offset -2^19 * 2^-149 * (scale * 2^100), and the finished sums are multiplied by 2^49.  All exact;
+// the intermediate sums stay far inside fp32's normal range for any f16 scales.
+constexpr uint32_t kRowScaleBits = 0x71800000u;      // 2^100
+constexpr uint32_t kOffsetBits = 0xB0800000u;        // -2^-30 = -2^19 * 2^-149 * 2^100
+constexpr uint32_t kSumScaleBits = 0x58000000u;      // 2^49
 
 struct GemmShared {
-    uint64_t full[kG_Stages];        // stage bytes have landed
-    uint64_t empty[kG_Stages];       // stage read by the MMAs and by the read-back warps (scales)
-    uint64_t tfull[2];               // the two accumulators of a block pair are complete
-    uint64_t tempty[2];              // ... have been read back
-    uint64_t sfull[kG_Sched];        // a tile index has been published
-    uint64_t sempty[kG_Sched];       // ... and taken by the MMA warp and every read-back warp
-    uint64_t ebar;                   // meeting point of the read-back warps in an epilogue
+    uint64_t full1[kG_RingSlotsSlim];                // ring 1: a stage's bytes have landed (kTypeOperand: those of ring 2 as well)
+    uint64_t empty1[kG_RingSlotsSlim];               // ... the stage has been read back, and both its slots are free
+    uint64_t xfull2[kG_ASlots];                      // ring 2: operand and scales expanded
+    uint64_t tfull[kG_TmemSlots], tempty[kG_TmemSlots];   // accumulators of a slot complete / read back (tempty: wide tiles only)
+    uint64_t sfull[kG_Sched], sempty[kG_Sched];      // a tile index has been published / taken by every other warp
+    uint64_t xfull, xempty;                          // a tile's sums are in the exchange buffer / have been stored
     int sched[kG_Sched];
     uint32_t tmem_base;
     int failed;
 };
 
-// What a CTA works on: its operands (mma128 tiles), the number of K blocks and of valid token columns.
+// One output tile: 128 weight rows (row tile rt of an expert's matrix) x the columns of a token tile.
 struct GemmWork {
-    const uint8_t* a_src; const uint8_t* b_src;
-    int nblocks, n_valid;
-    int aux0, aux1, aux2, aux3;   // policy specific
+    const uint8_t* b;            // token tile: [block][npad * 36 bytes]
+    int nb;                      // 32-wide blocks of K
+    int n_valid, npad;           // token columns / as laid out (16, 32, 64 or 128)
+    int expert, shared, rt, start, col16;
+    int aux0, aux1;
 };
-
-// Policy::work() names tile idx: kWorkOk, kWorkSkip (no such tile, go on) or kWorkEnd (nothing at or after idx).
-// Policy::store<W>() consumes the fp32 accumulators, thread = row; acc[c] belongs to token column part * W + c.
 constexpr int kWorkOk = 0, kWorkSkip = 1, kWorkEnd = 2;
 
-// Meeting point of the read-back warps with a bounded wait (a warp that gave up must not block the others
-// for good).  `phase` counts the meetings of this warp; false if the wait ran out.
-__device__ __forceinline__ bool epilogue_meet(GemmShared& sh, uint32_t& phase, int lane) {
-    __syncwarp();
-    if (lane == 0) mbar_arrive_cta(&sh.ebar);
-    const bool ok = mbar_wait(&sh.ebar, phase & 1u);
-    ++phase;
-    return ok;
+// Position in the two operand rings; every role walks the same sequence.  Ring 1 has two geometries (slots for tiles of
+// more than 32 columns, and more, smaller ones); on a change the producer lets the ring run empty first.
+struct RingPos {
+    int r = 0, e = 0, slim = 0;
+    uint32_t ph1 = 0, ph2 = 0;
+    __device__ __forceinline__ int slots1() const { return slim ? kG_RingSlotsSlim : kG_RingSlotsWide; }
+    __device__ __forceinline__ uint32_t slot1_off() const { return (uint32_t)r * (slim ? kG_RingSlotSlim : kG_RingSlotWide); }
+    __device__ __forceinline__ void geometry(int s) { if (s != slim) { slim = s; r = 0; } }
+    __device__ __forceinline__ uint32_t par1() const { return (ph1 >> r) & 1u; }
+    __device__ __forceinline__ uint32_t par2() const { return (ph2 >> e) & 1u; }
+    // the ring-1 slot of the stage that used A slot e before (three stages ago), and the parity its release completes
+    __device__ __forceinline__ int lag() const { return slim ? (r >= kG_ASlots ? r - kG_ASlots : r + kG_ASlots) : r; }
+    __device__ __forceinline__ uint32_t released(int slot) const { return ((ph1 >> slot) & 1u) ^ 1u; }
+    __device__ __forceinline__ void next(bool expanded) {
+        ph1 ^= 1u << r;
+        if (expanded) ph2 ^= 1u << e;
+        r = r + 1 == slots1() ? 0 : r + 1;
+        e = e + 1 == kG_ASlots ? 0 : e + 1;
+    }
+};
+// TMEM slots of a tile of npad columns (512 columns in all): two blocks per slot in a 128-column tile, else a whole stage.
+struct TmemPos {
+    int slot = 0, npad = 0, nslots = 0;
+    uint32_t ph = 0, ph_empty = 0;   // (ph_empty: the MMA warp's, of the slots that wait for their read-back)
+    __device__ __forceinline__ uint32_t par() const { return (ph >> slot) & 1u; }
+    __device__ __forceinline__ void next() { ph ^= 1u << slot; slot = slot + 1 == nslots ? 0 : slot + 1; }
+};
+__host__ __device__ constexpr int blocks_per_slot(int npad) { return npad == 128 ? 2 : 4; }
+
+// arrival of one thread for `n` of a barrier's count
+__device__ __forceinline__ void mbar_arrive_n(uint64_t* bar, uint32_t n) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(n) : "memory");
+}
+__device__ __forceinline__ void gemm_timeout(GemmShared& sh, int32_t* status, int lane) {
+    if (lane == 0 && status) atomicOr(status, kStatusWaitTimeout);
+    sh.failed = 1;
 }
 
-// two 64-bit words (four floats) from a 32-bit shared address, the same for every lane
-__device__ __forceinline__ void lds_2x64(uint32_t a, uint64_t& x, uint64_t& y) { asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(x), "=l"(y) : "r"(a)); }
-__device__ __forceinline__ float lds_f32(uint32_t a) { float v; asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a)); return v; }
+// ------------------------------------------------------------------ roles ----
+// First unit of stage s.  IQ3_S tiles keep a super-block's scales behind its eight units, so its second half is taken first
+// (one copy brings both) and the expanders keep the scales for the first half.
+__device__ __forceinline__ int stage_unit(int type, int s) { return kG_StageUnits * (type == CHIMERE_TYPE_IQ3_S ? s ^ 1 : s); }
 
-// One piece of one block: CH accumulator columns of this thread's row, already in registers as int32.
-//   acc[c] += (S * sa) * sb[col]      with S * sa = fma(float(S + magic), sa, -magic * sa)
-// The addend of the first step is exact when sa has at most 22 significant bits (every ggml scale is an f16 times
-// a small integer), so the step rounds S * sa once, like a plain multiplication.  sb: shared address of the token
-// scales of the piece's first column (16-byte aligned).
-template <int CH>
-__device__ __forceinline__ void block_piece(const int (&v)[CH], uint64_t sa2, uint32_t sb, uint64_t* acc2) {
-    const uint64_t c2 = mul2(sa2, pack2(__float_as_uint(-kMagic), __float_as_uint(-kMagic)));
+// Warp 0: copies of one tile, a few pieces per stage (a copy costs its warp about 50 cycles, whoever of its lanes asks).
+template <class Policy, class Params>
+__device__ __forceinline__ bool produce_tile(const Params& p, const GemmWork& w, GemmShared& sh, uint8_t* ring1, uint8_t* ring2, RingPos& pos, int lane) {
+    const int type = Policy::type(p, w);
+    const int slim = w.npad <= 32;
+    if (slim != pos.slim) {   // the other slot geometry: every slot of the old one has to be empty first
+        for (int r = 0; r < pos.slots1(); ++r)
+            if (!mbar_wait(&sh.empty1[r], pos.released(r))) { gemm_timeout(sh, p.status, lane); return false; }
+        pos.geometry(slim);
+    }
+    const uint8_t* data = Policy::tile(p, w, lane & 3);
+    const int ntiles = Policy::tiles_valid(p, w);
+    const int nstages = (w.nb + kG_StageUnits - 1) / kG_StageUnits;
+    for (int s = 0; s < nstages; ++s) {
+        const int u0 = stage_unit(type, s), nu = min(kG_StageUnits, w.nb - u0);
+        uint64_t* bar = &sh.full1[pos.r];
+        bool ok = mbar_wait(&sh.empty1[pos.r], pos.released(pos.r));
+        if (ok && type == kTypeOperand) ok = mbar_wait(&sh.empty1[pos.lag()], pos.released(pos.lag()));
+        if (!ok) { gemm_timeout(sh, p.status, lane); return false; }
+        uint8_t* raw = ring1 + pos.slot1_off();
+        const uint32_t bbytes = (uint32_t)(nu * w.npad * 36);
+        // bytes of one row tile (4-bit types), its offset in the matrix and in the slot
+        const uint32_t piece = type == CHIMERE_TYPE_Q4_0 ? (uint32_t)nu * 576u : (s & 1) ? 2048u : 2240u;
+        if (lane == 0) mbar_expect_tx(bar, (type == kTypeOperand ? (uint32_t)(nu * kG_MmaTile) : (uint32_t)ntiles * piece) + bbytes);
+        __syncwarp();
+        if (type == kTypeOperand) {
+            if (lane == 0) bulk_g2s(ring2 + (uint32_t)pos.e * kG_ASlot, data + (size_t)u0 * kG_MmaTile, (uint32_t)(nu * kG_MmaTile), bar);
+        } else if (lane < 4 && data) {
+            const uint32_t off = type == CHIMERE_TYPE_Q4_0 ? (uint32_t)u0 * 576u : (uint32_t)(u0 >> 3) * 4288u + (uint32_t)(u0 & 4) * 512u;
+            bulk_g2s(raw + lane * (kG_RawBytes / 4), data + off, piece, bar);
+        }
+        if (lane == 4) bulk_g2s(raw + kG_RawBytes, w.b + (size_t)u0 * w.npad * 36, bbytes, bar);
+        pos.next(type != kTypeOperand);
+    }
+    return true;
+}
+
+// Packed 4-bit units -> int8 operand rows.  A unit's 16 bytes per row hold elements 0..15 in the low nibbles (code + 8) and
+// 16..31 in the high ones (two's complement): the two halves are the row's 16 bytes of the operand's two K halves.
+// Warp x expands row tiles x and x + 2; the loads of two units' pieces are in flight together (the compiler keeps the order
+// of the shared-memory accesses as written).
+template <int TYPE>
+__device__ __forceinline__ void expand_units(uint32_t raw, uint32_t a, int nu, int x, int lane) {
+    constexpr uint32_t kOdd = TYPE == CHIMERE_TYPE_IQ3_S ? 0x08080808u : 0u;   // 8 * (2c + 1) = 16c + 8
+    constexpr uint32_t kTilePitch = kG_RawBytes / 4, kUnitPitch = TYPE == CHIMERE_TYPE_IQ3_S ? 512 : 576;
+    const uint32_t src = raw + (uint32_t)x * kTilePitch + lane * 16, dst = a + (uint32_t)x * 512 + lane * 16;
 #pragma unroll
-    for (int g = 0; g < CH / 4; ++g) {
+    for (int u = 0; u < kG_StageUnits; u += 2) {
+        if (u >= nu) break;
+        uint4 v[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) v[i] = lds128(src + (i & 1) * 2 * kTilePitch + (u + (i >> 1)) * kUnitPitch);   // (an odd last unit reads bytes nobody uses)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            uint4 lo, hi;
+            lo.x = ((v[i].x << 4) & 0xF0F0F0F0u) ^ (0x80808080u | kOdd); hi.x = (v[i].x & 0xF0F0F0F0u) | kOdd;
+            lo.y = ((v[i].y << 4) & 0xF0F0F0F0u) ^ (0x80808080u | kOdd); hi.y = (v[i].y & 0xF0F0F0F0u) | kOdd;
+            lo.z = ((v[i].z << 4) & 0xF0F0F0F0u) ^ (0x80808080u | kOdd); hi.z = (v[i].z & 0xF0F0F0F0u) | kOdd;
+            lo.w = ((v[i].w << 4) & 0xF0F0F0F0u) ^ (0x80808080u | kOdd); hi.w = (v[i].w & 0xF0F0F0F0u) | kOdd;
+            const uint32_t d = dst + (u + (i >> 1)) * kG_MmaTile + (i & 1) * 1024;
+            sts128(d, lo);
+            sts128(d + 2048, hi);
+        }
+    }
+}
+
+// Warps 2..3: warp x takes row tiles x and x + 2 of every stage.
+template <class Policy, class Params>
+__device__ __forceinline__ bool expand_tile(const Params& p, const GemmWork& w, GemmShared& sh, uint32_t ring1, uint32_t ring2, RingPos& pos, int x, int lane) {
+    const int type = Policy::type(p, w);
+    pos.geometry(w.npad <= 32);
+    const int nstages = (w.nb + kG_StageUnits - 1) / kG_StageUnits;
+    if (type == kTypeOperand) {   // nothing to do but keep step
+        for (int s = 0; s < nstages; ++s) pos.next(false);
+        return true;
+    }
+    float d3[2] = {0.0f, 0.0f};        // IQ3_S: this lane's rows' scales of the super-block, kept over its two stages
+    uint32_t sc3[2] = {0u, 0u};
+    for (int s = 0; s < nstages; ++s) {
+        const int u0 = stage_unit(type, s), nu = min(kG_StageUnits, w.nb - u0);
+        if (!mbar_wait(&sh.full1[pos.r], pos.par1()) || !mbar_wait(&sh.empty1[pos.lag()], pos.released(pos.lag()))) { gemm_timeout(sh, p.status, lane); return false; }
+        const uint32_t raw = ring1 + pos.slot1_off(), a = ring2 + (uint32_t)pos.e * kG_ASlot;
+        const uint32_t rec = a + 4096 + (x * 32 + lane) * 4;   // [unit] kG_MmaTile apart, row tile x + 2: 256 bytes further
+        if (type == CHIMERE_TYPE_Q4_0) {
+            expand_units<CHIMERE_TYPE_Q4_0>(raw, a, nu, x, lane);
+            uint32_t d[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) d[i] = lds16(raw + (x + 2 * (i & 1)) * (kG_RawBytes / 4) + (i >> 1) * 576 + 512 + lane * 2);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) sts_f32(rec + (i >> 1) * kG_MmaTile + (i & 1) * 256, h2f(d[i]) * 0.0625f);
+        } else {
+            expand_units<CHIMERE_TYPE_IQ3_S>(raw, a, nu, x, lane);
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                if (!(s & 1)) {   // the scales came behind these units
+                    const uint32_t t = raw + (x + 2 * h) * (kG_RawBytes / 4) + 2048;
+                    d3[h] = h2f(lds16(t + lane * 2)) * 0.125f;
+                    sc3[h] = lds32(t + 64 + lane * 4);
+                }
+                const uint32_t sc = sc3[h] >> (4 * (u0 & 4));
+#pragma unroll
+                for (int u = 0; u < 4; ++u)   // d * (1 + 2 * sub-scale) is exact in f32
+                    sts_f32(rec + u * kG_MmaTile + h * 256, d3[h] * (float)(1u + 2u * ((sc >> (4 * u)) & 15u)));
+            }
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the MMAs read what ordinary stores wrote
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cta(&sh.xfull2[pos.e]);
+        pos.next(true);
+    }
+    return true;
+}
+
+// Warp 1, lane 0: the MMAs of one tile.  A slim tile's TMEM slots need no barrier of their own: there are more of them than A
+// slots, and an A slot is refilled only after its stage has been read back.
+template <class Policy, class Params>
+__device__ __forceinline__ bool mma_tile(const Params& p, const GemmWork& w, GemmShared& sh, uint32_t cst, uint32_t ring1, uint32_t ring2, uint32_t tmem,
+                                         RingPos& pos, TmemPos& tp) {
+    const bool expanded = Policy::type(p, w) != kTypeOperand;
+    const bool wide = w.npad == 128, handshake = w.npad >= 64;
+    const int npad = w.npad, bps = blocks_per_slot(npad);
+    if (npad != tp.npad) {   // another width lays the accumulators out differently: everything has to be read back first
+        for (int r = 0; r < pos.slots1(); ++r)
+            if (!mbar_wait(&sh.empty1[r], pos.released(r))) { gemm_timeout(sh, p.status, 0); return false; }
+        tp.npad = npad; tp.slot = 0; tp.nslots = kG_TmemCols / (bps * npad);
+    }
+    pos.geometry(npad <= 32);
+    const uint32_t idesc = instr_desc_i8(npad), lbo_b = (uint32_t)npad * 16u, bstep = (uint32_t)(npad * 36) >> 4;
+    const uint64_t ca = smem_desc_kmajor(cst, 2048), cb = smem_desc_kmajor(cst, lbo_b);
+    const uint64_t a_base = smem_desc_kmajor(ring2, 2048), b_base = smem_desc_kmajor(ring1 + kG_RawBytes, lbo_b);
+    const int nstages = (w.nb + kG_StageUnits - 1) / kG_StageUnits;
+    for (int s = 0; s < nstages; ++s) {
+        const int nu = min(kG_StageUnits, w.nb - s * kG_StageUnits);
+        if (!(expanded ? mbar_wait(&sh.xfull2[pos.e], pos.par2()) : mbar_wait(&sh.full1[pos.r], pos.par1()))) { gemm_timeout(sh, p.status, 0); return false; }
+        const uint64_t a = a_base + (uint32_t)pos.e * (kG_ASlot >> 4), b = b_base + (pos.slot1_off() >> 4);
+#pragma unroll
+        for (int j = 0; j < kG_StageUnits; ++j) {
+            if (j >= nu) break;
+            const int js = wide ? j & 1 : j;   // block within the slot
+            if (js == 0) {
+                if (handshake) {
+                    if (!mbar_wait(&sh.tempty[tp.slot], ((tp.ph_empty >> tp.slot) & 1u) ^ 1u)) { gemm_timeout(sh, p.status, 0); return false; }
+                    tp.ph_empty ^= 1u << tp.slot;
+                }
+                tc_fence_after();
+            }
+            const uint32_t d = tmem + (uint32_t)((tp.slot * bps + js) * npad);
+            if (wide) tc_mma_i8(d, ca, cb, idesc, 0u);
+            tc_mma_i8(d, a + (uint32_t)j * (kG_MmaTile >> 4), b + (uint32_t)j * bstep, idesc, wide ? 1u : 0u);
+            if (j == nu - 1 || (wide && js == 1)) {   // (also tells the read-back warps that the operands have been read)
+                tc_commit(&sh.tfull[tp.slot]);
+                tp.next();
+            }
+        }
+        pos.next(expanded);
+    }
+    return true;
+}
+
+// W accumulator columns of this thread's row: acc[c] += (dot * sa) * sb[c] with dot * sa = fma(reading, sa, offset * sa),
+// rounded once like a plain product.  sb: shared address of the first column's token scale.
+template <int W, uint32_t kBias>
+__device__ __forceinline__ void block_values(const int (&v)[W], float sa, uint32_t sb, uint64_t* acc2) {
+    const float sr = sa * __uint_as_float(kRowScaleBits), c = sa * __uint_as_float(kOffsetBits);
+    const uint64_t sa2 = pack2f(sr, sr);
+    const uint64_t c2 = pack2f(c, c);
+#pragma unroll
+    for (int g = 0; g < W / 4; ++g) {
         uint64_t s01, s23;
         lds_2x64(sb + 16u * g, s01, s23);
-        const uint64_t u01 = fma2(pack2((uint32_t)v[4 * g + 0] + kMagicBits, (uint32_t)v[4 * g + 1] + kMagicBits), sa2, c2);
-        const uint64_t u23 = fma2(pack2((uint32_t)v[4 * g + 2] + kMagicBits, (uint32_t)v[4 * g + 3] + kMagicBits), sa2, c2);
+        const uint64_t u01 = fma2(pack2((uint32_t)v[4 * g + 0] + kBias, (uint32_t)v[4 * g + 1] + kBias), sa2, c2);
+        const uint64_t u23 = fma2(pack2((uint32_t)v[4 * g + 2] + kBias, (uint32_t)v[4 * g + 3] + kBias), sa2, c2);
         acc2[2 * g + 0] = fma2(u01, s01, acc2[2 * g + 0]);
         acc2[2 * g + 1] = fma2(u23, s23, acc2[2 * g + 1]);
     }
 }
 
-// The read-back of one output tile by one warp: W = CH * NCH token columns per warp, taken in pieces of CH columns.
-// Blocks come in pairs (never across a ring stage): one wait per pair, and the pair's TMEM buffers are handed back as
-// soon as their values are in registers.  The load of a piece is in flight while the piece before it is processed
-// (two register sets in turn); the last piece of a pair is processed under the first load of the next pair.
-template <int CH, int NCH>
-__device__ __forceinline__ bool readback_tile(GemmShared& sh, uint32_t smem_base, uint32_t tmem, int32_t* status, int nblocks, int q, int part,
-                                              int lane, uint32_t& sg, uint32_t& bg, uint64_t* acc2) {
-    constexpr int W = CH * NCH;
-    constexpr int kLast = (NCH - 1) * CH;        // first column of a block's last piece
-    const uint32_t row4 = (uint32_t)(q * 32 + lane) * 4u, col4 = (uint32_t)(part * W) * 4u;
-    const uint32_t trow = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(part * W);
-    int va[CH], vb[CH];                          // pieces with an even / odd number within their pair
-    uint64_t p_sa2 = 0; uint32_t p_sb = 0;       // scales of the piece waiting in vb
-    bool have = false;
-    int release_st = -1;                         // ring stage whose scales the waiting piece still needs
-    bool ok = true;
-    for (int blk = 0; blk < nblocks; ++bg) {
-        const int s = blk / kG_BlocksPerStage, j0 = blk - s * kG_BlocksPerStage;
-        const int st = (int)((sg + (uint32_t)s) % kG_Stages);
-        const int nb_stage = min(kG_BlocksPerStage, nblocks - s * kG_BlocksPerStage);
-        const int npair = min(2, nb_stage - j0);
-        const int pr = (int)(bg & 1u), tph = (int)((bg >> 1) & 1u);
-        if (!mbar_wait(&sh.tfull[pr], (uint32_t)tph)) { if (status) atomicOr(status, kStatusWaitTimeout); sh.failed = 1; ok = false; break; }
-        tc_fence_after();
-        // shared addresses of block j0's row scales (this thread's row) and token scales (this warp's first column)
-        const uint32_t a_sc = smem_base + (uint32_t)(st * kG_StageBytes + j0 * kG_TileBytes + 4096) + row4;
-        const uint32_t sb_0 = smem_base + (uint32_t)(st * kG_StageBytes + (kG_BlocksPerStage + j0) * kG_TileBytes + 4096) + col4;
-        const float sa_0 = lds_f32(a_sc);
-        const uint64_t sa2_0 = pack2(__float_as_uint(sa_0), __float_as_uint(sa_0));
-        const uint32_t t0 = trow + (uint32_t)((2 * pr) * 128);
-        if (npair == 2) {
-            const float sa_1 = lds_f32(a_sc + kG_TileBytes);
-            const uint64_t sa2_1 = pack2(__float_as_uint(sa_1), __float_as_uint(sa_1));
-            const uint32_t sb_1 = sb_0 + kG_TileBytes;
-#pragma unroll
-            for (int k = 0; k < 2 * NCH; ++k) {
-                const int h = k / NCH, c = k % NCH;
-                const uint32_t ta = t0 + (uint32_t)(h * 128 + c * CH);
-                if ((k & 1) == 0) tc_ld_nowait<CH>(ta, va); else tc_ld_nowait<CH>(ta, vb);
-                if (k == 0) {
-                    if (have) {
-                        block_piece<CH>(vb, p_sa2, p_sb, acc2 + kLast / 2);
-                        if (release_st >= 0) { __syncwarp(); if (lane == 0) mbar_arrive_cta(&sh.empty[release_st]); release_st = -1; }
-                    }
-                } else {
-                    const int hp = (k - 1) / NCH, cp = (k - 1) % NCH;
-                    if (((k - 1) & 1) == 0) block_piece<CH>(va, hp ? sa2_1 : sa2_0, (hp ? sb_1 : sb_0) + 4u * cp * CH, acc2 + cp * CH / 2);
-                    else block_piece<CH>(vb, hp ? sa2_1 : sa2_0, (hp ? sb_1 : sb_0) + 4u * cp * CH, acc2 + cp * CH / 2);
-                }
-                tc_wait_ld();
-            }
-            p_sa2 = sa2_1; p_sb = sb_1 + 4u * kLast; have = true;   // piece 2 * NCH - 1 waits in vb
+// The read-back of one tile by one warp: column group colg of W columns; in tiles of up to 64 columns the warps of a column
+// group also share the stages among them (KG shares, stage s to share s % KG), so that a warp has that much longer for the
+// latency of one stage (barrier, TMEM load, scales: about a thousand cycles).
+template <int COLG, int KG, int W>
+__device__ __forceinline__ bool readback_tile(GemmShared& sh, uint32_t ring1, uint32_t ring2, uint32_t tmem, int32_t* status, int nb, bool expanded, int q,
+                                              int part, int lane, RingPos& pos, TmemPos& tp, uint64_t* acc2) {
+    constexpr int kPad = COLG * W, kBps = blocks_per_slot(kPad);
+    constexpr bool kHandshake = kPad >= 64;
+    const int colg = part % COLG, kg = part / COLG;
+    if (tp.npad != kPad) { tp.npad = kPad; tp.slot = 0; tp.nslots = kG_TmemCols / (kBps * kPad); }
+    const uint32_t trow = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(colg * W);
+    const uint32_t rec0 = ring2 + 4096 + (uint32_t)(q * 32 + lane) * 4u;
+    const uint32_t sb0 = ring1 + kG_RawBytes + kPad * 32 + colg * (W * 4);
+    int share = 0;
+    for (int b0 = 0; b0 < nb; b0 += kG_StageUnits) {
+        const int nu = min(kG_StageUnits, nb - b0);
+        if (KG > 1 && share != kg) {   // another share's stage: keep step
+            // a barrier's phases are told apart by parity, so nobody may be a whole round of slots ahead: everyone waits for
+            // a tile's last stage (the stages between are never further behind than a warp's own last one)
+            if (nu == nb - b0 && !mbar_wait(&sh.tfull[tp.slot], tp.par())) { gemm_timeout(sh, status, lane); return false; }
+            tp.next();
         } else {
-            // an odd last block: no partner to overlap with
-            if (have) {
-                block_piece<CH>(vb, p_sa2, p_sb, acc2 + kLast / 2);
-                if (release_st >= 0) { __syncwarp(); if (lane == 0) mbar_arrive_cta(&sh.empty[release_st]); release_st = -1; }
-                have = false;
-            }
+            const uint32_t rec = rec0 + (uint32_t)pos.e * kG_ASlot, sb = sb0 + pos.slot1_off();
 #pragma unroll
-            for (int c = 0; c < NCH; ++c) {
-                tc_ld_nowait<CH>(t0 + (uint32_t)(c * CH), va);
-                tc_wait_ld();
-                block_piece<CH>(va, sa2_0, sb_0 + 4u * c * CH, acc2 + c * CH / 2);
+            for (int j0 = 0; j0 < kG_StageUnits; j0 += kBps) {
+                if (j0 >= nu) break;
+                if (!mbar_wait(&sh.tfull[tp.slot], tp.par())) { gemm_timeout(sh, status, lane); return false; }
+                tc_fence_after();
+                const uint32_t t0 = trow + (uint32_t)(tp.slot * (kBps * kPad));
+                const int cnt = min(kBps, nu - j0);
+#pragma unroll
+                for (int i = 0; i < kBps; ++i) {
+                    if (i < cnt) {
+                        int v[W];
+                        tc_ld_nowait<W>(t0 + (uint32_t)(i * kPad), v);
+                        const float sa = lds_f32(rec + (j0 + i) * kG_MmaTile);
+                        tc_wait_ld();
+                        if (kHandshake && i + 1 == cnt) {   // the slot's last values are in registers: the MMAs may overwrite it
+                            tc_fence_before();
+                            __syncwarp();
+                            if (lane == 0) mbar_arrive_n(&sh.tempty[tp.slot], KG);
+                        }
+                        block_values<W, kPad == 128 ? 0u : 1u << 19>(v, sa, sb + (uint32_t)((j0 + i) * (kPad * 36)), acc2);
+                    }
+                }
+                tp.next();
             }
+            if (!kHandshake) tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_n(&sh.empty1[pos.r], KG);
         }
-        // every value of the pair is in registers: the MMA warp may overwrite its two accumulators
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive_cta(&sh.tempty[pr]);
-        blk += npair;
-        if (j0 + npair == nb_stage) {   // the stage's scales are needed until the waiting piece has been processed
-            if (have) release_st = st;
-            else if (lane == 0) mbar_arrive_cta(&sh.empty[st]);
-        }
+        if (KG > 1) share = share + 1 == KG ? 0 : share + 1;
+        pos.next(expanded);
     }
-    if (ok && have) block_piece<CH>(vb, p_sa2, p_sb, acc2 + kLast / 2);
-    if (release_st >= 0) { __syncwarp(); if (lane == 0) mbar_arrive_cta(&sh.empty[release_st]); }
-    sg += (uint32_t)((nblocks + kG_BlocksPerStage - 1) / kG_BlocksPerStage);
-    return ok;
+    return true;
 }
 
-// One output tile by one read-back warp: accumulate over the blocks, then hand the sums to the policy's store.
-template <class Policy, class Params, int CH, int NCH>
-__device__ __forceinline__ bool readback_and_store(const Params& p, int idx, GemmShared& sh, uint32_t smem_base, uint8_t* xch, uint32_t tmem, int q,
-                                                   int part, int lane, uint32_t& sg, uint32_t& bg, uint32_t& ephase) {
-    constexpr int W = CH * NCH;
-    GemmWork item;
-    Policy::work(p, idx, item);
+// One output tile by one read-back warp: sums over its blocks, then into the exchange buffer.
+template <class Policy, class Params, int COLG, int KG, int W>
+__device__ __forceinline__ bool readback(const Params& p, const GemmWork& w, GemmShared& sh, uint32_t ring1, uint32_t ring2, float* xch, uint32_t tmem, int q,
+                                         int part, int lane, RingPos& pos, TmemPos& tp, uint32_t& xphase) {
+    pos.geometry(COLG * W <= 32);
     uint64_t acc2[W / 2];
 #pragma unroll
     for (int i = 0; i < W / 2; ++i) acc2[i] = 0ull;
-    const bool ok = readback_tile<CH, NCH>(sh, smem_base, tmem, p.status, item.nblocks, q, part, lane, sg, bg, acc2);
-    float acc[W];
+    bool ok = readback_tile<COLG, KG, W>(sh, ring1, ring2, tmem, p.status, w.nb, Policy::type(p, w) != kTypeOperand, q, part, lane, pos, tp, acc2);
+    if (!mbar_wait(&sh.xempty, (xphase & 1u) ^ 1u)) { gemm_timeout(sh, p.status, lane); ok = false; }   // the tile before has been stored
+    ++xphase;
+    float* mine = xch + part * (W * 128) + q * 32 + lane;   // (part = share * COLG + column group)
+    const uint64_t sc2 = pack2(kSumScaleBits, kSumScaleBits);
 #pragma unroll
-    for (int i = 0; i < W / 2; ++i) unpack2(acc2[i], acc[2 * i], acc[2 * i + 1]);
-    Policy::work(p, idx, item);   // named again here rather than kept in registers through the read-back
-    Policy::template store<W>(p, item, q * 32 + lane, q, part, lane, acc, xch, sh, ephase, ok);
+    for (int i = 0; i < W / 2; ++i) unpack2(mul2(acc2[i], sc2), mine[(2 * i) * 128], mine[(2 * i + 1) * 128]);
+    __syncwarp();
+    if (lane == 0) mbar_arrive_cta(&sh.xfull);
     return ok;
 }
-template <class Policy, class Params, int CH, int NCH>
-__device__ __noinline__ bool readback_and_store_call(const Params& p, int idx, GemmShared& sh, uint32_t smem_base, uint8_t* xch, uint32_t tmem, int q,
-                                                     int part, int lane, uint32_t& sg, uint32_t& bg, uint32_t& ephase) {
-    return readback_and_store<Policy, Params, CH, NCH>(p, idx, sh, smem_base, xch, tmem, q, part, lane, sg, bg, ephase);
+
+// Warps 4..7: what happens to a tile's sums, while the read-back warps are at the next tile.
+template <class Policy, class Params>
+__device__ __forceinline__ bool store_tile(const Params& p, const GemmWork& w, GemmShared& sh, const float* xch, int ew, int lane, uint32_t& xphase) {
+    const bool ok = mbar_wait(&sh.xfull, xphase & 1u);
+    ++xphase;
+    if (!ok) { gemm_timeout(sh, p.status, lane); return false; }
+    if (w.npad == 128) Policy::template store<1>(p, w, xch, ew, lane);
+    else if (w.npad == 64) Policy::template store<2>(p, w, xch, ew, lane);
+    else Policy::template store<4>(p, w, xch, ew, lane);
+    __syncwarp();
+    if (lane == 0) mbar_arrive_cta(&sh.xempty);
+    return true;
+}
+
+// The next tile of the schedule ring, for every warp but the scheduler's own; negative: no more (or a wait ran out).
+__device__ __forceinline__ int take_tile(GemmShared& sh, int32_t* status, uint32_t& tn, int lane) {
+    const int slot = (int)(tn % kG_Sched);
+    if (!mbar_wait(&sh.sfull[slot], (tn / kG_Sched) & 1u)) { gemm_timeout(sh, status, lane); return -1; }
+    const int idx = *reinterpret_cast<volatile int*>(&sh.sched[slot]);
+    __syncwarp();
+    if (lane == 0) mbar_arrive_cta(&sh.sempty[slot]);
+    ++tn;
+    return idx;
 }
 
 template <class Policy, class Params>
 __global__ void __launch_bounds__(kG_Threads, 1) gemm_i8_kernel(const Params p, int32_t* tile_counter) {
-    extern __shared__ __align__(1024) uint8_t smem[];
+    extern __shared__ uint8_t smem_raw[];
     __shared__ GemmShared sh;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+    uint8_t* ring1 = smem + kG_ConstBytes;
+    uint8_t* ring2 = ring1 + kG_RingBytes;
+    float* xch = reinterpret_cast<float*>(ring2 + kG_ASlots * kG_ASlot);
 
     if (tid == 0) {
-        for (int i = 0; i < kG_Stages; ++i) { mbar_init(&sh.full[i], 1); mbar_init(&sh.empty[i], 1 + kG_EpiWarps); }
-        for (int i = 0; i < 2; ++i) { mbar_init(&sh.tfull[i], 1); mbar_init(&sh.tempty[i], kG_EpiWarps); }
-        for (int i = 0; i < kG_Sched; ++i) { mbar_init(&sh.sfull[i], 1); mbar_init(&sh.sempty[i], 1 + kG_EpiWarps); }
-        mbar_init(&sh.ebar, kG_EpiWarps);
+        for (int i = 0; i < kG_RingSlotsSlim; ++i) { mbar_init(&sh.full1[i], 1); mbar_init(&sh.empty1[i], kG_RbWarps); }
+        for (int i = 0; i < kG_ASlots; ++i) { mbar_init(&sh.xfull2[i], kG_ExpWarps); }
+        for (int i = 0; i < kG_TmemSlots; ++i) { mbar_init(&sh.tfull[i], 1); mbar_init(&sh.tempty[i], kG_RbWarps); }
+        for (int i = 0; i < kG_Sched; ++i) { mbar_init(&sh.sfull[i], 1); mbar_init(&sh.sempty[i], 1 + kG_ExpWarps + kG_EpiWarps + kG_RbWarps); }
+        mbar_init(&sh.xfull, kG_RbWarps); mbar_init(&sh.xempty, kG_EpiWarps);
         sh.failed = 0;
         mbar_fence_init();
     }
+    for (int i = tid; i < kG_ConstBytes / 4; i += kG_Threads) reinterpret_cast<uint32_t*>(smem)[i] = 0x80808080u;   // int8 -128
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&sh.tmem_base)), "r"(kG_TmemCols) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -276,88 +484,73 @@ __global__ void __launch_bounds__(kG_Threads, 1) gemm_i8_kernel(const Params p, 
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = sh.tmem_base;
+    griddep_wait();                        // (the set-up above may run while the kernel that fills the operands finishes)
+    if (tid == 0) griddep_launch();
 
-    if (warp == 0) {
-        // ------------------------------ tile scheduler + operand producer ------------------------------
-        if (lane == 0) {
-            uint32_t sg = 0, tn = 0;   // ring stages issued / tile indices published so far
-            bool ok = true;
-            while (ok) {
-                // next tile (heavy tiles have the low indices); a skipped index costs one more atomic
-                GemmWork item;
-                int idx, ws;
-                do { idx = atomicAdd(tile_counter, 1); ws = Policy::work(p, idx, item); } while (ws == kWorkSkip);
-                const int slot = (int)(tn % kG_Sched), sph = (int)((tn / kG_Sched) & 1u);
-                if (!mbar_wait(&sh.sempty[slot], (uint32_t)(sph ^ 1))) { atomicOr(p.status, kStatusWaitTimeout); sh.failed = 1; break; }
-                sh.sched[slot] = ws == kWorkEnd ? -1 : idx;
-                mbar_arrive_cta(&sh.sfull[slot]);   // (release: the index is visible to whoever sees the arrival)
-                ++tn;
-                if (ws == kWorkEnd) break;
-                const int nstages = (item.nblocks + kG_BlocksPerStage - 1) / kG_BlocksPerStage;
-                for (int s = 0; s < nstages; ++s, ++sg) {
-                    const int st = (int)(sg % kG_Stages), ph = (int)((sg / kG_Stages) & 1u);
-                    if (!mbar_wait(&sh.empty[st], (uint32_t)(ph ^ 1))) { atomicOr(p.status, kStatusWaitTimeout); sh.failed = 1; ok = false; break; }
-                    const int b0 = s * kG_BlocksPerStage, nb = min(kG_BlocksPerStage, item.nblocks - b0);
-                    uint8_t* dst = smem + (size_t)st * kG_StageBytes;
-                    const uint32_t bytes = (uint32_t)nb * kG_TileBytes;
-                    mbar_expect_tx(&sh.full[st], 2 * bytes);
-                    bulk_g2s(dst, item.a_src + (size_t)b0 * kG_TileBytes, bytes, &sh.full[st]);
-                    bulk_g2s(dst + kG_BlocksPerStage * kG_TileBytes, item.b_src + (size_t)b0 * kG_TileBytes, bytes, &sh.full[st]);
-                }
+    // The read-back warps and the others take separate paths from here on, each with its own share of the registers.
+    if (warp >= kG_FirstRb) {
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kG_RegsRb));
+        const int q = warp & 3, part = (warp - kG_FirstRb) >> 2;   // TMEM lane quarter this warp may read; its share of columns and stages
+        RingPos pos;
+        TmemPos tp;
+        uint32_t tn = 0, xphase = 0;
+        int idx;
+        bool ok = true;
+        while (ok && (idx = take_tile(sh, p.status, tn, lane)) >= 0) {
+            GemmWork w;
+            Policy::work(p, idx, w);
+            const uint32_t r1 = smem_u32(ring1), r2 = smem_u32(ring2);
+            switch (w.npad) {
+                case 128: ok = readback<Policy, Params, 4, 1, 32>(p, w, sh, r1, r2, xch, tmem, q, part, lane, pos, tp, xphase); break;
+                case 64: ok = readback<Policy, Params, 2, 2, 32>(p, w, sh, r1, r2, xch, tmem, q, part, lane, pos, tp, xphase); break;
+                case 32: ok = readback<Policy, Params, 1, 4, 32>(p, w, sh, r1, r2, xch, tmem, q, part, lane, pos, tp, xphase); break;
+                default: ok = readback<Policy, Params, 1, 4, 16>(p, w, sh, r1, r2, xch, tmem, q, part, lane, pos, tp, xphase); break;
             }
         }
     } else {
-        // ------------------------------ MMA issuer (warp 1) and read-back warps (2..17) ------------------------------
-        const int q = warp & 3;                      // TMEM lane quarter a read-back warp may read
-        const int part = (warp - 2) >> 2;            // which share of the token columns
-        uint32_t sg = 0, bg = 0, tn = 0, ephase = 0; // ring stages / block pairs / tiles / epilogue meetings so far
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kG_RegsAux));
+        RingPos pos;
+        uint32_t tn = 0;
         bool ok = true;
-        while (ok) {
-            const int slot = (int)(tn % kG_Sched), sph = (int)((tn / kG_Sched) & 1u);
-            if (!mbar_wait(&sh.sfull[slot], (uint32_t)sph)) { if (lane == 0) atomicOr(p.status, kStatusWaitTimeout); sh.failed = 1; break; }
-            const int idx = *reinterpret_cast<volatile int*>(&sh.sched[slot]);
-            __syncwarp();
-            if (lane == 0) mbar_arrive_cta(&sh.sempty[slot]);
-            ++tn;
-            if (idx < 0) break;
-            GemmWork item;
-            Policy::work(p, idx, item);
-            const int nblocks = item.nblocks;
-            if (warp == 1) {
+        if (warp == 0) {
+            // ------------------------------ tile scheduler + operand producer ------------------------------
+            while (ok) {
+                GemmWork w;
+                int idx = 0, ws;
+                do {   // a skipped index costs one more atomic
+                    if (lane == 0) idx = atomicAdd(tile_counter, 1);
+                    idx = __shfl_sync(0xffffffffu, idx, 0);
+                    ws = Policy::work(p, idx, w);
+                } while (ws == kWorkSkip);
+                const int slot = (int)(tn % kG_Sched);
+                if (!mbar_wait(&sh.sempty[slot], ((tn / kG_Sched) & 1u) ^ 1u)) { gemm_timeout(sh, p.status, lane); ok = false; break; }
                 if (lane == 0) {
-                    const int n_mma = min(128, max(16, (item.n_valid + 15) & ~15));
-                    const uint32_t idesc = instr_desc_i8(n_mma);
-                    const int nstages = (nblocks + kG_BlocksPerStage - 1) / kG_BlocksPerStage;
-                    for (int s = 0; s < nstages && ok; ++s, ++sg) {
-                        const int st = (int)(sg % kG_Stages), ph = (int)((sg / kG_Stages) & 1u);
-                        if (!mbar_wait(&sh.full[st], (uint32_t)ph)) { atomicOr(p.status, kStatusWaitTimeout); sh.failed = 1; ok = false; break; }
-                        tc_fence_after();
-                        const int nb = min(kG_BlocksPerStage, nblocks - s * kG_BlocksPerStage);
-                        const uint32_t sa = smem_u32(smem + (size_t)st * kG_StageBytes);
-                        const uint32_t sb = sa + kG_BlocksPerStage * kG_TileBytes;
-                        // two blocks per hand-over: accumulator pair bg & 1 = TMEM buffers 2 * (bg & 1) and + 1
-                        for (int j = 0; j < nb; j += 2, ++bg) {
-                            const int pr = (int)(bg & 1u), tph = (int)((bg >> 1) & 1u);
-                            if (!mbar_wait(&sh.tempty[pr], (uint32_t)(tph ^ 1))) { atomicOr(p.status, kStatusWaitTimeout); sh.failed = 1; ok = false; break; }
-                            tc_fence_after();
-                            tc_mma_i8(tmem + (2 * pr) * 128, smem_desc_kmajor(sa + j * kG_TileBytes), smem_desc_kmajor(sb + j * kG_TileBytes), idesc);
-                            if (j + 1 < nb)
-                                tc_mma_i8(tmem + (2 * pr + 1) * 128, smem_desc_kmajor(sa + (j + 1) * kG_TileBytes), smem_desc_kmajor(sb + (j + 1) * kG_TileBytes), idesc);
-                            tc_commit(&sh.tfull[pr]);        // both accumulators ready when these MMAs have finished
-                        }
-                        if (ok) tc_commit(&sh.empty[st]);    // ... and the stage's int8 data is no longer needed
-                    }
+                    sh.sched[slot] = ws == kWorkEnd ? -1 : idx;
+                    mbar_arrive_cta(&sh.sfull[slot]);   // (release: the index is visible to whoever sees the arrival)
                 }
-                ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
-                continue;
+                ++tn;
+                if (ws == kWorkEnd) break;
+                ok = produce_tile<Policy>(p, w, sh, ring1, ring2, pos, lane);
             }
-            // ---- read-back: thread = output row; the narrower the tile, the fewer columns per warp ----
-            // (full tiles inline; the narrower classes are calls, so that they do not weigh on the registers of this loop)
-            const int n_valid = item.n_valid;
-            uint8_t* xch = smem + (size_t)kG_Stages * kG_StageBytes;
-            if (n_valid > 64) ok = readback_and_store<Policy, Params, 8, 4>(p, idx, sh, smem_u32(smem), xch, tmem, q, part, lane, sg, bg, ephase);
-            else if (n_valid > 32) ok = readback_and_store_call<Policy, Params, 8, 2>(p, idx, sh, smem_u32(smem), xch, tmem, q, part, lane, sg, bg, ephase);
-            else ok = readback_and_store_call<Policy, Params, 8, 1>(p, idx, sh, smem_u32(smem), xch, tmem, q, part, lane, sg, bg, ephase);
+            if (!ok)   // a wait ran out: the copies already asked for have to land before this CTA's memory goes away
+                for (int r = 0; r < pos.slots1(); ++r) mbar_wait(&sh.full1[r], pos.released(r));
+        } else {
+            TmemPos tp;
+            uint32_t xphase = 0;
+            int idx;
+            while (ok && (idx = take_tile(sh, p.status, tn, lane)) >= 0) {
+                GemmWork w;
+                Policy::work(p, idx, w);
+                const uint32_t r1 = smem_u32(ring1), r2 = smem_u32(ring2);
+                if (warp == 1) {
+                    if (lane == 0) ok = mma_tile<Policy>(p, w, sh, smem_u32(smem), r1, r2, tmem, pos, tp);
+                    ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+                } else if (warp < kG_FirstEpi) {
+                    ok = expand_tile<Policy>(p, w, sh, r1, r2, pos, warp - 2, lane);
+                } else {
+                    ok = store_tile<Policy>(p, w, sh, xch, warp - kG_FirstEpi, lane, xphase);
+                }
+            }
         }
     }
 
@@ -369,118 +562,140 @@ __global__ void __launch_bounds__(kG_Threads, 1) gemm_i8_kernel(const Params p, 
     }
 }
 
-// plain fp32 tile store: out[(row0 + r) * ldo + col0 + c] = D[r][c]  (the primitive)
+// ------------------------------------------------------------------ policies ----
+// plain fp32 tile store: out[(row0 + r) * ldo + col0 + c] = D[r][c]  (the primitive; operands in the mma128 form)
 struct PlainPolicy {
     __device__ static __forceinline__ int work(const GemmParams& p, int idx, GemmWork& w) {
         if (idx >= p.n_items) return kWorkEnd;
         const GemmItem it = p.items[idx];
-        w.a_src = p.a_base + it.a_offset; w.b_src = p.b_base + it.b_offset;
-        w.nblocks = p.nblocks; w.n_valid = it.n_valid;
-        w.aux0 = it.rows_valid; w.aux1 = it.out_row0; w.aux2 = it.out_col0; w.aux3 = 0;
+        w.b = p.b_base + it.b_offset;
+        w.nb = p.nblocks; w.n_valid = it.n_valid; w.npad = 128;
+        w.expert = idx; w.shared = 0; w.rt = it.rows_valid; w.start = 0; w.col16 = 0;
+        w.aux0 = it.out_row0; w.aux1 = it.out_col0;
         return kWorkOk;
     }
-    template <int W>
-    __device__ static __forceinline__ void store(const GemmParams& p, const GemmWork& w, int row, int, int part, int,
-                                                 const float (&acc)[W], uint8_t*, GemmShared&, uint32_t&, bool ok) {
-        if (!ok || row >= w.aux0) return;
-        float* out = p.out + (size_t)(w.aux1 + row) * p.ldo + w.aux2 + part * W;
-#pragma unroll
-        for (int c = 0; c < W; ++c)
-            if (part * W + c < w.n_valid) out[c] = acc[c];
+    __device__ static __forceinline__ int type(const GemmParams&, const GemmWork&) { return kTypeOperand; }
+    __device__ static __forceinline__ int tiles_valid(const GemmParams&, const GemmWork&) { return 4; }
+    __device__ static __forceinline__ const uint8_t* tile(const GemmParams& p, const GemmWork& w, int) { return p.a_base + p.items[w.expert].a_offset; }
+    template <int KG>
+    __device__ static __forceinline__ void store(const GemmParams& p, const GemmWork& w, const float* xch, int ew, int lane) {
+        for (int r = ew; r < w.rt; r += kG_EpiWarps)   // (all tiles of the primitive are 128 columns wide: one share)
+            for (int c = lane; c < w.n_valid; c += 32) p.out[(size_t)(w.aux0 + r) * p.ldo + w.aux1 + c] = xch[c * 128 + r];
     }
 };
 
-// ------------------------------------------------------------------ MoE prefill policies ----
-// Token tiles (built on the device after routing): {expert (-1 = shared expert), start, n_valid, 0}; word 0 of the
-// list = number of tiles, words 4 and 5 = the tile counters of the two GEMM launches (zero when the list is built).
-// Routed tile: pairs perm[start .. start + n_valid); shared tile: tokens start .. .
+// Token tiles (built on the device after routing): {expert (-1 = shared expert), start, pairs, first column / 16}; word 0 of
+// the list = number of tiles, words 4 and 5 = the tile counters of the two GEMM launches (zero when the list is built).
+// Routed tile: pairs perm[start .. start + n); shared tile: tokens start .. .  A tile of n pairs is tile_width(n) columns wide.
 constexpr int kTileHeader = 8;
+__device__ __forceinline__ int tile_width(int n) { return n <= 16 ? 16 : n <= 32 ? 32 : n <= 64 ? 64 : 128; }
 
-// gate/up: A tile = 64 gate rows | 64 up rows of the same 64 intermediate rows (or 128 up rows when there is no
-// gate).  The halves meet in shared memory; the activation is quantised to Q8_1 (32 consecutive rows = one warp)
-// straight into the down GEMM's token tile.
-struct GateUpPolicy {
+// What the gate/up and the down launch share: the tile list and where a row tile's weights are.
+struct MoePolicy {
     __device__ static __forceinline__ int work(const PrefillGemmParams& p, int idx, GemmWork& w) {
-        const int n_tiles = __ldcg(p.tiles);
         const int j = idx / p.row_tiles_max, rt = idx - j * p.row_tiles_max;
-        if (j >= n_tiles) return kWorkEnd;
+        if (j >= __ldcg(p.tiles)) return kWorkEnd;
         const int4 t = __ldcg(reinterpret_cast<const int4*>(p.tiles + kTileHeader) + j);
-        const bool shared = t.x < 0;
-        const int row_tiles = shared ? p.row_tiles_shared : p.row_tiles_routed;
-        if (rt >= row_tiles) return kWorkSkip;
-        const int nb = p.ncols_in / 32;
-        w.a_src = (shared ? p.sh_a : p.a_exps + (size_t)t.x * p.stride_a) + (size_t)rt * nb * kG_TileBytes;
-        w.b_src = p.b_tiles + (size_t)j * p.b_tile_stride;
-        w.nblocks = nb; w.n_valid = t.z;
-        w.aux0 = j; w.aux1 = rt; w.aux2 = shared ? 1 : 0; w.aux3 = t.y;
+        w.shared = t.x < 0 ? 1 : 0;
+        const PrefillGemmMats& m = p.m[w.shared];
+        if (rt >= m.row_tiles) return kWorkSkip;
+        w.expert = t.x < 0 ? 0 : t.x;
+        w.nb = m.ncols >> 5; w.n_valid = t.z; w.npad = tile_width(t.z);
+        w.rt = rt; w.start = t.y; w.col16 = t.w;
+        w.b = p.b_tiles + (size_t)t.w * p.b_col16_bytes;
+        w.aux0 = w.aux1 = 0;
         return kWorkOk;
     }
-    template <int W>
-    __device__ static __forceinline__ void store(const PrefillGemmParams& p, const GemmWork& w, int row, int q, int part, int lane,
-                                                 float (&acc)[W], uint8_t* smem, GemmShared& sh, uint32_t& ephase, bool ok) {
-        const bool dual = p.act == CHIMERE_ACT_SWIGLU;
-        float* xch = reinterpret_cast<float*>(smem);   // [128][129] floats behind the ring
-        // every read-back warp is done with the previous tile's exchange
-        if (!epilogue_meet(sh, ephase, lane) && lane == 0) atomicOr(p.status, kStatusWaitTimeout);
+    __device__ static __forceinline__ int type(const PrefillGemmParams& p, const GemmWork& w) { return p.m[w.shared].type; }
+    // gated: two 32-row tiles of the gate matrix, then the same two of the up matrix; else four of the one matrix
+    __device__ static __forceinline__ int tiles_valid(const PrefillGemmParams& p, const GemmWork& w) {
+        const int n = p.m[w.shared].rows32;
+        return p.dual ? 2 * min(2, n - 2 * w.rt) : min(4, n - 4 * w.rt);
+    }
+    __device__ static __forceinline__ const uint8_t* tile(const PrefillGemmParams& p, const GemmWork& w, int t) {
+        const PrefillGemmMats& m = p.m[w.shared];
+        if (m.type == kTypeOperand) return m.w0 + (size_t)w.expert * m.stride0 + (size_t)w.rt * w.nb * kG_MmaTile;
+        const int i = p.dual ? 2 * w.rt + (t & 1) : 4 * w.rt + t;
+        if (i >= m.rows32) return nullptr;
+        const bool second = p.dual && t >= 2;
+        return (second ? m.w1 + (size_t)w.expert * m.stride1 : m.w0 + (size_t)w.expert * m.stride0) + (size_t)i * m.tile_bytes;
+    }
+};
+
+// sums of the K shares, shares in order
+template <int KG>
+__device__ __forceinline__ float xch_sum(const float* xch, int npad, int row, int c) {
+    float v = xch[c * 128 + row];
 #pragma unroll
-        for (int c = 0; c < W; ++c) xch[row * 129 + part * W + c] = acc[c];
-        if (!epilogue_meet(sh, ephase, lane) && lane == 0) atomicOr(p.status, kStatusWaitTimeout);
-        if (!ok) return;
-        // units of work: (32-row block of the intermediate, token column); a warp takes a unit at a time, lane = row
-        const int nrb = dual ? 2 : 4;
-        const int ew = (part << 2) | q;                  // this warp's number among the read-back warps
-        const int nblk_limit = w.aux2 ? p.nblk_shared : p.nblk_routed;
-        const int khalf = lane >> 4, kin = lane & 15;
-        for (int u = ew; u < nrb * w.n_valid; u += kG_EpiWarps) {
-            const int rb = u % nrb, c = u / nrb;
-            const int blk = (dual ? w.aux1 * 2 : w.aux1 * 4) + rb;
-            if (blk >= nblk_limit) continue;             // rows of zero padding behind the last real row
-            const int r = rb * 32 + lane;
-            const float a = xch[r * 129 + c];
-            float v;
-            if (dual) v = silu_mul_ref(a, xch[(r + 64) * 129 + c]);
-            else { const float t = fmaxf(a, 0.0f); v = t * t; }
-            float amax = fabsf(v);
+    for (int k = 1; k < KG; ++k) v += xch[(k * npad + c) * 128 + row];
+    return v;
+}
+
+// gate/up: A tile = 64 gate rows | 64 up rows of the same 64 intermediate rows (or 128 up rows when there is no gate).  The
+// activation is quantised to Q8_1 (32 consecutive rows = one warp) straight into the down GEMM's token tile.  A warp takes
+// a 32-row block of the intermediate and every second or every column of the tile, two columns at a time so that the
+// divisions of one hide the other's.
+struct GateUpPolicy : MoePolicy {
+    template <int KG>
+    __device__ static __forceinline__ void store(const PrefillGemmParams& p, const GemmWork& w, const float* xch, int ew, int lane) {
+        const int nrb = p.dual ? 2 : 4, rb = ew & (nrb - 1), blk = w.rt * nrb + rb;
+        if (blk >= p.m[w.shared].rows32) return;     // (the last row tile may be partly filled)
+        const int cstep = kG_EpiWarps / nrb, r = rb * 32 + lane;
+        uint8_t* dst = p.out_tiles + (size_t)w.col16 * p.out_col16_bytes + (size_t)blk * (w.npad * 36);
+        int8_t* qdst = reinterpret_cast<int8_t*>(dst) + (lane >> 4) * (w.npad * 16) + (lane & 15);
+        float* ddst = reinterpret_cast<float*>(dst + w.npad * 32);
+        for (int c = ew / nrb; c < w.n_valid; c += 2 * cstep) {
+            float v[2];
 #pragma unroll
-            for (int s = 16; s > 0; s >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, s));
-            const float d = amax / 127.0f;
-            const int8_t qv = (amax == 0.0f) ? (int8_t)0 : (int8_t)roundf(v / d);
-            uint8_t* dst = p.out_tiles + (size_t)w.aux0 * p.out_tile_stride + (size_t)blk * kG_TileBytes;
-            reinterpret_cast<int8_t*>(dst)[khalf * 2048 + (c >> 3) * 128 + (c & 7) * 16 + kin] = qv;
-            if (lane == 0) *reinterpret_cast<float*>(dst + 4096 + c * 4) = __half2float(__float2half(d));
+            for (int i = 0; i < 2; ++i) {
+                const int ci = min(c + i * cstep, w.n_valid - 1);
+                const float a = xch_sum<KG>(xch, w.npad, r, ci);
+                if (p.dual) v[i] = silu_mul_near(a, xch_sum<KG>(xch, w.npad, r + 64, ci));
+                else { const float t = fmaxf(a, 0.0f); v[i] = t * t; }
+            }
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                const int ci = c + i * cstep;
+                // largest magnitude of the block: bit patterns of non-negative floats order like the values
+                const float amax = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(fabsf(v[i]))));
+                const float d = div_near(amax, 127.0f);
+                const int8_t qv = (amax == 0.0f) ? (int8_t)0 : (int8_t)round_int(div_near(v[i], d));
+                if (ci < w.n_valid) {
+                    qdst[(ci >> 3) * 128 + (ci & 7) * 16] = qv;
+                    if (lane == 0) ddst[ci] = __half2float(__float2half(d));
+                }
+            }
         }
         // Token columns past n_valid of the tile are left as they are: the down GEMM never stores them, and every
         // column's sums depend on that column alone.
     }
 };
 
-// down: rows of H; the tile's columns are pairs, written to pair_out[pair row][H]
-struct DownPolicy {
-    __device__ static __forceinline__ int work(const PrefillGemmParams& p, int idx, GemmWork& w) {
-        const int n_tiles = __ldcg(p.tiles);
-        const int j = idx / p.row_tiles_max, rt = idx - j * p.row_tiles_max;
-        if (j >= n_tiles) return kWorkEnd;
-        const int4 t = __ldcg(reinterpret_cast<const int4*>(p.tiles + kTileHeader) + j);
-        const bool shared = t.x < 0;
-        const int nb = (shared ? p.ncols_in_shared : p.ncols_in) / 32;
-        w.a_src = (shared ? p.sh_a : p.a_exps + (size_t)t.x * p.stride_a) + (size_t)rt * nb * kG_TileBytes;
-        w.b_src = p.b_tiles + (size_t)j * p.b_tile_stride;
-        w.nblocks = nb; w.n_valid = t.z;
-        w.aux0 = j; w.aux1 = rt; w.aux2 = shared ? 1 : 0; w.aux3 = t.y;
-        return kWorkOk;
-    }
-    template <int W>
-    __device__ static __forceinline__ void store(const PrefillGemmParams& p, const GemmWork& w, int row, int, int part, int,
-                                                 float (&acc)[W], uint8_t*, GemmShared&, uint32_t&, bool ok) {
-        if (!ok) return;
-        const int h = w.aux1 * 128 + row;
-        if (h >= p.H) return;
+// down: rows of H; the tile's columns are pairs, written to pair_out[pair row][H].  A warp stores the 128 rows of every fourth
+// column, four rows per lane (H is a multiple of 32).
+struct DownPolicy : MoePolicy {
+    template <int KG>
+    __device__ static __forceinline__ void store(const PrefillGemmParams& p, const GemmWork& w, const float* xch, int ew, int lane) {
+        const bool rows = w.rt * 128 + lane * 4 < p.H;
+        float* out = p.pair_out + w.rt * 128 + lane * 4;
+        const float* x = xch + lane * 4;
+        for (int c0 = 0; c0 < w.n_valid; c0 += 128) {
+            // this lane's pair rows: of columns ew + 4 * lane
+            const int cl = c0 + ew + 4 * lane;
+            int prow = 0;
+            if (cl < w.n_valid) prow = w.shared ? p.T * p.top_k + w.start + cl : __ldcg(p.perm + w.start + cl);
+            const int n = min(32, (w.n_valid - c0 - ew + 3) >> 2);
+#pragma unroll 4
+            for (int i = 0; i < n; ++i) {
+                const int c = c0 + ew + 4 * i;
+                float4 v = *reinterpret_cast<const float4*>(x + c * 128);
 #pragma unroll
-        for (int c = 0; c < W; ++c) {
-            const int col = part * W + c;
-            if (col < w.n_valid) {
-                const int prow = w.aux2 ? p.T * p.top_k + w.aux3 + col : __ldcg(p.perm + w.aux3 + col);
-                p.pair_out[(size_t)prow * p.H + h] = acc[c];
+                for (int k = 1; k < KG; ++k) {
+                    const float4 u = *reinterpret_cast<const float4*>(x + (k * w.npad + c) * 128);
+                    v.x += u.x; v.y += u.y; v.z += u.z; v.w += u.w;
+                }
+                const int row = __shfl_sync(0xffffffffu, prow, i);
+                if (rows) *reinterpret_cast<float4*>(out + (size_t)row * p.H) = v;
             }
         }
     }
@@ -495,7 +710,7 @@ __global__ void pack_mma128_kernel(const int8_t* q, const float* scales, uint8_t
     if (idx >= (int64_t)rows_pad * nb) return;
     const int row = (int)(idx % rows_pad), b = (int)(idx / rows_pad);
     const int tile = row >> 7, r = row & 127;
-    uint8_t* dst = out + ((size_t)tile * nb + b) * kG_TileBytes;
+    uint8_t* dst = out + ((size_t)tile * nb + b) * kG_MmaTile;
     uint4 lo = make_uint4(0, 0, 0, 0), hi = lo;
     float sc = 0.0f;
     if (row < rows) {
@@ -520,20 +735,20 @@ static int gemm_grid(int n_items) {
     const int n_sm = sm_count();
     return n_items < n_sm ? n_items : n_sm;
 }
-constexpr size_t kG_RingBytes = (size_t)kG_Stages * kG_StageBytes;
-constexpr size_t kG_XchBytes = 128 * 129 * sizeof(float);   // gate/up: where the two halves of a tile meet
+template <class Policy, class Params>
+static cudaError_t launch_gemm(const Params& p, int n_items, int32_t* counter, cudaStream_t stream) {
+    static bool attr_done[64] = {};
+    cudaError_t e = max_smem_once(gemm_i8_kernel<Policy, Params>, (int)kG_Smem, attr_done);
+    if (e != cudaSuccess) return e;
+    return launch_pdl(gemm_i8_kernel<Policy, Params>, dim3(gemm_grid(n_items)), kG_Threads, kG_Smem, stream, p, counter);
+}
 
 // tile_counter: one int32 of device memory that is zero when the kernel starts (it ends at n_items + the number of CTAs)
 cudaError_t launch_gemm_i8_f32(const GemmParams& p_in, int n_items, int32_t* tile_counter, cudaStream_t stream) {
     if (n_items <= 0) return cudaSuccess;
     GemmParams p = p_in;
     p.n_items = n_items;
-    const size_t smem = kG_RingBytes + 1024;
-    static bool attr_done[64] = {};
-    cudaError_t e = max_smem_once(gemm_i8_kernel<PlainPolicy, GemmParams>, (int)smem, attr_done);
-    if (e != cudaSuccess) return e;
-    gemm_i8_kernel<PlainPolicy, GemmParams><<<gemm_grid(n_items), kG_Threads, smem, stream>>>(p, tile_counter);
-    return cudaGetLastError();
+    return launch_gemm<PlainPolicy>(p, n_items, tile_counter, stream);
 }
 
 // The tile list's header words 4 (gate/up) and 5 (down) are the launches' tile counters; build_tiles_kernel zeroes them.
@@ -541,21 +756,7 @@ cudaError_t launch_prefill_gemm(const PrefillGemmParams& p, bool down, int n_til
     const int n_items = n_tiles_max * p.row_tiles_max;
     if (n_items <= 0) return cudaSuccess;
     int32_t* counter = const_cast<int32_t*>(p.tiles) + (down ? 5 : 4);
-    cudaError_t e;
-    if (down) {
-        const size_t smem = kG_RingBytes + 1024;
-        static bool attr_done[64] = {};
-        e = max_smem_once(gemm_i8_kernel<DownPolicy, PrefillGemmParams>, (int)smem, attr_done);
-        if (e != cudaSuccess) return e;
-        gemm_i8_kernel<DownPolicy, PrefillGemmParams><<<gemm_grid(n_items), kG_Threads, smem, stream>>>(p, counter);
-    } else {
-        const size_t smem = kG_RingBytes + kG_XchBytes + 1024;
-        static bool attr_done[64] = {};
-        e = max_smem_once(gemm_i8_kernel<GateUpPolicy, PrefillGemmParams>, (int)smem, attr_done);
-        if (e != cudaSuccess) return e;
-        gemm_i8_kernel<GateUpPolicy, PrefillGemmParams><<<gemm_grid(n_items), kG_Threads, smem, stream>>>(p, counter);
-    }
-    return cudaGetLastError();
+    return down ? launch_gemm<DownPolicy>(p, n_items, counter, stream) : launch_gemm<GateUpPolicy>(p, n_items, counter, stream);
 }
 
 // ------------------------------------------------------------------ tensor-pipe probe ----
@@ -583,7 +784,7 @@ __global__ void __launch_bounds__(128, 1) mma_i8_probe_kernel(int n_mma, int n_c
     if (tid == 0) {
         const uint32_t sa = smem_u32(smem), sb = sa + 4096;
         const uint32_t lbo_b = (uint32_t)n_cols * 16u;   // K halves of B are n_cols / 8 row groups of 128 bytes apart
-        const uint64_t adesc = smem_desc_kmajor(sa);
+        const uint64_t adesc = smem_desc_kmajor(sa, 2048);
         const uint64_t bdesc = (uint64_t)((sb & 0x3FFFFu) >> 4) | ((uint64_t)(lbo_b >> 4) << 16) | ((uint64_t)(128u >> 4) << 32) | (1ull << 46);
         const uint32_t idesc = (2u << 4) | (1u << 7) | (1u << 10) | (((uint32_t)n_cols >> 3) << 17) | ((128u >> 4) << 24);
         auto mma = [&](uint32_t d, uint32_t acc) {
@@ -629,140 +830,122 @@ int launch_mma_i8_probe(int n_mma, int n_cols, int n_acc, int32_t* status, cudaS
 }
 
 // ------------------------------------------------------------------ prefill plumbing kernels ----
-// ggml blocks -> mma128 tiles: int8 values and f32 block scales (IQ3_S: scale = d * (1 + 2*sub-scale), exact in f32).
+// ggml Q8_0 blocks -> mma128 tiles: int8 values in the MMA's operand order and f32 block scales.
 // dst row of source row r: plain (mode 0), gate half (mode 1: (r/64)*128 + r%64) or up half (mode 2: ... + 64).
 // One thread per (row, block); blockIdx.y = expert.
-template <int TYPE>
-__global__ void pack_mma128_ggml_kernel(const uint8_t* raw, uint8_t* out, int nrows, int ncols, int mode, int64_t raw_stride,
-                                        int64_t out_stride, const uint32_t* grid) {
+__global__ void pack_mma128_q8_0_kernel(const uint8_t* raw, uint8_t* out, int nrows, int ncols, int mode, int64_t raw_stride, int64_t out_stride) {
     const int nb = ncols >> 5;
     const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= (int64_t)nrows * nb) return;
     const int r = (int)(idx % nrows), b = (int)(idx / nrows);
     int w[8], mul;
     float dw;
-    Unit<TYPE>::load(raw + (size_t)blockIdx.y * raw_stride + (size_t)r * Unit<TYPE>::row_bytes(ncols), b, grid, w, dw, mul);
-    if (TYPE == CHIMERE_TYPE_Q4_0) {
-#pragma unroll
-        for (int g = 0; g < 8; ++g) {   // bytes hold 16 * (nibble - 8): arithmetic shift of every byte
-            const int x = w[g];
-            w[g] = (int)(((uint32_t)((int8_t)(x) >> 4) & 0xFFu) | (((uint32_t)((int8_t)(x >> 8) >> 4) & 0xFFu) << 8) |
-                         (((uint32_t)((int8_t)(x >> 16) >> 4) & 0xFFu) << 16) | (((uint32_t)((int8_t)(x >> 24) >> 4) & 0xFFu) << 24));
-        }
-    }
+    using U = Unit<CHIMERE_TYPE_Q8_0>;
+    U::load(raw + (size_t)blockIdx.y * raw_stride + (size_t)r * U::row_bytes(ncols), b, nullptr, w, dw, mul);
     const int dr = mode == 0 ? r : (r >> 6) * 128 + (r & 63) + (mode == 2 ? 64 : 0);
     const int tile = dr >> 7, rr = dr & 127;
-    uint8_t* dst = out + (size_t)blockIdx.y * out_stride + ((size_t)tile * nb + b) * kG_TileBytes;
+    uint8_t* dst = out + (size_t)blockIdx.y * out_stride + ((size_t)tile * nb + b) * kG_MmaTile;
     *reinterpret_cast<uint4*>(dst + (rr >> 3) * 128 + (rr & 7) * 16) = make_uint4(w[0], w[1], w[2], w[3]);
     *reinterpret_cast<uint4*>(dst + 2048 + (rr >> 3) * 128 + (rr & 7) * 16) = make_uint4(w[4], w[5], w[6], w[7]);
-    *reinterpret_cast<float*>(dst + 4096 + rr * 4) = dw * (float)mul;
+    *reinterpret_cast<float*>(dst + 4096 + rr * 4) = dw;
 }
 
-static __device__ const uint32_t g_iq3s_grid_mma[512] = {
-#include "iq3s_grid.inc"
-};
-
-cudaError_t launch_pack_mma128_ggml(int type, const void* raw, void* out, int n_mats, int nrows, int ncols, int mode,
-                                    int64_t raw_stride, int64_t out_stride, cudaStream_t stream) {
+cudaError_t launch_pack_mma128_q8_0(const void* raw, void* out, int n_mats, int nrows, int ncols, int mode, int64_t raw_stride, int64_t out_stride,
+                                    cudaStream_t stream) {
     if (n_mats <= 0) return cudaSuccess;
     const int64_t n = (int64_t)nrows * (ncols / 32);
-    const dim3 grid((unsigned)((n + 255) / 256), (unsigned)n_mats);
-    const uint32_t* g = nullptr;
-    cudaGetSymbolAddress((void**)&g, g_iq3s_grid_mma);
-    switch (type) {
-        case CHIMERE_TYPE_Q4_0: pack_mma128_ggml_kernel<CHIMERE_TYPE_Q4_0><<<grid, 256, 0, stream>>>((const uint8_t*)raw, (uint8_t*)out, nrows, ncols, mode, raw_stride, out_stride, g); break;
-        case CHIMERE_TYPE_Q8_0: pack_mma128_ggml_kernel<CHIMERE_TYPE_Q8_0><<<grid, 256, 0, stream>>>((const uint8_t*)raw, (uint8_t*)out, nrows, ncols, mode, raw_stride, out_stride, g); break;
-        case CHIMERE_TYPE_IQ3_S: pack_mma128_ggml_kernel<CHIMERE_TYPE_IQ3_S><<<grid, 256, 0, stream>>>((const uint8_t*)raw, (uint8_t*)out, nrows, ncols, mode, raw_stride, out_stride, g); break;
-        default: return cudaErrorInvalidValue;
-    }
+    pack_mma128_q8_0_kernel<<<dim3((unsigned)((n + 255) / 256), (unsigned)n_mats), 256, 0, stream>>>((const uint8_t*)raw, (uint8_t*)out, nrows, ncols, mode,
+                                                                                                     raw_stride, out_stride);
     return cudaGetLastError();
 }
 
-// After routing: token tiles for the experts with at least `gemm_min` pairs (and for the shared expert), and the
-// GEMV work list rewritten to hold only the smaller experts.  One CTA of 256 threads, thread e = expert e.
-// Full tiles (128 pairs) come first and the partly filled ones last, so that the persistent GEMM CTAs, which take
-// tiles round-robin, all get a similar mix of expensive and cheap tiles.
-__global__ void __launch_bounds__(256) build_tiles_kernel(const int32_t* offsets, const int32_t* perm, int32_t* tiles, int32_t* list,
-                                                          int E, int T, int top_k, int has_shared, int gemm_min) {
-    __shared__ int scan_f[8], scan_p[8], scan_e[8];
+// After routing: the token tiles of every expert that has pairs (and of the shared expert).  One CTA of 256 threads,
+// thread e = expert e.  Wide tiles come first and the narrow ones last, so that the persistent GEMM CTAs, which take tiles
+// in order, end on cheap ones; within a width the shared expert's tile leads.  Tiles per width are counted with one scan
+// (four 16-bit counters in a 64-bit word), and a tile's first column follows from its place, because all tiles of a width
+// are equally wide.
+__device__ __forceinline__ uint64_t width_bit(int n, uint64_t count) { return n > 64 ? count : n > 32 ? count << 16 : n > 16 ? count << 32 : count << 48; }
+__global__ void __launch_bounds__(256) build_tiles_kernel(const int32_t* offsets, int32_t* tiles, int E, int T, int has_shared) {
+    __shared__ uint64_t scan[8];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    griddep_wait();
+    if (tid == 0) griddep_launch();
     const int cnt = tid < E ? offsets[tid + 1] - offsets[tid] : 0, off = tid < E ? offsets[tid] : 0;
-    const bool big = cnt >= gemm_min;
-    const int nf = big ? cnt / 128 : 0;                   // full tiles
-    const int np = big && (cnt % 128) ? 1 : 0;            // the partly filled one
-    const int ne = big ? 0 : (cnt + kMaxGroupTokens - 1) / kMaxGroupTokens;
-    int jf = nf, jp = np, ie = ne;
+    const int nf = cnt >> 7, rem = cnt & 127;
+    const uint64_t own = (uint64_t)nf + (rem ? width_bit(rem, 1) : 0ull);
+    uint64_t incl = own;
 #pragma unroll
     for (int s = 1; s < 32; s <<= 1) {
-        const int a = __shfl_up_sync(0xffffffffu, jf, s), b = __shfl_up_sync(0xffffffffu, jp, s), c = __shfl_up_sync(0xffffffffu, ie, s);
-        if (lane >= s) { jf += a; jp += b; ie += c; }
+        const uint64_t a = __shfl_up_sync(0xffffffffu, incl, s);
+        if (lane >= s) incl += a;
     }
-    if (lane == 31) { scan_f[warp] = jf; scan_p[warp] = jp; scan_e[warp] = ie; }
+    if (lane == 31) scan[warp] = incl;
     __syncthreads();
-    int bf = 0, bp = 0, be = 0, tot_f = 0, tot_p = 0, tot_e = 0;
-    for (int w = 0; w < 8; ++w) {
-        if (w < warp) { bf += scan_f[w]; bp += scan_p[w]; be += scan_e[w]; }
-        tot_f += scan_f[w]; tot_p += scan_p[w]; tot_e += scan_e[w];
+    uint64_t before = incl - own, total = 0;
+    for (int w = 0; w < 8; ++w) { if (w < warp) before += scan[w]; total += scan[w]; }
+    const int sh_full = has_shared ? T >> 7 : 0, sh_rem = has_shared ? T & 127 : 0;
+    const uint64_t shared = (uint64_t)sh_full + (sh_rem ? width_bit(sh_rem, 1) : 0ull);
+    total += shared;
+    before += shared;   // the shared expert's tiles lead every width
+    int first[5], col16[5];   // first tile and first column / 16 of each width
+    first[0] = 0; col16[0] = 0;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const int n = (int)((total >> (16 * k)) & 0xFFFFu);
+        first[k + 1] = first[k] + n;
+        col16[k + 1] = col16[k] + n * (8 >> k);
     }
-    // shared-expert tiles: the full ones in front, its partly filled one with the other partly filled ones
-    const int nsh_full = has_shared ? T / 128 : 0, nsh_part = has_shared && (T % 128) ? 1 : 0;
     int4* tv = reinterpret_cast<int4*>(tiles + kTileHeader);
-    for (int i = tid; i < nsh_full; i += 256) tv[i] = make_int4(-1, i * 128, 128, 0);
-    const int f0 = nsh_full + bf + jf - nf;
-    for (int i = 0; i < nf; ++i) tv[f0 + i] = make_int4(tid, off + i * 128, 128, 0);
-    const int part0 = nsh_full + tot_f;
-    if (tid == 0 && nsh_part) tv[part0] = make_int4(-1, nsh_full * 128, T - nsh_full * 128, 0);
-    if (np) tv[part0 + nsh_part + bp + jp - np] = make_int4(tid, off + nf * 128, cnt - nf * 128, 0);
-    const int e0 = be + ie - ne;
-    for (int i = 0; i < ne; ++i) {
-        int* ent = list + kListHeader + kListEntry * (e0 + i);
-        const int mm = min(kMaxGroupTokens, cnt - i * kMaxGroupTokens);
-        ent[0] = tid; ent[1] = off + i * kMaxGroupTokens; ent[2] = mm; ent[3] = 0;
-        for (int j = 0; j < kMaxGroupTokens; ++j) ent[4 + j] = j < mm ? perm[off + i * kMaxGroupTokens + j] : 0;
+    auto put = [&](int k, int i, int expert, int start, int n) { tv[first[k] + i] = make_int4(expert, start, n, col16[k] + i * (8 >> k)); };
+    auto width_of = [](int n) { return n > 64 ? 0 : n > 32 ? 1 : n > 16 ? 2 : 3; };
+    for (int i = tid; i < sh_full; i += 256) put(0, i, -1, i * 128, 128);
+    if (tid == 0 && sh_rem) put(width_of(sh_rem), sh_rem > 64 ? sh_full : 0, -1, sh_full * 128, sh_rem);
+    const int f0 = (int)(before & 0xFFFFu);
+    for (int i = 0; i < nf; ++i) put(0, f0 + i, tid, off + i * 128, 128);
+    if (rem) {
+        const int k = width_of(rem);
+        put(k, (int)((before >> (16 * k)) & 0xFFFFu) + (k == 0 ? nf : 0), tid, off + nf * 128, rem);
     }
     if (tid == 0) {
-        tiles[0] = nsh_full + nsh_part + tot_f + tot_p; tiles[1] = nsh_full + nsh_part; tiles[2] = tot_f + tot_p; tiles[3] = 0;
+        tiles[0] = first[4]; tiles[1] = 0; tiles[2] = 0; tiles[3] = 0;
         tiles[4] = 0; tiles[5] = 0; tiles[6] = 0; tiles[7] = 0;   // the two GEMM launches' tile counters start at zero
-        list[0] = tot_e; list[1] = tot_e; list[2] = 0; list[3] = 0;
     }
 }
 
-// Token tiles of the gate/up GEMM: the Q8_1 planes of each tile's tokens in mma128 order.
+// Token tiles of the gate/up GEMM: the Q8_1 planes of each tile's tokens in the MMA's operand order.
 // grid = (max tiles, 16 groups of 8 token slots), 256 threads = 8 slots x 32 chunk lanes: the eight slots of a group
 // are the 8 x 16 bytes of one core-matrix row group, so every 128-byte segment of the tile is written whole, and a
-// token's 16-byte chunks are read four in a row.
+// token's 16-byte chunks are read four in a row.  Columns without a token are left as they are (nobody reads their sums).
 __global__ void __launch_bounds__(256) gather_tiles_kernel(const int32_t* tiles, const int32_t* perm, const int8_t* x_q, int64_t x_q_stride,
-                                                           const float* x_d, int x_d_stride, uint8_t* b_tiles, int64_t b_tile_stride, int H,
+                                                           const float* x_d, int x_d_stride, uint8_t* b_tiles, int64_t b_col16_bytes, int H,
                                                            int top_k) {
+    griddep_wait();
+    if (threadIdx.x == 0) griddep_launch();
     const int j = blockIdx.x, grp = blockIdx.y;
     if (j >= __ldcg(tiles)) return;
     const int4 t = __ldcg(reinterpret_cast<const int4*>(tiles + kTileHeader) + j);
     const int sl = threadIdx.x & 7, lane_ch = threadIdx.x >> 3;
-    const int c = grp * 8 + sl;                   // token slot of the tile
-    const bool valid = c < t.z;
-    const int tok = !valid ? 0 : (t.x < 0 ? t.y + c : __ldcg(perm + t.y + c) / top_k);
-    uint8_t* base = b_tiles + (size_t)j * b_tile_stride;
+    const int c = grp * 8 + sl, npad = tile_width(t.z);   // token slot of the tile
+    if (c >= t.z) return;
+    const int tok = t.x < 0 ? t.y + c : __ldcg(perm + t.y + c) / top_k;
+    uint8_t* base = b_tiles + (size_t)t.w * b_col16_bytes;
     for (int ch = lane_ch; ch < H / 16; ch += 32) {
-        const uint4 v = valid ? __ldcg(reinterpret_cast<const uint4*>(x_q + (size_t)tok * x_q_stride) + ch) : make_uint4(0, 0, 0, 0);
+        const uint4 v = __ldcg(reinterpret_cast<const uint4*>(x_q + (size_t)tok * x_q_stride) + ch);
         const int b = ch >> 1, khalf = ch & 1;
-        *reinterpret_cast<uint4*>(base + (size_t)b * kG_TileBytes + khalf * 2048 + grp * 128 + sl * 16) = v;
+        *reinterpret_cast<uint4*>(base + (size_t)b * (npad * 36) + khalf * (npad * 16) + grp * 128 + sl * 16) = v;
     }
     for (int b = lane_ch; b < H / 32; b += 32)
-        *reinterpret_cast<float*>(base + (size_t)b * kG_TileBytes + 4096 + c * 4) = valid ? __ldcg(x_d + (size_t)tok * x_d_stride + b) : 0.0f;
+        *reinterpret_cast<float*>(base + (size_t)b * (npad * 36) + npad * 32 + c * 4) = __ldcg(x_d + (size_t)tok * x_d_stride + b);
 }
 
-cudaError_t launch_build_tiles(const int32_t* offsets, const int32_t* perm, int32_t* tiles, int32_t* list, int E, int T, int top_k,
-                               int has_shared, int gemm_min, cudaStream_t stream) {
-    build_tiles_kernel<<<1, 256, 0, stream>>>(offsets, perm, tiles, list, E, T, top_k, has_shared, gemm_min);
-    return cudaGetLastError();
+cudaError_t launch_build_tiles(const int32_t* offsets, int32_t* tiles, int E, int T, int has_shared, cudaStream_t stream) {
+    return launch_pdl(build_tiles_kernel, dim3(1), 256, 0, stream, offsets, tiles, E, T, has_shared);
 }
 
 cudaError_t launch_gather_tiles(const int32_t* tiles, const int32_t* perm, const int8_t* x_q, int64_t x_q_stride, const float* x_d,
-                                int x_d_stride, uint8_t* b_tiles, int64_t b_tile_stride, int H, int top_k, int n_tiles_max, cudaStream_t stream) {
+                                int x_d_stride, uint8_t* b_tiles, int64_t b_col16_bytes, int H, int top_k, int n_tiles_max, cudaStream_t stream) {
     if (n_tiles_max <= 0) return cudaSuccess;
-    gather_tiles_kernel<<<dim3(n_tiles_max, 16), 256, 0, stream>>>(tiles, perm, x_q, x_q_stride, x_d, x_d_stride, b_tiles, b_tile_stride, H, top_k);
-    return cudaGetLastError();
+    return launch_pdl(gather_tiles_kernel, dim3(n_tiles_max, 16), 256, 0, stream, tiles, perm, x_q, x_q_stride, x_d, x_d_stride, b_tiles, b_col16_bytes, H, top_k);
 }
-
 
 }  // namespace chimere
