@@ -52,9 +52,10 @@ constexpr int kG_XchFloats = 128 * 128;      // exchange buffer [K share][column
 constexpr int kG_ExpWarps = 2, kG_EpiWarps = 4, kG_RbWarps = 16;
 constexpr int kG_FirstEpi = 4, kG_FirstRb = 8;
 constexpr int kG_Threads = 32 * (kG_FirstRb + kG_RbWarps);
-// Registers: the launch gives every thread 80; the read-back warps take 96 (512 x 96) and leave 48 to the others (256 x 48).
-// (With 80 the read-back spills inside its loop: 1150 cycles per block instead of 700.)
-constexpr int kG_RegsRb = 96, kG_RegsAux = 48;
+// Registers: the launch gives every thread 80; the read-back warps take 88 (512 x 88) and leave 64 to the others (256 x 64).
+// (With 80 for all the read-back spills inside its loop, 1150 cycles per block instead of 700; with 96 / 48 the expanders do: 520 us
+// for the Nemotron-H-style layer's 256 tokens instead of 450.)
+constexpr int kG_RegsRb = 88, kG_RegsAux = 64;
 static_assert(kG_RbWarps * kG_RegsRb + kG_FirstRb * kG_RegsAux == (kG_RbWarps + kG_FirstRb) * 80, "register shares add up to the launch's total");
 constexpr int kG_TmemCols = 512, kG_TmemSlots = 8;
 constexpr int kG_Sched = 4;                  // tile indices in flight between the scheduler and the other warps
@@ -64,14 +65,20 @@ __device__ __forceinline__ uint64_t smem_desc_kmajor(uint32_t saddr, uint32_t lb
     // start address (>>4) | leading (K) byte offset (>>4) << 16 | stride (8-row group) byte offset 128 (>>4) << 32 | version 1 << 46
     return (uint64_t)((saddr & 0x3FFFFu) >> 4) | ((uint64_t)(lbo >> 4) << 16) | ((uint64_t)(128u >> 4) << 32) | (1ull << 46);
 }
-// D format S32 (2 << 4), A and B signed int8 (1 << 7, 1 << 10), both K-major, N (>> 3 at bit 17), M = 128 (>> 4 at bit 24)
-__device__ __forceinline__ uint32_t instr_desc_i8(int n) { return (2u << 4) | (1u << 7) | (1u << 10) | (((uint32_t)n >> 3) << 17) | ((128u >> 4) << 24); }
-
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
+// One lane of a converged warp.  The single-thread roles keep their whole warp together and let the elected lane issue:
+// their state is then the same in every lane and stays in uniform registers, which the MMA and copy instructions read.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t r;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.b32 %0, 1, 0, p;\n\t}" : "=r"(r));
+    return r != 0;
+}
+__device__ __forceinline__ int uniform(int v) { return __shfl_sync(0xffffffffu, v, 0); }
+__device__ __forceinline__ const uint8_t* uniform(const uint8_t* v) { return (const uint8_t*)__shfl_sync(0xffffffffu, (unsigned long long)v, 0); }
 __device__ __forceinline__ void tc_mma_i8(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
         "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
@@ -132,6 +139,7 @@ struct GemmWork {
     int aux0, aux1;
 };
 constexpr int kWorkOk = 0, kWorkSkip = 1, kWorkEnd = 2;
+struct RowTiles { const uint8_t* src0; const uint8_t* src1; int tile_bytes, n0, n1; };   // the 32-row tiles of a GemmWork (see produce_tile)
 
 // Position in the two operand rings; every role walks the same sequence.  Ring 1 has two geometries (slots for tiles of
 // more than 32 columns, and more, smaller ones); on a change the producer lets the ring run empty first.
@@ -176,38 +184,50 @@ __device__ __forceinline__ void gemm_timeout(GemmShared& sh, int32_t* status, in
 // (one copy brings both) and the expanders keep the scales for the first half.
 __device__ __forceinline__ int stage_unit(int type, int s) { return kG_StageUnits * (type == CHIMERE_TYPE_IQ3_S ? s ^ 1 : s); }
 
-// Warp 0: copies of one tile, a few pieces per stage (a copy costs its warp about 50 cycles, whoever of its lanes asks).
+// Warp 0: copies of one tile, a few pieces per stage, all issued by the elected lane (a copy costs its warp about 50 cycles).
 template <class Policy, class Params>
 __device__ __forceinline__ bool produce_tile(const Params& p, const GemmWork& w, GemmShared& sh, uint8_t* ring1, uint8_t* ring2, RingPos& pos, int lane) {
-    const int type = Policy::type(p, w);
-    const int slim = w.npad <= 32;
+    const int type = uniform(Policy::type(p, w)), nb = uniform(w.nb), npad = uniform(w.npad);
+    const int slim = npad <= 32;
     if (slim != pos.slim) {   // the other slot geometry: every slot of the old one has to be empty first
         for (int r = 0; r < pos.slots1(); ++r)
             if (!mbar_wait(&sh.empty1[r], pos.released(r))) { gemm_timeout(sh, p.status, lane); return false; }
         pos.geometry(slim);
     }
-    const uint8_t* data = Policy::tile(p, w, lane & 3);
-    const int ntiles = Policy::tiles_valid(p, w);
-    const int nstages = (w.nb + kG_StageUnits - 1) / kG_StageUnits;
+    // four row tiles: two at src0, two at src1 (neighbours tile_bytes apart), n0 and n1 of them there
+    const RowTiles rt = Policy::rows(p, w);
+    const uint8_t* src0 = uniform(rt.src0);
+    const uint8_t* src1 = uniform(rt.src1);
+    const uint8_t* bsrc = uniform(w.b);
+    const uint32_t tile_bytes = (uint32_t)uniform(rt.tile_bytes), n0 = (uint32_t)uniform(rt.n0), n1 = (uint32_t)uniform(rt.n1);
+    const int nstages = (nb + kG_StageUnits - 1) / kG_StageUnits;
     for (int s = 0; s < nstages; ++s) {
-        const int u0 = stage_unit(type, s), nu = min(kG_StageUnits, w.nb - u0);
+        const int u0 = stage_unit(type, s), nu = min(kG_StageUnits, nb - u0);
         uint64_t* bar = &sh.full1[pos.r];
         bool ok = mbar_wait(&sh.empty1[pos.r], pos.released(pos.r));
         if (ok && type == kTypeOperand) ok = mbar_wait(&sh.empty1[pos.lag()], pos.released(pos.lag()));
         if (!ok) { gemm_timeout(sh, p.status, lane); return false; }
         uint8_t* raw = ring1 + pos.slot1_off();
-        const uint32_t bbytes = (uint32_t)(nu * w.npad * 36);
-        // bytes of one row tile (4-bit types), its offset in the matrix and in the slot
+        const uint32_t bbytes = (uint32_t)(nu * npad * 36);
+        // 4-bit types: bytes of one row tile, and where they start in it
         const uint32_t piece = type == CHIMERE_TYPE_Q4_0 ? (uint32_t)nu * 576u : (s & 1) ? 2048u : 2240u;
-        if (lane == 0) mbar_expect_tx(bar, (type == kTypeOperand ? (uint32_t)(nu * kG_MmaTile) : (uint32_t)ntiles * piece) + bbytes);
-        __syncwarp();
-        if (type == kTypeOperand) {
-            if (lane == 0) bulk_g2s(ring2 + (uint32_t)pos.e * kG_ASlot, data + (size_t)u0 * kG_MmaTile, (uint32_t)(nu * kG_MmaTile), bar);
-        } else if (lane < 4 && data) {
-            const uint32_t off = type == CHIMERE_TYPE_Q4_0 ? (uint32_t)u0 * 576u : (uint32_t)(u0 >> 3) * 4288u + (uint32_t)(u0 & 4) * 512u;
-            bulk_g2s(raw + lane * (kG_RawBytes / 4), data + off, piece, bar);
+        const uint32_t off = type == CHIMERE_TYPE_Q4_0 ? (uint32_t)u0 * 576u : (uint32_t)(u0 >> 3) * 4288u + (uint32_t)(u0 & 4) * 512u;
+        if (elect_one()) {
+            if (type == kTypeOperand) {
+                mbar_expect_tx(bar, (uint32_t)(nu * kG_MmaTile) + bbytes);
+                bulk_g2s(ring2 + (uint32_t)pos.e * kG_ASlot, src0 + (size_t)u0 * kG_MmaTile, (uint32_t)(nu * kG_MmaTile), bar);
+            } else {
+                mbar_expect_tx(bar, (n0 + n1) * piece + bbytes);
+                const uint8_t* a = src0 + off;
+                const uint8_t* b = src1 + off;
+                bulk_g2s(raw, a, piece, bar);
+                if (n0 > 1) bulk_g2s(raw + kG_RawBytes / 4, a + tile_bytes, piece, bar);
+                if (n1 > 0) bulk_g2s(raw + kG_RawBytes / 2, b, piece, bar);
+                if (n1 > 1) bulk_g2s(raw + 3 * (kG_RawBytes / 4), b + tile_bytes, piece, bar);
+            }
+            bulk_g2s(raw + kG_RawBytes, bsrc + (size_t)u0 * npad * 36, bbytes, bar);
         }
-        if (lane == 4) bulk_g2s(raw + kG_RawBytes, w.b + (size_t)u0 * w.npad * 36, bbytes, bar);
+        __syncwarp();
         pos.next(type != kTypeOperand);
     }
     return true;
@@ -215,39 +235,35 @@ __device__ __forceinline__ bool produce_tile(const Params& p, const GemmWork& w,
 
 // Packed 4-bit units -> int8 operand rows.  A unit's 16 bytes per row hold elements 0..15 in the low nibbles (code + 8) and
 // 16..31 in the high ones (two's complement): the two halves are the row's 16 bytes of the operand's two K halves.
-// Warp x expands row tiles x and x + 2; the loads of two units' pieces are in flight together (the compiler keeps the order
-// of the shared-memory accesses as written).
+// Warp x expands row tiles x and x + 2; all loads of a stage go out first (the compiler keeps the order of the
+// shared-memory accesses as written).
 template <int TYPE>
-__device__ __forceinline__ void expand_units(uint32_t raw, uint32_t a, int nu, int x, int lane) {
+__device__ __forceinline__ void expand_units(uint32_t raw, uint32_t a, int x, int lane) {
     constexpr uint32_t kOdd = TYPE == CHIMERE_TYPE_IQ3_S ? 0x08080808u : 0u;   // 8 * (2c + 1) = 16c + 8
     constexpr uint32_t kTilePitch = kG_RawBytes / 4, kUnitPitch = TYPE == CHIMERE_TYPE_IQ3_S ? 512 : 576;
     const uint32_t src = raw + (uint32_t)x * kTilePitch + lane * 16, dst = a + (uint32_t)x * 512 + lane * 16;
+    uint4 v[8];
 #pragma unroll
-    for (int u = 0; u < kG_StageUnits; u += 2) {
-        if (u >= nu) break;
-        uint4 v[4];
+    for (int i = 0; i < 8; ++i) v[i] = lds128(src + (i & 1) * 2 * kTilePitch + (i >> 1) * kUnitPitch);   // (units past nu: bytes nobody uses)
 #pragma unroll
-        for (int i = 0; i < 4; ++i) v[i] = lds128(src + (i & 1) * 2 * kTilePitch + (u + (i >> 1)) * kUnitPitch);   // (an odd last unit reads bytes nobody uses)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            uint4 lo, hi;
-            lo.x = ((v[i].x << 4) & 0xF0F0F0F0u) ^ (0x80808080u | kOdd); hi.x = (v[i].x & 0xF0F0F0F0u) | kOdd;
-            lo.y = ((v[i].y << 4) & 0xF0F0F0F0u) ^ (0x80808080u | kOdd); hi.y = (v[i].y & 0xF0F0F0F0u) | kOdd;
-            lo.z = ((v[i].z << 4) & 0xF0F0F0F0u) ^ (0x80808080u | kOdd); hi.z = (v[i].z & 0xF0F0F0F0u) | kOdd;
-            lo.w = ((v[i].w << 4) & 0xF0F0F0F0u) ^ (0x80808080u | kOdd); hi.w = (v[i].w & 0xF0F0F0F0u) | kOdd;
-            const uint32_t d = dst + (u + (i >> 1)) * kG_MmaTile + (i & 1) * 1024;
-            sts128(d, lo);
-            sts128(d + 2048, hi);
-        }
+    for (int i = 0; i < 8; ++i) {
+        uint4 lo, hi;
+        lo.x = ((v[i].x << 4) & 0xF0F0F0F0u) ^ (0x80808080u | kOdd); hi.x = (v[i].x & 0xF0F0F0F0u) | kOdd;
+        lo.y = ((v[i].y << 4) & 0xF0F0F0F0u) ^ (0x80808080u | kOdd); hi.y = (v[i].y & 0xF0F0F0F0u) | kOdd;
+        lo.z = ((v[i].z << 4) & 0xF0F0F0F0u) ^ (0x80808080u | kOdd); hi.z = (v[i].z & 0xF0F0F0F0u) | kOdd;
+        lo.w = ((v[i].w << 4) & 0xF0F0F0F0u) ^ (0x80808080u | kOdd); hi.w = (v[i].w & 0xF0F0F0F0u) | kOdd;
+        const uint32_t d = dst + (i >> 1) * kG_MmaTile + (i & 1) * 1024;
+        sts128(d, lo);
+        sts128(d + 2048, hi);
     }
 }
 
 // Warps 2..3: warp x takes row tiles x and x + 2 of every stage.
 template <class Policy, class Params>
 __device__ __forceinline__ bool expand_tile(const Params& p, const GemmWork& w, GemmShared& sh, uint32_t ring1, uint32_t ring2, RingPos& pos, int x, int lane) {
-    const int type = Policy::type(p, w);
-    pos.geometry(w.npad <= 32);
-    const int nstages = (w.nb + kG_StageUnits - 1) / kG_StageUnits;
+    const int type = uniform(Policy::type(p, w)), nb = uniform(w.nb);
+    pos.geometry(uniform(w.npad) <= 32);
+    const int nstages = (nb + kG_StageUnits - 1) / kG_StageUnits;
     if (type == kTypeOperand) {   // nothing to do but keep step
         for (int s = 0; s < nstages; ++s) pos.next(false);
         return true;
@@ -255,19 +271,19 @@ __device__ __forceinline__ bool expand_tile(const Params& p, const GemmWork& w, 
     float d3[2] = {0.0f, 0.0f};        // IQ3_S: this lane's rows' scales of the super-block, kept over its two stages
     uint32_t sc3[2] = {0u, 0u};
     for (int s = 0; s < nstages; ++s) {
-        const int u0 = stage_unit(type, s), nu = min(kG_StageUnits, w.nb - u0);
+        const int u0 = stage_unit(type, s), nu = min(kG_StageUnits, nb - u0);
         if (!mbar_wait(&sh.full1[pos.r], pos.par1()) || !mbar_wait(&sh.empty1[pos.lag()], pos.released(pos.lag()))) { gemm_timeout(sh, p.status, lane); return false; }
         const uint32_t raw = ring1 + pos.slot1_off(), a = ring2 + (uint32_t)pos.e * kG_ASlot;
         const uint32_t rec = a + 4096 + (x * 32 + lane) * 4;   // [unit] kG_MmaTile apart, row tile x + 2: 256 bytes further
         if (type == CHIMERE_TYPE_Q4_0) {
-            expand_units<CHIMERE_TYPE_Q4_0>(raw, a, nu, x, lane);
+            expand_units<CHIMERE_TYPE_Q4_0>(raw, a, x, lane);
             uint32_t d[8];
 #pragma unroll
             for (int i = 0; i < 8; ++i) d[i] = lds16(raw + (x + 2 * (i & 1)) * (kG_RawBytes / 4) + (i >> 1) * 576 + 512 + lane * 2);
 #pragma unroll
             for (int i = 0; i < 8; ++i) sts_f32(rec + (i >> 1) * kG_MmaTile + (i & 1) * 256, h2f(d[i]) * 0.0625f);
         } else {
-            expand_units<CHIMERE_TYPE_IQ3_S>(raw, a, nu, x, lane);
+            expand_units<CHIMERE_TYPE_IQ3_S>(raw, a, x, lane);
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 if (!(s & 1)) {   // the scales came behind these units
@@ -289,46 +305,56 @@ __device__ __forceinline__ bool expand_tile(const Params& p, const GemmWork& w, 
     return true;
 }
 
-// Warp 1, lane 0: the MMAs of one tile.  A slim tile's TMEM slots need no barrier of their own: there are more of them than A
-// slots, and an A slot is refilled only after its stage has been read back.
-template <class Policy, class Params>
+// Warp 1: the MMAs of one tile, issued by its elected lane.  A slim tile's TMEM slots need no barrier of their own: there are
+// more of them than A slots, and an A slot is refilled only after its stage has been read back.  Everything a block's MMA
+// needs is a constant away from the stage's values: with a slim tile the warp has about 400 cycles per stage, of which the
+// four MMAs and the commit take 360.
+template <class Policy, int NPAD, class Params>
 __device__ __forceinline__ bool mma_tile(const Params& p, const GemmWork& w, GemmShared& sh, uint32_t cst, uint32_t ring1, uint32_t ring2, uint32_t tmem,
-                                         RingPos& pos, TmemPos& tp) {
-    const bool expanded = Policy::type(p, w) != kTypeOperand;
-    const bool wide = w.npad == 128, handshake = w.npad >= 64;
-    const int npad = w.npad, bps = blocks_per_slot(npad);
-    if (npad != tp.npad) {   // another width lays the accumulators out differently: everything has to be read back first
+                                         RingPos& pos, TmemPos& tp, int lane) {
+    constexpr int kBps = blocks_per_slot(NPAD);
+    constexpr bool kWide = NPAD == 128, kHandshake = NPAD >= 64;
+    // D format S32 (2 << 4), A and B signed int8 (1 << 7, 1 << 10), both K-major, N (>> 3 at bit 17), M = 128 (>> 4 at bit 24)
+    constexpr uint32_t kIdesc = (2u << 4) | (1u << 7) | (1u << 10) | (((uint32_t)NPAD >> 3) << 17) | ((128u >> 4) << 24);
+    const bool expanded = uniform(Policy::type(p, w)) != kTypeOperand;
+    const int nb = uniform(w.nb);
+    if (NPAD != tp.npad) {   // another width lays the accumulators out differently: everything has to be read back first
         for (int r = 0; r < pos.slots1(); ++r)
-            if (!mbar_wait(&sh.empty1[r], pos.released(r))) { gemm_timeout(sh, p.status, 0); return false; }
-        tp.npad = npad; tp.slot = 0; tp.nslots = kG_TmemCols / (bps * npad);
+            if (!mbar_wait(&sh.empty1[r], pos.released(r))) { gemm_timeout(sh, p.status, lane); return false; }
+        tp.npad = NPAD; tp.slot = 0; tp.nslots = kG_TmemCols / (kBps * NPAD);
     }
-    pos.geometry(npad <= 32);
-    const uint32_t idesc = instr_desc_i8(npad), lbo_b = (uint32_t)npad * 16u, bstep = (uint32_t)(npad * 36) >> 4;
-    const uint64_t ca = smem_desc_kmajor(cst, 2048), cb = smem_desc_kmajor(cst, lbo_b);
-    const uint64_t a_base = smem_desc_kmajor(ring2, 2048), b_base = smem_desc_kmajor(ring1 + kG_RawBytes, lbo_b);
-    const int nstages = (w.nb + kG_StageUnits - 1) / kG_StageUnits;
-    for (int s = 0; s < nstages; ++s) {
-        const int nu = min(kG_StageUnits, w.nb - s * kG_StageUnits);
-        if (!(expanded ? mbar_wait(&sh.xfull2[pos.e], pos.par2()) : mbar_wait(&sh.full1[pos.r], pos.par1()))) { gemm_timeout(sh, p.status, 0); return false; }
+    pos.geometry(NPAD <= 32);
+    const uint64_t ca = smem_desc_kmajor(cst, 2048), cb = smem_desc_kmajor(cst, NPAD * 16);
+    const uint64_t a_base = smem_desc_kmajor(ring2, 2048), b_base = smem_desc_kmajor(ring1 + kG_RawBytes, NPAD * 16);
+    auto block = [&](uint64_t a, uint64_t b, uint32_t d, int j) {
+        d += (uint32_t)((j % kBps) * NPAD);
+        if (kWide) tc_mma_i8(d, ca, cb, kIdesc, 0u);
+        tc_mma_i8(d, a + (uint32_t)(j * (kG_MmaTile >> 4)), b + (uint32_t)(j * ((NPAD * 36) >> 4)), kIdesc, kWide ? 1u : 0u);
+    };
+    for (int b0 = 0; b0 < nb; b0 += kG_StageUnits) {
+        const int nu = min(kG_StageUnits, nb - b0);
+        if (!(expanded ? mbar_wait(&sh.xfull2[pos.e], pos.par2()) : mbar_wait(&sh.full1[pos.r], pos.par1()))) { gemm_timeout(sh, p.status, lane); return false; }
         const uint64_t a = a_base + (uint32_t)pos.e * (kG_ASlot >> 4), b = b_base + (pos.slot1_off() >> 4);
 #pragma unroll
-        for (int j = 0; j < kG_StageUnits; ++j) {
-            if (j >= nu) break;
-            const int js = wide ? j & 1 : j;   // block within the slot
-            if (js == 0) {
-                if (handshake) {
-                    if (!mbar_wait(&sh.tempty[tp.slot], ((tp.ph_empty >> tp.slot) & 1u) ^ 1u)) { gemm_timeout(sh, p.status, 0); return false; }
-                    tp.ph_empty ^= 1u << tp.slot;
+        for (int j0 = 0; j0 < kG_StageUnits; j0 += kBps) {
+            if (j0 >= nu) break;
+            if (kHandshake) {
+                if (!mbar_wait(&sh.tempty[tp.slot], ((tp.ph_empty >> tp.slot) & 1u) ^ 1u)) { gemm_timeout(sh, p.status, lane); return false; }
+                tp.ph_empty ^= 1u << tp.slot;
+            }
+            tc_fence_after();
+            const uint32_t d = tmem + (uint32_t)(tp.slot * (kBps * NPAD));
+            if (elect_one()) {
+                if (nu == kG_StageUnits) {
+#pragma unroll
+                    for (int j = 0; j < kBps; ++j) block(a, b, d, j0 + j);
+                } else {
+                    for (int j = j0; j < min(nu, j0 + kBps); ++j) block(a, b, d, j);
                 }
-                tc_fence_after();
+                tc_commit(&sh.tfull[tp.slot]);   // (also tells the read-back warps that the operands have been read)
             }
-            const uint32_t d = tmem + (uint32_t)((tp.slot * bps + js) * npad);
-            if (wide) tc_mma_i8(d, ca, cb, idesc, 0u);
-            tc_mma_i8(d, a + (uint32_t)j * (kG_MmaTile >> 4), b + (uint32_t)j * bstep, idesc, wide ? 1u : 0u);
-            if (j == nu - 1 || (wide && js == 1)) {   // (also tells the read-back warps that the operands have been read)
-                tc_commit(&sh.tfull[tp.slot]);
-                tp.next();
-            }
+            __syncwarp();
+            tp.next();
         }
         pos.next(expanded);
     }
@@ -418,7 +444,7 @@ __device__ __forceinline__ bool readback(const Params& p, const GemmWork& w, Gem
     uint64_t acc2[W / 2];
 #pragma unroll
     for (int i = 0; i < W / 2; ++i) acc2[i] = 0ull;
-    bool ok = readback_tile<COLG, KG, W>(sh, ring1, ring2, tmem, p.status, w.nb, Policy::type(p, w) != kTypeOperand, q, part, lane, pos, tp, acc2);
+    bool ok = readback_tile<COLG, KG, W>(sh, ring1, ring2, tmem, p.status, uniform(w.nb), uniform(Policy::type(p, w)) != kTypeOperand, q, part, lane, pos, tp, acc2);
     if (!mbar_wait(&sh.xempty, (xphase & 1u) ^ 1u)) { gemm_timeout(sh, p.status, lane); ok = false; }   // the tile before has been stored
     ++xphase;
     float* mine = xch + part * (W * 128) + q * 32 + lane;   // (part = share * COLG + column group)
@@ -459,7 +485,7 @@ template <class Policy, class Params>
 __global__ void __launch_bounds__(kG_Threads, 1) gemm_i8_kernel(const Params p, int32_t* tile_counter) {
     extern __shared__ uint8_t smem_raw[];
     __shared__ GemmShared sh;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x, lane = tid & 31, warp = uniform(tid >> 5);
     uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
     uint8_t* ring1 = smem + kG_ConstBytes;
     uint8_t* ring2 = ring1 + kG_RingBytes;
@@ -500,7 +526,7 @@ __global__ void __launch_bounds__(kG_Threads, 1) gemm_i8_kernel(const Params p, 
             GemmWork w;
             Policy::work(p, idx, w);
             const uint32_t r1 = smem_u32(ring1), r2 = smem_u32(ring2);
-            switch (w.npad) {
+            switch (uniform(w.npad)) {
                 case 128: ok = readback<Policy, Params, 4, 1, 32>(p, w, sh, r1, r2, xch, tmem, q, part, lane, pos, tp, xphase); break;
                 case 64: ok = readback<Policy, Params, 2, 2, 32>(p, w, sh, r1, r2, xch, tmem, q, part, lane, pos, tp, xphase); break;
                 case 32: ok = readback<Policy, Params, 1, 4, 32>(p, w, sh, r1, r2, xch, tmem, q, part, lane, pos, tp, xphase); break;
@@ -543,8 +569,13 @@ __global__ void __launch_bounds__(kG_Threads, 1) gemm_i8_kernel(const Params p, 
                 Policy::work(p, idx, w);
                 const uint32_t r1 = smem_u32(ring1), r2 = smem_u32(ring2);
                 if (warp == 1) {
-                    if (lane == 0) ok = mma_tile<Policy>(p, w, sh, smem_u32(smem), r1, r2, tmem, pos, tp);
-                    ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+                    const uint32_t cst = smem_u32(smem);
+                    switch (uniform(w.npad)) {
+                        case 128: ok = mma_tile<Policy, 128>(p, w, sh, cst, r1, r2, tmem, pos, tp, lane); break;
+                        case 64: ok = mma_tile<Policy, 64>(p, w, sh, cst, r1, r2, tmem, pos, tp, lane); break;
+                        case 32: ok = mma_tile<Policy, 32>(p, w, sh, cst, r1, r2, tmem, pos, tp, lane); break;
+                        default: ok = mma_tile<Policy, 16>(p, w, sh, cst, r1, r2, tmem, pos, tp, lane); break;
+                    }
                 } else if (warp < kG_FirstEpi) {
                     ok = expand_tile<Policy>(p, w, sh, r1, r2, pos, warp - 2, lane);
                 } else {
@@ -575,8 +606,7 @@ struct PlainPolicy {
         return kWorkOk;
     }
     __device__ static __forceinline__ int type(const GemmParams&, const GemmWork&) { return kTypeOperand; }
-    __device__ static __forceinline__ int tiles_valid(const GemmParams&, const GemmWork&) { return 4; }
-    __device__ static __forceinline__ const uint8_t* tile(const GemmParams& p, const GemmWork& w, int) { return p.a_base + p.items[w.expert].a_offset; }
+    __device__ static __forceinline__ RowTiles rows(const GemmParams& p, const GemmWork& w) { return RowTiles{p.a_base + p.items[w.expert].a_offset, nullptr, 0, 0, 0}; }
     template <int KG>
     __device__ static __forceinline__ void store(const GemmParams& p, const GemmWork& w, const float* xch, int ew, int lane) {
         for (int r = ew; r < w.rt; r += kG_EpiWarps)   // (all tiles of the primitive are 128 columns wide: one share)
@@ -607,18 +637,22 @@ struct MoePolicy {
         return kWorkOk;
     }
     __device__ static __forceinline__ int type(const PrefillGemmParams& p, const GemmWork& w) { return p.m[w.shared].type; }
-    // gated: two 32-row tiles of the gate matrix, then the same two of the up matrix; else four of the one matrix
-    __device__ static __forceinline__ int tiles_valid(const PrefillGemmParams& p, const GemmWork& w) {
-        const int n = p.m[w.shared].rows32;
-        return p.dual ? 2 * min(2, n - 2 * w.rt) : min(4, n - 4 * w.rt);
-    }
-    __device__ static __forceinline__ const uint8_t* tile(const PrefillGemmParams& p, const GemmWork& w, int t) {
+    // gated: two 32-row tiles of the gate matrix and the same two of the up matrix; else four of the one matrix
+    __device__ static __forceinline__ RowTiles rows(const PrefillGemmParams& p, const GemmWork& w) {
         const PrefillGemmMats& m = p.m[w.shared];
-        if (m.type == kTypeOperand) return m.w0 + (size_t)w.expert * m.stride0 + (size_t)w.rt * w.nb * kG_MmaTile;
-        const int i = p.dual ? 2 * w.rt + (t & 1) : 4 * w.rt + t;
-        if (i >= m.rows32) return nullptr;
-        const bool second = p.dual && t >= 2;
-        return (second ? m.w1 + (size_t)w.expert * m.stride1 : m.w0 + (size_t)w.expert * m.stride0) + (size_t)i * m.tile_bytes;
+        RowTiles r{m.w0 + (size_t)w.expert * m.stride0, nullptr, (int)m.tile_bytes, 0, 0};
+        if (m.type == kTypeOperand) { r.src0 += (size_t)w.rt * w.nb * kG_MmaTile; return r; }
+        if (p.dual) {
+            r.src0 += (size_t)(2 * w.rt) * m.tile_bytes;
+            r.src1 = m.w1 + (size_t)w.expert * m.stride1 + (size_t)(2 * w.rt) * m.tile_bytes;
+            r.n0 = r.n1 = min(2, m.rows32 - 2 * w.rt);
+        } else {
+            r.src0 += (size_t)(4 * w.rt) * m.tile_bytes;
+            r.src1 = r.src0 + 2 * m.tile_bytes;
+            r.n0 = min(2, m.rows32 - 4 * w.rt);
+            r.n1 = max(0, min(2, m.rows32 - 4 * w.rt - 2));
+        }
+        return r;
     }
 };
 
