@@ -34,6 +34,13 @@ inline chimere_moe_layer routed_only(const chimere_moe_layer* w) {
     return r;   // (keeps shexp_gate_w: the router still computes the gate logit)
 }
 
+// ... and whether that shared expert can go through the grouped GEMM (prefill-size batches): all three matrices Q4_K or Q5_K
+// (Q6_K has a scale per 16 weights, the MMA's blocks are 32 wide) and whole 64-row pairs of gate and up rows.
+inline bool kshared_gemm(const chimere_moe_layer* w) {
+    auto ok = [](int t) { return t == CHIMERE_TYPE_Q4_K || t == CHIMERE_TYPE_Q5_K; };
+    return kshared(w) && w->act == CHIMERE_ACT_SWIGLU && ok(w->type_sh_gate) && ok(w->type_sh_up) && ok(w->type_sh_down);
+}
+
 int validate_layer(const chimere_moe_layer* w) {
     if (!w) return -1;
     if (kshared(w)) {
@@ -88,8 +95,10 @@ int routed_entries_for(const chimere_moe_layer* w, int T) {
     return (w->E < P ? w->E : P) + extra + (w->F_s > 0 ? (T + shared_group_tokens(T) - 1) / shared_group_tokens(T) : 0);
 }
 
-Layout make_layout(const chimere_moe_layer* w, int T) {
-    if (kshared(w)) { const chimere_moe_layer r = routed_only(w); return make_layout(&r, T); }
+// extra_rows: per-pair output rows beyond the routed pairs' and the shared expert's own (a K-quant shared expert's rows on the
+// grouped GEMM; they come last, so that the rest of the layout does not depend on them)
+Layout make_layout(const chimere_moe_layer* w, int T, int extra_rows = 0) {
+    if (kshared(w)) { const chimere_moe_layer r = routed_only(w); return make_layout(&r, T, kshared_gemm(w) ? T : 0); }
     Layout L{};
     const int k = w->top_k, H = w->H, E = w->E;
     const int Fmax = w->F > w->F_s ? w->F : w->F_s;
@@ -113,7 +122,6 @@ Layout make_layout(const chimere_moe_layer* w, int T) {
     L.group_list = o; o += up256((size_t)(kListHeader + kListEntry * L.max_entries) * 4);
     L.counters = o; o += up256((size_t)L.n_counters * 4);
     L.inter_q8 = o; o += up256(pairs * L.inter_stride);
-    L.pair_out = o; o += up256(pairs * H * 4);
     L.Fmax = Fmax;
     L.x_d_stride = (H / 32 + 3) & ~3;
     L.inter_d_stride = (Fmax / 32 + 3) & ~3;
@@ -122,6 +130,7 @@ Layout make_layout(const chimere_moe_layer* w, int T) {
     L.inter_q = o; o += up256(pairs * Fmax);
     L.inter_d = o; o += up256(pairs * L.inter_d_stride * 4);
     L.status = o; o += 256;
+    L.pair_out = o; o += up256((pairs + extra_rows) * H * 4);
     L.total = o;
     return L;
 }
@@ -641,8 +650,9 @@ struct PrefillArena { size_t tiles, bx, b2, total; int64_t bx_col16, b2_col16; }
 PrefillArena prefill_arena(const chimere_moe_layer* w, int T) {
     PrefillArena A{};
     const int Fmax = w->F > w->F_s ? w->F : w->F_s;
-    A.bx_col16 = (int64_t)(w->H / 32) * 576;   // 16 columns: 36 bytes per column and block
-    A.b2_col16 = (int64_t)(Fmax / 32) * 576;
+    const int per = kshared_gemm(w) ? 640 : 576;   // 16 columns: 36 bytes per column and block, 40 with the blocks' sums
+    A.bx_col16 = (int64_t)(w->H / 32) * per;
+    A.b2_col16 = (int64_t)(Fmax / 32) * per;
     const int64_t cols = n_col16_max_for(w, T);
     size_t o = 0;
     A.tiles = o; o += up256((size_t)(8 + 4 * n_tiles_max_for(w, T)) * 4);
@@ -653,8 +663,8 @@ PrefillArena prefill_arena(const chimere_moe_layer* w, int T) {
 }
 }  // namespace
 
-// The GEMM reads 4-bit weights in the tiled32 form; only Q8_0 matrices get a copy in the MMA's own order (mma128 tiles; gate
-// and up rows interleaved per 64, so that one output tile holds both).
+// The GEMM reads 4-bit weights in the tiled32 form; Q8_0 matrices, and a shared expert in Q4_K / Q5_K super-blocks, get a copy
+// in the MMA's own order (mma128 tiles; gate and up rows interleaved per 64, so that one output tile holds both).
 namespace {
 struct PrefillPlan { size_t gu, down, sh_gu, sh_down, total; int64_t sgu, sdown, s_sh_gu, s_sh_down; };
 PrefillPlan prefill_plan(const chimere_moe_layer* w) {
@@ -665,6 +675,10 @@ PrefillPlan prefill_plan(const chimere_moe_layer* w) {
     P.sdown = w->type_down == CHIMERE_TYPE_Q8_0 ? tiles(w->H, 128, w->F) : 0;
     P.s_sh_gu = w->F_s > 0 && w->type_sh_up == CHIMERE_TYPE_Q8_0 ? tiles(w->F_s, rpt, w->H) : 0;
     P.s_sh_down = w->F_s > 0 && w->type_sh_down == CHIMERE_TYPE_Q8_0 ? tiles(w->H, 128, w->F_s) : 0;
+    if (kshared_gemm(w)) {
+        P.s_sh_gu = (int64_t)((w->F_s + 63) / 64) * (w->H / 128) * kOperandMinStage;
+        P.s_sh_down = (int64_t)(w->H / 128) * (w->F_s / 128) * kOperandMinStage;
+    }
     size_t o = 256;   // (never empty: the size doubles as the check of the dimensions)
     P.gu = o; o += up256((size_t)P.sgu * w->E);
     P.down = o; o += up256((size_t)P.sdown * w->E);
@@ -677,7 +691,7 @@ PrefillPlan prefill_plan(const chimere_moe_layer* w) {
 
 size_t chimere_b200_moe_pack_prefill_bytes(const chimere_moe_layer* raw) {
     if (validate_layer(raw) != 0) return 0;
-    if (kshared(raw)) { const chimere_moe_layer r = routed_only(raw); return chimere_b200_moe_pack_prefill_bytes(&r); }
+    if (kshared(raw) && !kshared_gemm(raw)) { const chimere_moe_layer r = routed_only(raw); return chimere_b200_moe_pack_prefill_bytes(&r); }
     if (raw->layout != CHIMERE_LAYOUT_GGML || !prefill_dims_ok(raw)) return 0;
     return prefill_plan(raw).total;
 }
@@ -687,7 +701,7 @@ int chimere_b200_moe_pack_prefill(const chimere_moe_layer* raw, void* d_arena, s
     int rc = validate_layer(raw);
     if (rc) return rc;
     if (!d_arena || !out) return -1;
-    if (kshared(raw)) { const chimere_moe_layer r = routed_only(raw); return chimere_b200_moe_pack_prefill(&r, d_arena, bytes, out, stream); }
+    if (kshared(raw) && !kshared_gemm(raw)) { const chimere_moe_layer r = routed_only(raw); return chimere_b200_moe_pack_prefill(&r, d_arena, bytes, out, stream); }
     if (raw->layout != CHIMERE_LAYOUT_GGML || !prefill_dims_ok(raw)) return -2;
     if ((uintptr_t)d_arena & 255) return -5;
     const PrefillPlan P = prefill_plan(raw);
@@ -707,6 +721,13 @@ int chimere_b200_moe_pack_prefill(const chimere_moe_layer* raw, void* d_arena, s
         if (e == cudaSuccess) e = launch_pack_mma128_q8_0(raw->down_exps, base + P.down, raw->E, raw->H, raw->F, 0, raw->stride_down, P.sdown, stream);
         out->down_exps = base + P.down; out->stride_down = P.sdown;
     }
+    if (kshared_gemm(raw)) {
+        if (e == cudaSuccess) e = launch_pack_operand_min(raw->type_sh_gate, raw->sh_gate, base + P.sh_gu, raw->F_s, raw->H, 1, stream);
+        if (e == cudaSuccess) e = launch_pack_operand_min(raw->type_sh_up, raw->sh_up, base + P.sh_gu, raw->F_s, raw->H, 2, stream);
+        if (e == cudaSuccess) e = launch_pack_operand_min(raw->type_sh_down, raw->sh_down, base + P.sh_down, raw->H, raw->F_s, 0, stream);
+        out->sh_gu = base + P.sh_gu; out->sh_down = base + P.sh_down;
+        return cuda_rc(e);
+    }
     if (P.s_sh_gu) { gate_up(raw->sh_gate, raw->sh_up, P.sh_gu, 1, raw->F_s, 0, 0, 0); out->sh_gu = base + P.sh_gu; }
     if (P.s_sh_down) {
         if (e == cudaSuccess) e = launch_pack_mma128_q8_0(raw->sh_down, base + P.sh_down, 1, raw->H, raw->F_s, 0, 0, 0, stream);
@@ -717,7 +738,7 @@ int chimere_b200_moe_pack_prefill(const chimere_moe_layer* raw, void* d_arena, s
 
 size_t chimere_b200_moe_prefill_bytes(const chimere_moe_layer* w, int max_T) {
     if (validate_layer(w) != 0 || max_T <= 0) return 0;
-    if (kshared(w)) { const chimere_moe_layer r = routed_only(w); return chimere_b200_moe_prefill_bytes(&r, max_T); }
+    if (kshared(w) && !kshared_gemm(w)) { const chimere_moe_layer r = routed_only(w); return chimere_b200_moe_prefill_bytes(&r, max_T); }
     if (!prefill_dims_ok(w)) return 0;
     return prefill_arena(w, max_T).total;
 }
@@ -756,6 +777,11 @@ static PrefillGemmMats gemm_mats(const chimere_moe_layer* w, const chimere_moe_p
     m.ncols = down ? width : w->H;
     m.rows32 = (down ? w->H : width) / 32;
     m.row_tiles = dual ? (m.rows32 + 1) / 2 : (m.rows32 + 3) / 4;
+    if (kquant_type(m.type)) {   // (a shared expert that kshared_gemm accepts: its copy with minimums)
+        m.type = kTypeOperandMin;
+        m.w0 = (const uint8_t*)(pw ? (down ? pw->sh_down : pw->sh_gu) : nullptr);
+        return m;
+    }
     m.tile_bytes = m.ncols > 0 ? tiled_matrix_bytes(m.type, 32, m.ncols) : 0;
     m.w0 = (const uint8_t*)(down ? dn : dual ? gate : up);
     m.w1 = dual ? (const uint8_t*)up : nullptr;
@@ -788,12 +814,13 @@ static int gemm_experts(const chimere_moe_layer* w, const chimere_moe_prefill_we
     // the rows' Q8_1 planes: the workspace's, or (expert-parallel owner) the received packed rows in place
     const int8_t* xq = d_packed ? (const int8_t*)d_packed : ws->x_q;
     const float* xd = d_packed ? (const float*)((const uint8_t*)d_packed + w->H) : ws->x_d;
-    e = launch_gather_tiles(tiles, ws->perm, xq, d_packed ? row_bytes : w->H, xd, d_packed ? row_bytes / 4 : L.x_d_stride, base + A.bx, A.bx_col16,
-                            w->H, w->top_k, n_tiles_max, stream);
+    const bool sums = kshared(w);   // the shared expert's token tiles carry the blocks' sums
+    e = launch_gather_tiles(tiles, ws->perm, xq, d_packed ? row_bytes : w->H, xd, d_packed ? row_bytes / 4 : L.x_d_stride, ws->x_q8, base + A.bx, A.bx_col16,
+                            w->H, w->top_k, n_tiles_max, sums, stream);
     if (e != cudaSuccess) return cuda_rc(e);
     PrefillGemmParams g{};
     g.tiles = tiles; g.perm = ws->perm; g.status = ws->status;
-    g.T = T; g.top_k = w->top_k; g.H = w->H;
+    g.T = T; g.top_k = w->top_k; g.H = w->H; g.shared_sums = sums;
     for (int down = 0; down < 2 && e == cudaSuccess; ++down) {
         g.dual = !down && w->act == CHIMERE_ACT_SWIGLU;
         g.m[0] = gemm_mats(w, pw, false, down != 0);
@@ -813,11 +840,13 @@ int chimere_b200_moe_forward_prefill(const chimere_moe_layer* w, const chimere_m
     int rc = check_call(w, d_x, d_y, T, ws, true);
     if (rc) return rc;
     if (!pw || !ws->prefill_arena) return -1;
-    const bool ks = kshared(w);   // (a K-quant shared expert runs as GEMVs per token behind the routed part, at any batch size)
-    const chimere_moe_layer wr_ = ks ? routed_only(w) : *w;
+    // A K-quant shared expert goes through the GEMM with the routed ones where it can, else it follows as GEMVs per token.
+    const bool ks = kshared(w), gemm = ks && kshared_gemm(w) && pw->sh_gu && pw->sh_down;
+    const chimere_moe_layer wr_ = ks && !gemm ? routed_only(w) : *w;
     const chimere_moe_layer* wr = &wr_;
     if (wr->layout != CHIMERE_LAYOUT_TILED32 || !prefill_dims_ok(wr)) return -2;
-    RouteParams rp = route_params(wr, d_x, T, ws, ks);
+    const chimere_moe_layer route_ = ks ? routed_only(w) : *w;
+    RouteParams rp = route_params(&route_, d_x, T, ws, ks);
     rp.list_mode = 2;   // no work entries: the tile builder makes its own list
     cudaError_t e = launch_route(rp, stream);
     if (e != cudaSuccess) return cuda_rc(e);
@@ -827,7 +856,7 @@ int chimere_b200_moe_forward_prefill(const chimere_moe_layer* w, const chimere_m
     const float* shared_rows = wr->F_s > 0 ? ws->pair_out + (size_t)T * wr->top_k * wr->H : nullptr;
     const float* logit = (wr->F_s > 0 && wr->shexp_gate_w) ? ws->sh_gate_logit : nullptr;
     e = launch_ep_finish(ws->pair_out, nullptr, ws->topk_w, shared_rows, logit, d_y, T, wr->H, wr->top_k, stream);
-    if (e != cudaSuccess || !ks) return cuda_rc(e);
+    if (e != cudaSuccess || !ks || gemm) return cuda_rc(e);
     return kshared_chain(w, T, d_y, ws, stream);
 }
 

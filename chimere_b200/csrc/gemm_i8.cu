@@ -41,9 +41,9 @@ namespace chimere {
 constexpr int kG_MmaTile = 4096 + 512;       // operand of one block: 128 rows x 32 int8 in the MMA's order, then 128 f32 scales
 constexpr int kG_StageUnits = 4;             // 32-wide blocks per ring stage
 constexpr int kG_RawBytes = 9216;            // packed weights of a stage: 4 row tiles x 4 units x 576 (Q4_0, the largest)
-constexpr int kG_ASlot = kG_StageUnits * kG_MmaTile, kG_ASlots = 3;   // ring 2: the A operand
-constexpr int kG_RingSlotWide = kG_RawBytes + kG_StageUnits * 128 * 36, kG_RingSlotsWide = 3;
-constexpr int kG_RingSlotSlim = kG_RawBytes + kG_StageUnits * 32 * 36, kG_RingSlotsSlim = 6;   // tiles of up to 32 columns
+constexpr int kG_ASlot = kOperandMinStage, kG_ASlots = 3;   // ring 2: the A operand [4][kG_MmaTile], then (kTypeOperandMin) [4][128] minimums
+constexpr int kG_RingSlotWide = kG_RawBytes + kG_StageUnits * 128 * 40, kG_RingSlotsWide = 3;
+constexpr int kG_RingSlotSlim = kG_RawBytes + kG_StageUnits * 32 * 40, kG_RingSlotsSlim = 6;   // tiles of up to 32 columns
 constexpr int kG_RingBytes = kG_RingSlotWide * kG_RingSlotsWide;
 static_assert(kG_RingSlotSlim * kG_RingSlotsSlim <= kG_RingBytes, "both ring geometries share one area");
 static_assert(kG_RingSlotsWide == kG_ASlots && kG_RingSlotsSlim == 2 * kG_ASlots, "an A slot's last user is found from the ring-1 slot of that stage");
@@ -188,6 +188,7 @@ __device__ __forceinline__ int stage_unit(int type, int s) { return kG_StageUnit
 template <class Policy, class Params>
 __device__ __forceinline__ bool produce_tile(const Params& p, const GemmWork& w, GemmShared& sh, uint8_t* ring1, uint8_t* ring2, RingPos& pos, int lane) {
     const int type = uniform(Policy::type(p, w)), nb = uniform(w.nb), npad = uniform(w.npad);
+    const bool operand = type >= kTypeOperand;
     const int slim = npad <= 32;
     if (slim != pos.slim) {   // the other slot geometry: every slot of the old one has to be empty first
         for (int r = 0; r < pos.slots1(); ++r)
@@ -205,17 +206,19 @@ __device__ __forceinline__ bool produce_tile(const Params& p, const GemmWork& w,
         const int u0 = stage_unit(type, s), nu = min(kG_StageUnits, nb - u0);
         uint64_t* bar = &sh.full1[pos.r];
         bool ok = mbar_wait(&sh.empty1[pos.r], pos.released(pos.r));
-        if (ok && type == kTypeOperand) ok = mbar_wait(&sh.empty1[pos.lag()], pos.released(pos.lag()));
+        if (ok && operand) ok = mbar_wait(&sh.empty1[pos.lag()], pos.released(pos.lag()));
         if (!ok) { gemm_timeout(sh, p.status, lane); return false; }
         uint8_t* raw = ring1 + pos.slot1_off();
-        const uint32_t bbytes = (uint32_t)(nu * npad * 36);
+        // a token block: 32 values and a scale per column, beside weights with minimums the column's sum as well (by stages)
+        const uint32_t bcol = type == kTypeOperandMin ? 40u : 36u, bbytes = (uint32_t)(nu * npad) * bcol;
         // 4-bit types: bytes of one row tile, and where they start in it
         const uint32_t piece = type == CHIMERE_TYPE_Q4_0 ? (uint32_t)nu * 576u : (s & 1) ? 2048u : 2240u;
         const uint32_t off = type == CHIMERE_TYPE_Q4_0 ? (uint32_t)u0 * 576u : (uint32_t)(u0 >> 3) * 4288u + (uint32_t)(u0 & 4) * 512u;
         if (elect_one()) {
-            if (type == kTypeOperand) {
-                mbar_expect_tx(bar, (uint32_t)(nu * kG_MmaTile) + bbytes);
-                bulk_g2s(ring2 + (uint32_t)pos.e * kG_ASlot, src0 + (size_t)u0 * kG_MmaTile, (uint32_t)(nu * kG_MmaTile), bar);
+            if (operand) {
+                const uint32_t abytes = (uint32_t)nu * (type == kTypeOperand ? kG_MmaTile : kOperandMinStage / kG_StageUnits);
+                mbar_expect_tx(bar, abytes + bbytes);
+                bulk_g2s(ring2 + (uint32_t)pos.e * kG_ASlot, src0 + (size_t)u0 * (type == kTypeOperand ? kG_MmaTile : kOperandMinStage / kG_StageUnits), abytes, bar);
             } else {
                 mbar_expect_tx(bar, (n0 + n1) * piece + bbytes);
                 const uint8_t* a = src0 + off;
@@ -225,10 +228,10 @@ __device__ __forceinline__ bool produce_tile(const Params& p, const GemmWork& w,
                 if (n1 > 0) bulk_g2s(raw + kG_RawBytes / 2, b, piece, bar);
                 if (n1 > 1) bulk_g2s(raw + 3 * (kG_RawBytes / 4), b + tile_bytes, piece, bar);
             }
-            bulk_g2s(raw + kG_RawBytes, bsrc + (size_t)u0 * npad * 36, bbytes, bar);
+            bulk_g2s(raw + kG_RawBytes, bsrc + (size_t)u0 * (npad * bcol), bbytes, bar);
         }
         __syncwarp();
-        pos.next(type != kTypeOperand);
+        pos.next(!operand);
     }
     return true;
 }
@@ -264,7 +267,7 @@ __device__ __forceinline__ bool expand_tile(const Params& p, const GemmWork& w, 
     const int type = uniform(Policy::type(p, w)), nb = uniform(w.nb);
     pos.geometry(uniform(w.npad) <= 32);
     const int nstages = (nb + kG_StageUnits - 1) / kG_StageUnits;
-    if (type == kTypeOperand) {   // nothing to do but keep step
+    if (type >= kTypeOperand) {   // nothing to do but keep step
         for (int s = 0; s < nstages; ++s) pos.next(false);
         return true;
     }
@@ -316,7 +319,7 @@ __device__ __forceinline__ bool mma_tile(const Params& p, const GemmWork& w, Gem
     constexpr bool kWide = NPAD == 128, kHandshake = NPAD >= 64;
     // D format S32 (2 << 4), A and B signed int8 (1 << 7, 1 << 10), both K-major, N (>> 3 at bit 17), M = 128 (>> 4 at bit 24)
     constexpr uint32_t kIdesc = (2u << 4) | (1u << 7) | (1u << 10) | (((uint32_t)NPAD >> 3) << 17) | ((128u >> 4) << 24);
-    const bool expanded = uniform(Policy::type(p, w)) != kTypeOperand;
+    const bool expanded = uniform(Policy::type(p, w)) < kTypeOperand;
     const int nb = uniform(w.nb);
     if (NPAD != tp.npad) {   // another width lays the accumulators out differently: everything has to be read back first
         for (int r = 0; r < pos.slots1(); ++r)
@@ -379,10 +382,23 @@ __device__ __forceinline__ void block_values(const int (&v)[W], float sa, uint32
     }
 }
 
+// ... and the minimums of a block: acc[c] += m * s[c], s the token's sum over the block
+template <int W>
+__device__ __forceinline__ void block_minimums(float m, uint32_t sums, uint64_t* acc2) {
+    const uint64_t m2 = pack2f(m, m);
+#pragma unroll
+    for (int g = 0; g < W / 4; ++g) {
+        uint64_t s01, s23;
+        lds_2x64(sums + 16u * g, s01, s23);
+        acc2[2 * g + 0] = fma2(m2, s01, acc2[2 * g + 0]);
+        acc2[2 * g + 1] = fma2(m2, s23, acc2[2 * g + 1]);
+    }
+}
+
 // The read-back of one tile by one warp: column group colg of W columns; in tiles of up to 64 columns the warps of a column
 // group also share the stages among them (KG shares, stage s to share s % KG), so that a warp has that much longer for the
 // latency of one stage (barrier, TMEM load, scales: about a thousand cycles).
-template <int COLG, int KG, int W>
+template <int COLG, int KG, int W, bool MIN>
 __device__ __forceinline__ bool readback_tile(GemmShared& sh, uint32_t ring1, uint32_t ring2, uint32_t tmem, int32_t* status, int nb, bool expanded, int q,
                                               int part, int lane, RingPos& pos, TmemPos& tp, uint64_t* acc2) {
     constexpr int kPad = COLG * W, kBps = blocks_per_slot(kPad);
@@ -422,6 +438,9 @@ __device__ __forceinline__ bool readback_tile(GemmShared& sh, uint32_t ring1, ui
                             if (lane == 0) mbar_arrive_n(&sh.tempty[tp.slot], KG);
                         }
                         block_values<W, kPad == 128 ? 0u : 1u << 19>(v, sa, sb + (uint32_t)((j0 + i) * (kPad * 36)), acc2);
+                        if (MIN)
+                            block_minimums<W>(lds_f32(rec - 4096 + 4 * kG_MmaTile + (j0 + i) * 512),
+                                              sb - kPad * 32 + kG_StageUnits * kPad * 36 + (uint32_t)((j0 + i) * (kPad * 4)), acc2);
                     }
                 }
                 tp.next();
@@ -444,7 +463,9 @@ __device__ __forceinline__ bool readback(const Params& p, const GemmWork& w, Gem
     uint64_t acc2[W / 2];
 #pragma unroll
     for (int i = 0; i < W / 2; ++i) acc2[i] = 0ull;
-    bool ok = readback_tile<COLG, KG, W>(sh, ring1, ring2, tmem, p.status, uniform(w.nb), uniform(Policy::type(p, w)) != kTypeOperand, q, part, lane, pos, tp, acc2);
+    const int type = uniform(Policy::type(p, w)), nb = uniform(w.nb);
+    bool ok = type == kTypeOperandMin ? readback_tile<COLG, KG, W, true>(sh, ring1, ring2, tmem, p.status, nb, false, q, part, lane, pos, tp, acc2)
+                                      : readback_tile<COLG, KG, W, false>(sh, ring1, ring2, tmem, p.status, nb, type < kTypeOperand, q, part, lane, pos, tp, acc2);
     if (!mbar_wait(&sh.xempty, (xphase & 1u) ^ 1u)) { gemm_timeout(sh, p.status, lane); ok = false; }   // the tile before has been stored
     ++xphase;
     float* mine = xch + part * (W * 128) + q * 32 + lane;   // (part = share * COLG + column group)
@@ -641,7 +662,7 @@ struct MoePolicy {
     __device__ static __forceinline__ RowTiles rows(const PrefillGemmParams& p, const GemmWork& w) {
         const PrefillGemmMats& m = p.m[w.shared];
         RowTiles r{m.w0 + (size_t)w.expert * m.stride0, nullptr, (int)m.tile_bytes, 0, 0};
-        if (m.type == kTypeOperand) { r.src0 += (size_t)w.rt * w.nb * kG_MmaTile; return r; }
+        if (m.type >= kTypeOperand) { r.src0 += (size_t)w.rt * w.nb * (m.type == kTypeOperand ? kG_MmaTile : kOperandMinStage / kG_StageUnits); return r; }
         if (p.dual) {
             r.src0 += (size_t)(2 * w.rt) * m.tile_bytes;
             r.src1 = m.w1 + (size_t)w.expert * m.stride1 + (size_t)(2 * w.rt) * m.tile_bytes;
@@ -675,7 +696,10 @@ struct GateUpPolicy : MoePolicy {
         const int nrb = p.dual ? 2 : 4, rb = ew & (nrb - 1), blk = w.rt * nrb + rb;
         if (blk >= p.m[w.shared].rows32) return;     // (the last row tile may be partly filled)
         const int cstep = kG_EpiWarps / nrb, r = rb * 32 + lane;
-        uint8_t* dst = p.out_tiles + (size_t)w.col16 * p.out_col16_bytes + (size_t)blk * (w.npad * 36);
+        const bool sums = w.shared && p.shared_sums;   // the down matrix of the shared expert has minimums: it wants the blocks' sums too
+        uint8_t* tile = p.out_tiles + (size_t)w.col16 * p.out_col16_bytes;
+        uint8_t* dst = sums ? tile + (size_t)(blk >> 2) * (w.npad * 160) + (blk & 3) * (w.npad * 36) : tile + (size_t)blk * (w.npad * 36);
+        float* sdst = reinterpret_cast<float*>(tile + (size_t)(blk >> 2) * (w.npad * 160) + w.npad * 144 + (blk & 3) * (w.npad * 4));
         int8_t* qdst = reinterpret_cast<int8_t*>(dst) + (lane >> 4) * (w.npad * 16) + (lane & 15);
         float* ddst = reinterpret_cast<float*>(dst + w.npad * 32);
         for (int c = ew / nrb; c < w.n_valid; c += 2 * cstep) {
@@ -697,6 +721,12 @@ struct GateUpPolicy : MoePolicy {
                 if (ci < w.n_valid) {
                     qdst[(ci >> 3) * 128 + (ci & 7) * 16] = qv;
                     if (lane == 0) ddst[ci] = __half2float(__float2half(d));
+                }
+                if (sums) {
+                    float sum = v[i];
+#pragma unroll
+                    for (int k = 16; k > 0; k >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, k);
+                    if (lane == 0 && ci < w.n_valid) sdst[ci] = __half2float(__float2half(sum));
                 }
             }
         }
@@ -951,8 +981,8 @@ __global__ void __launch_bounds__(256) build_tiles_kernel(const int32_t* offsets
 // are the 8 x 16 bytes of one core-matrix row group, so every 128-byte segment of the tile is written whole, and a
 // token's 16-byte chunks are read four in a row.  Columns without a token are left as they are (nobody reads their sums).
 __global__ void __launch_bounds__(256) gather_tiles_kernel(const int32_t* tiles, const int32_t* perm, const int8_t* x_q, int64_t x_q_stride,
-                                                           const float* x_d, int x_d_stride, uint8_t* b_tiles, int64_t b_col16_bytes, int H,
-                                                           int top_k) {
+                                                           const float* x_d, int x_d_stride, const uint8_t* x_q8, uint8_t* b_tiles,
+                                                           int64_t b_col16_bytes, int H, int top_k, int shared_sums) {
     griddep_wait();
     if (threadIdx.x == 0) griddep_launch();
     const int j = blockIdx.x, grp = blockIdx.y;
@@ -963,13 +993,20 @@ __global__ void __launch_bounds__(256) gather_tiles_kernel(const int32_t* tiles,
     if (c >= t.z) return;
     const int tok = t.x < 0 ? t.y + c : __ldcg(perm + t.y + c) / top_k;
     uint8_t* base = b_tiles + (size_t)t.w * b_col16_bytes;
+    // a shared expert with minimums: stages of four blocks, each with the blocks' sums (the Q8_1 rows' second half) behind it
+    const bool sums = t.x < 0 && shared_sums;
+    auto block = [&](int b) { return base + (sums ? (size_t)(b >> 2) * (npad * 160) + (b & 3) * (npad * 36) : (size_t)b * (npad * 36)); };
     for (int ch = lane_ch; ch < H / 16; ch += 32) {
         const uint4 v = __ldcg(reinterpret_cast<const uint4*>(x_q + (size_t)tok * x_q_stride) + ch);
-        const int b = ch >> 1, khalf = ch & 1;
-        *reinterpret_cast<uint4*>(base + (size_t)b * (npad * 36) + khalf * (npad * 16) + grp * 128 + sl * 16) = v;
+        *reinterpret_cast<uint4*>(block(ch >> 1) + (ch & 1) * (npad * 16) + grp * 128 + sl * 16) = v;
     }
-    for (int b = lane_ch; b < H / 32; b += 32)
-        *reinterpret_cast<float*>(base + (size_t)b * (npad * 36) + npad * 32 + c * 4) = __ldcg(x_d + (size_t)tok * x_d_stride + b);
+    for (int b = lane_ch; b < H / 32; b += 32) {
+        *reinterpret_cast<float*>(block(b) + npad * 32 + c * 4) = __ldcg(x_d + (size_t)tok * x_d_stride + b);
+        if (sums) {
+            const uint32_t ds = __ldcg(reinterpret_cast<const uint32_t*>(x_q8 + ((size_t)tok * (H / 32) + b) * kQ81Bytes));
+            *reinterpret_cast<float*>(base + (size_t)(b >> 2) * (npad * 160) + npad * 144 + (b & 3) * (npad * 4) + c * 4) = h2f(ds >> 16);
+        }
+    }
 }
 
 cudaError_t launch_build_tiles(const int32_t* offsets, int32_t* tiles, int E, int T, int has_shared, cudaStream_t stream) {
@@ -977,9 +1014,11 @@ cudaError_t launch_build_tiles(const int32_t* offsets, int32_t* tiles, int E, in
 }
 
 cudaError_t launch_gather_tiles(const int32_t* tiles, const int32_t* perm, const int8_t* x_q, int64_t x_q_stride, const float* x_d,
-                                int x_d_stride, uint8_t* b_tiles, int64_t b_col16_bytes, int H, int top_k, int n_tiles_max, cudaStream_t stream) {
+                                int x_d_stride, const uint8_t* x_q8, uint8_t* b_tiles, int64_t b_col16_bytes, int H, int top_k, int n_tiles_max,
+                                bool shared_sums, cudaStream_t stream) {
     if (n_tiles_max <= 0) return cudaSuccess;
-    return launch_pdl(gather_tiles_kernel, dim3(n_tiles_max, 16), 256, 0, stream, tiles, perm, x_q, x_q_stride, x_d, x_d_stride, b_tiles, b_col16_bytes, H, top_k);
+    return launch_pdl(gather_tiles_kernel, dim3(n_tiles_max, 16), 256, 0, stream, tiles, perm, x_q, x_q_stride, x_d, x_d_stride, x_q8, b_tiles, b_col16_bytes,
+                      H, top_k, shared_sums ? 1 : 0);
 }
 
 }  // namespace chimere

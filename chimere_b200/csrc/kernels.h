@@ -157,13 +157,18 @@ struct PrefillGemmParams {
     float* pair_out;                                 // down: per-pair rows [pairs][H]
     int row_tiles_max;
     int dual, T, top_k, H;
+    int shared_sums;                 // gate/up: the shared expert's token tiles of the down GEMM carry block sums (kTypeOperandMin)
     int32_t* status;
 };
 cudaError_t launch_prefill_gemm(const PrefillGemmParams& p, bool down, int n_tiles_max, cudaStream_t stream);
 cudaError_t launch_build_tiles(const int32_t* offsets, int32_t* tiles, int E, int T, int has_shared, cudaStream_t stream);
 cudaError_t launch_gather_tiles(const int32_t* tiles, const int32_t* perm, const int8_t* x_q, int64_t x_q_stride, const float* x_d,
-                                int x_d_stride, uint8_t* b_tiles, int64_t b_col16_bytes, int H, int top_k, int n_tiles_max, cudaStream_t stream);
+                                int x_d_stride, const uint8_t* x_q8, uint8_t* b_tiles, int64_t b_col16_bytes, int H, int top_k, int n_tiles_max,
+                                bool shared_sums, cudaStream_t stream);
 constexpr int kTypeOperand = 100;    // PrefillGemmMats::type of weights in the MMA's own order (mma128 tiles)
+constexpr int kTypeOperandMin = 101; // ... with a minimum per row and block beside the scale (Q4_K, Q5_K), grouped by stages of four blocks
+constexpr int kOperandMinStage = 4 * (4096 + 512 + 512);
+cudaError_t launch_pack_operand_min(int type, const void* raw, void* out, int nrows, int ncols, int mode, cudaStream_t stream);
 cudaError_t launch_pack_mma128_q8_0(const void* raw, void* out, int n_mats, int nrows, int ncols, int mode, int64_t raw_stride, int64_t out_stride,
                                     cudaStream_t stream);
 cudaError_t launch_pack_mma128(const int8_t* q, const float* scales, uint8_t* out, int rows, int cols, cudaStream_t stream);

@@ -286,9 +286,9 @@ int chimere_b200_mma_i8_probe(int n_mma, int n_cols, int n_acc, int32_t* d_statu
 
 /* ------------------------------------------------------------ prefill-size batches -------- */
 /* For many tokens per call the expert products run as grouped block-scaled int8 GEMMs on the tensor cores
- * (the primitive above): experts with at least 8 routed tokens and the shared expert go to the GEMM, the rest
- * stay on the GEMV kernels.  The GEMM needs a second weight copy in its own layout (int8 values + f32 block
- * scales, gate and up rows interleaved per 64 rows): about 1.06x the Q8_0 bytes, 2x Q4_0, 2.3x IQ3_S. */
+ * (the primitive above).  Q4_0 and IQ3_S weights are read in the TILED32 form itself; Q8_0 matrices, and a shared expert in
+ * Q4_K / Q5_K super-blocks, need a copy in the MMA's own order (int8 values + f32 block scales, gate and up rows interleaved
+ * per 64 rows; 1.06x the Q8_0 bytes).  Pointers of matrices without a copy are null. */
 typedef struct chimere_moe_prefill_weights {
     const void* gu_exps;   int64_t stride_gu;     /* routed: gate|up tiles */
     const void* down_exps; int64_t stride_down;
@@ -304,7 +304,7 @@ int chimere_b200_moe_pack_prefill(const chimere_moe_layer* raw, void* d_arena, s
                                   chimere_moe_prefill_weights* out, cudaStream_t stream);
 /* Extra scratch the prefill path needs for up to max_T tokens; pass it with ws->prefill_arena / prefill_bytes. */
 size_t chimere_b200_moe_prefill_bytes(const chimere_moe_layer* w, int max_T);
-/* y = MoE(x) like chimere_b200_moe_forward; `w` TILED32 (used for the small experts), `pw` its GEMM copy. */
+/* y = MoE(x) like chimere_b200_moe_forward; `w` TILED32, `pw` what chimere_b200_moe_pack_prefill made of the same layer. */
 int chimere_b200_moe_forward_prefill(const chimere_moe_layer* w, const chimere_moe_prefill_weights* pw,
                                      const float* d_x, float* d_y, int T, chimere_moe_workspace* ws,
                                      cudaStream_t stream);
