@@ -200,6 +200,10 @@ static RouteParams route_params(const chimere_moe_layer* w, const float* d_x, in
     const Layout L = make_layout(w, ws->max_T);
     const size_t combine_ints = (size_t)L.n_counters - kCtrRouteTile - (ws->max_T + 7) / 8;
     const size_t need = (size_t)((T * w->top_k + 127) / 128) * 256 + 260;
+    // the router of a large batch rewrites its rows into the per-pair output area, which the down stage fills only later; its
+    // first T rows may hold the input (the residual + norm entry)
+    p.scratch = ws->pair_out + (size_t)T * w->H;
+    p.scratch_floats = ((size_t)ws->max_T * (w->top_k + (w->F_s > 0 ? 1 : 0)) - T) * w->H;
     p.dispatch_scratch = need <= combine_ints ? ws->counters + kCtrRouteTile + (ws->max_T + 7) / 8 : nullptr;
     return p;
 }

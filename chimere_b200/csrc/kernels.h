@@ -36,6 +36,8 @@ struct RouteParams {
     int32_t* status;            // workspace status word (may be null): a bounded wait that ran out raises a bit here
     int32_t* wait_flags;        // dispatch step alone (expert-parallel owner): counters of the peer-store exchange to wait for first
     int wait_n, wait_expect;    // ... `wait_n` of them, each has to reach `wait_expect`; they are taken down again (null = none)
+    float* scratch;             // room for the rewritten rows of a large batch's router (16-byte aligned; may be null)
+    size_t scratch_floats;
     int32_t* dispatch_scratch;  // zeroed scratch for the dispatch of large batches: ceil(T*top_k / 128) * 256 + 260 ints, left
                                 // zeroed again; null = always sort in one CTA
 };

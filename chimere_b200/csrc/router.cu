@@ -30,14 +30,11 @@ __device__ __forceinline__ float tree256(const float* r, int lane) {
 
 // Q8_1 of one 32-float block by one warp; lane = element.
 __device__ __forceinline__ void quantize_block_q8_1(float xi, uint8_t* out, int lane, int8_t* plane_q, float* plane_d) {
-    float amax = fabsf(xi), sum = xi;
+    float sum = xi;
 #pragma unroll
-    for (int m = 16; m > 0; m >>= 1) {
-        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, m));
-        sum += __shfl_xor_sync(0xffffffffu, sum, m);
-    }
-    const float d = amax / 127.0f;
-    const int8_t q = (amax == 0.0f) ? (int8_t)0 : (int8_t)roundf(xi / d);
+    for (int m = 16; m > 0; m >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, m);
+    float d;
+    const int8_t q = q8_1_warp(xi, d);
     reinterpret_cast<int8_t*>(out)[4 + lane] = q;
     const __half dh = __float2half(d);
     if (lane == 0) *reinterpret_cast<__half2*>(out) = __halves2half2(dh, __float2half(sum));
@@ -433,159 +430,198 @@ __global__ void __launch_bounds__(256) route_kernel(const RouteParams p) {
     build_dispatch(p, reinterpret_cast<int*>(smem_f), nullptr, (int)(TT * TE * 256) - kDispatchSmemInts);
 }
 
-// Larger batches.  The order of the additions is fixed (256 partial sums per output, tree of strides 128 .. 1), so
-// a thread can only ever own one partial of an output, and the operands of an output tile have to pass through the
-// SM once per tile: the kernel is bound by how many outputs a CTA can hold per router row it fetches.
-// CTA = kBigGroups token groups of 256 threads.  Thread (g, p) keeps elements p, p+256, ... of eight token rows in
-// registers and owns partial p of every output of its group; the router rows come four at a time through a ring of bulk
-// copies shared by the CTA's groups.  The 32 x 256 partial sums a group makes per step are left in shared memory and summed
-// by the group's eight warps, four outputs each, in the reference's order.  One group per CTA and two CTAs per SM measured
-// faster than two groups in one CTA (747 against 834 us at T = 8192, the same at T = 2048): the phases of a step
-// (multiply-adds, partial sums to shared memory, tree) use different units, and two independent CTAs overlap them where
-// two groups that share their barriers cannot.  A CTA whose row group starts at row 0
-// also writes the Q8_1 form of its tokens, from the values it holds anyway.
-// grid = (row groups, token tiles of kBigGroups * 8); NC = ceil(H / 256) <= 8 columns per thread; H a multiple of 32.
-constexpr int kBigGroups = 1;   // token groups (of 256 threads and kBigTT tokens) per CTA
-constexpr int kBigTT = 8, kBigTE = 4, kBigThreads = 256 * kBigGroups, kBigRing = kBigGroups == 1 ? 2 : 4;
-constexpr int kBigCtasPerSm = kBigGroups == 1 ? 2 : 1;
-constexpr int kBigRedFloats = kBigGroups * kBigTT * kBigTE * 256;        // [group][token][row][256] partial sums of one step
-static size_t big_route_smem(int H) { return (size_t)(kBigRedFloats + kBigRing * kBigTE * H) * sizeof(float); }
-// The same tree for two outputs whose partials are interleaved (partial i of the pair at r[2 * i], r[2 * i + 1]): one
-// 64-bit load serves both, two-wide adds keep each lane's order.  Valid in lane 0.
-__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) { uint64_t d; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
-__device__ __forceinline__ void tree256_pair(const float* r, int lane, float& v0, float& v1) {
-    const uint64_t* q = reinterpret_cast<const uint64_t*>(r);
-    const uint64_t a0 = add2(q[lane], q[lane + 128]);
-    const uint64_t a1 = add2(q[lane + 32], q[lane + 160]);
-    const uint64_t a2 = add2(q[lane + 64], q[lane + 192]);
-    const uint64_t a3 = add2(q[lane + 96], q[lane + 224]);
-    const uint64_t b0 = add2(a0, a2);
-    const uint64_t b1 = add2(a1, a3);
-    unpack2(add2(b0, b1), v0, v1);
+// Larger batches, as a register-tiled product.  The order of the additions is fixed (256 partial sums per output, partial p over
+// elements p, p+256, ..., then a tree of strides 128 .. 1), but a single thread can follow it: taking the partials in
+// bit-reversed order turns the tree into one over neighbours, which a binary counter of pending sums walks with one add per
+// partial.  So a thread owns 4 x 4 outputs (tokens x experts) and nothing is exchanged until the top levels of the tree, which
+// are split over WP warps of the CTA and meet in shared memory once at the end.
+//   route_prep_kernel : one CTA per token or router row: the row rewritten in that order (below), and for a token the Q8_1 form
+//                       and the shared expert's gate logit
+//   route_tile_kernel : CTA tile of 32 WT tokens x 16 WE experts; chunks of four partials come through a ring of bulk copies
+// Bound by the FMA pipe: 8 LDS.128 per 64 multiply-adds and thread.  (The form before it kept one partial of 32 outputs per
+// thread and passed 256 partials of every output through shared memory: 563 us at T = 8192, E = 256, H = 2048, 68 us at T = 512.)
+// Order of a row's copy: [chunk of 4 partials][row][4 partials x NQ x 4 elements, 4 floats of padding]; partial number n stands for
+// p = bit-reversed n.  The padding puts the rows a warp reads together on different banks.
+constexpr int kRoutePartials = 4, kRouteChunks = 256 / kRoutePartials;
+__host__ __device__ constexpr int route_pitch(int nq) { return 16 * nq + 4; }   // floats of a row in a chunk
+__host__ __device__ constexpr int route_nq(int H) { return (H + 1023) / 1024; }
+static size_t route_scratch_floats(int T, int E, int H) { return (size_t)(T + E) * kRouteChunks * route_pitch(route_nq(H)); }
+
+template <int NQ>
+__global__ void __launch_bounds__(256) route_prep_kernel(const RouteParams p) {
+    __shared__ float red[256];
+    constexpr int kPitch = route_pitch(NQ);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, H = p.H;
+    const bool token = (int)blockIdx.x < p.T;
+    const int row = token ? blockIdx.x : blockIdx.x - p.T, rows = token ? p.T : p.E;
+    const float* src = token ? p.x + (size_t)row * H : p.router_w + (size_t)row * H;
+    float v[4 * NQ];
+    if (token) griddep_wait();
 #pragma unroll
-    for (int s = 16; s > 0; s >>= 1) {
-        v0 += __shfl_down_sync(0xffffffffu, v0, s);
-        v1 += __shfl_down_sync(0xffffffffu, v1, s);
+    for (int i = 0; i < 4 * NQ; ++i) v[i] = i * 256 + tid < H ? src[i * 256 + tid] : 0.0f;
+    if (!token) griddep_wait();   // (the router's rows are constants; the scratch may still be in use)
+    if (tid == 0) griddep_launch();
+    const int n = (int)(__brev((unsigned)tid) >> 24);
+    float* dst = p.scratch + (token ? 0 : (size_t)p.T * kRouteChunks * kPitch);
+    dst += ((size_t)(n / kRoutePartials) * rows + row) * kPitch + (n % kRoutePartials) * (4 * NQ);
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) *reinterpret_cast<float4*>(dst + 4 * q) = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+    if (!token) return;
+    if (p.shexp_gate_w) {
+        float acc = 0.0f;
+#pragma unroll
+        for (int i = 0; i < 4 * NQ; ++i)
+            if (i * 256 + tid < H) acc = fmaf(__ldg(p.shexp_gate_w + i * 256 + tid), v[i], acc);
+        red[tid] = acc;
+    }
+    const int nbH = H >> 5;
+#pragma unroll
+    for (int i = 0; i < 4 * NQ; ++i) {
+        const int b = i * 8 + warp;
+        if (b < nbH) quantize_block_q8_1(v[i], p.x_q8 + ((size_t)row * nbH + b) * kQ81Bytes, lane, p.x_soa_q + (size_t)row * H + b * 32,
+                                         p.x_soa_d + (size_t)row * p.x_soa_d_stride + b);
+    }
+    if (p.shexp_gate_w) {
+        __syncthreads();
+        if (warp == 0) {
+            const float g = tree256(red, lane);
+            if (lane == 0) p.sh_gate_logit[row] = g;
+        }
     }
 }
 
-// EXACT: H == NC * 256 (the common case, H = 2048): no bounds tests and constant offsets in the inner loop.
-// The partial sums of two neighbouring tokens travel together (two-wide fused multiply-adds, each lane rounded like the
-// scalar instruction), so the sums of a step sit in shared memory as [group][token pair][row][partial][2].
-template <int NC, bool EXACT>
-__global__ void __launch_bounds__(kBigThreads, kBigCtasPerSm) route_big_kernel(const RouteParams p, int rows_per_group, int split_dispatch) {
-    extern __shared__ __align__(16) float smem_f[];   // [kBigRedFloats] partial sums, then [kBigRing][kBigTE][H] router rows
-    __shared__ __align__(8) uint64_t s_full[kBigRing];
+template <int NQ, int WT, int WE, int WP> struct RouteTile {
+    static constexpr int kTok = 32 * WT, kExp = 16 * WE, kPitch = route_pitch(NQ), kSteps = kRouteChunks / WP;
+    static constexpr int kGroup = (kTok + kExp) * kPitch, kStage = WP * kGroup;   // floats
+    static constexpr int kRing = WP == 8 ? 2 : 4;
+    static constexpr int kThreads = 32 * WT * WE * WP;
+    static constexpr size_t kSmem = (size_t)kRing * kStage * 4;
+    static_assert(kThreads == 256, "the dispatch step at the end is written for 256 threads");
+    static_assert(WP * kTok * kExp <= kRing * kStage && kRing * kStage >= kDispatchSmemInts + 8192, "what follows the product reuses the ring");
+};
+
+__device__ __forceinline__ float4 lds_f4(uint32_t a) {
+    float4 v;
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a));
+    return v;
+}
+
+// grid = (expert tiles, token tiles)
+template <int NQ, int WT, int WE, int WP>
+__global__ void __launch_bounds__(256, WP == 8 ? 2 : 1) route_tile_kernel(const RouteParams p, int split_dispatch) {
+    using R = RouteTile<NQ, WT, WE, WP>;
+    extern __shared__ __align__(128) float smem_f[];
+    __shared__ __align__(8) uint64_t s_full[R::kRing], s_empty[R::kRing];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int g = tid >> 8, pt = tid & 255;
-    const int H = EXACT ? NC * 256 : p.H, E = p.E;
-    const int nrows = E + (p.shexp_gate_w ? 1 : 0);
-    const int t0 = blockIdx.y * (kBigGroups * kBigTT) + g * kBigTT;
-    const int r_begin = blockIdx.x * rows_per_group, r_end = min(nrows, r_begin + rows_per_group);
-    const int nsteps = (r_end - r_begin + kBigTE - 1) / kBigTE;
-    if (tid == 0) griddep_launch();
-    float* ring = smem_f + kBigRedFloats;
-    auto wrow = [&](int r) -> const float* { return r < E ? p.router_w + (size_t)r * H : p.shexp_gate_w; };
-    // thread 0: the rows of step k into ring slot k % kBigRing (rows past r_end are not copied; what the slot holds in
-    // their place is multiplied and never stored)
+    const int T = p.T, E = p.E, t0 = blockIdx.y * R::kTok, e0 = blockIdx.x * R::kExp;
+    const int wp = warp % WP, we = (warp / WP) % WE, wt = warp / (WP * WE);
+    const float* xp = p.scratch;
+    const float* wpm = p.scratch + (size_t)T * kRouteChunks * R::kPitch;
+    // step k: chunk k of every warp's share of the partials
     auto ask = [&](int k) {
-        const int r = r_begin + kBigTE * k, slot = k % kBigRing;
-        const uint32_t bytes = (uint32_t)H * 4u;
-        const int n = min(kBigTE, r_end - r);
-        mbar_expect_tx(&s_full[slot], bytes * n);
-        for (int b = 0; b < n; ++b) bulk_g2s(ring + ((size_t)slot * kBigTE + b) * H, wrow(r + b), bytes, &s_full[slot]);
+        const int slot = k % R::kRing;
+        const uint32_t xb = (uint32_t)min(R::kTok, T - t0) * (R::kPitch * 4), wb = (uint32_t)min(R::kExp, E - e0) * (R::kPitch * 4);
+        mbar_expect_tx(&s_full[slot], WP * (xb + wb));
+        for (int g = 0; g < WP; ++g) {
+            const int c = g * R::kSteps + k;
+            float* d = smem_f + slot * R::kStage + g * R::kGroup;
+            bulk_g2s(d, xp + ((size_t)c * T + t0) * R::kPitch, xb, &s_full[slot]);
+            bulk_g2s(d + R::kTok * R::kPitch, wpm + ((size_t)c * E + e0) * R::kPitch, wb, &s_full[slot]);
+        }
     };
     if (tid == 0) {
-        for (int i = 0; i < kBigRing; ++i) mbar_init(&s_full[i], 1);
+        for (int i = 0; i < R::kRing; ++i) { mbar_init(&s_full[i], 1); mbar_init(&s_empty[i], 8); }
         mbar_fence_init();
-        for (int k = 0; k < kBigRing && k < nsteps; ++k) ask(k);
     }
-    // what is added to a row's sums before they are stored (a load from global memory at that point would put a trip
-    // to L2 behind every output of every step)
-    __shared__ float s_bias[kMaxExperts + 1];
-    for (int e = tid; e <= kMaxExperts; e += kBigThreads) s_bias[e] = (p.router_bias && e < E) ? p.router_bias[e] : 0.0f;
-    uint64_t xv2[kBigTT / 2][NC];   // elements pt + 256 i of tokens (2 a2, 2 a2 + 1)
-    {
-        const int nbH = H >> 5;
-#pragma unroll
-        for (int a2 = 0; a2 < kBigTT / 2; ++a2)
-#pragma unroll
-            for (int i = 0; i < NC; ++i) {
-                const int j = i * 256 + pt, ta = t0 + 2 * a2;
-                const bool in = EXACT || j < H;
-                const float x0 = (in && ta < p.T) ? p.x[(size_t)ta * H + j] : 0.0f;
-                const float x1 = (in && ta + 1 < p.T) ? p.x[(size_t)(ta + 1) * H + j] : 0.0f;
-                xv2[a2][i] = pack2f(x0, x1);
-                if (blockIdx.x == 0) {
-                    // Q8_1 of this group's tokens: a warp's 32 threads hold one 32-element block per (token, i)
-                    const int b = i * 8 + (pt >> 5);
-                    if (b < nbH && ta < p.T)   // (uniform over the warp)
-                        quantize_block_q8_1(x0, p.x_q8 + ((size_t)ta * nbH + b) * kQ81Bytes, lane, p.x_soa_q + (size_t)ta * H + b * 32,
-                                            p.x_soa_d + (size_t)ta * p.x_soa_d_stride + b);
-                    if (b < nbH && ta + 1 < p.T)
-                        quantize_block_q8_1(x1, p.x_q8 + ((size_t)(ta + 1) * nbH + b) * kQ81Bytes, lane, p.x_soa_q + (size_t)(ta + 1) * H + b * 32,
-                                            p.x_soa_d + (size_t)(ta + 1) * p.x_soa_d_stride + b);
-                }
-            }
+    __syncthreads();
+    griddep_wait();
+    if (tid == 0) {
+        griddep_launch();
+        for (int k = 0; k < R::kRing && k < R::kSteps; ++k) ask(k);
     }
-    __syncthreads();   // barriers initialised
-    float* red = smem_f + g * (kBigTT * kBigTE * 256) + 2 * pt;   // this thread's pair slot of every (token pair, row)
-    for (int k = 0; k < nsteps; ++k) {
-        const int r = r_begin + kBigTE * k, slot = k % kBigRing;
-        if (!mbar_wait(&s_full[slot], (uint32_t)((k / kBigRing) & 1))) {
-            if (p.status && tid == 0) atomicOr(p.status, kStatusWaitTimeout);   // a wait ran out: leave a mark, go on
-            mbar_wait(&s_full[slot], (uint32_t)((k / kBigRing) & 1));
+    // this thread: tokens tg + 8 a, experts eg + 4 b of its warp's 32 x 16
+    const int tg = lane & 7, eg = lane >> 3;
+    const uint32_t xs0 = smem_u32(smem_f) + 4u * (wp * R::kGroup + (wt * 32 + tg) * R::kPitch);
+    const uint32_t ws0 = smem_u32(smem_f) + 4u * (wp * R::kGroup + (R::kTok + we * 16 + eg) * R::kPitch);
+    constexpr int kLevels = R::kSteps == 8 ? 3 : R::kSteps == 16 ? 4 : 5;
+    float st[kLevels][16], v[16];
+    bool ok = true;
+    for (int k = 0; k < R::kSteps; ++k) {
+        const int slot = k % R::kRing;
+        if (tid == 0 && k > 0 && k - 1 + R::kRing < R::kSteps) {   // the slot of the step before is free when every warp has read it
+            ok = ok && mbar_wait(&s_empty[(k - 1) % R::kRing], (uint32_t)(((k - 1) / R::kRing) & 1));
+            if (ok) ask(k - 1 + R::kRing);
         }
-        const float* w0 = ring + (size_t)slot * kBigTE * H + pt;
-        uint64_t acc2[kBigTT / 2][kBigTE];
+        __syncwarp();
+        if (!mbar_wait(&s_full[slot], (uint32_t)((k / R::kRing) & 1))) { ok = false; break; }
+        const uint32_t xs = xs0 + 4u * (slot * R::kStage), ws = ws0 + 4u * (slot * R::kStage);
+        float pend[16];
 #pragma unroll
-        for (int a2 = 0; a2 < kBigTT / 2; ++a2)
+        for (int j = 0; j < kRoutePartials; ++j) {
+            float acc[16];
 #pragma unroll
-            for (int b = 0; b < kBigTE; ++b) acc2[a2][b] = 0ull;
+            for (int i = 0; i < 16; ++i) acc[i] = 0.0f;
 #pragma unroll
-        for (int i = 0; i < NC; ++i) {   // ascending j, one fused multiply-add per output each
-            if (EXACT || i * 256 + pt < H) {
+            for (int q = 0; q < NQ; ++q) {
+                float4 w[4];
 #pragma unroll
-                for (int b = 0; b < kBigTE; ++b) {
-                    const float w = w0[b * H + i * 256];
-                    const uint64_t w2 = pack2f(w, w);
+                for (int b = 0; b < 4; ++b) w[b] = lds_f4(ws + 4u * (4 * b * R::kPitch + (j * NQ + q) * 4));
 #pragma unroll
-                    for (int a2 = 0; a2 < kBigTT / 2; ++a2) acc2[a2][b] = fma2(w2, xv2[a2][i], acc2[a2][b]);
-                }
-            }
-        }
-        if (k > 0) __syncthreads();   // the sums of the previous step have been read
+                for (int a = 0; a < 4; ++a) {
+                    const float4 x = lds_f4(xs + 4u * (8 * a * R::kPitch + (j * NQ + q) * 4));
 #pragma unroll
-        for (int a2 = 0; a2 < kBigTT / 2; ++a2)
-#pragma unroll
-            for (int b = 0; b < kBigTE; ++b) *reinterpret_cast<uint64_t*>(red + (a2 * kBigTE + b) * 512) = acc2[a2][b];
-        __syncthreads();   // partial sums complete; every thread is done with this ring slot
-        if (tid == 0 && k + kBigRing < nsteps) {
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            ask(k + kBigRing);
-        }
-        // sixteen warps, two (token pair, row) sums each: warp = (group, token pair, row half)
-        {
-            const int og = warp >> 3, a2 = (warp >> 1) & 3, bh = warp & 1;
-            const float* rb = smem_f + og * (kBigTT * kBigTE * 256) + a2 * (kBigTE * 512);
-            const int t = blockIdx.y * (kBigGroups * kBigTT) + og * kBigTT + 2 * a2;
-#pragma unroll
-            for (int bb = 0; bb < kBigTE / 2; ++bb) {
-                const int b = bh * (kBigTE / 2) + bb, rr = r + b;
-                float v0, v1;
-                tree256_pair(rb + b * 512, lane, v0, v1);
-                if (lane == 0 && rr < r_end) {
-                    const float bias = s_bias[rr];
-                    if (rr < E) {
-                        if (t < p.T) p.router_logits[(size_t)t * E + rr] = p.router_bias ? v0 + bias : v0;
-                        if (t + 1 < p.T) p.router_logits[(size_t)(t + 1) * E + rr] = p.router_bias ? v1 + bias : v1;
-                    } else {
-                        if (t < p.T) p.sh_gate_logit[t] = v0;
-                        if (t + 1 < p.T) p.sh_gate_logit[t + 1] = v1;
+                    for (int b = 0; b < 4; ++b) {   // ascending elements, one fused multiply-add each
+                        acc[4 * a + b] = fmaf(w[b].x, x.x, acc[4 * a + b]);
+                        acc[4 * a + b] = fmaf(w[b].y, x.y, acc[4 * a + b]);
+                        acc[4 * a + b] = fmaf(w[b].z, x.z, acc[4 * a + b]);
+                        acc[4 * a + b] = fmaf(w[b].w, x.w, acc[4 * a + b]);
                     }
                 }
             }
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+                if (j == 0) v[i] = acc[i];
+                else if (j == 1) v[i] += acc[i];
+                else if (j == 2) pend[i] = acc[i];
+                else v[i] += pend[i] + acc[i];
+            }
         }
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cta(&s_empty[slot]);
+        // the binary counter: v completes level after level as long as that level has a pending left half
+#pragma unroll
+        for (int l = 0; l < kLevels; ++l) {
+            if ((k >> l) & 1) {
+#pragma unroll
+                for (int i = 0; i < 16; ++i) v[i] += st[l][i];
+            } else {
+#pragma unroll
+                for (int i = 0; i < 16; ++i) st[l][i] = v[i];
+                break;
+            }
+        }
+    }
+    if (!ok && lane == 0 && p.status) atomicOr(p.status, kStatusWaitTimeout);
+    if (tid == 0) {   // (only after a wait ran out are there copies in flight here)
+        if (!ok) for (int i = 0; i < R::kRing; ++i) mbar_wait(&s_full[i], 0), mbar_wait(&s_full[i], 1);
+    }
+    __syncthreads();   // the ring is no longer read: the warps' shares of every output meet in its memory
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int b = 0; b < 4; ++b)
+            smem_f[(wp * R::kTok + wt * 32 + tg + 8 * a) * R::kExp + we * 16 + eg + 4 * b] = v[4 * a + b];
+    __syncthreads();
+    for (int o = tid; o < R::kTok * R::kExp; o += 256) {
+        float s[WP];
+#pragma unroll
+        for (int g = 0; g < WP; ++g) s[g] = smem_f[g * (R::kTok * R::kExp) + o];
+#pragma unroll
+        for (int h = 1; h < WP; h <<= 1)
+#pragma unroll
+            for (int g = 0; g < WP; g += 2 * h) s[g] += s[g + h];
+        const int t = t0 + o / R::kExp, e = e0 + o % R::kExp;
+        if (t < T && e < E) p.router_logits[(size_t)t * E + e] = p.router_bias ? s[0] + p.router_bias[e] : s[0];
     }
 
     // ---- last CTA of the token tile: scores and top-k, one warp per token ----
@@ -595,18 +631,16 @@ __global__ void __launch_bounds__(kBigThreads, kBigCtasPerSm) route_big_kernel(c
     __syncthreads();
     if (!s_flag) return;
     if (tid == 0) p.counters[kCtrRouteTile + blockIdx.y] = 0;
-    {
-        const int t = blockIdx.y * (kBigGroups * kBigTT) + warp;
-        if (t < p.T) topk_warp(p, p.router_logits + (size_t)t * E, t, lane, smem_f + warp * 256, nullptr);
-    }
-    if (split_dispatch) return;   // three small launches follow and do the dispatch over the whole GPU
-    // ---- last token tile overall: dispatch permutation and work list (the first 256 threads) ----
+    for (int i = warp; i < R::kTok; i += 8)
+        if (t0 + i < T) topk_warp(p, p.router_logits + (size_t)(t0 + i) * E, t0 + i, lane, smem_f + warp * 256, nullptr);
+    if (split_dispatch) return;   // small launches follow and do the dispatch over the whole GPU
+    // ---- last token tile overall: dispatch permutation and work list ----
     __syncthreads();   // every thread's writes are ordered before thread 0's counter increment, which releases them
     if (tid == 0) s_flag = (atom_add_acq_rel_gpu(&p.counters[kCtrRouteAll], 1) == (int)gridDim.y - 1);   // ... and acquires the other CTAs'
     __syncthreads();
-    if (!s_flag || tid >= 256) return;
+    if (!s_flag) return;
     if (tid == 0) p.counters[kCtrRouteAll] = 0;
-    build_dispatch(p, reinterpret_cast<int*>(smem_f), nullptr, kBigRedFloats - kDispatchSmemInts);
+    build_dispatch(p, reinterpret_cast<int*>(smem_f), nullptr, R::kRing * R::kStage - kDispatchSmemInts);
 }
 
 // ---- dispatch of a large batch in three small launches --------------------------------------
@@ -635,21 +669,38 @@ __global__ void __launch_bounds__(kDispatchChunk) dispatch_hist_kernel(const Rou
     }
 }
 
-// One CTA of 256: thread = expert.  hist[chunk][e] becomes the number of pairs of expert e in earlier chunks.
-__global__ void __launch_bounds__(256) dispatch_scan_kernel(const RouteParams p, int32_t* hist, int nchunks) {
+// One CTA of 1024: thread = (quarter of the chunks, expert).  hist[chunk][e] becomes the number of pairs of expert e in earlier
+// chunks.  Two passes over the counts (sums of the quarters, then the running counts), sixteen independent loads in flight: the
+// latency of a serial walk over the chunks was the kernel (26 us at 512 chunks by 256 threads with eight loads in flight).
+__global__ void __launch_bounds__(1024) dispatch_scan_kernel(const RouteParams p, int32_t* hist, int nchunks) {
     __shared__ int scan[16];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    int run = 0;
+    __shared__ int part[4][256];
+    const int tid = threadIdx.x & 255, quarter = threadIdx.x >> 8, lane = tid & 31, warp = tid >> 5;
+    const int per = (nchunks + 3) / 4, c0 = min(nchunks, quarter * per), c1 = min(nchunks, c0 + per);
     int32_t* col = hist + tid;
-    int c = 0;
-    for (; c + 8 <= nchunks; c += 8) {   // eight independent loads in flight
-        int v[8];
+    constexpr int kBatch = 16;
+    int sum = 0;
+    for (int c = c0; c < c1; c += kBatch) {
+        int v[kBatch];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) v[i] = col[(size_t)(c + i) * 256];
+        for (int i = 0; i < kBatch; ++i) v[i] = c + i < c1 ? col[(size_t)(c + i) * 256] : 0;
 #pragma unroll
-        for (int i = 0; i < 8; ++i) { col[(size_t)(c + i) * 256] = run; run += v[i]; }
+        for (int i = 0; i < kBatch; ++i) sum += v[i];
     }
-    for (; c < nchunks; ++c) { const int v = col[(size_t)c * 256]; col[(size_t)c * 256] = run; run += v; }
+    part[quarter][tid] = sum;
+    __syncthreads();
+    int run = 0;
+    for (int q = 0; q < quarter; ++q) run += part[q][tid];
+    for (int c = c0; c < c1; c += kBatch) {
+        int v[kBatch];
+#pragma unroll
+        for (int i = 0; i < kBatch; ++i) v[i] = c + i < c1 ? col[(size_t)(c + i) * 256] : 0;
+#pragma unroll
+        for (int i = 0; i < kBatch; ++i)
+            if (c + i < c1) { col[(size_t)(c + i) * 256] = run; run += v[i]; }
+    }
+    if (quarter > 0) return;
+    run = part[0][tid] + part[1][tid] + part[2][tid] + part[3][tid];
     const int cnt = tid < p.E ? run : 0;
     const int nent = (cnt + kMaxGroupTokens - 1) / kMaxGroupTokens;
     int incl_c = cnt, incl_n = nent;
@@ -659,7 +710,7 @@ __global__ void __launch_bounds__(256) dispatch_scan_kernel(const RouteParams p,
         if (lane >= sft) { incl_c += a; incl_n += b; }
     }
     if (lane == 31) { scan[warp] = incl_c; scan[8 + warp] = incl_n; }
-    __syncthreads();
+    dispatch_sync();   // (the first quarter's 256 threads)
     int base_c = 0, base_n = 0;
     for (int w = 0; w < warp; ++w) { base_c += scan[w]; base_n += scan[8 + w]; }
     int32_t* ent_base = hist + (size_t)nchunks * 256;   // [257] first routed entry of each expert, then their number
@@ -726,7 +777,7 @@ __global__ void __launch_bounds__(kDispatchChunk) dispatch_place_kernel(const Ro
 static cudaError_t launch_dispatch_split(const RouteParams& p, cudaStream_t stream) {
     const int nchunks = dispatch_chunks(p.T * p.top_k);
     dispatch_hist_kernel<<<nchunks, kDispatchChunk, 0, stream>>>(p, p.dispatch_scratch);
-    dispatch_scan_kernel<<<1, 256, 0, stream>>>(p, p.dispatch_scratch, nchunks);
+    dispatch_scan_kernel<<<1, 1024, 0, stream>>>(p, p.dispatch_scratch, nchunks);
     dispatch_place_kernel<<<nchunks, kDispatchChunk, 0, stream>>>(p, p.dispatch_scratch, nchunks);
     return cudaGetLastError();
 }
@@ -764,22 +815,38 @@ __global__ void __launch_bounds__(256) permute_kernel(const RouteParams p) {
 // Final step of an expert-parallel layer on the tokens' home rank: routing-weighted sum of the k expert
 // rows of every token in slot order (weighted_combine_kernel, chimere_kernels.cu:1551-1565) plus the
 // sigmoid-gated shared expert (sigmoid_gate_add_kernel, scratch_pool.rs:266-277).
-__global__ void ep_finish_kernel(const float* rows, const int32_t* slot, const float* topk_w, const float* shared_rows,
-                                 const float* sh_logit, float* y, int T, int H, int k) {
+// HBM-bound: T * (k + 1) rows in, T out.  Four elements per thread and every row's load issued before the first is used
+// (k <= kMaxTopK): 161 us with one element and one load at a time at T = 8192, k = 8, H = 2048.
+__global__ void __launch_bounds__(256) ep_finish_kernel(const float* __restrict__ rows, const int32_t* __restrict__ slot, const float* __restrict__ topk_w,
+                                                        const float* __restrict__ shared_rows, const float* __restrict__ sh_logit, float* __restrict__ y,
+                                                        int T, int H, int k) {
+    griddep_wait();
+    if (threadIdx.x == 0) griddep_launch();
     const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= (int64_t)T * H) return;
-    const int t = (int)(idx / H), h = (int)(idx - (int64_t)t * H);
-    float sum = 0.0f;
-    for (int j = 0; j < k; ++j) {
-        const size_t r = slot ? (size_t)slot[t * k + j] : (size_t)t * k + j;   // where pair (t, j) came back
-        sum = fmaf(topk_w[(size_t)t * k + j], rows[r * H + h], sum);
-    }
+    const int h4 = H >> 2;
+    if (idx >= (int64_t)T * h4) return;
+    const int t = (int)(idx / h4), h = (int)(idx - (int64_t)t * h4) * 4;
+    float4 v[kMaxTopK], sh;
+    float w[kMaxTopK];
+#pragma unroll
+    for (int j = 0; j < kMaxTopK; ++j)
+        if (j < k) {
+            const size_t r = slot ? (size_t)slot[t * k + j] : (size_t)t * k + j;   // where pair (t, j) came back
+            v[j] = __ldcs(reinterpret_cast<const float4*>(rows + r * H + h));
+            w[j] = topk_w[(size_t)t * k + j];
+        }
+    if (shared_rows) sh = __ldcs(reinterpret_cast<const float4*>(shared_rows + (size_t)t * H + h));
+    float4 sum = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+    for (int j = 0; j < kMaxTopK; ++j)
+        if (j < k) { sum.x = fmaf(w[j], v[j].x, sum.x); sum.y = fmaf(w[j], v[j].y, sum.y); sum.z = fmaf(w[j], v[j].z, sum.z); sum.w = fmaf(w[j], v[j].w, sum.w); }
     if (shared_rows) {
-        const float sh = shared_rows[(size_t)t * H + h];
-        if (sh_logit) sum = fmaf(sh, sigmoid_ref(sh_logit[t]), sum);
-        else sum = sh + sum;
+        if (sh_logit) {
+            const float g = sigmoid_ref(sh_logit[t]);
+            sum.x = fmaf(sh.x, g, sum.x); sum.y = fmaf(sh.y, g, sum.y); sum.z = fmaf(sh.z, g, sum.z); sum.w = fmaf(sh.w, g, sum.w);
+        } else { sum.x += sh.x; sum.y += sh.y; sum.z += sh.z; sum.w += sh.w; }
     }
-    y[idx] = sum;
+    *reinterpret_cast<float4*>(y + (size_t)t * H + h) = sum;
 }
 
 // Fixed-size dispatch of an expert-parallel layer.  Slot s = (destination rank d, position i) of the send
@@ -1026,10 +1093,9 @@ cudaError_t launch_routing_trace(const int32_t* topk_idx, uint8_t* trace, int32_
 
 cudaError_t launch_ep_finish(const float* rows, const int32_t* slot, const float* topk_w, const float* shared_rows, const float* sh_logit,
                              float* y, int T, int H, int k, cudaStream_t stream) {
-    const int64_t n = (int64_t)T * H;
+    const int64_t n = (int64_t)T * (H / 4);   // (H is a multiple of 32)
     if (n <= 0) return cudaSuccess;
-    ep_finish_kernel<<<(unsigned)((n + 255) / 256), 256, 0, stream>>>(rows, slot, topk_w, shared_rows, sh_logit, y, T, H, k);
-    return cudaGetLastError();
+    return launch_pdl(ep_finish_kernel, dim3((unsigned)((n + 255) / 256)), 256, 0, stream, rows, slot, topk_w, shared_rows, sh_logit, y, T, H, k);
 }
 
 // Exact-size dispatch (prefill-size batches): the routing kernel's dispatch has already sorted the pairs by expert, and the
@@ -1063,35 +1129,40 @@ cudaError_t launch_ep_pack(const int32_t* topk_idx, const int8_t* x_q, const flo
     return cudaGetLastError();
 }
 
+template <int NQ, int WT, int WE, int WP>
+static cudaError_t launch_route_tile_t(const RouteParams& p, cudaStream_t stream) {
+    using R = RouteTile<NQ, WT, WE, WP>;
+    static bool attr_done[64] = {};
+    cudaError_t e = max_smem_once(route_tile_kernel<NQ, WT, WE, WP>, (int)R::kSmem, attr_done);
+    if (e != cudaSuccess) return e;
+    const bool split = use_split_dispatch(p);
+    e = launch_pdl(route_tile_kernel<NQ, WT, WE, WP>, dim3((p.E + R::kExp - 1) / R::kExp, (p.T + R::kTok - 1) / R::kTok), R::kThreads, R::kSmem, stream, p,
+                   split ? 1 : 0);
+    return e == cudaSuccess && split ? launch_dispatch_split(p, stream) : e;
+}
+// A tile of 64 tokens x 32 experts reads half the bytes per output of one of 32 x 16, but a CTA takes 20 us over it whatever the
+// batch: small tiles (5 us, eight warps sharing the partials) until the large ones fill the GPU.
+template <int NQ>
+static cudaError_t launch_route_tiles(const RouteParams& p, cudaStream_t stream) {
+    cudaError_t e = launch_pdl(route_prep_kernel<NQ>, dim3(p.T + p.E), 256, 0, stream, p);
+    if (e != cudaSuccess) return e;
+    const bool large = (int64_t)((p.T + 63) / 64) * ((p.E + 31) / 32) >= sm_count();
+    return large ? launch_route_tile_t<NQ, 2, 2, 2>(p, stream) : launch_route_tile_t<NQ, 1, 1, 8>(p, stream);
+}
+
 cudaError_t launch_route(const RouteParams& p, cudaStream_t stream) {
     const int nrows = p.E + (p.shexp_gate_w ? 1 : 0);
     if (p.T <= 32) {
         constexpr int TT = 8, TE = 2;
         dim3 grid((nrows + TE - 1) / TE, (p.T + TT - 1) / TT);
         return launch_pdl(route_kernel<TT, TE>, grid, 256, route_smem(TT, TE), stream, p);
-    } else if (p.H <= 2048 && p.H % 32 == 0) {
-        // token tiles of kBigGroups * 8; the router rows are cut into row groups (multiples of four rows) only while there are too few
-        // token tiles to fill the GPU, because every row group fetches its tokens again
-        const int token_tiles = (p.T + kBigGroups * kBigTT - 1) / (kBigGroups * kBigTT);
-        int groups = sm_count() * kBigCtasPerSm / token_tiles;   // (rounded down: a second wave of a few CTAs would double the time)
-        const int max_groups = (nrows + kBigTE - 1) / kBigTE;
-        groups = groups < 1 ? 1 : (groups > max_groups ? max_groups : groups);
-        const int rows_per_group = kBigTE * (((nrows + groups - 1) / groups + kBigTE - 1) / kBigTE);
-        const dim3 grid((nrows + rows_per_group - 1) / rows_per_group, token_tiles);
-        const size_t smem = big_route_smem(p.H);
-        static bool attr_done[64] = {};
-        static bool attr_done_x[64] = {};
-        const bool split = use_split_dispatch(p);
-        if (p.H == 2048) {
-            cudaError_t e = max_smem_once(route_big_kernel<8, true>, (int)big_route_smem(2048), attr_done_x);
-            if (e != cudaSuccess) return e;
-            route_big_kernel<8, true><<<grid, kBigThreads, smem, stream>>>(p, rows_per_group, split ? 1 : 0);
-        } else {
-            cudaError_t e = max_smem_once(route_big_kernel<8, false>, (int)big_route_smem(2048), attr_done);
-            if (e != cudaSuccess) return e;
-            route_big_kernel<8, false><<<grid, kBigThreads, smem, stream>>>(p, rows_per_group, split ? 1 : 0);
+    } else if (p.scratch && p.H <= 4096 && route_scratch_floats(p.T, p.E, p.H) <= p.scratch_floats) {
+        switch (route_nq(p.H)) {
+            case 1: return launch_route_tiles<1>(p, stream);
+            case 2: return launch_route_tiles<2>(p, stream);
+            case 3: return launch_route_tiles<3>(p, stream);
+            default: return launch_route_tiles<4>(p, stream);
         }
-        if (split) return launch_dispatch_split(p, stream);
     } else {
         constexpr int TT = 8, TE = 8;
         static bool attr_done[64] = {};
