@@ -437,13 +437,17 @@ __global__ void __launch_bounds__(256) route_kernel(const RouteParams p) {
 // are split over WP warps of the CTA and meet in shared memory once at the end.
 //   route_prep_kernel : one CTA per token or router row: the row rewritten in that order (below), and for a token the Q8_1 form
 //                       and the shared expert's gate logit
-//   route_tile_kernel : CTA tile of 32 WT tokens x 16 WE experts; chunks of four partials come through a ring of bulk copies
-// Bound by the FMA pipe: 8 LDS.128 per 64 multiply-adds and thread.  (The form before it kept one partial of 32 outputs per
-// thread and passed 256 partials of every output through shared memory: 563 us at T = 8192, E = 256, H = 2048, 68 us at T = 512.)
-// Order of a row's copy: [chunk of 4 partials][row][4 partials x NQ x 4 elements, 4 floats of padding]; partial number n stands for
+//   route_tile_kernel : CTA tile of 32 tokens x 16 experts, its eight warps with an eighth of the partials each; chunks of two
+//                       partials come through a ring of bulk copies of every warp's own (no CTA barrier until the end)
+//   route_topk_kernel : scores and top-k, one warp per token; the last CTA does the dispatch
+// Bound by the FMA pipe and its operands: 8 LDS.128 per 64 multiply-adds and thread.  (The form before it kept one partial of 32
+// outputs per thread and passed all 256 partials of every output through shared memory: 563 us at T = 8192, E = 256, H = 2048, 68 us
+// at T = 512.  Tiles of 64 x 32 with the partials split over two warps read half the bytes per output, but a CTA of them takes 40 us
+// whatever the batch, and at T = 8192 they are no faster.)
+// Order of a row's copy: [chunk of 2 partials][row][2 partials x NQ x 4 elements, 4 floats of padding]; partial number n stands for
 // p = bit-reversed n.  The padding puts the rows a warp reads together on different banks.
-constexpr int kRoutePartials = 4, kRouteChunks = 256 / kRoutePartials;
-__host__ __device__ constexpr int route_pitch(int nq) { return 16 * nq + 4; }   // floats of a row in a chunk
+constexpr int kRoutePartials = 2, kRouteChunks = 256 / kRoutePartials;
+__host__ __device__ constexpr int route_pitch(int nq) { return 4 * kRoutePartials * nq + 4; }   // floats of a row in a chunk
 __host__ __device__ constexpr int route_nq(int H) { return (H + 1023) / 1024; }
 static size_t route_scratch_floats(int T, int E, int H) { return (size_t)(T + E) * kRouteChunks * route_pitch(route_nq(H)); }
 
@@ -490,14 +494,11 @@ __global__ void __launch_bounds__(256) route_prep_kernel(const RouteParams p) {
     }
 }
 
-template <int NQ, int WT, int WE, int WP> struct RouteTile {
-    static constexpr int kTok = 32 * WT, kExp = 16 * WE, kPitch = route_pitch(NQ), kSteps = kRouteChunks / WP;
-    static constexpr int kGroup = (kTok + kExp) * kPitch, kStage = WP * kGroup;   // floats
-    static constexpr int kRing = WP == 8 ? 2 : 4;
-    static constexpr int kThreads = 32 * WT * WE * WP;
-    static constexpr size_t kSmem = (size_t)kRing * kStage * 4;
-    static_assert(kThreads == 256, "the dispatch step at the end is written for 256 threads");
-    static_assert(WP * kTok * kExp <= kRing * kStage && kRing * kStage >= kDispatchSmemInts + 8192, "what follows the product reuses the ring");
+template <int NQ> struct RouteTile {
+    static constexpr int kTok = 32, kExp = 16, kWarps = 8, kPitch = route_pitch(NQ), kSteps = kRouteChunks / kWarps;
+    static constexpr int kStage = (kTok + kExp) * kPitch, kRing = NQ <= 2 ? 3 : 2;   // floats of a warp's stage; two CTAs per SM
+    static constexpr size_t kSmem = (size_t)kWarps * kRing * kStage * 4;
+    static_assert(kTok * kExp <= kRing * kStage, "the shares of the outputs meet in the ring's memory");
 };
 
 __device__ __forceinline__ float4 lds_f4(uint32_t a) {
@@ -507,55 +508,46 @@ __device__ __forceinline__ float4 lds_f4(uint32_t a) {
 }
 
 // grid = (expert tiles, token tiles)
-template <int NQ, int WT, int WE, int WP>
-__global__ void __launch_bounds__(256, WP == 8 ? 2 : 1) route_tile_kernel(const RouteParams p, int split_dispatch) {
-    using R = RouteTile<NQ, WT, WE, WP>;
+template <int NQ>
+__global__ void __launch_bounds__(256, 2) route_tile_kernel(const RouteParams p) {
+    using R = RouteTile<NQ>;
     extern __shared__ __align__(128) float smem_f[];
-    __shared__ __align__(8) uint64_t s_full[R::kRing], s_empty[R::kRing];
+    __shared__ __align__(8) uint64_t s_full[R::kWarps][R::kRing];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int T = p.T, E = p.E, t0 = blockIdx.y * R::kTok, e0 = blockIdx.x * R::kExp;
-    const int wp = warp % WP, we = (warp / WP) % WE, wt = warp / (WP * WE);
-    const float* xp = p.scratch;
-    const float* wpm = p.scratch + (size_t)T * kRouteChunks * R::kPitch;
-    // step k: chunk k of every warp's share of the partials
-    auto ask = [&](int k) {
-        const int slot = k % R::kRing;
-        const uint32_t xb = (uint32_t)min(R::kTok, T - t0) * (R::kPitch * 4), wb = (uint32_t)min(R::kExp, E - e0) * (R::kPitch * 4);
-        mbar_expect_tx(&s_full[slot], WP * (xb + wb));
-        for (int g = 0; g < WP; ++g) {
-            const int c = g * R::kSteps + k;
-            float* d = smem_f + slot * R::kStage + g * R::kGroup;
-            bulk_g2s(d, xp + ((size_t)c * T + t0) * R::kPitch, xb, &s_full[slot]);
-            bulk_g2s(d + R::kTok * R::kPitch, wpm + ((size_t)c * E + e0) * R::kPitch, wb, &s_full[slot]);
-        }
+    float* ring = smem_f + warp * (R::kRing * R::kStage);
+    uint64_t* full = s_full[warp];
+    const uint32_t xb = (uint32_t)min(R::kTok, T - t0) * (R::kPitch * 4), wb = (uint32_t)min(R::kExp, E - e0) * (R::kPitch * 4);
+    const float* xsrc = p.scratch + ((size_t)(warp * R::kSteps) * T + t0) * R::kPitch;
+    const float* wsrc = p.scratch + ((size_t)T * kRouteChunks + (size_t)(warp * R::kSteps) * E + e0) * R::kPitch;
+    auto ask = [&](int slot) {   // the warp's next chunk (lane 0)
+        mbar_expect_tx(&full[slot], xb + wb);
+        bulk_g2s(ring + slot * R::kStage, xsrc, xb, &full[slot]);
+        bulk_g2s(ring + slot * R::kStage + R::kTok * R::kPitch, wsrc, wb, &full[slot]);
+        xsrc += (size_t)T * R::kPitch;
+        wsrc += (size_t)E * R::kPitch;
     };
-    if (tid == 0) {
-        for (int i = 0; i < R::kRing; ++i) { mbar_init(&s_full[i], 1); mbar_init(&s_empty[i], 8); }
+    if (lane == 0) {
+        for (int i = 0; i < R::kRing; ++i) mbar_init(&full[i], 1);
         mbar_fence_init();
     }
-    __syncthreads();
     griddep_wait();
-    if (tid == 0) {
-        griddep_launch();
-        for (int k = 0; k < R::kRing && k < R::kSteps; ++k) ask(k);
-    }
-    // this thread: tokens tg + 8 a, experts eg + 4 b of its warp's 32 x 16
+    if (tid == 0) griddep_launch();
+    if (lane == 0)
+        for (int k = 0; k < R::kRing; ++k) ask(k);
+    __syncwarp();
+    // this thread: tokens tg + 8 a, experts eg + 4 b
     const int tg = lane & 7, eg = lane >> 3;
-    const uint32_t xs0 = smem_u32(smem_f) + 4u * (wp * R::kGroup + (wt * 32 + tg) * R::kPitch);
-    const uint32_t ws0 = smem_u32(smem_f) + 4u * (wp * R::kGroup + (R::kTok + we * 16 + eg) * R::kPitch);
-    constexpr int kLevels = R::kSteps == 8 ? 3 : R::kSteps == 16 ? 4 : 5;
+    const uint32_t xs0 = smem_u32(ring) + 4u * (tg * R::kPitch), ws0 = smem_u32(ring) + 4u * ((R::kTok + eg) * R::kPitch);
+    constexpr int kLevels = 4;
+    static_assert(R::kSteps == 1 << kLevels, "a warp's chunks are the leaves of its part of the tree");
     float st[kLevels][16], v[16];
     bool ok = true;
+    uint32_t phase = 0;
+    int slot = 0;
     for (int k = 0; k < R::kSteps; ++k) {
-        const int slot = k % R::kRing;
-        if (tid == 0 && k > 0 && k - 1 + R::kRing < R::kSteps) {   // the slot of the step before is free when every warp has read it
-            ok = ok && mbar_wait(&s_empty[(k - 1) % R::kRing], (uint32_t)(((k - 1) / R::kRing) & 1));
-            if (ok) ask(k - 1 + R::kRing);
-        }
-        __syncwarp();
-        if (!mbar_wait(&s_full[slot], (uint32_t)((k / R::kRing) & 1))) { ok = false; break; }
+        if (!mbar_wait(&full[slot], phase)) { ok = false; break; }
         const uint32_t xs = xs0 + 4u * (slot * R::kStage), ws = ws0 + 4u * (slot * R::kStage);
-        float pend[16];
 #pragma unroll
         for (int j = 0; j < kRoutePartials; ++j) {
             float acc[16];
@@ -579,15 +571,11 @@ __global__ void __launch_bounds__(256, WP == 8 ? 2 : 1) route_tile_kernel(const 
                 }
             }
 #pragma unroll
-            for (int i = 0; i < 16; ++i) {
-                if (j == 0) v[i] = acc[i];
-                else if (j == 1) v[i] += acc[i];
-                else if (j == 2) pend[i] = acc[i];
-                else v[i] += pend[i] + acc[i];
-            }
+            for (int i = 0; i < 16; ++i) v[i] = j == 0 ? acc[i] : v[i] + acc[i];
         }
-        __syncwarp();
-        if (lane == 0) mbar_arrive_cta(&s_empty[slot]);
+        __syncwarp();   // every lane has read the slot
+        if (lane == 0 && k + R::kRing < R::kSteps) ask(slot);
+        if (++slot == R::kRing) { slot = 0; phase ^= 1u; }
         // the binary counter: v completes level after level as long as that level has a pending left half
 #pragma unroll
         for (int l = 0; l < kLevels; ++l) {
@@ -601,46 +589,43 @@ __global__ void __launch_bounds__(256, WP == 8 ? 2 : 1) route_tile_kernel(const 
             }
         }
     }
-    if (!ok && lane == 0 && p.status) atomicOr(p.status, kStatusWaitTimeout);
-    if (tid == 0) {   // (only after a wait ran out are there copies in flight here)
-        if (!ok) for (int i = 0; i < R::kRing; ++i) mbar_wait(&s_full[i], 0), mbar_wait(&s_full[i], 1);
+    if (!ok && lane == 0) {
+        if (p.status) atomicOr(p.status, kStatusWaitTimeout);
+        for (int i = 0; i < R::kRing; ++i) { mbar_wait(&full[i], 0); mbar_wait(&full[i], 1); }   // its copies have to land before this memory goes away
     }
-    __syncthreads();   // the ring is no longer read: the warps' shares of every output meet in its memory
+    __syncwarp();
+    // the warps' shares of every output, each in its own ring's memory (row pitch 17: the lanes of a store on different banks)
 #pragma unroll
     for (int a = 0; a < 4; ++a)
 #pragma unroll
-        for (int b = 0; b < 4; ++b)
-            smem_f[(wp * R::kTok + wt * 32 + tg + 8 * a) * R::kExp + we * 16 + eg + 4 * b] = v[4 * a + b];
+        for (int b = 0; b < 4; ++b) ring[(tg + 8 * a) * 17 + eg + 4 * b] = v[4 * a + b];
     __syncthreads();
     for (int o = tid; o < R::kTok * R::kExp; o += 256) {
-        float s[WP];
+        const int r = o / R::kExp, c = o % R::kExp, t = t0 + r, e = e0 + c;
+        float s[R::kWarps];
 #pragma unroll
-        for (int g = 0; g < WP; ++g) s[g] = smem_f[g * (R::kTok * R::kExp) + o];
-#pragma unroll
-        for (int h = 1; h < WP; h <<= 1)
-#pragma unroll
-            for (int g = 0; g < WP; g += 2 * h) s[g] += s[g + h];
-        const int t = t0 + o / R::kExp, e = e0 + o % R::kExp;
-        if (t < T && e < E) p.router_logits[(size_t)t * E + e] = p.router_bias ? s[0] + p.router_bias[e] : s[0];
+        for (int g = 0; g < R::kWarps; ++g) s[g] = smem_f[g * (R::kRing * R::kStage) + r * 17 + c];
+        const float sum = ((s[0] + s[1]) + (s[2] + s[3])) + ((s[4] + s[5]) + (s[6] + s[7]));
+        if (t < T && e < E) p.router_logits[(size_t)t * E + e] = p.router_bias ? sum + p.router_bias[e] : sum;
     }
+}
 
-    // ---- last CTA of the token tile: scores and top-k, one warp per token ----
+// Scores and top-k, one warp per token; unless the dispatch follows as launches of its own, the last CTA does it.
+constexpr int kTopkIdsRoom = 4096;
+__global__ void __launch_bounds__(256) route_topk_kernel(const RouteParams p, int split_dispatch) {
+    extern __shared__ __align__(16) float smem_f[];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, t = blockIdx.x * 8 + warp;
     __shared__ int s_flag;
+    griddep_wait();
+    if (tid == 0) griddep_launch();
+    if (t < p.T) topk_warp(p, p.router_logits + (size_t)t * p.E, t, lane, smem_f + warp * 256, nullptr);
+    if (split_dispatch) return;
     __syncthreads();   // every thread's writes are ordered before thread 0's counter increment, which releases them
-    if (tid == 0) s_flag = (atom_add_acq_rel_gpu(&p.counters[kCtrRouteTile + blockIdx.y], 1) == (int)gridDim.x - 1);   // ... and acquires the other CTAs'
-    __syncthreads();
-    if (!s_flag) return;
-    if (tid == 0) p.counters[kCtrRouteTile + blockIdx.y] = 0;
-    for (int i = warp; i < R::kTok; i += 8)
-        if (t0 + i < T) topk_warp(p, p.router_logits + (size_t)(t0 + i) * E, t0 + i, lane, smem_f + warp * 256, nullptr);
-    if (split_dispatch) return;   // small launches follow and do the dispatch over the whole GPU
-    // ---- last token tile overall: dispatch permutation and work list ----
-    __syncthreads();   // every thread's writes are ordered before thread 0's counter increment, which releases them
-    if (tid == 0) s_flag = (atom_add_acq_rel_gpu(&p.counters[kCtrRouteAll], 1) == (int)gridDim.y - 1);   // ... and acquires the other CTAs'
+    if (tid == 0) s_flag = (atom_add_acq_rel_gpu(&p.counters[kCtrRouteAll], 1) == (int)gridDim.x - 1);   // ... and acquires the other CTAs'
     __syncthreads();
     if (!s_flag) return;
     if (tid == 0) p.counters[kCtrRouteAll] = 0;
-    build_dispatch(p, reinterpret_cast<int*>(smem_f), nullptr, R::kRing * R::kStage - kDispatchSmemInts);
+    build_dispatch(p, reinterpret_cast<int*>(smem_f), nullptr, kTopkIdsRoom);
 }
 
 // ---- dispatch of a large batch in three small launches --------------------------------------
@@ -1129,25 +1114,18 @@ cudaError_t launch_ep_pack(const int32_t* topk_idx, const int8_t* x_q, const flo
     return cudaGetLastError();
 }
 
-template <int NQ, int WT, int WE, int WP>
-static cudaError_t launch_route_tile_t(const RouteParams& p, cudaStream_t stream) {
-    using R = RouteTile<NQ, WT, WE, WP>;
-    static bool attr_done[64] = {};
-    cudaError_t e = max_smem_once(route_tile_kernel<NQ, WT, WE, WP>, (int)R::kSmem, attr_done);
-    if (e != cudaSuccess) return e;
-    const bool split = use_split_dispatch(p);
-    e = launch_pdl(route_tile_kernel<NQ, WT, WE, WP>, dim3((p.E + R::kExp - 1) / R::kExp, (p.T + R::kTok - 1) / R::kTok), R::kThreads, R::kSmem, stream, p,
-                   split ? 1 : 0);
-    return e == cudaSuccess && split ? launch_dispatch_split(p, stream) : e;
-}
-// A tile of 64 tokens x 32 experts reads half the bytes per output of one of 32 x 16, but a CTA takes 20 us over it whatever the
-// batch: small tiles (5 us, eight warps sharing the partials) until the large ones fill the GPU.
 template <int NQ>
 static cudaError_t launch_route_tiles(const RouteParams& p, cudaStream_t stream) {
-    cudaError_t e = launch_pdl(route_prep_kernel<NQ>, dim3(p.T + p.E), 256, 0, stream, p);
+    using R = RouteTile<NQ>;
+    static bool attr_done[64] = {};
+    cudaError_t e = max_smem_once(route_tile_kernel<NQ>, (int)R::kSmem, attr_done);
+    if (e == cudaSuccess) e = launch_pdl(route_prep_kernel<NQ>, dim3(p.T + p.E), 256, 0, stream, p);
+    if (e == cudaSuccess) e = launch_pdl(route_tile_kernel<NQ>, dim3((p.E + R::kExp - 1) / R::kExp, (p.T + R::kTok - 1) / R::kTok), 256, R::kSmem, stream, p);
     if (e != cudaSuccess) return e;
-    const bool large = (int64_t)((p.T + 63) / 64) * ((p.E + 31) / 32) >= sm_count();
-    return large ? launch_route_tile_t<NQ, 2, 2, 2>(p, stream) : launch_route_tile_t<NQ, 1, 1, 8>(p, stream);
+    const bool split = use_split_dispatch(p);
+    const size_t smem = (split ? 2048 : kDispatchSmemInts + kTopkIdsRoom) * 4;
+    e = launch_pdl(route_topk_kernel, dim3((p.T + 7) / 8), 256, smem, stream, p, split ? 1 : 0);
+    return e == cudaSuccess && split ? launch_dispatch_split(p, stream) : e;
 }
 
 cudaError_t launch_route(const RouteParams& p, cudaStream_t stream) {
