@@ -496,8 +496,10 @@ __global__ void __launch_bounds__(256) route_prep_kernel(const RouteParams p) {
 
 template <int NQ> struct RouteTile {
     static constexpr int kTok = 32, kExp = 16, kWarps = 8, kPitch = route_pitch(NQ), kSteps = kRouteChunks / kWarps;
-    static constexpr int kStage = (kTok + kExp) * kPitch, kRing = NQ <= 2 ? 3 : 2;   // floats of a warp's stage; two CTAs per SM
-    static constexpr size_t kSmem = (size_t)kWarps * kRing * kStage * 4;
+    static constexpr int kStage = (kTok + kExp) * kPitch, kRing = 2;   // floats of a warp's stage; two CTAs per SM up to NQ = 2
+    static constexpr int kLevels = 4, kPending = (kLevels - 1) * 16 * 256;   // pending sums of the levels above the first
+    static constexpr size_t kSmem = ((size_t)kWarps * kRing * kStage + kPending) * 4;
+    static_assert(kSteps == 1 << kLevels, "a warp's chunks are the leaves of its part of the tree");
     static_assert(kTok * kExp <= kRing * kStage, "the shares of the outputs meet in the ring's memory");
 };
 
@@ -539,9 +541,10 @@ __global__ void __launch_bounds__(256, 2) route_tile_kernel(const RouteParams p)
     // this thread: tokens tg + 8 a, experts eg + 4 b
     const int tg = lane & 7, eg = lane >> 3;
     const uint32_t xs0 = smem_u32(ring) + 4u * (tg * R::kPitch), ws0 = smem_u32(ring) + 4u * ((R::kTok + eg) * R::kPitch);
-    constexpr int kLevels = 4;
-    static_assert(R::kSteps == 1 << kLevels, "a warp's chunks are the leaves of its part of the tree");
-    float st[kLevels][16], v[16];
+    // pending sums: the first level's in registers, the others in shared memory, thread beside thread (a register file of them
+    // would leave one CTA per SM, local memory costs a small batch 10 us of first touches)
+    float* st = smem_f + R::kWarps * R::kRing * R::kStage + tid;
+    float pend[16], v[16];
     bool ok = true;
     uint32_t phase = 0;
     int slot = 0;
@@ -562,12 +565,13 @@ __global__ void __launch_bounds__(256, 2) route_tile_kernel(const RouteParams p)
                 for (int a = 0; a < 4; ++a) {
                     const float4 x = lds_f4(xs + 4u * (8 * a * R::kPitch + (j * NQ + q) * 4));
 #pragma unroll
-                    for (int b = 0; b < 4; ++b) {   // ascending elements, one fused multiply-add each
-                        acc[4 * a + b] = fmaf(w[b].x, x.x, acc[4 * a + b]);
-                        acc[4 * a + b] = fmaf(w[b].y, x.y, acc[4 * a + b]);
-                        acc[4 * a + b] = fmaf(w[b].z, x.z, acc[4 * a + b]);
-                        acc[4 * a + b] = fmaf(w[b].w, x.w, acc[4 * a + b]);
-                    }
+                    for (int b = 0; b < 4; ++b) acc[4 * a + b] = fmaf(w[b].x, x.x, acc[4 * a + b]);   // ascending elements, one fused multiply-add each
+#pragma unroll
+                    for (int b = 0; b < 4; ++b) acc[4 * a + b] = fmaf(w[b].y, x.y, acc[4 * a + b]);
+#pragma unroll
+                    for (int b = 0; b < 4; ++b) acc[4 * a + b] = fmaf(w[b].z, x.z, acc[4 * a + b]);
+#pragma unroll
+                    for (int b = 0; b < 4; ++b) acc[4 * a + b] = fmaf(w[b].w, x.w, acc[4 * a + b]);
                 }
             }
 #pragma unroll
@@ -577,14 +581,22 @@ __global__ void __launch_bounds__(256, 2) route_tile_kernel(const RouteParams p)
         if (lane == 0 && k + R::kRing < R::kSteps) ask(slot);
         if (++slot == R::kRing) { slot = 0; phase ^= 1u; }
         // the binary counter: v completes level after level as long as that level has a pending left half
+        if (!(k & 1)) {
 #pragma unroll
-        for (int l = 0; l < kLevels; ++l) {
+            for (int i = 0; i < 16; ++i) pend[i] = v[i];
+            continue;
+        }
+#pragma unroll
+        for (int i = 0; i < 16; ++i) v[i] += pend[i];
+#pragma unroll
+        for (int l = 1; l < R::kLevels; ++l) {
+            float* sl = st + (l - 1) * 16 * 256;
             if ((k >> l) & 1) {
 #pragma unroll
-                for (int i = 0; i < 16; ++i) v[i] += st[l][i];
+                for (int i = 0; i < 16; ++i) v[i] += sl[i * 256];
             } else {
 #pragma unroll
-                for (int i = 0; i < 16; ++i) st[l][i] = v[i];
+                for (int i = 0; i < 16; ++i) sl[i * 256] = v[i];
                 break;
             }
         }
@@ -1114,6 +1126,9 @@ cudaError_t launch_ep_pack(const int32_t* topk_idx, const int8_t* x_q, const flo
     return cudaGetLastError();
 }
 
+// The tiled product's three launches start to pay where the simple kernel (a CTA per 8 tokens x 8 experts, partials through shared
+// memory) fills the GPU more than once: 19.6 against 29 us at 61 x 257 outputs of H = 2048, 32 against 33 at 130 x 257.
+constexpr int64_t kRouteTileWork = 32768;
 template <int NQ>
 static cudaError_t launch_route_tiles(const RouteParams& p, cudaStream_t stream) {
     using R = RouteTile<NQ>;
@@ -1134,7 +1149,7 @@ cudaError_t launch_route(const RouteParams& p, cudaStream_t stream) {
         constexpr int TT = 8, TE = 2;
         dim3 grid((nrows + TE - 1) / TE, (p.T + TT - 1) / TT);
         return launch_pdl(route_kernel<TT, TE>, grid, 256, route_smem(TT, TE), stream, p);
-    } else if (p.scratch && p.H <= 4096 && route_scratch_floats(p.T, p.E, p.H) <= p.scratch_floats) {
+    } else if (p.scratch && (int64_t)p.T * p.E > kRouteTileWork && p.H <= 4096 && route_scratch_floats(p.T, p.E, p.H) <= p.scratch_floats) {
         switch (route_nq(p.H)) {
             case 1: return launch_route_tiles<1>(p, stream);
             case 2: return launch_route_tiles<2>(p, stream);
