@@ -49,7 +49,7 @@ static_assert(kG_RingSlotSlim * kG_RingSlotsSlim <= kG_RingBytes, "both ring geo
 static_assert(kG_RingSlotsWide == kG_ASlots && kG_RingSlotsSlim == 2 * kG_ASlots, "an A slot's last user is found from the ring-1 slot of that stage");
 constexpr int kG_ConstBytes = 4096;          // operand of the constant MMA
 constexpr int kG_XchFloats = 128 * 128;      // exchange buffer [K share][column][128 rows]: 1 x 128, 2 x 64 or 4 x 32 columns
-constexpr int kG_ExpWarps = 2, kG_EpiWarps = 4, kG_RbWarps = 16;
+constexpr int kG_ExpWarps = 2, kG_EpiWarps = 4, kG_RbWarps = 16, kG_SlimExpWarps = 8;
 constexpr int kG_FirstEpi = 4, kG_FirstRb = 8;
 constexpr int kG_Threads = 32 * (kG_FirstRb + kG_RbWarps);
 // Registers: the launch gives every thread 80; the read-back warps take 88 (512 x 88) and leave 64 to the others (256 x 64).
@@ -241,34 +241,40 @@ __device__ __forceinline__ bool produce_tile(const Params& p, const GemmWork& w,
 // Warp x expands row tiles x and x + 2; all loads of a stage go out first (the compiler keeps the order of the
 // shared-memory accesses as written).
 template <int TYPE>
-__device__ __forceinline__ void expand_units(uint32_t raw, uint32_t a, int x, int lane) {
+__device__ __forceinline__ void expand_unit(const uint4& v, uint32_t dst) {
     constexpr uint32_t kOdd = TYPE == CHIMERE_TYPE_IQ3_S ? 0x08080808u : 0u;   // 8 * (2c + 1) = 16c + 8
-    constexpr uint32_t kTilePitch = kG_RawBytes / 4, kUnitPitch = TYPE == CHIMERE_TYPE_IQ3_S ? 512 : 576;
-    const uint32_t src = raw + (uint32_t)x * kTilePitch + lane * 16, dst = a + (uint32_t)x * 512 + lane * 16;
+    uint4 lo, hi;
+    lo.x = ((v.x << 4) & 0xF0F0F0F0u) ^ (0x80808080u | kOdd); hi.x = (v.x & 0xF0F0F0F0u) | kOdd;
+    lo.y = ((v.y << 4) & 0xF0F0F0F0u) ^ (0x80808080u | kOdd); hi.y = (v.y & 0xF0F0F0F0u) | kOdd;
+    lo.z = ((v.z << 4) & 0xF0F0F0F0u) ^ (0x80808080u | kOdd); hi.z = (v.z & 0xF0F0F0F0u) | kOdd;
+    lo.w = ((v.w << 4) & 0xF0F0F0F0u) ^ (0x80808080u | kOdd); hi.w = (v.w & 0xF0F0F0F0u) | kOdd;
+    sts128(dst, lo);
+    sts128(dst + 2048, hi);
+}
+constexpr uint32_t kRawTile = kG_RawBytes / 4;   // a row tile's packed units in a ring slot
+template <int TYPE> __host__ __device__ constexpr uint32_t raw_unit() { return TYPE == CHIMERE_TYPE_IQ3_S ? 512 : 576; }
+template <int TYPE>
+__device__ __forceinline__ void expand_units(uint32_t raw, uint32_t a, int x, int lane) {
+    const uint32_t src = raw + (uint32_t)x * kRawTile + lane * 16, dst = a + (uint32_t)x * 512 + lane * 16;
     uint4 v[8];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) v[i] = lds128(src + (i & 1) * 2 * kTilePitch + (i >> 1) * kUnitPitch);   // (units past nu: bytes nobody uses)
+    for (int i = 0; i < 8; ++i) v[i] = lds128(src + (i & 1) * 2 * kRawTile + (i >> 1) * raw_unit<TYPE>());   // (units past nu: bytes nobody uses)
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        uint4 lo, hi;
-        lo.x = ((v[i].x << 4) & 0xF0F0F0F0u) ^ (0x80808080u | kOdd); hi.x = (v[i].x & 0xF0F0F0F0u) | kOdd;
-        lo.y = ((v[i].y << 4) & 0xF0F0F0F0u) ^ (0x80808080u | kOdd); hi.y = (v[i].y & 0xF0F0F0F0u) | kOdd;
-        lo.z = ((v[i].z << 4) & 0xF0F0F0F0u) ^ (0x80808080u | kOdd); hi.z = (v[i].z & 0xF0F0F0F0u) | kOdd;
-        lo.w = ((v[i].w << 4) & 0xF0F0F0F0u) ^ (0x80808080u | kOdd); hi.w = (v[i].w & 0xF0F0F0F0u) | kOdd;
-        const uint32_t d = dst + (i >> 1) * kG_MmaTile + (i & 1) * 1024;
-        sts128(d, lo);
-        sts128(d + 2048, hi);
-    }
+    for (int i = 0; i < 8; ++i) expand_unit<TYPE>(v[i], dst + (i >> 1) * kG_MmaTile + (i & 1) * 1024);
 }
 
 // Warps 2..3: warp x takes row tiles x and x + 2 of every stage.
 template <class Policy, class Params>
 __device__ __forceinline__ bool expand_tile(const Params& p, const GemmWork& w, GemmShared& sh, uint32_t ring1, uint32_t ring2, RingPos& pos, int x, int lane) {
     const int type = uniform(Policy::type(p, w)), nb = uniform(w.nb);
-    pos.geometry(uniform(w.npad) <= 32);
+    const bool slim = uniform(w.npad) <= 32;
+    pos.geometry(slim);
     const int nstages = (nb + kG_StageUnits - 1) / kG_StageUnits;
-    if (type >= kTypeOperand) {   // nothing to do but keep step
-        for (int s = 0; s < nstages; ++s) pos.next(false);
+    if (type >= kTypeOperand || slim) {   // nothing to do (slim tiles: half of the read-back warps expand) but keep step
+        for (int s = 0; s + 1 < nstages; ++s) pos.next(type < kTypeOperand);
+        // (parity tells a barrier's phases apart only within a round: see the tile's last bytes arrive before going on)
+        if (!mbar_wait(&sh.full1[pos.r], pos.par1())) { gemm_timeout(sh, p.status, lane); return false; }
+        pos.next(type < kTypeOperand);
         return true;
     }
     float d3[2] = {0.0f, 0.0f};        // IQ3_S: this lane's rows' scales of the super-block, kept over its two stages
@@ -302,7 +308,7 @@ __device__ __forceinline__ bool expand_tile(const Params& p, const GemmWork& w, 
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the MMAs read what ordinary stores wrote
         __syncwarp();
-        if (lane == 0) mbar_arrive_cta(&sh.xfull2[pos.e]);
+        if (lane == 0) mbar_arrive_n(&sh.xfull2[pos.e], kG_SlimExpWarps / kG_ExpWarps);
         pos.next(true);
     }
     return true;
@@ -435,7 +441,7 @@ __device__ __forceinline__ bool readback_tile(GemmShared& sh, uint32_t ring1, ui
                         if (kHandshake && i + 1 == cnt) {   // the slot's last values are in registers: the MMAs may overwrite it
                             tc_fence_before();
                             __syncwarp();
-                            if (lane == 0) mbar_arrive_n(&sh.tempty[tp.slot], KG);
+                            if (lane == 0) mbar_arrive_n(&sh.tempty[tp.slot], 4 / COLG);
                         }
                         block_values<W, kPad == 128 ? 0u : 1u << 19>(v, sa, sb + (uint32_t)((j0 + i) * (kPad * 36)), acc2);
                         if (MIN)
@@ -447,7 +453,7 @@ __device__ __forceinline__ bool readback_tile(GemmShared& sh, uint32_t ring1, ui
             }
             if (!kHandshake) tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive_n(&sh.empty1[pos.r], KG);
+            if (lane == 0) mbar_arrive_n(&sh.empty1[pos.r], 4 / COLG);   // 4 * COLG warps per stage, 16 arrivals
         }
         if (KG > 1) share = share + 1 == KG ? 0 : share + 1;
         pos.next(expanded);
@@ -477,6 +483,59 @@ __device__ __forceinline__ bool readback(const Params& p, const GemmWork& w, Gem
     return ok;
 }
 
+// Slim tiles of packed weights: the read-back needs few of its warps and the two expander warps would be what bounds the kernel
+// (1000 of 1490 cycles per stage with 16 columns), so parts 2 and 3 of the read-back warps expand instead, a row tile and
+// two of a stage's four units each: warp x of eight.
+template <class Policy, class Params, int W>
+__device__ __forceinline__ bool expand_slim(const Params& p, const GemmWork& w, GemmShared& sh, uint32_t ring1, uint32_t ring2, int x, int lane, RingPos& pos,
+                                            TmemPos& tp, uint32_t& xphase) {
+    const int type = uniform(Policy::type(p, w)), nb = uniform(w.nb);
+    pos.geometry(1);
+    if (tp.npad != W) { tp.npad = W; tp.slot = 0; tp.nslots = kG_TmemCols / (blocks_per_slot(W) * W); }
+    const uint32_t t = x & 3, h = x >> 2;
+    const uint32_t src = ring1 + t * kRawTile, dst = ring2 + h * (2 * kG_MmaTile) + t * 512 + lane * 16, rec = ring2 + 4096 + h * (2 * kG_MmaTile) + (t * 32 + lane) * 4;
+    const int nstages = (nb + kG_StageUnits - 1) / kG_StageUnits;
+    float d3 = 0.0f;        // IQ3_S: this lane's row's scales of the super-block, kept over its two stages
+    uint32_t sc3 = 0u;
+    bool ok = true;
+    for (int s = 0; s < nstages && ok; ++s) {
+        const int u0 = stage_unit(type, s);
+        if (!mbar_wait(&sh.full1[pos.r], pos.par1()) || !mbar_wait(&sh.empty1[pos.lag()], pos.released(pos.lag()))) { ok = false; break; }
+        const uint32_t raw = src + pos.slot1_off(), a = (uint32_t)pos.e * kG_ASlot;
+        if (type == CHIMERE_TYPE_Q4_0) {
+            const uint4 v0 = lds128(raw + (2 * h) * 576 + lane * 16), v1 = lds128(raw + (2 * h + 1) * 576 + lane * 16);
+            const uint32_t e0 = lds16(raw + (2 * h) * 576 + 512 + lane * 2), e1 = lds16(raw + (2 * h + 1) * 576 + 512 + lane * 2);
+            expand_unit<CHIMERE_TYPE_Q4_0>(v0, dst + a);
+            expand_unit<CHIMERE_TYPE_Q4_0>(v1, dst + a + kG_MmaTile);
+            sts_f32(rec + a, h2f(e0) * 0.0625f);
+            sts_f32(rec + a + kG_MmaTile, h2f(e1) * 0.0625f);
+        } else {
+            const uint4 v0 = lds128(raw + (2 * h) * 512 + lane * 16), v1 = lds128(raw + (2 * h + 1) * 512 + lane * 16);
+            if (!(s & 1)) {   // the scales came behind these units
+                d3 = h2f(lds16(raw + 2048 + lane * 2)) * 0.125f;
+                sc3 = lds32(raw + 2048 + 64 + lane * 4);
+            }
+            const uint32_t sc = sc3 >> (4 * (u0 & 4) + 8 * h);
+            expand_unit<CHIMERE_TYPE_IQ3_S>(v0, dst + a);
+            expand_unit<CHIMERE_TYPE_IQ3_S>(v1, dst + a + kG_MmaTile);
+            sts_f32(rec + a, d3 * (float)(1u + 2u * (sc & 15u)));
+            sts_f32(rec + a + kG_MmaTile, d3 * (float)(1u + 2u * ((sc >> 4) & 15u)));
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the MMAs read what ordinary stores wrote
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cta(&sh.xfull2[pos.e]);
+        // (as in readback_tile: see the tile's last stage complete before going on)
+        if (s + 1 == nstages && !mbar_wait(&sh.tfull[tp.slot], tp.par())) ok = false;
+        tp.next();
+        pos.next(true);
+    }
+    if (ok && !mbar_wait(&sh.xempty, (xphase & 1u) ^ 1u)) ok = false;
+    ++xphase;
+    if (!ok) gemm_timeout(sh, p.status, lane);
+    if (lane == 0) mbar_arrive_cta(&sh.xfull);   // nothing of this warp's to store
+    return ok;
+}
+
 // Warps 4..7: what happens to a tile's sums, while the read-back warps are at the next tile.
 template <class Policy, class Params>
 __device__ __forceinline__ bool store_tile(const Params& p, const GemmWork& w, GemmShared& sh, const float* xch, int ew, int lane, uint32_t& xphase) {
@@ -484,7 +543,7 @@ __device__ __forceinline__ bool store_tile(const Params& p, const GemmWork& w, G
     ++xphase;
     if (!ok) { gemm_timeout(sh, p.status, lane); return false; }
     if (w.npad == 128) Policy::template store<1>(p, w, xch, ew, lane);
-    else if (w.npad == 64) Policy::template store<2>(p, w, xch, ew, lane);
+    else if (w.npad == 64 || Policy::type(p, w) < kTypeOperand) Policy::template store<2>(p, w, xch, ew, lane);
     else Policy::template store<4>(p, w, xch, ew, lane);
     __syncwarp();
     if (lane == 0) mbar_arrive_cta(&sh.xempty);
@@ -514,7 +573,7 @@ __global__ void __launch_bounds__(kG_Threads, 1) gemm_i8_kernel(const Params p, 
 
     if (tid == 0) {
         for (int i = 0; i < kG_RingSlotsSlim; ++i) { mbar_init(&sh.full1[i], 1); mbar_init(&sh.empty1[i], kG_RbWarps); }
-        for (int i = 0; i < kG_ASlots; ++i) { mbar_init(&sh.xfull2[i], kG_ExpWarps); }
+        for (int i = 0; i < kG_ASlots; ++i) { mbar_init(&sh.xfull2[i], kG_SlimExpWarps); }
         for (int i = 0; i < kG_TmemSlots; ++i) { mbar_init(&sh.tfull[i], 1); mbar_init(&sh.tempty[i], kG_RbWarps); }
         for (int i = 0; i < kG_Sched; ++i) { mbar_init(&sh.sfull[i], 1); mbar_init(&sh.sempty[i], 1 + kG_ExpWarps + kG_EpiWarps + kG_RbWarps); }
         mbar_init(&sh.xfull, kG_RbWarps); mbar_init(&sh.xempty, kG_EpiWarps);
@@ -550,8 +609,16 @@ __global__ void __launch_bounds__(kG_Threads, 1) gemm_i8_kernel(const Params p, 
             switch (uniform(w.npad)) {
                 case 128: ok = readback<Policy, Params, 4, 1, 32>(p, w, sh, r1, r2, xch, tmem, q, part, lane, pos, tp, xphase); break;
                 case 64: ok = readback<Policy, Params, 2, 2, 32>(p, w, sh, r1, r2, xch, tmem, q, part, lane, pos, tp, xphase); break;
-                case 32: ok = readback<Policy, Params, 1, 4, 32>(p, w, sh, r1, r2, xch, tmem, q, part, lane, pos, tp, xphase); break;
-                default: ok = readback<Policy, Params, 1, 4, 16>(p, w, sh, r1, r2, xch, tmem, q, part, lane, pos, tp, xphase); break;
+                case 32:
+                    if (uniform(Policy::type(p, w)) >= kTypeOperand) ok = readback<Policy, Params, 1, 4, 32>(p, w, sh, r1, r2, xch, tmem, q, part, lane, pos, tp, xphase);
+                    else if (part < 2) ok = readback<Policy, Params, 1, 2, 32>(p, w, sh, r1, r2, xch, tmem, q, part, lane, pos, tp, xphase);
+                    else ok = expand_slim<Policy, Params, 32>(p, w, sh, r1, r2, warp - kG_FirstRb - 8, lane, pos, tp, xphase);
+                    break;
+                default:
+                    if (uniform(Policy::type(p, w)) >= kTypeOperand) ok = readback<Policy, Params, 1, 4, 16>(p, w, sh, r1, r2, xch, tmem, q, part, lane, pos, tp, xphase);
+                    else if (part < 2) ok = readback<Policy, Params, 1, 2, 16>(p, w, sh, r1, r2, xch, tmem, q, part, lane, pos, tp, xphase);
+                    else ok = expand_slim<Policy, Params, 16>(p, w, sh, r1, r2, warp - kG_FirstRb - 8, lane, pos, tp, xphase);
+                    break;
             }
         }
     } else {
