@@ -74,6 +74,48 @@ int validate_layer(const chimere_moe_layer* w) {
     return 0;
 }
 
+// From this many tokens on the decode entry's experts run on the grouped GEMM.
+constexpr int kForwardGemmTokens = 17;
+// ---------------------------------------------------------------- grouped GEMM path ----
+// Token tiles of a batch: at most P / 128 full ones and one partial one per expert with pairs, and the shared expert's.
+int n_tiles_max_for(const chimere_moe_layer* w, int T) {
+    const int P = T * w->top_k;
+    return P / 128 + (w->E < P ? w->E : P) + (w->F_s > 0 ? (T + 127) / 128 : 0);
+}
+// ... and their columns / 16: a tile of n pairs is at most max(16, 2 n) columns wide.
+int64_t n_col16_max_for(const chimere_moe_layer* w, int T) {
+    const int64_t P = (int64_t)T * w->top_k, E = w->E < P ? w->E : P;
+    const int64_t sh = w->F_s > 0 ? T : 0;
+    return (2 * (P + sh) + 15) / 16 + E + 1;
+}
+int prefill_dims_ok(const chimere_moe_layer* w) {
+    const int rpt = w->act == CHIMERE_ACT_SWIGLU ? 64 : 32;
+    if (w->H % 128 || w->F % rpt || w->F_s % rpt) return 0;
+    return 1;
+}
+struct PrefillArena { size_t tiles, bx, b2, total; int64_t bx_col16, b2_col16; };
+PrefillArena prefill_arena(const chimere_moe_layer* w, int T) {
+    PrefillArena A{};
+    const int Fmax = w->F > w->F_s ? w->F : w->F_s;
+    const int per = kshared_gemm(w) ? 640 : 576;   // 16 columns: 36 bytes per column and block, 40 with the blocks' sums
+    A.bx_col16 = (int64_t)(w->H / 32) * per;
+    A.b2_col16 = (int64_t)(Fmax / 32) * per;
+    const int64_t cols = n_col16_max_for(w, T);
+    size_t o = 0;
+    A.tiles = o; o += up256((size_t)(8 + 4 * n_tiles_max_for(w, T)) * 4);
+    A.bx = o; o += up256((size_t)(cols * A.bx_col16));
+    A.b2 = o; o += up256((size_t)(cols * A.b2_col16));
+    A.total = o;
+    return A;
+}
+// Whether the decode entry may take the grouped GEMM for T tokens of a layer (w without a K-quant shared expert): weights it
+// reads in the tiled32 form, and enough tokens.
+bool forward_gemm(const chimere_moe_layer* w, int T) {
+    if (T < kForwardGemmTokens || w->layout != CHIMERE_LAYOUT_TILED32 || !prefill_dims_ok(w)) return false;
+    auto ok = [](int t) { return t == CHIMERE_TYPE_Q4_0 || t == CHIMERE_TYPE_IQ3_S; };
+    return ok(w->type_up) && ok(w->type_down) && (w->F_s == 0 || (ok(w->type_sh_up) && ok(w->type_sh_down)));
+}
+
 struct Layout {
     size_t topk_idx, topk_w, logits, sh_logit, x_q8, perm, offsets, group_list, counters, inter_q8, pair_out, status, total;
     size_t x_q, x_d, inter_q, inter_d;
@@ -81,6 +123,7 @@ struct Layout {
     int max_entries, n_row_tiles, tile_rows, n_counters;
     int n_row_tiles_tiled;
     size_t inter_stride;
+    size_t gemm, gemm_bytes;   // the decode entry's token tiles (gemm_bytes = 0: never on the GEMM)
 };
 
 int max_entries_for(const chimere_moe_layer* w, int T) {
@@ -131,6 +174,9 @@ Layout make_layout(const chimere_moe_layer* w, int T, int extra_rows = 0) {
     L.inter_d = o; o += up256(pairs * L.inter_d_stride * 4);
     L.status = o; o += 256;
     L.pair_out = o; o += up256((pairs + extra_rows) * H * 4);
+    L.gemm = o;
+    L.gemm_bytes = forward_gemm(w, T) ? prefill_arena(w, T).total : 0;
+    o += up256(L.gemm_bytes);
     L.total = o;
     return L;
 }
@@ -177,6 +223,7 @@ int chimere_b200_moe_workspace_init(chimere_moe_workspace* ws, void* d_arena, si
     ws->inter_q = (int8_t*)(base + L.inter_q);
     ws->inter_d = (float*)(base + L.inter_d);
     ws->status = (int32_t*)(base + L.status);
+    if (L.gemm_bytes) { ws->prefill_arena = base + L.gemm; ws->prefill_bytes = L.gemm_bytes; }
     cudaError_t e = cudaMemsetAsync(ws->counters, 0, (size_t)L.n_counters * 4, stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(ws->status, 0, 256, stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(ws->group_list, 0, (size_t)(kListHeader + kListEntry * L.max_entries) * 4, stream);
@@ -226,6 +273,9 @@ int chimere_b200_moe_route(const chimere_moe_layer* w, const float* d_x, int T, 
 }
 
 static int kshared_chain(const chimere_moe_layer* w, int T, float* d_y, chimere_moe_workspace* ws, cudaStream_t stream);
+static int gemm_experts(const chimere_moe_layer* w, const chimere_moe_prefill_weights* pw, int E, int T, chimere_moe_workspace* ws, cudaStream_t stream,
+                        const void* d_packed = nullptr, int row_bytes = 0, bool taps = false);
+static cudaError_t finish_tokens(const chimere_moe_layer* w, float* d_y, int T, chimere_moe_workspace* ws, cudaStream_t stream);
 static GemvParams gate_up_params(const chimere_moe_layer* w, int T, chimere_moe_workspace* ws, const Layout& L);
 static GemvParams down_params(const chimere_moe_layer* w, float* d_y, int T, chimere_moe_workspace* ws, const Layout& L);
 
@@ -541,13 +591,24 @@ int chimere_b200_moe_forward(const chimere_moe_layer* w, const float* d_x, float
     const bool ks = kshared(w);
     const chimere_moe_layer wr_ = ks ? routed_only(w) : *w;
     const chimere_moe_layer* wr = &wr_;
-    const Layout L = make_layout(wr, ws->max_T);
-    const int max_entries = routed_entries_for(wr, T);
-    cudaError_t e = launch_route(route_params(wr, d_x, T, ws, ks), stream);
-    if (e != cudaSuccess) return cuda_rc(e);
-    e = run_gate_up(wr, gate_up_params(wr, T, ws, L), max_entries, stream);
-    if (e != cudaSuccess) return cuda_rc(e);
-    e = run_down(wr, down_params(wr, d_y, T, ws, L), max_entries, stream);
+    cudaError_t e;
+    if (forward_gemm(wr, T) && ws->prefill_arena && ws->prefill_bytes >= prefill_arena(wr, ws->max_T).total) {
+        RouteParams rp = route_params(wr, d_x, T, ws, ks);
+        rp.list_mode = 2;
+        e = launch_route(rp, stream);
+        if (e != cudaSuccess) return cuda_rc(e);
+        rc = gemm_experts(wr, nullptr, wr->E, T, ws, stream, nullptr, 0, true);
+        if (rc) return rc;
+        e = finish_tokens(wr, d_y, T, ws, stream);
+    } else {
+        const Layout L = make_layout(wr, ws->max_T);
+        const int max_entries = routed_entries_for(wr, T);
+        e = launch_route(route_params(wr, d_x, T, ws, ks), stream);
+        if (e != cudaSuccess) return cuda_rc(e);
+        e = run_gate_up(wr, gate_up_params(wr, T, ws, L), max_entries, stream);
+        if (e != cudaSuccess) return cuda_rc(e);
+        e = run_down(wr, down_params(wr, d_y, T, ws, L), max_entries, stream);
+    }
     if (e != cudaSuccess || !ks) return cuda_rc(e);
     return kshared_chain(w, T, d_y, ws, stream);
 }
@@ -632,40 +693,6 @@ int chimere_b200_mma_i8_probe(int n_mma, int n_cols, int n_acc, int32_t* d_statu
     return launch_mma_i8_probe(n_mma, n_cols, n_acc, d_status, stream);
 }
 
-// ---------------------------------------------------------------- grouped GEMM path ----
-namespace {
-// Token tiles of a batch: at most P / 128 full ones and one partial one per expert with pairs, and the shared expert's.
-int n_tiles_max_for(const chimere_moe_layer* w, int T) {
-    const int P = T * w->top_k;
-    return P / 128 + (w->E < P ? w->E : P) + (w->F_s > 0 ? (T + 127) / 128 : 0);
-}
-// ... and their columns / 16: a tile of n pairs is at most max(16, 2 n) columns wide.
-int64_t n_col16_max_for(const chimere_moe_layer* w, int T) {
-    const int64_t P = (int64_t)T * w->top_k, E = w->E < P ? w->E : P;
-    const int64_t sh = w->F_s > 0 ? T : 0;
-    return (2 * (P + sh) + 15) / 16 + E + 1;
-}
-int prefill_dims_ok(const chimere_moe_layer* w) {
-    const int rpt = w->act == CHIMERE_ACT_SWIGLU ? 64 : 32;
-    if (w->H % 128 || w->F % rpt || w->F_s % rpt) return 0;
-    return 1;
-}
-struct PrefillArena { size_t tiles, bx, b2, total; int64_t bx_col16, b2_col16; };
-PrefillArena prefill_arena(const chimere_moe_layer* w, int T) {
-    PrefillArena A{};
-    const int Fmax = w->F > w->F_s ? w->F : w->F_s;
-    const int per = kshared_gemm(w) ? 640 : 576;   // 16 columns: 36 bytes per column and block, 40 with the blocks' sums
-    A.bx_col16 = (int64_t)(w->H / 32) * per;
-    A.b2_col16 = (int64_t)(Fmax / 32) * per;
-    const int64_t cols = n_col16_max_for(w, T);
-    size_t o = 0;
-    A.tiles = o; o += up256((size_t)(8 + 4 * n_tiles_max_for(w, T)) * 4);
-    A.bx = o; o += up256((size_t)(cols * A.bx_col16));
-    A.b2 = o; o += up256((size_t)(cols * A.b2_col16));
-    A.total = o;
-    return A;
-}
-}  // namespace
 
 // The GEMM reads 4-bit weights in the tiled32 form; Q8_0 matrices, and a shared expert in Q4_K / Q5_K super-blocks, get a copy
 // in the MMA's own order (mma128 tiles; gate and up rows interleaved per 64, so that one output tile holds both).
@@ -804,7 +831,7 @@ static PrefillGemmMats gemm_mats(const chimere_moe_layer* w, const chimere_moe_p
 // of an exchange) are in place: token tiles of every expert with pairs (and of the shared expert; E = 0: of it alone), the
 // gate/up GEMM with the activation and the Q8_1 step, the down GEMM; per-pair rows land in ws->pair_out.
 static int gemm_experts(const chimere_moe_layer* w, const chimere_moe_prefill_weights* pw, int E, int T, chimere_moe_workspace* ws, cudaStream_t stream,
-                        const void* d_packed = nullptr, int row_bytes = 0) {
+                        const void* d_packed, int row_bytes, bool taps) {
     if (!ws->prefill_arena) return -1;
     if (w->layout != CHIMERE_LAYOUT_TILED32 || !prefill_dims_ok(w)) return -2;
     const PrefillArena A = prefill_arena(w, ws->max_T);
@@ -834,9 +861,17 @@ static int gemm_experts(const chimere_moe_layer* w, const chimere_moe_prefill_we
         g.b_tiles = base + (down ? A.b2 : A.bx); g.b_col16_bytes = down ? A.b2_col16 : A.bx_col16;
         g.out_tiles = base + A.b2; g.out_col16_bytes = A.b2_col16;
         g.pair_out = ws->pair_out;
+        if (taps) { g.inter_q8 = ws->inter_q8; g.inter_stride = (int64_t)L.inter_stride; }
         e = launch_prefill_gemm(g, down != 0, n_tiles_max, stream);
     }
     return cuda_rc(e);
+}
+
+// routing-weighted sum of every token's pair rows in slot order + the sigmoid-gated shared expert
+static cudaError_t finish_tokens(const chimere_moe_layer* w, float* d_y, int T, chimere_moe_workspace* ws, cudaStream_t stream) {
+    const float* shared_rows = w->F_s > 0 ? ws->pair_out + (size_t)T * w->top_k * w->H : nullptr;
+    const float* logit = (w->F_s > 0 && w->shexp_gate_w) ? ws->sh_gate_logit : nullptr;
+    return launch_ep_finish(ws->pair_out, nullptr, ws->topk_w, shared_rows, logit, d_y, T, w->H, w->top_k, stream);
 }
 
 int chimere_b200_moe_forward_prefill(const chimere_moe_layer* w, const chimere_moe_prefill_weights* pw, const float* d_x, float* d_y,
@@ -856,10 +891,7 @@ int chimere_b200_moe_forward_prefill(const chimere_moe_layer* w, const chimere_m
     if (e != cudaSuccess) return cuda_rc(e);
     rc = gemm_experts(wr, pw, wr->E, T, ws, stream);
     if (rc) return rc;
-    // routing-weighted sum of every token's pair rows in slot order + the sigmoid-gated shared expert
-    const float* shared_rows = wr->F_s > 0 ? ws->pair_out + (size_t)T * wr->top_k * wr->H : nullptr;
-    const float* logit = (wr->F_s > 0 && wr->shexp_gate_w) ? ws->sh_gate_logit : nullptr;
-    e = launch_ep_finish(ws->pair_out, nullptr, ws->topk_w, shared_rows, logit, d_y, T, wr->H, wr->top_k, stream);
+    e = finish_tokens(wr, d_y, T, ws, stream);
     if (e != cudaSuccess || !ks || gemm) return cuda_rc(e);
     return kshared_chain(w, T, d_y, ws, stream);
 }

@@ -789,11 +789,18 @@ struct GateUpPolicy : MoePolicy {
                     qdst[(ci >> 3) * 128 + (ci & 7) * 16] = qv;
                     if (lane == 0) ddst[ci] = __half2float(__float2half(d));
                 }
-                if (sums) {
+                if (sums || p.inter_q8) {
                     float sum = v[i];
 #pragma unroll
                     for (int k = 16; k > 0; k >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, k);
-                    if (lane == 0 && ci < w.n_valid) sdst[ci] = __half2float(__float2half(sum));
+                    const __half sh = __float2half(sum);
+                    if (sums && lane == 0 && ci < w.n_valid) sdst[ci] = __half2float(sh);
+                    if (p.inter_q8 && ci < w.n_valid) {   // the decode entry's rows of intermediates
+                        const int row = w.shared ? p.T * p.top_k + w.start + ci : __ldcg(p.perm + w.start + ci);
+                        uint8_t* tap = p.inter_q8 + (size_t)row * p.inter_stride + (size_t)blk * kQ81Bytes;
+                        reinterpret_cast<int8_t*>(tap)[4 + lane] = qv;
+                        if (lane == 0) *reinterpret_cast<__half2*>(tap) = __halves2half2(__float2half(d), sh);
+                    }
                 }
             }
         }

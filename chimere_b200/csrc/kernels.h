@@ -159,6 +159,7 @@ struct PrefillGemmParams {
     float* pair_out;                                 // down: per-pair rows [pairs][H]
     int row_tiles_max;
     int dual, T, top_k, H;
+    uint8_t* inter_q8; int64_t inter_stride;   // gate/up: Q8_1 rows of the intermediates as the GEMV kernels leave them (null = not wanted)
     int shared_sums;                 // gate/up: the shared expert's token tiles of the down GEMM carry block sums (kTypeOperandMin)
     int32_t* status;
 };
