@@ -74,8 +74,11 @@ int validate_layer(const chimere_moe_layer* w) {
     return 0;
 }
 
-// From this many tokens on the decode entry's experts run on the grouped GEMM.
-constexpr int kForwardGemmTokens = 17;
+// From this many tokens on the decode entry sends experts with at least kForwardGemmPairs pairs, and the shared expert, to the
+// grouped GEMM and the others to the GEMV kernels: a GEMM tile costs the same with 1 pair as with 16, a GEMV entry grows with
+// every pair.
+constexpr int kForwardGemmTokens = 17, kForwardGemmPairs = 3;
+static_assert(kForwardGemmPairs <= kMaxGroupTokens + 1, "a small expert must fit one work entry");
 // ---------------------------------------------------------------- grouped GEMM path ----
 // Token tiles of a batch: at most P / 128 full ones and one partial one per expert with pairs, and the shared expert's.
 int n_tiles_max_for(const chimere_moe_layer* w, int T) {
@@ -274,7 +277,7 @@ int chimere_b200_moe_route(const chimere_moe_layer* w, const float* d_x, int T, 
 
 static int kshared_chain(const chimere_moe_layer* w, int T, float* d_y, chimere_moe_workspace* ws, cudaStream_t stream);
 static int gemm_experts(const chimere_moe_layer* w, const chimere_moe_prefill_weights* pw, int E, int T, chimere_moe_workspace* ws, cudaStream_t stream,
-                        const void* d_packed = nullptr, int row_bytes = 0, bool taps = false);
+                        const void* d_packed = nullptr, int row_bytes = 0, bool mixed = false);
 static cudaError_t finish_tokens(const chimere_moe_layer* w, float* d_y, int T, chimere_moe_workspace* ws, cudaStream_t stream);
 static GemvParams gate_up_params(const chimere_moe_layer* w, int T, chimere_moe_workspace* ws, const Layout& L);
 static GemvParams down_params(const chimere_moe_layer* w, float* d_y, int T, chimere_moe_workspace* ws, const Layout& L);
@@ -831,7 +834,7 @@ static PrefillGemmMats gemm_mats(const chimere_moe_layer* w, const chimere_moe_p
 // of an exchange) are in place: token tiles of every expert with pairs (and of the shared expert; E = 0: of it alone), the
 // gate/up GEMM with the activation and the Q8_1 step, the down GEMM; per-pair rows land in ws->pair_out.
 static int gemm_experts(const chimere_moe_layer* w, const chimere_moe_prefill_weights* pw, int E, int T, chimere_moe_workspace* ws, cudaStream_t stream,
-                        const void* d_packed, int row_bytes, bool taps) {
+                        const void* d_packed, int row_bytes, bool mixed) {
     if (!ws->prefill_arena) return -1;
     if (w->layout != CHIMERE_LAYOUT_TILED32 || !prefill_dims_ok(w)) return -2;
     const PrefillArena A = prefill_arena(w, ws->max_T);
@@ -840,7 +843,7 @@ static int gemm_experts(const chimere_moe_layer* w, const chimere_moe_prefill_we
     int32_t* tiles = (int32_t*)(base + A.tiles);
     const Layout L = make_layout(w, ws->max_T);
     const int n_tiles_max = E > 0 ? n_tiles_max_for(w, T) : (T + 127) / 128;
-    cudaError_t e = launch_build_tiles(ws->offsets, tiles, E, T, w->F_s > 0, stream);
+    cudaError_t e = launch_build_tiles(ws->offsets, ws->perm, tiles, mixed ? ws->group_list : nullptr, E, T, w->F_s > 0, mixed ? kForwardGemmPairs : 1, stream);
     if (e != cudaSuccess) return cuda_rc(e);
     // the rows' Q8_1 planes: the workspace's, or (expert-parallel owner) the received packed rows in place
     const int8_t* xq = d_packed ? (const int8_t*)d_packed : ws->x_q;
@@ -849,6 +852,18 @@ static int gemm_experts(const chimere_moe_layer* w, const chimere_moe_prefill_we
     e = launch_gather_tiles(tiles, ws->perm, xq, d_packed ? row_bytes : w->H, xd, d_packed ? row_bytes / 4 : L.x_d_stride, ws->x_q8, base + A.bx, A.bx_col16,
                             w->H, w->top_k, n_tiles_max, sums, stream);
     if (e != cudaSuccess) return cuda_rc(e);
+    if (mixed) {   // the small experts: GEMV kernels on the list that the tile builder wrote, per-pair rows only
+        const int max_entries = w->E < T * w->top_k ? w->E : T * w->top_k;
+        GemvParams gu = gate_up_params(w, T, ws, L);
+        gu.nrows_shared = 0; gu.ncols_shared = 0; gu.sh_a = nullptr; gu.sh_b = nullptr; gu.few_tokens = 1;
+        e = launch_gate_up_tiled(gu, max_entries, stream);
+        if (e != cudaSuccess) return cuda_rc(e);
+        GemvParams dn = down_params(w, nullptr, T, ws, L);
+        dn.no_combine = 1; dn.few_tokens = 1;
+        dn.nrows_shared = 0; dn.ncols_shared = 0; dn.sh_a = nullptr; dn.sh_b = nullptr;
+        e = launch_down_tiled(dn, max_entries, stream);
+        if (e != cudaSuccess) return cuda_rc(e);
+    }
     PrefillGemmParams g{};
     g.tiles = tiles; g.perm = ws->perm; g.status = ws->status;
     g.T = T; g.top_k = w->top_k; g.H = w->H; g.shared_sums = sums;
@@ -861,7 +876,7 @@ static int gemm_experts(const chimere_moe_layer* w, const chimere_moe_prefill_we
         g.b_tiles = base + (down ? A.b2 : A.bx); g.b_col16_bytes = down ? A.b2_col16 : A.bx_col16;
         g.out_tiles = base + A.b2; g.out_col16_bytes = A.b2_col16;
         g.pair_out = ws->pair_out;
-        if (taps) { g.inter_q8 = ws->inter_q8; g.inter_stride = (int64_t)L.inter_stride; }
+        if (mixed) { g.inter_q8 = ws->inter_q8; g.inter_stride = (int64_t)L.inter_stride; }
         e = launch_prefill_gemm(g, down != 0, n_tiles_max, stream);
     }
     return cuda_rc(e);

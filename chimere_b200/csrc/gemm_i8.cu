@@ -997,18 +997,37 @@ cudaError_t launch_pack_mma128_q8_0(const void* raw, void* out, int n_mats, int 
     return cudaGetLastError();
 }
 
-// After routing: the token tiles of every expert that has pairs (and of the shared expert).  One CTA of 256 threads,
+// After routing: the token tiles of every expert with at least gemm_min pairs (and of the shared expert), and, if `list` is given, the
+// GEMV work list of the others (gemm_min <= kMaxGroupTokens + 1).  One CTA of 256 threads,
 // thread e = expert e.  Wide tiles come first and the narrow ones last, so that the persistent GEMM CTAs, which take tiles
 // in order, end on cheap ones; within a width the shared expert's tile leads.  Tiles per width are counted with one scan
 // (four 16-bit counters in a 64-bit word), and a tile's first column follows from its place, because all tiles of a width
 // are equally wide.
 __device__ __forceinline__ uint64_t width_bit(int n, uint64_t count) { return n > 64 ? count : n > 32 ? count << 16 : n > 16 ? count << 32 : count << 48; }
-__global__ void __launch_bounds__(256) build_tiles_kernel(const int32_t* offsets, int32_t* tiles, int E, int T, int has_shared) {
+__global__ void __launch_bounds__(256) build_tiles_kernel(const int32_t* offsets, const int32_t* perm, int32_t* tiles, int32_t* list, int E, int T,
+                                                          int has_shared, int gemm_min) {
     __shared__ uint64_t scan[8];
+    __shared__ int scan_n[8];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     griddep_wait();
     if (tid == 0) griddep_launch();
-    const int cnt = tid < E ? offsets[tid + 1] - offsets[tid] : 0, off = tid < E ? offsets[tid] : 0;
+    const int pairs = tid < E ? offsets[tid + 1] - offsets[tid] : 0, off = tid < E ? offsets[tid] : 0;
+    // experts of fewer than gemm_min pairs go to the GEMV kernels, one work entry each
+    const bool small = pairs > 0 && pairs < gemm_min;
+    const int cnt = small ? 0 : pairs;
+    if (list) {
+        const unsigned m = __ballot_sync(0xffffffffu, small);
+        if (lane == 0) scan_n[warp] = __popc(m);
+        __syncthreads();
+        int first = __popc(m & ((1u << lane) - 1u)), total = 0;
+        for (int w = 0; w < 8; ++w) { if (w < warp) first += scan_n[w]; total += scan_n[w]; }
+        if (small) {
+            int* ent = list + kListHeader + kListEntry * first;
+            ent[0] = tid; ent[1] = off; ent[2] = pairs; ent[3] = 0;
+            for (int j = 0; j < kMaxGroupTokens; ++j) ent[4 + j] = j < pairs ? perm[off + j] : 0;
+        }
+        if (tid == 0) { list[0] = total; list[1] = total; list[2] = 0; list[3] = 0; }
+    }
     const int nf = cnt >> 7, rem = cnt & 127;
     const uint64_t own = (uint64_t)nf + (rem ? width_bit(rem, 1) : 0ull);
     uint64_t incl = own;
@@ -1083,8 +1102,9 @@ __global__ void __launch_bounds__(256) gather_tiles_kernel(const int32_t* tiles,
     }
 }
 
-cudaError_t launch_build_tiles(const int32_t* offsets, int32_t* tiles, int E, int T, int has_shared, cudaStream_t stream) {
-    return launch_pdl(build_tiles_kernel, dim3(1), 256, 0, stream, offsets, tiles, E, T, has_shared);
+cudaError_t launch_build_tiles(const int32_t* offsets, const int32_t* perm, int32_t* tiles, int32_t* list, int E, int T, int has_shared, int gemm_min,
+                               cudaStream_t stream) {
+    return launch_pdl(build_tiles_kernel, dim3(1), 256, 0, stream, offsets, perm, tiles, list, E, T, has_shared, gemm_min);
 }
 
 cudaError_t launch_gather_tiles(const int32_t* tiles, const int32_t* perm, const int8_t* x_q, int64_t x_q_stride, const float* x_d,

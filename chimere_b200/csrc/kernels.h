@@ -164,7 +164,8 @@ struct PrefillGemmParams {
     int32_t* status;
 };
 cudaError_t launch_prefill_gemm(const PrefillGemmParams& p, bool down, int n_tiles_max, cudaStream_t stream);
-cudaError_t launch_build_tiles(const int32_t* offsets, int32_t* tiles, int E, int T, int has_shared, cudaStream_t stream);
+cudaError_t launch_build_tiles(const int32_t* offsets, const int32_t* perm, int32_t* tiles, int32_t* list, int E, int T, int has_shared, int gemm_min,
+                               cudaStream_t stream);
 cudaError_t launch_gather_tiles(const int32_t* tiles, const int32_t* perm, const int8_t* x_q, int64_t x_q_stride, const float* x_d,
                                 int x_d_stride, const uint8_t* x_q8, uint8_t* b_tiles, int64_t b_col16_bytes, int H, int top_k, int n_tiles_max,
                                 bool shared_sums, cudaStream_t stream);
