@@ -334,7 +334,7 @@ __global__ void __launch_bounds__(kThreadsT, 4) tile_kernel(const GemvParams p, 
 // 128-bit-per-lane pattern (conflict-free).  A CTA holds all its weights at once; several CTAs per SM keep
 // enough bytes in flight.  Tokens are taken `mt` at a time so that the planes stay small.
 struct BulkSmem { uint32_t w_slot, aq, ad, red, total, q_row, d_row; };
-__host__ __device__ inline BulkSmem bulk_smem(uint32_t tile_bytes_max, int ncols_max, int wr, int wk, int nmat, int mt, bool need_red) {
+__host__ __device__ inline BulkSmem bulk_smem(uint32_t tile_bytes_max, int ncols_max, int wr, int wk, int nmat, int mt, bool need_red, bool overlay) {
     BulkSmem s;
     s.w_slot = (tile_bytes_max + 127u) & ~127u;
     s.q_row = (uint32_t)ncols_max;
@@ -342,7 +342,10 @@ __host__ __device__ inline BulkSmem bulk_smem(uint32_t tile_bytes_max, int ncols
     uint32_t o = (uint32_t)nmat * wr * s.w_slot;
     s.aq = o; o += (uint32_t)mt * s.q_row;
     s.ad = o; o += (uint32_t)mt * s.d_row;
-    s.red = o; o += need_red ? (uint32_t)nmat * wk * mt * 32 * wr * 4 : 0u;
+    // the partial sums behind the activations, or (overlay) in their place once every warp has read them
+    const uint32_t red = need_red ? (uint32_t)nmat * wk * mt * 32 * wr * 4 : 0u;
+    s.red = overlay ? s.aq : o;
+    if (overlay) { if (s.aq + red > o) o = s.aq + red; } else o += red;
     s.total = o;
     return s;
 }
@@ -376,7 +379,7 @@ __device__ __forceinline__ void dot_pass_pair_s(uint32_t tile_a, uint32_t tile_b
 
 // grid = (row items, max entries), block = 32 * wr * wk threads (wk = 1 << wk_shift, wr = 1 << wr_shift).
 template <int TYPE, int STAGE, bool DUAL, int MT>
-__global__ void __launch_bounds__(kThreadsT, 3) bulk_kernel(const GemvParams p, int wk_shift, int wr_shift, uint32_t tile_bytes_max) {
+__global__ void __launch_bounds__(kThreadsT, 3) bulk_kernel(const GemvParams p, int wk_shift, int wr_shift, uint32_t tile_bytes_max, int overlay) {
     constexpr int mt = MT;   // tokens per pass
     extern __shared__ __align__(128) uint8_t smem[];
     __shared__ int s_row[kMaxGroupTokens];
@@ -411,7 +414,7 @@ __global__ void __launch_bounds__(kThreadsT, 3) bulk_kernel(const GemvParams p, 
     // bring its CTAs in; it waits for this grid before it touches the workspace
     if (STAGE == kStageDown && tid == 0) griddep_launch();
     const bool need_red = STAGE == kStageGateUp || wk > 1;
-    const BulkSmem bs = bulk_smem(tile_bytes_max, max(p.ncols_routed, p.ncols_shared), wr, wk, kMat, mt, need_red);
+    const BulkSmem bs = bulk_smem(tile_bytes_max, max(p.ncols_routed, p.ncols_shared), wr, wk, kMat, mt, need_red, overlay != 0);
     float* red = reinterpret_cast<float*>(smem + bs.red);
     const uint32_t aq = smem_u32(smem + bs.aq), ad = smem_u32(smem + bs.ad);
     const int qrow = (int)bs.q_row, drow = (int)bs.d_row;
@@ -468,6 +471,7 @@ __global__ void __launch_bounds__(kThreadsT, 3) bulk_kernel(const GemvParams p, 
             // one token, gate and up rows of the tile together: the token's values are fetched once for both
             float au = 0.0f, ag = 0.0f;
             if (bytes > 0) dot_pass_pair_s<TYPE>(ws0, ws1, g0, g1, lane, nb, aq, ad, au, ag);
+            if (overlay) __syncthreads();   // (every warp has read the activations)
             red[(wk_id * mt) * width + wr_id * 32 + lane] = au;
             red[((wk + wk_id) * mt) * width + wr_id * 32 + lane] = ag;
         } else
@@ -500,6 +504,7 @@ __global__ void __launch_bounds__(kThreadsT, 3) bulk_kernel(const GemvParams p, 
                 }
             }
             if (need_red) {
+                if (overlay) __syncthreads();   // (one matrix, see plan_bulk: every warp has read the activations)
 #pragma unroll
                 for (int i = 0; i < MT; ++i)
                     if (i < mp) red[((mat * wk + wk_id) * mt + i) * width + wr_id * 32 + lane] = acc[i];
@@ -633,9 +638,9 @@ static cudaError_t launch_tile_t(const GemvParams& p, int max_entries, int wk, i
 
 // How the bulk-copy kernel fits an SM: CTAs per SM and tokens per pass.  ok = false: the weights of one CTA do not
 // fit, or something is not 16-byte aligned; the caller then takes the kernel that loads through registers.
-struct BulkPlan { bool ok; int mt; uint32_t tile_bytes_max, smem; };
+struct BulkPlan { bool ok; int mt; uint32_t tile_bytes_max, smem; int overlay; };
 static BulkPlan plan_bulk(const GemvParams& p, int stage, bool dual, int wk, int wr) {
-    BulkPlan b{false, 0, 0, 0};
+    BulkPlan b{false, 0, 0, 0, 0};
     const bool gu = stage == kStageGateUp;
     int64_t tb = tile_bytes_of(p.type_routed, p.ncols_routed);
     if (p.nrows_shared > 0) tb = max(tb, tile_bytes_of(p.type_shared, p.ncols_shared));
@@ -652,14 +657,21 @@ static BulkPlan plan_bulk(const GemvParams& p, int stage, bool dual, int wk, int
     // larger batches: at least four tokens per pass if that fits at all
     const int mt_floor = (p.T > 16 && !p.few_tokens) ? 4 : 1;
     for (int floor_mt = mt_floor; floor_mt >= 1 && !b.ok; floor_mt = (floor_mt == 1 ? 0 : 1)) {
-        int ctas = 0;
-        for (int c = max_ctas; c >= 1; --c)
-            if ((int64_t)bulk_smem((uint32_t)tb, ncols_max, wr, wk, nmat, floor_mt, need_red).total <= sm_bytes / c - per_cta) { ctas = c; break; }
+        auto bytes = [&](int mt, bool overlay) { return (int64_t)bulk_smem((uint32_t)tb, ncols_max, wr, wk, nmat, mt, need_red, overlay).total; };
+        auto ctas_of = [&](int mt, bool overlay) {
+            for (int c = max_ctas; c >= 1; --c)
+                if (bytes(mt, overlay) <= sm_bytes / c - per_cta) return c;
+            return 0;
+        };
+        // One token per pass, the partial sums may take the place of the activations (one more CTA barrier): worth it where that
+        // fits another CTA per SM -- Q4_0 gate and up of 2048 columns: 3 instead of 2
+        const bool overlay = need_red && floor_mt == 1 && ctas_of(1, true) > ctas_of(1, false);
+        const int ctas = ctas_of(floor_mt, overlay);
         if (!ctas) continue;
-        for (int mt = kMaxGroupTokens; mt >= floor_mt; mt >>= 1)
-            if ((int64_t)bulk_smem((uint32_t)tb, ncols_max, wr, wk, nmat, mt, need_red).total <= sm_bytes / ctas - per_cta) {
-                b.ok = true; b.mt = mt; b.tile_bytes_max = (uint32_t)tb;
-                b.smem = bulk_smem((uint32_t)tb, ncols_max, wr, wk, nmat, mt, need_red).total;
+        for (int mt = overlay ? 1 : kMaxGroupTokens; mt >= floor_mt; mt >>= 1)
+            if (bytes(mt, overlay) <= sm_bytes / ctas - per_cta) {
+                b.ok = true; b.mt = mt; b.tile_bytes_max = (uint32_t)tb; b.overlay = overlay;
+                b.smem = (uint32_t)bytes(mt, overlay);
                 break;
             }
     }
@@ -674,7 +686,7 @@ static cudaError_t launch_bulk_m(const GemvParams& p, int max_entries, int wk, i
     const int rows = max(p.nrows_routed, p.nrows_shared);
     const int items = (rows / 32 + wr - 1) / wr;
     return launch_pdl(bulk_kernel<TYPE, STAGE, DUAL, MT>, dim3(items, max_entries), 32 * wk * wr, b.smem, stream, p, log2i(wk), log2i(wr),
-                      b.tile_bytes_max);
+                      b.tile_bytes_max, b.overlay);
 }
 template <int TYPE, int STAGE, bool DUAL>
 static cudaError_t launch_bulk_t(const GemvParams& p, int max_entries, int wk, int wr, const BulkPlan& b, cudaStream_t stream) {
