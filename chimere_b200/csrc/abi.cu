@@ -74,10 +74,12 @@ int validate_layer(const chimere_moe_layer* w) {
     return 0;
 }
 
-// From this many tokens on the decode entry sends experts with at least kForwardGemmPairs pairs, and the shared expert, to the
-// grouped GEMM and the others to the GEMV kernels: a GEMM tile costs the same with 1 pair as with 16, a GEMV entry grows with
-// every pair.
-constexpr int kForwardGemmTokens = 17, kForwardGemmPairs = 3;
+// From forward_gemm_tokens() tokens on the decode entry sends experts with at least kForwardGemmPairs pairs, and the shared expert,
+// to the grouped GEMM and the others to the GEMV kernels: a GEMM tile costs the same with 1 pair as with 16, a GEMV entry grows
+// with every pair.  Uniform routing over 256 experts of 512 x 2048 breaks even near 40 tokens, 128 experts of 1856 x 2688 at 17 (there
+// the GEMV kernels have no room for a third CTA per SM); skewed routing gains earlier, but the host does not know the routing.
+constexpr int kForwardGemmPairs = 3;
+int forward_gemm_tokens(const chimere_moe_layer* w) { return (int64_t)w->F * w->H > (1 << 21) ? 17 : 41; }
 static_assert(kForwardGemmPairs <= kMaxGroupTokens + 1, "a small expert must fit one work entry");
 // ---------------------------------------------------------------- grouped GEMM path ----
 // Token tiles of a batch: at most P / 128 full ones and one partial one per expert with pairs, and the shared expert's.
@@ -114,7 +116,7 @@ PrefillArena prefill_arena(const chimere_moe_layer* w, int T) {
 // Whether the decode entry may take the grouped GEMM for T tokens of a layer (w without a K-quant shared expert): weights it
 // reads in the tiled32 form, and enough tokens.
 bool forward_gemm(const chimere_moe_layer* w, int T) {
-    if (T < kForwardGemmTokens || w->layout != CHIMERE_LAYOUT_TILED32 || !prefill_dims_ok(w)) return false;
+    if (T < forward_gemm_tokens(w) || w->layout != CHIMERE_LAYOUT_TILED32 || !prefill_dims_ok(w)) return false;
     auto ok = [](int t) { return t == CHIMERE_TYPE_Q4_0 || t == CHIMERE_TYPE_IQ3_S; };
     return ok(w->type_up) && ok(w->type_down) && (w->F_s == 0 || (ok(w->type_sh_up) && ok(w->type_sh_down)));
 }
@@ -130,15 +132,9 @@ struct Layout {
 };
 
 int max_entries_for(const chimere_moe_layer* w, int T) {
-    const int P = T * w->top_k;
-    return (w->E < P ? w->E : P) + P / kMaxGroupTokens + (w->F_s > 0 ? (T + shared_group_tokens(T) - 1) / shared_group_tokens(T) : 0);
-}
-// The same bound when the ids come from the library's own top-k (distinct within a token): an expert's pairs are cut into
-// entries of kMaxGroupTokens, so with at most that many tokens no expert needs a second entry.  Sizes launch grids only.
-int routed_entries_for(const chimere_moe_layer* w, int T) {
-    const int P = T * w->top_k;
-    const int extra = T <= kMaxGroupTokens ? 0 : P / kMaxGroupTokens;
-    return (w->E < P ? w->E : P) + extra + (w->F_s > 0 ? (T + shared_group_tokens(T) - 1) / shared_group_tokens(T) : 0);
+    const int P = T * w->top_k, g = group_tokens(T, (int64_t)w->F * w->H);
+    const int routed = (w->E < P ? w->E : P) + P / g;
+    return (routed < P ? routed : P) + (w->F_s > 0 ? (T + shared_group_tokens(T) - 1) / shared_group_tokens(T) : 0);
 }
 
 // extra_rows: per-pair output rows beyond the routed pairs' and the shared expert's own (a K-quant shared expert's rows on the
@@ -150,7 +146,8 @@ Layout make_layout(const chimere_moe_layer* w, int T, int extra_rows = 0) {
     const int Fmax = w->F > w->F_s ? w->F : w->F_s;
     const size_t pairs = (size_t)T * k + (w->F_s > 0 ? T : 0);
     L.max_entries = max_entries_for(w, T);   // T = the workspace's capacity; a smaller batch may need a few more entries
-    if (T > 8 && max_entries_for(w, 8) > L.max_entries) L.max_entries = max_entries_for(w, 8);   // (one-token shared entries up to T = 8)
+    for (int t : {8, kFewTokens})   // (smaller entries up to these batch sizes)
+        if (T > t && max_entries_for(w, t) > L.max_entries) L.max_entries = max_entries_for(w, t);
     L.tile_rows = down_tile_rows(w->type_down, w->F, w->type_sh_down, w->F_s);
     L.n_row_tiles = (H + L.tile_rows - 1) / L.tile_rows;
     L.n_row_tiles_tiled = (H + 31) / 32;   // counters for the finest row tiling any batch size may choose
@@ -238,6 +235,7 @@ static RouteParams route_params(const chimere_moe_layer* w, const float* d_x, in
     p.T = T; p.H = w->H; p.E = w->E; p.top_k = w->top_k; p.route_mode = w->route_mode;
     p.has_shared = w->F_s > 0;
     p.route_scale = w->route_scale;
+    p.group = group_tokens(T, (int64_t)w->F * w->H);
     p.x = d_x; p.router_w = w->router_w; p.router_bias = w->router_bias;
     p.shexp_gate_w = (w->F_s > 0 || keep_gate_vector) ? w->shexp_gate_w : nullptr;
     p.router_logits = ws->router_logits; p.sh_gate_logit = ws->sh_gate_logit;
@@ -605,7 +603,7 @@ int chimere_b200_moe_forward(const chimere_moe_layer* w, const float* d_x, float
         e = finish_tokens(wr, d_y, T, ws, stream);
     } else {
         const Layout L = make_layout(wr, ws->max_T);
-        const int max_entries = routed_entries_for(wr, T);
+        const int max_entries = max_entries_for(wr, T);
         e = launch_route(route_params(wr, d_x, T, ws, ks), stream);
         if (e != cudaSuccess) return cuda_rc(e);
         e = run_gate_up(wr, gate_up_params(wr, T, ws, L), max_entries, stream);

@@ -18,6 +18,12 @@ constexpr int kSharedGroupTokens = 2;  // ... for the shared expert (every token
 // Decode-size batches give every token its own shared-expert entry: the kernels stage one token per pass there, and
 // a second pass in the same CTA is a longer chain than a second CTA reading the shared matrices from L2.
 __host__ __device__ inline int shared_group_tokens(int T) { return T <= 8 ? 1 : kSharedGroupTokens; }
+// Tokens per routed entry.  In a decode-size batch every pair is an entry of its own: a popular expert's pairs are spread over
+// the SMs (its matrices then come from L2 again) instead of being a chain of passes in one CTA -- 8 skewed tokens through 256
+// experts of 512 x 2048 65 -> 37 us, 8 uniform ones 43 -> 38.  Matrices of more than 2M weights (1856 x 2688) cost more to fetch
+// twice than a second pass: two pairs per entry.
+constexpr int kFewTokens = 40;   // the largest batch for which the GEMV kernels are sized for one or two pairs per expert
+__host__ __device__ inline int group_tokens(int T, int64_t weights) { return T > kFewTokens ? kMaxGroupTokens : weights > (1 << 21) || T > 24 ? 2 : 1; }
 constexpr int kMaxTopK = 8;
 constexpr int kMaxExperts = 256;
 
@@ -169,6 +175,21 @@ __device__ __forceinline__ int unit_sumi(const int (&w)[8], int mul, const int* 
 #pragma unroll
     for (int g = 0; g < 8; ++g) s = __dp4a(w[g], q8words[g], s);
     return Unit<TYPE>::finish(s, mul);
+}
+
+// Sum of 256 partials held in shared memory in the order of a binary tree with strides
+// 128, 64, ..., 1 (element i+stride added into element i), done by one warp.
+__device__ __forceinline__ float tree256(const float* r, int lane) {
+    float a0 = r[lane] + r[lane + 128];
+    float a1 = r[lane + 32] + r[lane + 160];
+    float a2 = r[lane + 64] + r[lane + 192];
+    float a3 = r[lane + 96] + r[lane + 224];
+    float b0 = a0 + a2;
+    float b1 = a1 + a3;
+    float v = b0 + b1;
+#pragma unroll
+    for (int s = 16; s > 0; s >>= 1) v += __shfl_down_sync(0xffffffffu, v, s);
+    return v;  // valid in lane 0
 }
 
 // Sigmoid and SiLU exactly as the reference spells them (chimere_kernels.cu:1545, scratch_pool.rs:272).

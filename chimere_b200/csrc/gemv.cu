@@ -8,8 +8,7 @@
 //                    intermediates; the CTA that completes a token's last contribution for a row
 //                    tile adds them up in slot order with the routing weights and the sigmoid-gated
 //                    shared expert.  Replaces moe_ffn.rs:1325-1384 and :1700-1766.
-//   mmvq_kernel    : the same tile code behind the legacy operator entries
-//                    (ffi/ggml_cuda_gemv.cu:105-116, 243-279).
+//   mmvq_kernel    : the legacy operator entries (ffi/ggml_cuda_gemv.cu:105-116, 243-279).
 //
 // A CTA first asks the copy engine for its whole weight tile (cp.async.bulk, 8-row pieces, one
 // mbarrier each), stages the activations as an int8 plane + f32 scale plane while the weights
@@ -208,37 +207,24 @@ __global__ void __launch_bounds__(kThreads) gate_up_kernel(const GemvParams p) {
     }
 }
 
-// ------------------------------------------------------------------ down stage / plain -----
-// PLAIN = false: work-list driven; writes pair_out rows and combines them per token.
-// PLAIN = true : slot driven (legacy operator entries): blockIdx.y = slot, expert id from ids,
-//                output y[slot][row].
-struct PlainParams {
-    const uint8_t* w; const uint8_t* xq8; float* y; const int* ids;
-    int ncols, nrows; int64_t expert_stride, input_stride;
-};
-
-template <int TYPE, bool PLAIN>
-__global__ void __launch_bounds__(kThreads) down_kernel(const GemvParams p, const PlainParams pp, int tile_rows) {
+// ------------------------------------------------------------------ down stage -------------
+// Work-list driven: writes pair_out rows and combines them per token.
+template <int TYPE>
+__global__ void __launch_bounds__(kThreads) down_kernel(const GemvParams p, int tile_rows) {
     extern __shared__ __align__(128) uint8_t smem[];
     __shared__ const uint8_t* s_rows[kMaxGroupTokens];
     __shared__ int s_out_row[kMaxGroupTokens];
     __shared__ int s_tok[kMaxGroupTokens];
     __shared__ int s_done[kMaxGroupTokens];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    int expert, start, m, nrows, ncols;
-    bool shared = false;
-    if (PLAIN) {
-        expert = pp.ids ? pp.ids[blockIdx.y] : 0; start = blockIdx.y; m = 1; nrows = pp.nrows; ncols = pp.ncols;
-    } else {
-        const int n_entries = __ldcg(p.group_list);
-        if ((int)blockIdx.y >= n_entries) return;
-        const int* ent = p.group_list + kListHeader + kListEntry * blockIdx.y;
-        expert = __ldcg(ent); start = __ldcg(ent + 1); m = __ldcg(ent + 2);
-        shared = expert < 0;
-        if ((shared ? p.type_shared : p.type_routed) != TYPE) return;
-        nrows = shared ? p.nrows_shared : p.nrows_routed;
-        ncols = shared ? p.ncols_shared : p.ncols_routed;
-    }
+    const int n_entries = __ldcg(p.group_list);
+    if ((int)blockIdx.y >= n_entries) return;
+    const int* ent = p.group_list + kListHeader + kListEntry * blockIdx.y;
+    const int expert = __ldcg(ent), start = __ldcg(ent + 1), m = __ldcg(ent + 2);
+    const bool shared = expert < 0;
+    if ((shared ? p.type_shared : p.type_routed) != TYPE) return;
+    const int nrows = shared ? p.nrows_shared : p.nrows_routed;
+    const int ncols = shared ? p.ncols_shared : p.ncols_routed;
     const int r0 = blockIdx.x * tile_rows;
     if (r0 >= nrows) return;
     const int rows_here = min(tile_rows, nrows - r0);
@@ -251,8 +237,7 @@ __global__ void __launch_bounds__(kThreads) down_kernel(const GemvParams p, cons
     float* ad = reinterpret_cast<float*>(smem + sp.ad);
     uint8_t* wt = smem + sp.w0;
 
-    const uint8_t* wsrc = PLAIN ? pp.w + (size_t)expert * pp.expert_stride
-                                : (shared ? p.sh_a : p.w_a + (size_t)expert * p.stride_a);
+    const uint8_t* wsrc = shared ? p.sh_a : p.w_a + (size_t)expert * p.stride_a;
     wsrc += (size_t)r0 * rb;
     const int npieces = (rows_here + kPieceRows - 1) / kPieceRows;
     if (tid == 0) {
@@ -269,16 +254,12 @@ __global__ void __launch_bounds__(kThreads) down_kernel(const GemvParams p, cons
         for (int i = tid; i < 512; i += kThreads) grid_s[i] = g_iq3s_grid[i];
 
     if (tid < m) {
-        if (PLAIN) {
-            s_rows[0] = pp.xq8 + (size_t)start * pp.input_stride;
-        } else {
-            int t, irow;
-            if (shared) { t = start + tid; irow = p.T * p.top_k + t; }
-            else { irow = __ldcg(p.perm + start + tid); t = irow / p.top_k; }
-            s_rows[tid] = p.in_q8 + (size_t)irow * p.in_stride;
-            s_out_row[tid] = irow;
-            s_tok[tid] = t;
-        }
+        int t, irow;
+        if (shared) { t = start + tid; irow = p.T * p.top_k + t; }
+        else { irow = __ldcg(p.perm + start + tid); t = irow / p.top_k; }
+        s_rows[tid] = p.in_q8 + (size_t)irow * p.in_stride;
+        s_out_row[tid] = irow;
+        s_tok[tid] = t;
     }
     __syncthreads();
     stage_q8(s_rows, m, nb, ncols, aq, ad, tid);
@@ -295,17 +276,11 @@ __global__ void __launch_bounds__(kThreads) down_kernel(const GemvParams p, cons
         if (valid) row_dot<TYPE>(wt + (size_t)row * rb, l8, nb, ncols, aq, ad, m, grid_s, acc);
         reduce8(acc, m);
         if (valid && l8 == 0) {
-            if (PLAIN) {
-                pp.y[(size_t)blockIdx.y * nrows + r0 + row] = acc[0];
-            } else {
 #pragma unroll
-                for (int i = 0; i < kMaxGroupTokens; ++i)
-                    if (i < m) p.pair_out[(size_t)s_out_row[i] * p.H + r0 + row] = acc[i];
-            }
+            for (int i = 0; i < kMaxGroupTokens; ++i)
+                if (i < m) p.pair_out[(size_t)s_out_row[i] * p.H + r0 + row] = acc[i];
         }
     }
-    if (PLAIN) return;
-
     // ---- combine: whoever completes a token's contributions for this row tile adds them up ----
     __threadfence();
     __syncthreads();
@@ -339,6 +314,41 @@ __global__ void __launch_bounds__(kThreads) down_kernel(const GemvParams p, cons
     }
 }
 
+// ------------------------------------------------------------------ plain GEMV -------------
+// The legacy operator entries: y[slot][row] = W[ids[slot]][row] . xq8[slot] on raw blocks.  A group of 2^lanes_shift lanes owns a
+// row, lane l takes the 32-weight units l, l + lanes, ...; the lanes' sums meet in a butterfly.  A launch reads a few MB, so what
+// bounds it is the latency of one chain: weights are read straight into registers by as many warps as there are rows (staging
+// 64-row tiles in shared memory with 8 lanes per row and up to 8 units each in sequence took 8.5 us for 8 x 512 x 2048 IQ3_S).
+struct PlainParams {
+    const uint8_t* w; const uint8_t* xq8; float* y; const int* ids;
+    int ncols, nrows; int64_t expert_stride, input_stride;
+};
+template <int TYPE>
+__global__ void __launch_bounds__(kThreads) mmvq_kernel(const PlainParams pp, int lanes_shift) {
+    griddep_wait();
+    if (threadIdx.x == 0) griddep_launch();
+    const int lane = threadIdx.x & ((1 << lanes_shift) - 1), step = 1 << lanes_shift, nb = pp.ncols >> 5;
+    const int row = blockIdx.x * (kThreads >> lanes_shift) + (threadIdx.x >> lanes_shift);
+    const bool valid = row < pp.nrows;
+    const int expert = pp.ids ? pp.ids[blockIdx.y] : 0;
+    const uint8_t* rowp = pp.w + (size_t)expert * pp.expert_stride + (size_t)(valid ? row : 0) * Unit<TYPE>::row_bytes(pp.ncols);
+    const uint8_t* x = pp.xq8 + (size_t)blockIdx.y * pp.input_stride;
+    float acc = 0.0f;
+#pragma unroll 2
+    for (int b = lane; b < nb; b += step) {
+        int w[8], q[8], mul;
+        float dw;
+        const uint32_t* xb = reinterpret_cast<const uint32_t*>(x + (size_t)b * kQ81Bytes);
+        const float dx = h2f(xb[0] & 0xFFFFu);
+#pragma unroll
+        for (int g = 0; g < 8; ++g) q[g] = (int)xb[1 + g];
+        Unit<TYPE>::load(rowp, b, g_iq3s_grid, w, dw, mul);
+        acc = fmaf(dw * dx, (float)unit_sumi<TYPE>(w, mul, q), acc);
+    }
+    for (int s = step >> 1; s > 0; s >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, s);
+    if (valid && lane == 0) pp.y[(size_t)blockIdx.y * pp.nrows + row] = acc;
+}
+
 // ------------------------------------------------------------------ small kernels ----------
 // Parity tap: exact integer dot of every (row, 32-wide block) against one Q8_1 row.
 template <int TYPE>
@@ -359,6 +369,8 @@ __global__ void block_sumi_kernel(const uint8_t* w, const uint8_t* xq8, int32_t*
 // Q8_1 of `batch` rows of ncols floats; output rows of ncols_padded/32 blocks, tail blocks zero.
 // One warp per block.  quantize_row_q8_1_cuda as called from ffi/ggml_cuda_gemv.cu:184-194,393-404.
 __global__ void quantize_q8_1_kernel(const float* x, uint8_t* out, int64_t ncols, int64_t ncols_padded, int batch) {
+    griddep_wait();
+    if (threadIdx.x == 0) griddep_launch();
     const int lane = threadIdx.x & 31;
     const int64_t nbp = ncols_padded >> 5;
     const int64_t gw = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -399,29 +411,50 @@ __global__ void rmsnorm_kernel(const float* x, float* y, int H, float eps) {
 // fused_add_residual_rmsnorm (chimere-server/src/kernels/fused_ops.rs:91-140) for T rows at once, in its order:
 // thread i sums the squares of elements i, i+256, ... (one fused multiply-add each), the 256 sums meet in a tree
 // of strides 128 .. 1, and every element is scaled as (residual * inv_rms) * weight.
-__global__ void __launch_bounds__(256) add_residual_rmsnorm_kernel(const float* hidden, float* residual, const float* weight, float* normed,
-                                                                   int H, float eps) {
+// Latency-bound at a few rows: a thread's loads all go out before its first store (rows of up to 256 * 16 elements stay in
+// registers, longer ones are read again), and every warp sums the 256 partial sums itself instead of meeting eight times (10.5 us
+// -> 3.5 at 2 rows of 2048, cold).
+constexpr int kNormRegs = 16;
+__global__ void __launch_bounds__(256) add_residual_rmsnorm_kernel(const float* __restrict__ hidden, float* __restrict__ residual,
+                                                                   const float* __restrict__ weight, float* __restrict__ normed, int H, float eps) {
     __shared__ float s_sum[256];
+    const int tid = threadIdx.x, lane = tid & 31;
+    float w[kNormRegs];
+#pragma unroll
+    for (int j = 0; j < kNormRegs; ++j) w[j] = j * 256 + tid < H ? weight[j * 256 + tid] : 0.0f;   // (a constant of the layer)
     griddep_wait();                       // the rows may come from the previous kernel of the stream
-    if (threadIdx.x == 0) griddep_launch();
-    const int tid = threadIdx.x;
+    if (tid == 0) griddep_launch();
     const float* h = hidden + (size_t)blockIdx.x * H;
     float* r = residual + (size_t)blockIdx.x * H;
+    float* out = normed + (size_t)blockIdx.x * H;
+    float v[kNormRegs], hv[kNormRegs];
+#pragma unroll
+    for (int j = 0; j < kNormRegs; ++j) {
+        const int i = j * 256 + tid;
+        hv[j] = i < H ? h[i] : 0.0f;
+        v[j] = i < H ? r[i] : 0.0f;
+    }
     float sum_sq = 0.0f;
-    for (int i = tid; i < H; i += 256) {
+#pragma unroll
+    for (int j = 0; j < kNormRegs; ++j) {
+        const int i = j * 256 + tid;
+        v[j] = hv[j] + v[j];
+        if (i < H) { r[i] = v[j]; sum_sq = fmaf(v[j], v[j], sum_sq); }
+    }
+    for (int i = kNormRegs * 256 + tid; i < H; i += 256) {
         const float val = h[i] + r[i];
         r[i] = val;
         sum_sq = fmaf(val, val, sum_sq);
     }
     s_sum[tid] = sum_sq;
     __syncthreads();
-    for (int s = 128; s > 0; s >>= 1) {
-        if (tid < s) s_sum[tid] += s_sum[tid + s];
-        __syncthreads();
-    }
-    const float rms = sqrtf(s_sum[0] / (float)H + eps);
+    const float total = __shfl_sync(0xffffffffu, tree256(s_sum, lane), 0);
+    const float rms = sqrtf(total / (float)H + eps);
     const float inv_rms = 1.0f / rms;
-    for (int i = tid; i < H; i += 256) normed[(size_t)blockIdx.x * H + i] = r[i] * inv_rms * weight[i];
+#pragma unroll
+    for (int j = 0; j < kNormRegs; ++j)
+        if (j * 256 + tid < H) out[j * 256 + tid] = v[j] * inv_rms * w[j];
+    for (int i = kNormRegs * 256 + tid; i < H; i += 256) out[i] = r[i] * inv_rms * weight[i];
 }
 
 cudaError_t launch_add_residual_rmsnorm(const float* hidden, float* residual, const float* weight, float* normed, int T, int H, float eps,
@@ -434,9 +467,8 @@ cudaError_t launch_add_residual_rmsnorm(const float* hidden, float* residual, co
 constexpr int kSmemCap = 200 * 1024;
 
 template <typename K>
-static cudaError_t set_smem(K kernel, size_t bytes) {
-    if (bytes > (size_t)kSmemCap) return cudaErrorInvalidValue;
-    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemCap);
+static cudaError_t set_smem(K kernel, size_t bytes, bool (&done)[64]) {
+    return bytes > (size_t)kSmemCap ? cudaErrorInvalidValue : max_smem_once(kernel, kSmemCap, done);
 }
 
 static int64_t host_row_bytes(int type, int ncols) {
@@ -452,7 +484,8 @@ template <int TYPE>
 static cudaError_t launch_gate_up_t(const GemvParams& p, int max_entries, cudaStream_t stream) {
     const bool dual = p.act == CHIMERE_ACT_SWIGLU;
     const size_t smem = plan_smem(p.H, 32, host_row_bytes(TYPE, p.H), dual).total;
-    cudaError_t e = set_smem(gate_up_kernel<TYPE>, smem);
+    static bool attr_done[64] = {};
+    cudaError_t e = set_smem(gate_up_kernel<TYPE>, smem, attr_done);
     if (e != cudaSuccess) return e;
     const int tiles = (max(p.nrows_routed, p.nrows_shared) + 31) / 32;
     gate_up_kernel<TYPE><<<dim3(tiles, max_entries), kThreads, smem, stream>>>(p);
@@ -491,9 +524,10 @@ static cudaError_t launch_down_t(const GemvParams& p, int max_entries, cudaStrea
     if (p.type_routed == TYPE) smem = plan_smem(p.ncols_routed, p.tile_rows, host_row_bytes(TYPE, p.ncols_routed), false).total;
     if (p.nrows_shared > 0 && p.type_shared == TYPE)
         smem = max(smem, (size_t)plan_smem(p.ncols_shared, p.tile_rows, host_row_bytes(TYPE, p.ncols_shared), false).total);
-    cudaError_t e = set_smem(down_kernel<TYPE, false>, smem);
+    static bool attr_done[64] = {};
+    cudaError_t e = set_smem(down_kernel<TYPE>, smem, attr_done);
     if (e != cudaSuccess) return e;
-    down_kernel<TYPE, false><<<dim3(p.n_row_tiles, max_entries), kThreads, smem, stream>>>(p, PlainParams{}, p.tile_rows);
+    down_kernel<TYPE><<<dim3(p.n_row_tiles, max_entries), kThreads, smem, stream>>>(p, p.tile_rows);
     return cudaGetLastError();
 }
 
@@ -515,15 +549,10 @@ cudaError_t launch_down(const GemvParams& p, int max_entries, cudaStream_t strea
 
 template <int TYPE>
 static cudaError_t launch_mmvq_t(const PlainParams& pp, int nslots, cudaStream_t stream) {
-    const int64_t rb = host_row_bytes(TYPE, pp.ncols);
-    int rows = 64;
-    while (rows > 8 && rows * rb > 48 * 1024) rows >>= 1;
-    const size_t smem = plan_smem(pp.ncols, rows, rb, false).total;
-    cudaError_t e = set_smem(down_kernel<TYPE, true>, smem);
-    if (e != cudaSuccess) return e;
-    GemvParams p{};
-    down_kernel<TYPE, true><<<dim3((pp.nrows + rows - 1) / rows, nslots), kThreads, smem, stream>>>(p, pp, rows);
-    return cudaGetLastError();
+    int shift = 0;
+    while (shift < 5 && (1 << shift) < pp.ncols / 32) ++shift;
+    const int rows = kThreads >> shift;
+    return launch_pdl(mmvq_kernel<TYPE>, dim3((pp.nrows + rows - 1) / rows, nslots), kThreads, 0, stream, pp, shift);
 }
 
 cudaError_t launch_mmvq(int wtype, const void* w, const void* xq8, float* y, const int* ids, int ncols, int nrows,
@@ -556,8 +585,7 @@ cudaError_t launch_quantize_q8_1(const float* x, void* out, int64_t ncols, int64
                                  cudaStream_t stream) {
     const int64_t warps = (ncols_padded / 32) * batch;
     if (warps <= 0) return cudaSuccess;
-    quantize_q8_1_kernel<<<(unsigned)((warps + 7) / 8), 256, 0, stream>>>(x, (uint8_t*)out, ncols, ncols_padded, batch);
-    return cudaGetLastError();
+    return launch_pdl(quantize_q8_1_kernel, dim3((unsigned)((warps + 7) / 8)), 256, 0, stream, x, (uint8_t*)out, ncols, ncols_padded, batch);
 }
 
 cudaError_t launch_rmsnorm(const float* x, float* y, int T, int H, float eps, cudaStream_t stream) {

@@ -16,6 +16,7 @@ struct RouteParams {
     int idx_stride;             // permute only: distance in int32 between consecutive ids (0 or 1 = dense)
     int list_mode;              // 0: work list for routed + shared entries; 1: shared-expert entries only (expert-parallel home
                                 // rank); 2: an empty list (the prefill path builds its own from offsets and perm)
+    int group;                  // pairs per routed work entry (0 = kMaxGroupTokens)
     float route_scale;
     const float* x;             // [T][H]
     const float* router_w;      // [E][H]

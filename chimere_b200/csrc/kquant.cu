@@ -222,7 +222,7 @@ cudaError_t launch_mmvq_kquant_batched(int wtype, const void* w, const void* w2,
 }
 
 cudaError_t launch_mmvq_kquant(int wtype, const void* w, const void* xq8, float* y, int ncols, int nrows, cudaStream_t stream) {
-    return launch_mmvq_kquant_batched(wtype, w, nullptr, xq8, 0, y, nullptr, 0, 1, ncols, nrows, 0, nullptr, false, stream);
+    return launch_mmvq_kquant_batched(wtype, w, nullptr, xq8, 0, y, nullptr, 0, 1, ncols, nrows, 0, nullptr, true, stream);
 }
 
 cudaError_t launch_act_q8_1(const float* g, const float* u, int64_t in_stride, void* out, int64_t out_stride, int T, int F, cudaStream_t stream) {

@@ -13,21 +13,6 @@
 
 namespace chimere {
 
-// Sum of 256 partials held in shared memory in the order of a binary tree with strides
-// 128, 64, ..., 1 (element i+stride added into element i), done by one warp.
-__device__ __forceinline__ float tree256(const float* r, int lane) {
-    float a0 = r[lane] + r[lane + 128];
-    float a1 = r[lane + 32] + r[lane + 160];
-    float a2 = r[lane + 64] + r[lane + 192];
-    float a3 = r[lane + 96] + r[lane + 224];
-    float b0 = a0 + a2;
-    float b1 = a1 + a3;
-    float v = b0 + b1;
-#pragma unroll
-    for (int s = 16; s > 0; s >>= 1) v += __shfl_down_sync(0xffffffffu, v, s);
-    return v;  // valid in lane 0
-}
-
 // Q8_1 of one 32-float block by one warp; lane = element.
 __device__ __forceinline__ void quantize_block_q8_1(float xi, uint8_t* out, int lane, int8_t* plane_q, float* plane_d) {
     float sum = xi;
@@ -142,6 +127,7 @@ __device__ void build_dispatch_small(const RouteParams& p, int* smem_i, const in
     const int E = p.E, P = p.T * p.top_k;
     int* s_sid = smem_i;          // [64] expert ids in sorted order (room for two warps of positions)
     int* s_perm = smem_i + 64;    // [64] the permutation
+    const int gt = p.group > 0 ? p.group : kMaxGroupTokens;
     int* s_lead = smem_i + 128;   // [2] distinct experts among sorted positions 0..31 / 32..63
     const int my_e = tid < P ? s_ids[tid] : -1;
     const bool valid = my_e >= 0 && my_e < E;
@@ -176,7 +162,10 @@ __device__ void build_dispatch_small(const RouteParams& p, int* smem_i, const in
     // sorted position tid starts a new expert?  (warps 0 and 1 hold the 64 positions)
     unsigned lead = 0u;
     if (warp < 2) {
-        const bool first = tid < total && (tid == 0 || s_sid[tid] != s_sid[tid - 1]);
+        // (entry starts: every gt-th pair of an expert; an expert has at most T <= 4 pairs here)
+        int rank = 0;
+        while (rank < tid && tid < total && s_sid[tid - rank - 1] == s_sid[tid]) ++rank;
+        const bool first = tid < total && rank % gt == 0;
         lead = __ballot_sync(0xffffffffu, first);
         if (lane == 0) s_lead[warp] = __popc(lead);
     }
@@ -192,7 +181,7 @@ __device__ void build_dispatch_small(const RouteParams& p, int* smem_i, const in
         const int idx = __popc(lead & ((1u << lane) - 1u)) + (warp == 1 ? s_lead[0] : 0);
         const int e = s_sid[tid];
         int mm = 1;
-        while (mm < kMaxGroupTokens && tid + mm < total && s_sid[tid + mm] == e) ++mm;   // (an expert has at most T <= 8 pairs here)
+        while (mm < gt && tid + mm < total && s_sid[tid + mm] == e) ++mm;
         int* ent = p.group_list + kListHeader + kListEntry * (nsh + idx);
         ent[0] = e; ent[1] = tid; ent[2] = mm; ent[3] = 0;
         for (int j = 0; j < kMaxGroupTokens; ++j) ent[4 + j] = j < mm ? s_perm[tid + j] : 0;
@@ -244,7 +233,8 @@ __device__ void build_dispatch(const RouteParams& p, int* smem_i, const int* s_i
     }
     hist[tid] = cnt;
     // exclusive scans over the experts: pair offsets and work-entry offsets
-    const int nent = (cnt + kMaxGroupTokens - 1) / kMaxGroupTokens;
+    const int gt = p.group > 0 ? p.group : kMaxGroupTokens;
+    const int nent = (cnt + gt - 1) / gt;
     int incl_c = cnt, incl_n = nent;
 #pragma unroll
     for (int s = 1; s < 32; s <<= 1) {
@@ -310,14 +300,14 @@ __device__ void build_dispatch(const RouteParams& p, int* smem_i, const int* s_i
             if (ent_base[mid] <= idx) lo = mid; else hi = mid;
         }
         const int e = lo, i = idx - ent_base[e], c = hist[e], o = cursor[e];
-        const int mm = min(kMaxGroupTokens, c - i * kMaxGroupTokens);
+        const int mm = min(gt, c - i * gt);
         int* ent = p.group_list + kListHeader + kListEntry * (nsh + idx);
         ent[0] = e;
-        ent[1] = o + i * kMaxGroupTokens;
+        ent[1] = o + i * gt;
         ent[2] = mm;
         ent[3] = 0;
         for (int j = 0; j < kMaxGroupTokens; ++j)
-            ent[4 + j] = j < mm ? (perm_in_smem ? s_perm[o + i * kMaxGroupTokens + j] : p.perm[o + i * kMaxGroupTokens + j]) : 0;
+            ent[4 + j] = j < mm ? (perm_in_smem ? s_perm[o + i * gt + j] : p.perm[o + i * gt + j]) : 0;
     }
 }
 
