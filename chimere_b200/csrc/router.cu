@@ -335,7 +335,7 @@ __global__ void __launch_bounds__(256) route_kernel(const RouteParams p) {
         const int r = r0 + b;
         wrow[b] = (r < E) ? p.router_w + (size_t)r * H : ((r == E && r < nrows) ? p.shexp_gate_w : nullptr);
     }
-    constexpr int kStep = (TE <= 2) ? 8 : 2;   // elements per thread whose loads are in flight together
+    constexpr int kStep = TE == 1 ? 12 : TE == 2 ? 8 : 2;   // elements per thread whose loads are in flight together
     for (int j0 = 0; j0 < H; j0 += kStep * 256) {
         float wv[kStep][TE];
 #pragma unroll
@@ -1135,7 +1135,10 @@ static cudaError_t launch_route_tiles(const RouteParams& p, cudaStream_t stream)
 
 cudaError_t launch_route(const RouteParams& p, cudaStream_t stream) {
     const int nrows = p.E + (p.shexp_gate_w ? 1 : 0);
-    if (p.T <= 32) {
+    if (p.T <= 32 && nrows <= sm_count()) {   // few experts: a row per CTA, up to 3072 columns in flight at once
+        constexpr int TT = 8, TE = 1;
+        return launch_pdl(route_kernel<TT, TE>, dim3(nrows, (p.T + TT - 1) / TT), 256, route_smem(TT, TE), stream, p);
+    } else if (p.T <= 32) {
         constexpr int TT = 8, TE = 2;
         dim3 grid((nrows + TE - 1) / TE, (p.T + TT - 1) / TT);
         return launch_pdl(route_kernel<TT, TE>, grid, 256, route_smem(TT, TE), stream, p);
