@@ -281,7 +281,7 @@ def measure_secondary(lib, dev, hbm_peak, i8_peak_tops, prefill_tokens):
         del tiled, pw
         torch.cuda.empty_cache()
     return {"how": "one layer, one call per sample, L2 flushed (256 MB written) before every sample, CUDA events on the launching "
-                   "stream, median of 7; gemm = chimere_b200_moe_forward_prefill (tcgen05 grouped GEMM for experts with >= 8 tokens), "
+                   "stream, median of 7; gemm = chimere_b200_moe_forward_prefill (tcgen05 grouped GEMM), "
                    "gemv = chimere_b200_moe_forward; frac = max(algorithmic bytes / measured HBM peak, int8 operations / measured "
                    "int8 tensor peak) / time",
             "results": out}

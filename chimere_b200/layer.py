@@ -136,8 +136,9 @@ class MoeWeightsTiled:
 
 
 class MoeWeightsPrefill:
-    """The GEMM copy of a layer's expert matrices (chimere_b200_moe_pack_prefill): int8 values and f32 block scales in
-    the tensor-core operand order.  Built from the raw ggml form; used together with the tiled32 form."""
+    """What the grouped GEMM needs beside the tiled32 form (chimere_b200_moe_pack_prefill): copies in the tensor-core operand order
+    of Q8_0 matrices and of a Q4_K / Q5_K shared expert; 4-bit routed experts are read from the tiled32 form itself.  Built from
+    the raw ggml form; used together with the tiled32 form."""
 
     def __init__(self, raw: MoeWeightsRaw):
         lib = abi.load()
@@ -230,7 +231,7 @@ def forward_moe(w, scratch: MoeScratch, x: torch.Tensor, out: Optional[torch.Ten
 
 
 def forward_moe_prefill(w, pw: MoeWeightsPrefill, scratch: MoeScratch, x: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
-    """y = MoE(x) with the large experts on the tensor-core GEMM (w: tiled32 layer, pw: its GEMM copy)."""
+    """y = MoE(x) with the experts on the tensor-core GEMM (w: tiled32 layer, pw: its GEMM copies)."""
     lib = abi.load()
     if scratch.prefill is None:
         scratch.enable_prefill()

@@ -327,7 +327,7 @@ int chimere_b200_moe_routing_trace(const chimere_moe_layer* w, int T, const chim
                                    int32_t* d_expert_load, cudaStream_t stream);
 
 /* Expert-parallel owner rank, prefill-size batches: as chimere_b200_moe_experts (planes in ws->x_q / ws->x_d, local expert
- * ids in ws->topk_idx[n_rows], results in ws->pair_out[row][H]), with the local experts that received at least 8 rows on the
+ * ids in ws->topk_idx[n_rows], results in ws->pair_out[row][H]), with the local experts on the
  * grouped GEMM.  pw_local: the GEMM copy of the local shard (chimere_b200_moe_pack_prefill of the shard); ws needs the
  * prefill arena.  No counterpart in the reference (single GPU, no prefill kernel). */
 int chimere_b200_moe_experts_prefill(const chimere_moe_layer* w_local, const chimere_moe_prefill_weights* pw_local, int n_rows,

@@ -1,0 +1,71 @@
+"""Batch sizes and row widths on both sides of every line at which the whole-layer entries change their kernels or tile widths,
+against the CPU oracle: token tiles of 16 / 32 / 64 / 128 columns, ragged last row tiles, one or two pairs per GEMV entry, the
+decode entry's step to the GEMM, the tiled router and its padding for every row width."""
+import numpy as np
+import pytest
+import torch
+
+import oracle
+from chimere_b200 import configs, formats
+from chimere_b200.layer import MoeScratch, MoeWeightsPrefill, MoeWeightsTiled, forward_moe, forward_moe_prefill
+from parity_util import check_rows, oracle_on_gpu_routing
+
+pytestmark = pytest.mark.gpu
+Q4, Q8, IQ3 = configs.QWEN_Q4_0, configs.QWEN_Q8_0, configs.QWEN_IQ3S
+
+
+def _check(cfg, T, prefill):
+    raw = configs.make_layer(cfg, device="cuda")
+    tiled = MoeWeightsTiled(raw)
+    x = configs.make_input(cfg, T, device="cuda")
+    sc = MoeScratch(tiled, T)
+    y = forward_moe_prefill(tiled, MoeWeightsPrefill(raw), sc, x) if prefill else forward_moe(tiled, sc, x)
+    torch.cuda.synchronize()
+    assert sc.status() == 0
+    idx = sc.topk_indices(T).cpu().numpy()
+    o = oracle_on_gpu_routing(raw.to("cpu"), x.cpu().numpy(), idx)
+    assert np.array_equal(sc.router_logits(T).cpu().numpy(), o["logits"])
+    assert np.array_equal(sc.x_q8(T).cpu().numpy(), o["x_q8"])
+    perm, offs = oracle.permute(idx, cfg.E)
+    assert np.array_equal(sc.perm(T).cpu().numpy(), perm) and np.array_equal(sc.offsets().cpu().numpy(), offs)
+    check_rows(y.cpu().numpy(), o["y"])
+
+
+# one expert that every token uses: the token count is the tile's column count
+@pytest.mark.parametrize("base", [Q4, IQ3, Q8], ids=lambda c: c.name)
+@pytest.mark.parametrize("T", [1, 15, 16, 17, 32, 33, 64, 65, 127, 128, 129, 161])
+def test_token_tile_widths(base, T):
+    _check(configs.scaled(base, E=1, top_k=1, H=512, F=256, F_s=256, zipf_bias=False), T, prefill=True)
+
+
+# 32-row tiles that do not fill the last 128-row tile, K that does not fill the last stage of four blocks
+@pytest.mark.parametrize("kw", [dict(F=96, F_s=160, H=384), dict(F=160, F_s=32, H=128), dict(F=224, F_s=96, H=640)], ids=str)
+@pytest.mark.parametrize("T", [9, 70])
+def test_partly_filled_row_tiles(kw, T):
+    _check(configs.scaled(configs.NEMOTRON_Q4_0, E=4, top_k=2, **kw), T, prefill=True)
+
+
+@pytest.mark.parametrize("types", [(formats.TYPE_Q5_K, formats.TYPE_Q5_K), (formats.TYPE_Q4_K, formats.TYPE_Q5_K), (formats.TYPE_Q5_K, formats.TYPE_Q6_K)], ids=str)
+@pytest.mark.parametrize("T", [8, 33, 129])
+def test_kquant_shared_expert_beside_packed_experts(types, T):
+    _check(configs.scaled(IQ3, E=4, top_k=2, H=512, F=256, F_s=512, type_sh_gate_up=types[0], type_sh_down=types[1]), T, prefill=True)
+
+
+# weights read packed and weights in operand order in one launch
+@pytest.mark.parametrize("T", [20, 90])
+def test_mixed_operand_forms(T):
+    _check(configs.scaled(Q4, E=4, top_k=2, H=512, F=256, F_s=256, type_sh_gate_up=configs.Q8_0, type_sh_down=configs.Q8_0), T, prefill=True)
+
+
+@pytest.mark.parametrize("cfg,T", [(configs.scaled(Q4, E=16, F=128, F_s=128, H=512), t) for t in (16, 17, 24, 25, 40, 41, 64)] +
+                                  [(configs.scaled(configs.NEMOTRON_Q4_0, E=8, H=2688, F=800, F_s=1600, name="wide experts"), t) for t in (8, 16, 17, 33)],
+                         ids=lambda v: getattr(v, "name", str(v)))
+def test_decode_entry_steps(cfg, T):
+    _check(cfg, T, prefill=False)
+
+
+# rows of 1 .. 4 kilo-elements (one to four quads per partial), ragged ones, token counts around a tile of 32
+@pytest.mark.parametrize("H", [256, 1024, 1152, 2048, 2688, 3200, 4096])
+@pytest.mark.parametrize("T", [129, 160, 545])
+def test_tiled_router(H, T):
+    _check(configs.scaled(Q4, E=256, H=H, F=64, F_s=64), T, prefill=False)
