@@ -35,10 +35,10 @@ inline chimere_moe_layer routed_only(const chimere_moe_layer* w) {
 }
 
 // ... and whether that shared expert can go through the grouped GEMM (prefill-size batches): all three matrices Q4_K or Q5_K
-// (Q6_K has a scale per 16 weights, the MMA's blocks are 32 wide) and whole 64-row pairs of gate and up rows.
+// (Q6_K has a scale per 16 weights, the MMA's blocks are 32 wide), rows of whole rounds of 32 blocks, gated.
 inline bool kshared_gemm(const chimere_moe_layer* w) {
     auto ok = [](int t) { return t == CHIMERE_TYPE_Q4_K || t == CHIMERE_TYPE_Q5_K; };
-    return kshared(w) && w->act == CHIMERE_ACT_SWIGLU && ok(w->type_sh_gate) && ok(w->type_sh_up) && ok(w->type_sh_down);
+    return kshared(w) && w->H % 1024 == 0 && w->act == CHIMERE_ACT_SWIGLU && ok(w->type_sh_gate) && ok(w->type_sh_up) && ok(w->type_sh_down);
 }
 
 int validate_layer(const chimere_moe_layer* w) {
@@ -85,7 +85,7 @@ static_assert(kForwardGemmPairs <= kMaxGroupTokens + 1, "a small expert must fit
 // Token tiles of a batch: at most P / 128 full ones and one partial one per expert with pairs, and the shared expert's.
 int n_tiles_max_for(const chimere_moe_layer* w, int T) {
     const int P = T * w->top_k;
-    return P / 128 + (w->E < P ? w->E : P) + (w->F_s > 0 ? (T + 127) / 128 : 0);
+    return P / 128 + (w->E < P ? w->E : P) + (w->F_s > 0 ? kshared(w) ? (T + 31) / 32 : (T + 127) / 128 : 0);
 }
 // ... and their columns / 16: a tile of n pairs is at most max(16, 2 n) columns wide.
 int64_t n_col16_max_for(const chimere_moe_layer* w, int T) {
@@ -841,14 +841,14 @@ static int gemm_experts(const chimere_moe_layer* w, const chimere_moe_prefill_we
     int32_t* tiles = (int32_t*)(base + A.tiles);
     const Layout L = make_layout(w, ws->max_T);
     const int n_tiles_max = E > 0 ? n_tiles_max_for(w, T) : (T + 127) / 128;
-    cudaError_t e = launch_build_tiles(ws->offsets, ws->perm, tiles, mixed ? ws->group_list : nullptr, E, T, w->F_s > 0, mixed ? kForwardGemmPairs : 1, stream);
+    cudaError_t e = launch_build_tiles(ws->offsets, ws->perm, tiles, mixed ? ws->group_list : nullptr, E, T, w->F_s > 0, mixed ? kForwardGemmPairs : 1, kshared(w), stream);
     if (e != cudaSuccess) return cuda_rc(e);
     // the rows' Q8_1 planes: the workspace's, or (expert-parallel owner) the received packed rows in place
     const int8_t* xq = d_packed ? (const int8_t*)d_packed : ws->x_q;
     const float* xd = d_packed ? (const float*)((const uint8_t*)d_packed + w->H) : ws->x_d;
     const bool sums = kshared(w);   // the shared expert's token tiles carry the blocks' sums
     e = launch_gather_tiles(tiles, ws->perm, xq, d_packed ? row_bytes : w->H, xd, d_packed ? row_bytes / 4 : L.x_d_stride, ws->x_q8, base + A.bx, A.bx_col16,
-                            w->H, w->top_k, n_tiles_max, sums, stream);
+                            w->H, w->top_k, n_tiles_max, sums, T, stream);
     if (e != cudaSuccess) return cuda_rc(e);
     if (mixed) {   // the small experts: GEMV kernels on the list that the tile builder wrote, per-pair rows only
         const int max_entries = w->E < T * w->top_k ? w->E : T * w->top_k;
@@ -864,8 +864,9 @@ static int gemm_experts(const chimere_moe_layer* w, const chimere_moe_prefill_we
     }
     PrefillGemmParams g{};
     g.tiles = tiles; g.perm = ws->perm; g.status = ws->status;
-    g.T = T; g.top_k = w->top_k; g.H = w->H; g.shared_sums = sums;
+    g.T = T; g.top_k = w->top_k; g.H = w->H;
     for (int down = 0; down < 2 && e == cudaSuccess; ++down) {
+        g.shared_sums = sums && !down;
         g.dual = !down && w->act == CHIMERE_ACT_SWIGLU;
         g.m[0] = gemm_mats(w, pw, false, down != 0);
         g.m[1] = gemm_mats(w, pw, true, down != 0);

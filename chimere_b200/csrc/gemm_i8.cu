@@ -104,6 +104,10 @@ template <> __device__ __forceinline__ void tc_ld_nowait<16>(uint32_t taddr, int
           "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
         : "r"(taddr) : "memory");
 }
+template <> __device__ __forceinline__ void tc_ld_nowait<8>(uint32_t taddr, int (&v)[8]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]) : "r"(taddr) : "memory");
+}
 __device__ __forceinline__ void tc_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 // two 64-bit words (four floats) from a 32-bit shared address, the same for every lane
 __device__ __forceinline__ void lds_2x64(uint32_t a, uint64_t& x, uint64_t& y) { asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(x), "=l"(y) : "r"(a)); }
@@ -388,23 +392,10 @@ __device__ __forceinline__ void block_values(const int (&v)[W], float sa, uint32
     }
 }
 
-// ... and the minimums of a block: acc[c] += m * s[c], s the token's sum over the block
-template <int W>
-__device__ __forceinline__ void block_minimums(float m, uint32_t sums, uint64_t* acc2) {
-    const uint64_t m2 = pack2f(m, m);
-#pragma unroll
-    for (int g = 0; g < W / 4; ++g) {
-        uint64_t s01, s23;
-        lds_2x64(sums + 16u * g, s01, s23);
-        acc2[2 * g + 0] = fma2(m2, s01, acc2[2 * g + 0]);
-        acc2[2 * g + 1] = fma2(m2, s23, acc2[2 * g + 1]);
-    }
-}
-
 // The read-back of one tile by one warp: column group colg of W columns; in tiles of up to 64 columns the warps of a column
 // group also share the stages among them (KG shares, stage s to share s % KG), so that a warp has that much longer for the
 // latency of one stage (barrier, TMEM load, scales: about a thousand cycles).
-template <int COLG, int KG, int W, bool MIN>
+template <int COLG, int KG, int W>
 __device__ __forceinline__ bool readback_tile(GemmShared& sh, uint32_t ring1, uint32_t ring2, uint32_t tmem, int32_t* status, int nb, bool expanded, int q,
                                               int part, int lane, RingPos& pos, TmemPos& tp, uint64_t* acc2) {
     constexpr int kPad = COLG * W, kBps = blocks_per_slot(kPad);
@@ -444,9 +435,6 @@ __device__ __forceinline__ bool readback_tile(GemmShared& sh, uint32_t ring1, ui
                             if (lane == 0) mbar_arrive_n(&sh.tempty[tp.slot], 4 / COLG);
                         }
                         block_values<W, kPad == 128 ? 0u : 1u << 19>(v, sa, sb + (uint32_t)((j0 + i) * (kPad * 36)), acc2);
-                        if (MIN)
-                            block_minimums<W>(lds_f32(rec - 4096 + 4 * kG_MmaTile + (j0 + i) * 512),
-                                              sb - kPad * 32 + kG_StageUnits * kPad * 36 + (uint32_t)((j0 + i) * (kPad * 4)), acc2);
                     }
                 }
                 tp.next();
@@ -461,6 +449,94 @@ __device__ __forceinline__ bool readback_tile(GemmShared& sh, uint32_t ring1, ui
     return true;
 }
 
+// The binary counter of readback_min: sum completes level after level as long as that level has a pending left half.
+template <int L>
+__device__ __forceinline__ void count_up(int n, uint64_t (&sum)[4], uint64_t (&st)[5][4]) {
+    if constexpr (L < 5) {
+        if ((n >> L) & 1) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) sum[i] = add2(st[L][i], sum[i]);
+            count_up<L + 1>(n, sum, st);
+        } else {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) st[L][i] = sum[i];
+        }
+    }
+}
+
+// A warp's sums of a tile into the exchange buffer (part = share * column groups + column group).
+template <int W>
+__device__ __forceinline__ bool publish_sums(int32_t* status, GemmShared& sh, float* xch, int q, int part, int lane, uint32_t& xphase, const uint64_t* acc2, bool ok) {
+    if (!mbar_wait(&sh.xempty, (xphase & 1u) ^ 1u)) { gemm_timeout(sh, status, lane); ok = false; }   // the tile before has been stored
+    ++xphase;
+    float* mine = xch + part * (W * 128) + q * 32 + lane;
+    const uint64_t sc2 = pack2(kSumScaleBits, kSumScaleBits);
+#pragma unroll
+    for (int i = 0; i < W / 2; ++i) unpack2(mul2(acc2[i], sc2), mine[(2 * i) * 128], mine[(2 * i + 1) * 128]);
+    __syncwarp();
+    if (lane == 0) mbar_arrive_cta(&sh.xfull);
+    return ok;
+}
+
+// The read-back of a tile with minimums (Q4_K / Q5_K weights), 32 columns wide, eight of them per warp, bit for bit what
+// kquant_mmvq_kernel computes: a block's value is fma(-dmin * m, s, (d * d8) * float(sc * dot)), a lane's blocks (leaf of them, in
+// sequence) make a leaf, and the leaves of the 32 lanes, which come in bit-reversed order (operand_min_block), go up a binary counter
+// of pending sums.  The 8-bit rounding of the intermediates would show a different order of additions: these weights reach 4 sigma,
+// and one step of an intermediate moves an output by up to 3 % of the outputs' rms.  leaf = nb: plain sequence.
+// (Tiles with minimums have a kernel instance of their own, so that these registers do not weigh on the other tiles' loops.)
+__device__ __forceinline__ bool readback_min(GemmShared& sh, uint32_t ring1, uint32_t ring2, float* xch, uint32_t tmem, int32_t* status, int nb, int leaf, int q,
+                                          int part, int lane, RingPos& pos, TmemPos& tp, uint32_t& xphase) {
+    constexpr int W = 8, kPad = 32;
+    pos.geometry(1);
+    if (tp.npad != kPad) { tp.npad = kPad; tp.slot = 0; tp.nslots = kG_TmemCols / (blocks_per_slot(kPad) * kPad); }
+    const uint32_t trow = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(part * W);
+    const uint32_t rec0 = ring2 + (uint32_t)(q * 32 + lane) * 4u, sb0 = ring1 + kG_RawBytes + part * (W * 4);
+    uint64_t sum[W / 2], st[5][W / 2];
+    int in_leaf = 0, n = 0;
+    bool ok = true;
+    for (int b0 = 0; b0 < nb && ok; b0 += kG_StageUnits) {
+        const uint32_t rec = rec0 + (uint32_t)pos.e * kG_ASlot, sb = sb0 + pos.slot1_off();
+        if (!mbar_wait(&sh.tfull[tp.slot], tp.par())) { ok = false; break; }
+        tc_fence_after();
+        const uint32_t t0 = trow + (uint32_t)(tp.slot * (kG_StageUnits * kPad));
+#pragma unroll 1
+        for (int j = 0; j < kG_StageUnits; ++j) {
+            int v[W];
+            tc_ld_nowait<W>(t0 + (uint32_t)(j * kPad), v);
+            const uint32_t ds = lds32(rec + 4096 + j * kG_MmaTile);
+            const float m = lds_f32(rec + 4 * kG_MmaTile + j * 512), d = h2f(ds >> 16), sc = (float)(ds & 63u);
+            const uint64_t sc2 = pack2f(sc * __uint_as_float(kRowScaleBits), sc * __uint_as_float(kRowScaleBits));
+            const uint64_t c2 = pack2f(sc * __uint_as_float(kOffsetBits), sc * __uint_as_float(kOffsetBits)), d2 = pack2f(d, d), m2 = pack2f(m, m);
+            const uint32_t scale = sb + kPad * 32 + j * (kPad * 36), sums = sb + kG_StageUnits * kPad * 36 + j * (kPad * 4);
+            tc_wait_ld();
+#pragma unroll
+            for (int g = 0; g < W / 4; ++g) {
+                uint64_t x[2], s[2];
+                lds_2x64(scale + 16u * g, x[0], x[1]);
+                lds_2x64(sums + 16u * g, s[0], s[1]);
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    const uint64_t f = fma2(pack2((uint32_t)v[4 * g + 2 * i] + (1u << 19), (uint32_t)v[4 * g + 2 * i + 1] + (1u << 19)), sc2, c2);   // exact
+                    const uint64_t t = fma2(m2, s[i], mul2(mul2(d2, x[i]), f));
+                    sum[2 * g + i] = in_leaf ? add2(sum[2 * g + i], t) : t;
+                }
+            }
+            if (++in_leaf == leaf) {
+                in_leaf = 0;
+                count_up<0>(n, sum, st);
+                ++n;
+            }
+        }
+        tp.next();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cta(&sh.empty1[pos.r]);
+        pos.next(false);
+    }
+    if (!ok) gemm_timeout(sh, status, lane);
+    return publish_sums<W>(status, sh, xch, q, part, lane, xphase, sum, ok);
+}
+
 // One output tile by one read-back warp: sums over its blocks, then into the exchange buffer.
 template <class Policy, class Params, int COLG, int KG, int W>
 __device__ __forceinline__ bool readback(const Params& p, const GemmWork& w, GemmShared& sh, uint32_t ring1, uint32_t ring2, float* xch, uint32_t tmem, int q,
@@ -469,18 +545,8 @@ __device__ __forceinline__ bool readback(const Params& p, const GemmWork& w, Gem
     uint64_t acc2[W / 2];
 #pragma unroll
     for (int i = 0; i < W / 2; ++i) acc2[i] = 0ull;
-    const int type = uniform(Policy::type(p, w)), nb = uniform(w.nb);
-    bool ok = type == kTypeOperandMin ? readback_tile<COLG, KG, W, true>(sh, ring1, ring2, tmem, p.status, nb, false, q, part, lane, pos, tp, acc2)
-                                      : readback_tile<COLG, KG, W, false>(sh, ring1, ring2, tmem, p.status, nb, type < kTypeOperand, q, part, lane, pos, tp, acc2);
-    if (!mbar_wait(&sh.xempty, (xphase & 1u) ^ 1u)) { gemm_timeout(sh, p.status, lane); ok = false; }   // the tile before has been stored
-    ++xphase;
-    float* mine = xch + part * (W * 128) + q * 32 + lane;   // (part = share * COLG + column group)
-    const uint64_t sc2 = pack2(kSumScaleBits, kSumScaleBits);
-#pragma unroll
-    for (int i = 0; i < W / 2; ++i) unpack2(mul2(acc2[i], sc2), mine[(2 * i) * 128], mine[(2 * i + 1) * 128]);
-    __syncwarp();
-    if (lane == 0) mbar_arrive_cta(&sh.xfull);
-    return ok;
+    bool ok = readback_tile<COLG, KG, W>(sh, ring1, ring2, tmem, p.status, uniform(w.nb), uniform(Policy::type(p, w)) < kTypeOperand, q, part, lane, pos, tp, acc2);
+    return publish_sums<W>(p.status, sh, xch, q, part, lane, xphase, acc2, ok);
 }
 
 // Slim tiles of packed weights: the read-back needs few of its warps and the two expander warps would be what bounds the kernel
@@ -537,14 +603,14 @@ __device__ __forceinline__ bool expand_slim(const Params& p, const GemmWork& w, 
 }
 
 // Warps 4..7: what happens to a tile's sums, while the read-back warps are at the next tile.
-template <class Policy, class Params>
+template <class Policy, bool MIN, class Params>
 __device__ __forceinline__ bool store_tile(const Params& p, const GemmWork& w, GemmShared& sh, const float* xch, int ew, int lane, uint32_t& xphase) {
     const bool ok = mbar_wait(&sh.xfull, xphase & 1u);
     ++xphase;
     if (!ok) { gemm_timeout(sh, p.status, lane); return false; }
-    if (w.npad == 128) Policy::template store<1>(p, w, xch, ew, lane);
-    else if (w.npad == 64 || Policy::type(p, w) < kTypeOperand) Policy::template store<2>(p, w, xch, ew, lane);
-    else Policy::template store<4>(p, w, xch, ew, lane);
+    if (MIN || w.npad == 128) Policy::template store<1, MIN>(p, w, xch, ew, lane);
+    else if (w.npad == 64 || Policy::type(p, w) < kTypeOperand) Policy::template store<2, false>(p, w, xch, ew, lane);
+    else Policy::template store<4, false>(p, w, xch, ew, lane);
     __syncwarp();
     if (lane == 0) mbar_arrive_cta(&sh.xempty);
     return true;
@@ -561,7 +627,8 @@ __device__ __forceinline__ int take_tile(GemmShared& sh, int32_t* status, uint32
     return idx;
 }
 
-template <class Policy, class Params>
+// MIN: the tiles with minimums (Q4_K / Q5_K shared expert) and no others
+template <class Policy, class Params, bool MIN = false>
 __global__ void __launch_bounds__(kG_Threads, 1) gemm_i8_kernel(const Params p, int32_t* tile_counter) {
     extern __shared__ uint8_t smem_raw[];
     __shared__ GemmShared sh;
@@ -604,8 +671,13 @@ __global__ void __launch_bounds__(kG_Threads, 1) gemm_i8_kernel(const Params p, 
         bool ok = true;
         while (ok && (idx = take_tile(sh, p.status, tn, lane)) >= 0) {
             GemmWork w;
-            Policy::work(p, idx, w);
+            Policy::template work<MIN>(p, idx, w);
             const uint32_t r1 = smem_u32(ring1), r2 = smem_u32(ring2);
+            if (MIN) {
+                const int nb = uniform(w.nb);
+                ok = readback_min(sh, r1, r2, xch, tmem, p.status, nb, Policy::tree_order(p) ? nb >> 5 : nb, q, part, lane, pos, tp, xphase);
+                continue;
+            }
             switch (uniform(w.npad)) {
                 case 128: ok = readback<Policy, Params, 4, 1, 32>(p, w, sh, r1, r2, xch, tmem, q, part, lane, pos, tp, xphase); break;
                 case 64: ok = readback<Policy, Params, 2, 2, 32>(p, w, sh, r1, r2, xch, tmem, q, part, lane, pos, tp, xphase); break;
@@ -634,7 +706,7 @@ __global__ void __launch_bounds__(kG_Threads, 1) gemm_i8_kernel(const Params p, 
                 do {   // a skipped index costs one more atomic
                     if (lane == 0) idx = atomicAdd(tile_counter, 1);
                     idx = __shfl_sync(0xffffffffu, idx, 0);
-                    ws = Policy::work(p, idx, w);
+                    ws = Policy::template work<MIN>(p, idx, w);
                 } while (ws == kWorkSkip);
                 const int slot = (int)(tn % kG_Sched);
                 if (!mbar_wait(&sh.sempty[slot], ((tn / kG_Sched) & 1u) ^ 1u)) { gemm_timeout(sh, p.status, lane); ok = false; break; }
@@ -654,11 +726,12 @@ __global__ void __launch_bounds__(kG_Threads, 1) gemm_i8_kernel(const Params p, 
             int idx;
             while (ok && (idx = take_tile(sh, p.status, tn, lane)) >= 0) {
                 GemmWork w;
-                Policy::work(p, idx, w);
+                Policy::template work<MIN>(p, idx, w);
                 const uint32_t r1 = smem_u32(ring1), r2 = smem_u32(ring2);
                 if (warp == 1) {
                     const uint32_t cst = smem_u32(smem);
-                    switch (uniform(w.npad)) {
+                    if (MIN) ok = mma_tile<Policy, 32>(p, w, sh, cst, r1, r2, tmem, pos, tp, lane);
+                    else switch (uniform(w.npad)) {
                         case 128: ok = mma_tile<Policy, 128>(p, w, sh, cst, r1, r2, tmem, pos, tp, lane); break;
                         case 64: ok = mma_tile<Policy, 64>(p, w, sh, cst, r1, r2, tmem, pos, tp, lane); break;
                         case 32: ok = mma_tile<Policy, 32>(p, w, sh, cst, r1, r2, tmem, pos, tp, lane); break;
@@ -667,7 +740,7 @@ __global__ void __launch_bounds__(kG_Threads, 1) gemm_i8_kernel(const Params p, 
                 } else if (warp < kG_FirstEpi) {
                     ok = expand_tile<Policy>(p, w, sh, r1, r2, pos, warp - 2, lane);
                 } else {
-                    ok = store_tile<Policy>(p, w, sh, xch, warp - kG_FirstEpi, lane, xphase);
+                    ok = store_tile<Policy, MIN>(p, w, sh, xch, warp - kG_FirstEpi, lane, xphase);
                 }
             }
         }
@@ -684,6 +757,7 @@ __global__ void __launch_bounds__(kG_Threads, 1) gemm_i8_kernel(const Params p, 
 // ------------------------------------------------------------------ policies ----
 // plain fp32 tile store: out[(row0 + r) * ldo + col0 + c] = D[r][c]  (the primitive; operands in the mma128 form)
 struct PlainPolicy {
+    template <bool>
     __device__ static __forceinline__ int work(const GemmParams& p, int idx, GemmWork& w) {
         if (idx >= p.n_items) return kWorkEnd;
         const GemmItem it = p.items[idx];
@@ -694,8 +768,9 @@ struct PlainPolicy {
         return kWorkOk;
     }
     __device__ static __forceinline__ int type(const GemmParams&, const GemmWork&) { return kTypeOperand; }
+    __device__ static __forceinline__ bool tree_order(const GemmParams&) { return false; }
     __device__ static __forceinline__ RowTiles rows(const GemmParams& p, const GemmWork& w) { return RowTiles{p.a_base + p.items[w.expert].a_offset, nullptr, 0, 0, 0}; }
-    template <int KG>
+    template <int KG, bool MIN>
     __device__ static __forceinline__ void store(const GemmParams& p, const GemmWork& w, const float* xch, int ew, int lane) {
         for (int r = ew; r < w.rt; r += kG_EpiWarps)   // (all tiles of the primitive are 128 columns wide: one share)
             for (int c = lane; c < w.n_valid; c += 32) p.out[(size_t)(w.aux0 + r) * p.ldo + w.aux1 + c] = xch[c * 128 + r];
@@ -710,7 +785,19 @@ __device__ __forceinline__ int tile_width(int n) { return n <= 16 ? 16 : n <= 32
 
 // What the gate/up and the down launch share: the tile list and where a row tile's weights are.
 struct MoePolicy {
+    template <bool MIN>
     __device__ static __forceinline__ int work(const PrefillGemmParams& p, int idx, GemmWork& w) {
+        if (MIN) {   // shared-expert tiles of 32 tokens; word 1 of the list: their first column / 16
+            const PrefillGemmMats& m = p.m[1];
+            const int j = idx / m.row_tiles, t0 = j * 32;
+            if (t0 >= p.T) return kWorkEnd;
+            w.shared = 1; w.expert = 0; w.rt = idx - j * m.row_tiles;
+            w.nb = m.ncols >> 5; w.n_valid = min(32, p.T - t0); w.npad = 32;
+            w.start = t0; w.col16 = __ldcg(p.tiles + 1) + 2 * j;
+            w.b = p.b_tiles + (size_t)w.col16 * p.b_col16_bytes;
+            w.aux0 = w.aux1 = 0;
+            return kWorkOk;
+        }
         const int j = idx / p.row_tiles_max, rt = idx - j * p.row_tiles_max;
         if (j >= __ldcg(p.tiles)) return kWorkEnd;
         const int4 t = __ldcg(reinterpret_cast<const int4*>(p.tiles + kTileHeader) + j);
@@ -725,6 +812,7 @@ struct MoePolicy {
         return kWorkOk;
     }
     __device__ static __forceinline__ int type(const PrefillGemmParams& p, const GemmWork& w) { return p.m[w.shared].type; }
+    __device__ static __forceinline__ bool tree_order(const PrefillGemmParams& p) { return p.shared_sums != 0; }   // (set for the gate/up launch)
     // gated: two 32-row tiles of the gate matrix and the same two of the up matrix; else four of the one matrix
     __device__ static __forceinline__ RowTiles rows(const PrefillGemmParams& p, const GemmWork& w) {
         const PrefillGemmMats& m = p.m[w.shared];
@@ -758,12 +846,12 @@ __device__ __forceinline__ float xch_sum(const float* xch, int npad, int row, in
 // a 32-row block of the intermediate and every second or every column of the tile, two columns at a time so that the
 // divisions of one hide the other's.
 struct GateUpPolicy : MoePolicy {
-    template <int KG>
+    template <int KG, bool MIN>
     __device__ static __forceinline__ void store(const PrefillGemmParams& p, const GemmWork& w, const float* xch, int ew, int lane) {
         const int nrb = p.dual ? 2 : 4, rb = ew & (nrb - 1), blk = w.rt * nrb + rb;
         if (blk >= p.m[w.shared].rows32) return;     // (the last row tile may be partly filled)
         const int cstep = kG_EpiWarps / nrb, r = rb * 32 + lane;
-        const bool sums = w.shared && p.shared_sums;   // the down matrix of the shared expert has minimums: it wants the blocks' sums too
+        const bool sums = MIN;   // the down matrix has minimums too: it wants the blocks' sums
         uint8_t* tile = p.out_tiles + (size_t)w.col16 * p.out_col16_bytes;
         uint8_t* dst = sums ? tile + (size_t)(blk >> 2) * (w.npad * 160) + (blk & 3) * (w.npad * 36) : tile + (size_t)blk * (w.npad * 36);
         float* sdst = reinterpret_cast<float*>(tile + (size_t)(blk >> 2) * (w.npad * 160) + w.npad * 144 + (blk & 3) * (w.npad * 4));
@@ -775,16 +863,14 @@ struct GateUpPolicy : MoePolicy {
             for (int i = 0; i < 2; ++i) {
                 const int ci = min(c + i * cstep, w.n_valid - 1);
                 const float a = xch_sum<KG>(xch, w.npad, r, ci);
-                if (p.dual) v[i] = silu_mul_near(a, xch_sum<KG>(xch, w.npad, r + 64, ci));
+                if (p.dual) { const float u = xch_sum<KG>(xch, w.npad, r + 64, ci); v[i] = MIN ? silu_mul_ref(a, u) : silu_mul_near(a, u); }
                 else { const float t = fmaxf(a, 0.0f); v[i] = t * t; }
             }
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
                 const int ci = c + i * cstep;
-                // largest magnitude of the block: bit patterns of non-negative floats order like the values
-                const float amax = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(fabsf(v[i]))));
-                const float d = div_near(amax, 127.0f);
-                const int8_t qv = (amax == 0.0f) ? (int8_t)0 : (int8_t)round_int(div_near(v[i], d));
+                float d;
+                const int8_t qv = q8_1_warp(v[i], d);
                 if (ci < w.n_valid) {
                     qdst[(ci >> 3) * 128 + (ci & 7) * 16] = qv;
                     if (lane == 0) ddst[ci] = __half2float(__float2half(d));
@@ -812,7 +898,7 @@ struct GateUpPolicy : MoePolicy {
 // down: rows of H; the tile's columns are pairs, written to pair_out[pair row][H].  A warp stores the 128 rows of every fourth
 // column, four rows per lane (H is a multiple of 32).
 struct DownPolicy : MoePolicy {
-    template <int KG>
+    template <int KG, bool MIN>
     __device__ static __forceinline__ void store(const PrefillGemmParams& p, const GemmWork& w, const float* xch, int ew, int lane) {
         const bool rows = w.rt * 128 + lane * 4 < p.H;
         float* out = p.pair_out + w.rt * 128 + lane * 4;
@@ -873,12 +959,12 @@ static int gemm_grid(int n_items) {
     const int n_sm = sm_count();
     return n_items < n_sm ? n_items : n_sm;
 }
-template <class Policy, class Params>
+template <class Policy, bool MIN = false, class Params>
 static cudaError_t launch_gemm(const Params& p, int n_items, int32_t* counter, cudaStream_t stream) {
     static bool attr_done[64] = {};
-    cudaError_t e = max_smem_once(gemm_i8_kernel<Policy, Params>, (int)kG_Smem, attr_done);
+    cudaError_t e = max_smem_once(gemm_i8_kernel<Policy, Params, MIN>, (int)kG_Smem, attr_done);
     if (e != cudaSuccess) return e;
-    return launch_pdl(gemm_i8_kernel<Policy, Params>, dim3(gemm_grid(n_items)), kG_Threads, kG_Smem, stream, p, counter);
+    return launch_pdl(gemm_i8_kernel<Policy, Params, MIN>, dim3(gemm_grid(n_items)), kG_Threads, kG_Smem, stream, p, counter);
 }
 
 // tile_counter: one int32 of device memory that is zero when the kernel starts (it ends at n_items + the number of CTAs)
@@ -894,6 +980,11 @@ cudaError_t launch_prefill_gemm(const PrefillGemmParams& p, bool down, int n_til
     const int n_items = n_tiles_max * p.row_tiles_max;
     if (n_items <= 0) return cudaSuccess;
     int32_t* counter = const_cast<int32_t*>(p.tiles) + (down ? 5 : 4);
+    if (p.m[1].type == kTypeOperandMin) {   // (words 6 / 7: these launches' counters)
+        const int n_min = (p.T + 31) / 32 * p.m[1].row_tiles;
+        const cudaError_t e = down ? launch_gemm<DownPolicy, true>(p, n_min, counter + 2, stream) : launch_gemm<GateUpPolicy, true>(p, n_min, counter + 2, stream);
+        if (e != cudaSuccess) return e;
+    }
     return down ? launch_gemm<DownPolicy>(p, n_items, counter, stream) : launch_gemm<GateUpPolicy>(p, n_items, counter, stream);
 }
 
@@ -1005,7 +1096,7 @@ cudaError_t launch_pack_mma128_q8_0(const void* raw, void* out, int n_mats, int 
 // are equally wide.
 __device__ __forceinline__ uint64_t width_bit(int n, uint64_t count) { return n > 64 ? count : n > 32 ? count << 16 : n > 16 ? count << 32 : count << 48; }
 __global__ void __launch_bounds__(256) build_tiles_kernel(const int32_t* offsets, const int32_t* perm, int32_t* tiles, int32_t* list, int E, int T,
-                                                          int has_shared, int gemm_min) {
+                                                          int has_shared, int gemm_min, int shared_32) {
     __shared__ uint64_t scan[8];
     __shared__ int scan_n[8];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -1040,7 +1131,9 @@ __global__ void __launch_bounds__(256) build_tiles_kernel(const int32_t* offsets
     __syncthreads();
     uint64_t before = incl - own, total = 0;
     for (int w = 0; w < 8; ++w) { if (w < warp) before += scan[w]; total += scan[w]; }
-    const int sh_full = has_shared ? T >> 7 : 0, sh_rem = has_shared ? T & 127 : 0;
+    // the shared expert's tiles: 128 columns and a rest, or (shared_32) tiles of 32 that are not on the list, their columns behind all
+    // others'
+    const int sh_full = has_shared && !shared_32 ? T >> 7 : 0, sh_rem = has_shared && !shared_32 ? T & 127 : 0;
     const uint64_t shared = (uint64_t)sh_full + (sh_rem ? width_bit(sh_rem, 1) : 0ull);
     total += shared;
     before += shared;   // the shared expert's tiles lead every width
@@ -1064,7 +1157,7 @@ __global__ void __launch_bounds__(256) build_tiles_kernel(const int32_t* offsets
         put(k, (int)((before >> (16 * k)) & 0xFFFFu) + (k == 0 ? nf : 0), tid, off + nf * 128, rem);
     }
     if (tid == 0) {
-        tiles[0] = first[4]; tiles[1] = 0; tiles[2] = 0; tiles[3] = 0;
+        tiles[0] = first[4]; tiles[1] = col16[4]; tiles[2] = 0; tiles[3] = 0;
         tiles[4] = 0; tiles[5] = 0; tiles[6] = 0; tiles[7] = 0;   // the two GEMM launches' tile counters start at zero
     }
 }
@@ -1075,44 +1168,52 @@ __global__ void __launch_bounds__(256) build_tiles_kernel(const int32_t* offsets
 // token's 16-byte chunks are read four in a row.  Columns without a token are left as they are (nobody reads their sums).
 __global__ void __launch_bounds__(256) gather_tiles_kernel(const int32_t* tiles, const int32_t* perm, const int8_t* x_q, int64_t x_q_stride,
                                                            const float* x_d, int x_d_stride, const uint8_t* x_q8, uint8_t* b_tiles,
-                                                           int64_t b_col16_bytes, int H, int top_k, int shared_sums) {
+                                                           int64_t b_col16_bytes, int H, int top_k, int shared_sums, int T) {
     griddep_wait();
     if (threadIdx.x == 0) griddep_launch();
     const int j = blockIdx.x, grp = blockIdx.y;
-    if (j >= __ldcg(tiles)) return;
-    const int4 t = __ldcg(reinterpret_cast<const int4*>(tiles + kTileHeader) + j);
+    const int listed = __ldcg(tiles);
+    int4 t;
+    if (j < listed) t = __ldcg(reinterpret_cast<const int4*>(tiles + kTileHeader) + j);
+    else {
+        const int i = j - listed;   // a shared expert's tiles of 32 tokens
+        if (!shared_sums || i * 32 >= T) return;
+        t = make_int4(-1, i * 32, min(32, T - i * 32), __ldcg(tiles + 1) + 2 * i);
+    }
     const int sl = threadIdx.x & 7, lane_ch = threadIdx.x >> 3;
-    const int c = grp * 8 + sl, npad = tile_width(t.z);   // token slot of the tile
+    const bool sums = t.x < 0 && shared_sums;   // a shared expert with minimums
+    const int c = grp * 8 + sl, npad = sums ? 32 : tile_width(t.z);   // token slot of the tile
     if (c >= t.z) return;
     const int tok = t.x < 0 ? t.y + c : __ldcg(perm + t.y + c) / top_k;
     uint8_t* base = b_tiles + (size_t)t.w * b_col16_bytes;
-    // a shared expert with minimums: stages of four blocks, each with the blocks' sums (the Q8_1 rows' second half) behind it
-    const bool sums = t.x < 0 && shared_sums;
+    // a shared expert with minimums: blocks in tree order, stages of four, each with the blocks' sums (the Q8_1 rows' second half) behind it
+    auto place = [&](int b) { return sums ? operand_min_block(b, H / 32) : b; };
     auto block = [&](int b) { return base + (sums ? (size_t)(b >> 2) * (npad * 160) + (b & 3) * (npad * 36) : (size_t)b * (npad * 36)); };
     for (int ch = lane_ch; ch < H / 16; ch += 32) {
         const uint4 v = __ldcg(reinterpret_cast<const uint4*>(x_q + (size_t)tok * x_q_stride) + ch);
-        *reinterpret_cast<uint4*>(block(ch >> 1) + (ch & 1) * (npad * 16) + grp * 128 + sl * 16) = v;
+        *reinterpret_cast<uint4*>(block(place(ch >> 1)) + (ch & 1) * (npad * 16) + grp * 128 + sl * 16) = v;
     }
     for (int b = lane_ch; b < H / 32; b += 32) {
-        *reinterpret_cast<float*>(block(b) + npad * 32 + c * 4) = __ldcg(x_d + (size_t)tok * x_d_stride + b);
+        const int at = place(b);
+        *reinterpret_cast<float*>(block(at) + npad * 32 + c * 4) = __ldcg(x_d + (size_t)tok * x_d_stride + b);
         if (sums) {
             const uint32_t ds = __ldcg(reinterpret_cast<const uint32_t*>(x_q8 + ((size_t)tok * (H / 32) + b) * kQ81Bytes));
-            *reinterpret_cast<float*>(base + (size_t)(b >> 2) * (npad * 160) + npad * 144 + (b & 3) * (npad * 4) + c * 4) = h2f(ds >> 16);
+            *reinterpret_cast<float*>(base + (size_t)(at >> 2) * (npad * 160) + npad * 144 + (at & 3) * (npad * 4) + c * 4) = h2f(ds >> 16);
         }
     }
 }
 
 cudaError_t launch_build_tiles(const int32_t* offsets, const int32_t* perm, int32_t* tiles, int32_t* list, int E, int T, int has_shared, int gemm_min,
-                               cudaStream_t stream) {
-    return launch_pdl(build_tiles_kernel, dim3(1), 256, 0, stream, offsets, perm, tiles, list, E, T, has_shared, gemm_min);
+                               int shared_32, cudaStream_t stream) {
+    return launch_pdl(build_tiles_kernel, dim3(1), 256, 0, stream, offsets, perm, tiles, list, E, T, has_shared, gemm_min, shared_32);
 }
 
 cudaError_t launch_gather_tiles(const int32_t* tiles, const int32_t* perm, const int8_t* x_q, int64_t x_q_stride, const float* x_d,
                                 int x_d_stride, const uint8_t* x_q8, uint8_t* b_tiles, int64_t b_col16_bytes, int H, int top_k, int n_tiles_max,
-                                bool shared_sums, cudaStream_t stream) {
+                                bool shared_sums, int T, cudaStream_t stream) {
     if (n_tiles_max <= 0) return cudaSuccess;
     return launch_pdl(gather_tiles_kernel, dim3(n_tiles_max, 16), 256, 0, stream, tiles, perm, x_q, x_q_stride, x_d, x_d_stride, x_q8, b_tiles, b_col16_bytes,
-                      H, top_k, shared_sums ? 1 : 0);
+                      H, top_k, shared_sums ? 1 : 0, T);
 }
 
 }  // namespace chimere

@@ -166,13 +166,20 @@ struct PrefillGemmParams {
 };
 cudaError_t launch_prefill_gemm(const PrefillGemmParams& p, bool down, int n_tiles_max, cudaStream_t stream);
 cudaError_t launch_build_tiles(const int32_t* offsets, const int32_t* perm, int32_t* tiles, int32_t* list, int E, int T, int has_shared, int gemm_min,
-                               cudaStream_t stream);
+                               int shared_32, cudaStream_t stream);
 cudaError_t launch_gather_tiles(const int32_t* tiles, const int32_t* perm, const int8_t* x_q, int64_t x_q_stride, const float* x_d,
                                 int x_d_stride, const uint8_t* x_q8, uint8_t* b_tiles, int64_t b_col16_bytes, int H, int top_k, int n_tiles_max,
-                                bool shared_sums, cudaStream_t stream);
+                                bool shared_sums, int T, cudaStream_t stream);
 constexpr int kTypeOperand = 100;    // PrefillGemmMats::type of weights in the MMA's own order (mma128 tiles)
 constexpr int kTypeOperandMin = 101; // ... with a minimum per row and block beside the scale (Q4_K, Q5_K), grouped by stages of four blocks
 constexpr int kOperandMinStage = 4 * (4096 + 512 + 512);
+// Place of block b among nb (a multiple of 32) in the order in which a running tree can add them up as the GEMV kernel's lanes do
+// (lane l: blocks l, l + 32, ... in sequence; then lanes 16, 8, 4, 2, 1 apart): lanes in bit-reversed order, a lane's blocks together.
+__host__ __device__ inline int operand_min_block(int b, int nb) {
+    const int l = b & 31;
+    const int n = ((l & 1) << 4) | ((l & 2) << 2) | (l & 4) | ((l & 8) >> 2) | ((l & 16) >> 4);
+    return n * (nb >> 5) + (b >> 5);
+}
 cudaError_t launch_pack_operand_min(int type, const void* raw, void* out, int nrows, int ncols, int mode, cudaStream_t stream);
 cudaError_t launch_pack_mma128_q8_0(const void* raw, void* out, int n_mats, int nrows, int ncols, int mode, int64_t raw_stride, int64_t out_stride,
                                     cudaStream_t stream);

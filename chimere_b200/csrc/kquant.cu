@@ -160,8 +160,9 @@ __global__ void __launch_bounds__(256) act_q8_1_kernel(const float* __restrict__
 }
 
 // Q4_K / Q5_K rows -> the grouped GEMM's operand with minimums: per (128-row tile, stage of four 32-weight sub-blocks) four mma128
-// tiles (int8 quants, f32 d * sc) and then [4][128] f32 -dmin * m * 2^-49 (the power of two the GEMM's sums carry).  mode as for
-// the plain operand: 0 rows as they are, 1 / 2 gate / up rows interleaved per 64.  One thread per (row, sub-block).
+// tiles (int8 quants, words of f16 d << 16 | sc) and then [4][128] f32 -dmin * m * 2^-49 (the power of two the GEMM's sums carry).  mode as for
+// the plain operand: 0 rows as they are, 1 / 2 gate / up rows interleaved per 64 and sub-blocks in tree order (operand_min_block).
+// One thread per (row, sub-block).
 template <int TYPE>
 __global__ void __launch_bounds__(256) pack_operand_min_kernel(const uint8_t* __restrict__ raw, uint8_t* __restrict__ out, int nrows, int ncols, int mode) {
     const int nb = ncols >> 5;
@@ -171,12 +172,12 @@ __global__ void __launch_bounds__(256) pack_operand_min_kernel(const uint8_t* __
     SubBlock s;
     decode_sub<TYPE>(raw + ((size_t)r * (ncols >> 8) + (b >> 3)) * KBlock<TYPE>::kBytes, b & 7, s);
     const int dr = mode == 0 ? r : (r >> 6) * 128 + (r & 63) + (mode == 2 ? 64 : 0);
-    const int tile = dr >> 7, rr = dr & 127, u = b & 3;
-    uint8_t* stage = out + ((size_t)tile * (nb >> 2) + (b >> 2)) * kOperandMinStage;
+    const int at = mode == 0 ? b : operand_min_block(b, nb), tile = dr >> 7, rr = dr & 127, u = at & 3;
+    uint8_t* stage = out + ((size_t)tile * (nb >> 2) + (at >> 2)) * kOperandMinStage;
     uint8_t* dst = stage + u * 4608;
     *reinterpret_cast<uint4*>(dst + (rr >> 3) * 128 + (rr & 7) * 16) = make_uint4(s.w[0], s.w[1], s.w[2], s.w[3]);
     *reinterpret_cast<uint4*>(dst + 2048 + (rr >> 3) * 128 + (rr & 7) * 16) = make_uint4(s.w[4], s.w[5], s.w[6], s.w[7]);
-    *reinterpret_cast<float*>(dst + 4096 + rr * 4) = s.d * (float)s.sc;
+    *reinterpret_cast<uint32_t*>(dst + 4096 + rr * 4) = ((uint32_t)__half_as_ushort(__float2half(s.d)) << 16) | (uint32_t)s.sc;
     *reinterpret_cast<float*>(stage + 4 * 4608 + u * 512 + rr * 4) = -(s.dmin * (float)s.mn) * __uint_as_float(0x27000000u);   // 2^-49
 }
 

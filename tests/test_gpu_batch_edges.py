@@ -46,9 +46,10 @@ def test_partly_filled_row_tiles(kw, T):
 
 
 @pytest.mark.parametrize("types", [(formats.TYPE_Q5_K, formats.TYPE_Q5_K), (formats.TYPE_Q4_K, formats.TYPE_Q5_K), (formats.TYPE_Q5_K, formats.TYPE_Q6_K)], ids=str)
-@pytest.mark.parametrize("T", [8, 33, 129])
-def test_kquant_shared_expert_beside_packed_experts(types, T):
-    _check(configs.scaled(IQ3, E=4, top_k=2, H=512, F=256, F_s=512, type_sh_gate_up=types[0], type_sh_down=types[1]), T, prefill=True)
+@pytest.mark.parametrize("H", [512, 1024, 3072])
+@pytest.mark.parametrize("T", [8, 32, 33, 129])
+def test_kquant_shared_expert_beside_packed_experts(types, H, T):
+    _check(configs.scaled(IQ3, E=4, top_k=2, H=H, F=256, F_s=512, type_sh_gate_up=types[0], type_sh_down=types[1]), T, prefill=True)
 
 
 # weights read packed and weights in operand order in one launch
