@@ -162,10 +162,11 @@ __device__ void build_dispatch_small(const RouteParams& p, int* smem_i, const in
     // sorted position tid starts a new expert?  (warps 0 and 1 hold the 64 positions)
     unsigned lead = 0u;
     if (warp < 2) {
-        // (entry starts: every gt-th pair of an expert; an expert has at most T <= 4 pairs here)
+        // (entry starts: every gt-th pair of an expert, gt a power of two; an expert has at most T <= 4 pairs here.  One pair per
+        // entry needs no look at the neighbours: this is on the chain of a single token's layer)
         int rank = 0;
-        while (rank < tid && tid < total && s_sid[tid - rank - 1] == s_sid[tid]) ++rank;
-        const bool first = tid < total && rank % gt == 0;
+        if (gt > 1) while (rank < tid && tid < total && s_sid[tid - rank - 1] == s_sid[tid]) ++rank;
+        const bool first = tid < total && (rank & (gt - 1)) == 0;
         lead = __ballot_sync(0xffffffffu, first);
         if (lane == 0) s_lead[warp] = __popc(lead);
     }
