@@ -82,10 +82,11 @@ constexpr int kForwardGemmPairs = 3;
 int forward_gemm_tokens(const chimere_moe_layer* w) { return (int64_t)w->F * w->H > (1 << 21) ? 17 : 41; }
 static_assert(kForwardGemmPairs <= kMaxGroupTokens + 1, "a small expert must fit one work entry");
 // ---------------------------------------------------------------- grouped GEMM path ----
-// Token tiles of a batch: at most P / 128 full ones and one partial one per expert with pairs, and the shared expert's.
-int n_tiles_max_for(const chimere_moe_layer* w, int T) {
+// Token tiles of a batch: at most P / widest full ones and one partial one per expert with pairs, and the shared expert's.
+constexpr int kTileColumns = 128, kForwardTileColumns = 64;   // columns of a full token tile: prefill / decode entry
+int n_tiles_max_for(const chimere_moe_layer* w, int T, int widest) {
     const int P = T * w->top_k;
-    return P / 128 + (w->E < P ? w->E : P) + (w->F_s > 0 ? kshared(w) ? (T + 31) / 32 : (T + 127) / 128 : 0);
+    return P / widest + (w->E < P ? w->E : P) + (w->F_s > 0 ? kshared(w) ? (T + 31) / 32 : (T + widest - 1) / widest : 0);
 }
 // ... and their columns / 16: a tile of n pairs is at most max(16, 2 n) columns wide.
 int64_t n_col16_max_for(const chimere_moe_layer* w, int T) {
@@ -107,7 +108,7 @@ PrefillArena prefill_arena(const chimere_moe_layer* w, int T) {
     A.b2_col16 = (int64_t)(Fmax / 32) * per;
     const int64_t cols = n_col16_max_for(w, T);
     size_t o = 0;
-    A.tiles = o; o += up256((size_t)(8 + 4 * n_tiles_max_for(w, T)) * 4);
+    A.tiles = o; o += up256((size_t)(8 + 4 * n_tiles_max_for(w, T, kForwardTileColumns)) * 4);
     A.bx = o; o += up256((size_t)(cols * A.bx_col16));
     A.b2 = o; o += up256((size_t)(cols * A.b2_col16));
     A.total = o;
@@ -593,7 +594,9 @@ int chimere_b200_moe_forward(const chimere_moe_layer* w, const float* d_x, float
     const chimere_moe_layer wr_ = ks ? routed_only(w) : *w;
     const chimere_moe_layer* wr = &wr_;
     cudaError_t e;
-    if (forward_gemm(wr, T) && ws->prefill_arena && ws->prefill_bytes >= prefill_arena(wr, ws->max_T).total) {
+    const Layout L = make_layout(wr, ws->max_T);
+    if (forward_gemm(wr, T) && ws->prefill_arena && ws->prefill_bytes >= prefill_arena(wr, ws->max_T).total &&
+        tiled_bulk_runs(gate_up_params(wr, T, ws, L), down_params(wr, d_y, T, ws, L))) {
         RouteParams rp = route_params(wr, d_x, T, ws, ks);
         rp.list_mode = 2;
         e = launch_route(rp, stream);
@@ -602,7 +605,6 @@ int chimere_b200_moe_forward(const chimere_moe_layer* w, const float* d_x, float
         if (rc) return rc;
         e = finish_tokens(wr, d_y, T, ws, stream);
     } else {
-        const Layout L = make_layout(wr, ws->max_T);
         const int max_entries = max_entries_for(wr, T);
         e = launch_route(route_params(wr, d_x, T, ws, ks), stream);
         if (e != cudaSuccess) return cuda_rc(e);
@@ -840,8 +842,9 @@ static int gemm_experts(const chimere_moe_layer* w, const chimere_moe_prefill_we
     uint8_t* base = (uint8_t*)ws->prefill_arena;
     int32_t* tiles = (int32_t*)(base + A.tiles);
     const Layout L = make_layout(w, ws->max_T);
-    const int n_tiles_max = E > 0 ? n_tiles_max_for(w, T) : (T + 127) / 128;
-    cudaError_t e = launch_build_tiles(ws->offsets, ws->perm, tiles, mixed ? ws->group_list : nullptr, E, T, w->F_s > 0, mixed ? kForwardGemmPairs : 1, kshared(w), stream);
+    const int widest = mixed ? kForwardTileColumns : kTileColumns;
+    const int n_tiles_max = E > 0 ? n_tiles_max_for(w, T, widest) : (T + 127) / 128;
+    cudaError_t e = launch_build_tiles(ws->offsets, ws->perm, tiles, mixed ? ws->group_list : nullptr, E, T, w->F_s > 0, mixed ? kForwardGemmPairs : 1, kshared(w), widest, stream);
     if (e != cudaSuccess) return cuda_rc(e);
     // the rows' Q8_1 planes: the workspace's, or (expert-parallel owner) the received packed rows in place
     const int8_t* xq = d_packed ? (const int8_t*)d_packed : ws->x_q;
@@ -858,7 +861,7 @@ static int gemm_experts(const chimere_moe_layer* w, const chimere_moe_prefill_we
         if (e != cudaSuccess) return cuda_rc(e);
         GemvParams dn = down_params(w, nullptr, T, ws, L);
         dn.no_combine = 1; dn.few_tokens = 1;
-        dn.nrows_shared = 0; dn.ncols_shared = 0; dn.sh_a = nullptr; dn.sh_b = nullptr;
+        dn.nrows_shared = 0; dn.ncols_shared = 0; dn.sh_a = nullptr; dn.sh_b = nullptr; dn.split_cols_shared = w->F_s;
         e = launch_down_tiled(dn, max_entries, stream);
         if (e != cudaSuccess) return cuda_rc(e);
     }
@@ -875,7 +878,13 @@ static int gemm_experts(const chimere_moe_layer* w, const chimere_moe_prefill_we
         g.b_tiles = base + (down ? A.b2 : A.bx); g.b_col16_bytes = down ? A.b2_col16 : A.bx_col16;
         g.out_tiles = base + A.b2; g.out_col16_bytes = A.b2_col16;
         g.pair_out = ws->pair_out;
-        if (mixed) { g.inter_q8 = ws->inter_q8; g.inter_stride = (int64_t)L.inter_stride; }
+        if (mixed) {   // sums as the GEMV kernels form them: a token's result does not depend on its batch
+            g.inter_q8 = ws->inter_q8; g.inter_stride = (int64_t)L.inter_stride;
+            g.as_gemv = 1;
+            const int wk = down ? tiled_down_geom(w->type_down, w->F, w->type_sh_down, w->F_s, T).wk
+                                : tiled_gate_up_geom(w->type_up, w->type_sh_up, w->H, w->F_s > 0).wk;
+            for (PrefillGemmMats& m : g.m) m.slice = m.ncols > 0 ? tiled_slice_units(m.type, m.ncols, wk) / 4 : 1;
+        }
         e = launch_prefill_gemm(g, down != 0, n_tiles_max, stream);
     }
     return cuda_rc(e);

@@ -143,6 +143,9 @@ struct GemmWork {
     int aux0, aux1;
 };
 constexpr int kWorkOk = 0, kWorkSkip = 1, kWorkEnd = 2;
+// Kernel instances.  kMin: the tiles with minimums (Q4_K / Q5_K shared expert) and no others.  kOrdered: the decode entry's tiles, whose
+// sums are bit for bit the GEMV kernels' (readback_ordered): packed weights, tiles of up to 64 columns.
+constexpr int kPlain = 0, kMin = 1, kOrdered = 2;
 struct RowTiles { const uint8_t* src0; const uint8_t* src1; int tile_bytes, n0, n1; };   // the 32-row tiles of a GemmWork (see produce_tile)
 
 // Position in the two operand rings; every role walks the same sequence.  Ring 1 has two geometries (slots for tiles of
@@ -185,14 +188,16 @@ __device__ __forceinline__ void gemm_timeout(GemmShared& sh, int32_t* status, in
 
 // ------------------------------------------------------------------ roles ----
 // First unit of stage s.  IQ3_S tiles keep a super-block's scales behind its eight units, so its second half is taken first
-// (one copy brings both) and the expanders keep the scales for the first half.
-__device__ __forceinline__ int stage_unit(int type, int s) { return kG_StageUnits * (type == CHIMERE_TYPE_IQ3_S ? s ^ 1 : s); }
+// (one copy brings both) and the expanders keep the scales for the first half; kOrdered takes the units as they come and the
+// scales with a copy of their own.
+template <int MODE>
+__device__ __forceinline__ int stage_unit(int type, int s) { return kG_StageUnits * (MODE != kOrdered && type == CHIMERE_TYPE_IQ3_S ? s ^ 1 : s); }
 
 // Warp 0: copies of one tile, a few pieces per stage, all issued by the elected lane (a copy costs its warp about 50 cycles).
-template <class Policy, class Params>
+template <class Policy, int MODE, class Params>
 __device__ __forceinline__ bool produce_tile(const Params& p, const GemmWork& w, GemmShared& sh, uint8_t* ring1, uint8_t* ring2, RingPos& pos, int lane) {
     const int type = uniform(Policy::type(p, w)), nb = uniform(w.nb), npad = uniform(w.npad);
-    const bool operand = type >= kTypeOperand;
+    const bool operand = MODE != kOrdered && type >= kTypeOperand;
     const int slim = npad <= 32;
     if (slim != pos.slim) {   // the other slot geometry: every slot of the old one has to be empty first
         for (int r = 0; r < pos.slots1(); ++r)
@@ -207,7 +212,7 @@ __device__ __forceinline__ bool produce_tile(const Params& p, const GemmWork& w,
     const uint32_t tile_bytes = (uint32_t)uniform(rt.tile_bytes), n0 = (uint32_t)uniform(rt.n0), n1 = (uint32_t)uniform(rt.n1);
     const int nstages = (nb + kG_StageUnits - 1) / kG_StageUnits;
     for (int s = 0; s < nstages; ++s) {
-        const int u0 = stage_unit(type, s), nu = min(kG_StageUnits, nb - u0);
+        const int u0 = stage_unit<MODE>(type, s), nu = min(kG_StageUnits, nb - u0);
         uint64_t* bar = &sh.full1[pos.r];
         bool ok = mbar_wait(&sh.empty1[pos.r], pos.released(pos.r));
         if (ok && operand) ok = mbar_wait(&sh.empty1[pos.lag()], pos.released(pos.lag()));
@@ -216,7 +221,8 @@ __device__ __forceinline__ bool produce_tile(const Params& p, const GemmWork& w,
         // a token block: 32 values and a scale per column, beside weights with minimums the column's sum as well (by stages)
         const uint32_t bcol = type == kTypeOperandMin ? 40u : 36u, bbytes = (uint32_t)(nu * npad) * bcol;
         // 4-bit types: bytes of one row tile, and where they start in it
-        const uint32_t piece = type == CHIMERE_TYPE_Q4_0 ? (uint32_t)nu * 576u : (s & 1) ? 2048u : 2240u;
+        const uint32_t piece = type == CHIMERE_TYPE_Q4_0 ? (uint32_t)nu * 576u : (s & 1) || MODE == kOrdered ? 2048u : 2240u;
+        const bool scales = MODE == kOrdered && type == CHIMERE_TYPE_IQ3_S && !(s & 1);   // (behind the super-block's units, 192 bytes)
         const uint32_t off = type == CHIMERE_TYPE_Q4_0 ? (uint32_t)u0 * 576u : (uint32_t)(u0 >> 3) * 4288u + (uint32_t)(u0 & 4) * 512u;
         if (elect_one()) {
             if (operand) {
@@ -224,13 +230,19 @@ __device__ __forceinline__ bool produce_tile(const Params& p, const GemmWork& w,
                 mbar_expect_tx(bar, abytes + bbytes);
                 bulk_g2s(ring2 + (uint32_t)pos.e * kG_ASlot, src0 + (size_t)u0 * (type == kTypeOperand ? kG_MmaTile : kOperandMinStage / kG_StageUnits), abytes, bar);
             } else {
-                mbar_expect_tx(bar, (n0 + n1) * piece + bbytes);
+                mbar_expect_tx(bar, (n0 + n1) * (piece + (scales ? 192u : 0u)) + bbytes);
                 const uint8_t* a = src0 + off;
                 const uint8_t* b = src1 + off;
                 bulk_g2s(raw, a, piece, bar);
                 if (n0 > 1) bulk_g2s(raw + kG_RawBytes / 4, a + tile_bytes, piece, bar);
                 if (n1 > 0) bulk_g2s(raw + kG_RawBytes / 2, b, piece, bar);
                 if (n1 > 1) bulk_g2s(raw + 3 * (kG_RawBytes / 4), b + tile_bytes, piece, bar);
+                if (scales) {
+                    bulk_g2s(raw + 2048, a + 4096, 192u, bar);
+                    if (n0 > 1) bulk_g2s(raw + kG_RawBytes / 4 + 2048, a + tile_bytes + 4096, 192u, bar);
+                    if (n1 > 0) bulk_g2s(raw + kG_RawBytes / 2 + 2048, b + 4096, 192u, bar);
+                    if (n1 > 1) bulk_g2s(raw + 3 * (kG_RawBytes / 4) + 2048, b + tile_bytes + 4096, 192u, bar);
+                }
             }
             bulk_g2s(raw + kG_RawBytes, bsrc + (size_t)u0 * (npad * bcol), bbytes, bar);
         }
@@ -267,24 +279,31 @@ __device__ __forceinline__ void expand_units(uint32_t raw, uint32_t a, int x, in
     for (int i = 0; i < 8; ++i) expand_unit<TYPE>(v[i], dst + (i >> 1) * kG_MmaTile + (i & 1) * 1024);
 }
 
+// The word beside an expanded IQ3_S row of a unit: d * (1 + 2 * sub-scale) / 8 (exact in f32), or (kOrdered, which multiplies by the two
+// factors where the GEMV kernels do) f16 d in the upper half and 1 + 2 * sub-scale in the lower.
+template <int MODE>
+__device__ __forceinline__ uint32_t iq3s_word(uint32_t d16, uint32_t sub) {
+    return MODE == kOrdered ? (d16 << 16) | (1u + 2u * sub) : __float_as_uint(h2f(d16) * 0.125f * (float)(1u + 2u * sub));
+}
+__device__ __forceinline__ void sts_u32(uint32_t a, uint32_t v) { asm volatile("st.shared.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory"); }
+
 // Warps 2..3: warp x takes row tiles x and x + 2 of every stage.
-template <class Policy, class Params>
+template <class Policy, int MODE, class Params>
 __device__ __forceinline__ bool expand_tile(const Params& p, const GemmWork& w, GemmShared& sh, uint32_t ring1, uint32_t ring2, RingPos& pos, int x, int lane) {
     const int type = uniform(Policy::type(p, w)), nb = uniform(w.nb);
     const bool slim = uniform(w.npad) <= 32;
     pos.geometry(slim);
     const int nstages = (nb + kG_StageUnits - 1) / kG_StageUnits;
-    if (type >= kTypeOperand || slim) {   // nothing to do (slim tiles: half of the read-back warps expand) but keep step
-        for (int s = 0; s + 1 < nstages; ++s) pos.next(type < kTypeOperand);
+    if ((MODE != kOrdered && type >= kTypeOperand) || slim) {   // nothing to do (slim tiles: half of the read-back warps expand) but keep step
+        for (int s = 0; s + 1 < nstages; ++s) pos.next(MODE == kOrdered || type < kTypeOperand);
         // (parity tells a barrier's phases apart only within a round: see the tile's last bytes arrive before going on)
         if (!mbar_wait(&sh.full1[pos.r], pos.par1())) { gemm_timeout(sh, p.status, lane); return false; }
-        pos.next(type < kTypeOperand);
+        pos.next(MODE == kOrdered || type < kTypeOperand);
         return true;
     }
-    float d3[2] = {0.0f, 0.0f};        // IQ3_S: this lane's rows' scales of the super-block, kept over its two stages
-    uint32_t sc3[2] = {0u, 0u};
+    uint32_t d3[2] = {0u, 0u}, sc3[2] = {0u, 0u};   // IQ3_S: this lane's rows' scales of the super-block, kept over its two stages
     for (int s = 0; s < nstages; ++s) {
-        const int u0 = stage_unit(type, s), nu = min(kG_StageUnits, nb - u0);
+        const int u0 = stage_unit<MODE>(type, s);
         if (!mbar_wait(&sh.full1[pos.r], pos.par1()) || !mbar_wait(&sh.empty1[pos.lag()], pos.released(pos.lag()))) { gemm_timeout(sh, p.status, lane); return false; }
         const uint32_t raw = ring1 + pos.slot1_off(), a = ring2 + (uint32_t)pos.e * kG_ASlot;
         const uint32_t rec = a + 4096 + (x * 32 + lane) * 4;   // [unit] kG_MmaTile apart, row tile x + 2: 256 bytes further
@@ -301,13 +320,12 @@ __device__ __forceinline__ bool expand_tile(const Params& p, const GemmWork& w, 
             for (int h = 0; h < 2; ++h) {
                 if (!(s & 1)) {   // the scales came behind these units
                     const uint32_t t = raw + (x + 2 * h) * (kG_RawBytes / 4) + 2048;
-                    d3[h] = h2f(lds16(t + lane * 2)) * 0.125f;
+                    d3[h] = lds16(t + lane * 2);
                     sc3[h] = lds32(t + 64 + lane * 4);
                 }
                 const uint32_t sc = sc3[h] >> (4 * (u0 & 4));
 #pragma unroll
-                for (int u = 0; u < 4; ++u)   // d * (1 + 2 * sub-scale) is exact in f32
-                    sts_f32(rec + u * kG_MmaTile + h * 256, d3[h] * (float)(1u + 2u * ((sc >> (4 * u)) & 15u)));
+                for (int u = 0; u < 4; ++u) sts_u32(rec + u * kG_MmaTile + h * 256, iq3s_word<MODE>(d3[h], (sc >> (4 * u)) & 15u));
             }
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the MMAs read what ordinary stores wrote
@@ -322,14 +340,14 @@ __device__ __forceinline__ bool expand_tile(const Params& p, const GemmWork& w, 
 // more of them than A slots, and an A slot is refilled only after its stage has been read back.  Everything a block's MMA
 // needs is a constant away from the stage's values: with a slim tile the warp has about 400 cycles per stage, of which the
 // four MMAs and the commit take 360.
-template <class Policy, int NPAD, class Params>
+template <class Policy, int MODE, int NPAD, class Params>
 __device__ __forceinline__ bool mma_tile(const Params& p, const GemmWork& w, GemmShared& sh, uint32_t cst, uint32_t ring1, uint32_t ring2, uint32_t tmem,
                                          RingPos& pos, TmemPos& tp, int lane) {
     constexpr int kBps = blocks_per_slot(NPAD);
     constexpr bool kWide = NPAD == 128, kHandshake = NPAD >= 64;
     // D format S32 (2 << 4), A and B signed int8 (1 << 7, 1 << 10), both K-major, N (>> 3 at bit 17), M = 128 (>> 4 at bit 24)
     constexpr uint32_t kIdesc = (2u << 4) | (1u << 7) | (1u << 10) | (((uint32_t)NPAD >> 3) << 17) | ((128u >> 4) << 24);
-    const bool expanded = uniform(Policy::type(p, w)) < kTypeOperand;
+    const bool expanded = MODE == kOrdered || uniform(Policy::type(p, w)) < kTypeOperand;
     const int nb = uniform(w.nb);
     if (NPAD != tp.npad) {   // another width lays the accumulators out differently: everything has to be read back first
         for (int r = 0; r < pos.slots1(); ++r)
@@ -449,6 +467,83 @@ __device__ __forceinline__ bool readback_tile(GemmShared& sh, uint32_t ring1, ui
     return true;
 }
 
+// The read-back of one tile of packed weights by one warp, W of its columns and every stage, bit for bit what the GEMV kernels compute
+// for a token (gemv_tiled.cu), so that a token of a decode batch does not depend on how many others chose the same expert: with the
+// exact block dot t,  acc = fma(d * dx, t, acc) per block of Q4_0;  part = fma(t, dx, part) over the four blocks of a stage and
+// acc = fma(d, part, acc) for IQ3_S (t with the sub-block's factor);  slices of K (`slice` stages each) added up in order.  All sums carry 2^-49: t comes out of the
+// accumulator's float reading with one exact multiply-add (IQ3_S operands are 8, Q4_0 ones 16 times the weight; the Q4_0 scale in
+// shared memory is d / 16).
+template <int TYPE, int COLG, int W>
+__device__ __forceinline__ bool readback_ordered(GemmShared& sh, uint32_t ring1, uint32_t ring2, uint32_t tmem, int32_t* status, int nb, int slice, int q,
+                                                 int colg, int lane, RingPos& pos, TmemPos& tp, uint64_t (&total)[W / 2]) {
+    constexpr int kPad = COLG * W;
+    constexpr bool kHandshake = kPad >= 64, kGroup = TYPE == CHIMERE_TYPE_IQ3_S;
+    if (tp.npad != kPad) { tp.npad = kPad; tp.slot = 0; tp.nslots = kG_TmemCols / (kG_StageUnits * kPad); }
+    const uint32_t trow = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(colg * W);
+    const uint32_t rec0 = ring2 + 4096 + (uint32_t)(q * 32 + lane) * 4u, sb0 = ring1 + kG_RawBytes + kPad * 32 + colg * (W * 4);
+    uint64_t acc[W / 2];
+#pragma unroll
+    for (int i = 0; i < W / 2; ++i) acc[i] = total[i] = 0ull;
+    int left = slice;
+    for (int b0 = 0; b0 < nb; b0 += kG_StageUnits) {
+        const int nu = min(kG_StageUnits, nb - b0);
+        const uint32_t rec = rec0 + (uint32_t)pos.e * kG_ASlot, sb = sb0 + pos.slot1_off();
+        if (!mbar_wait(&sh.tfull[tp.slot], tp.par())) { gemm_timeout(sh, status, lane); return false; }
+        tc_fence_after();
+        const uint32_t t0 = trow + (uint32_t)(tp.slot * (kG_StageUnits * kPad));
+        uint64_t part[W / 2];
+        uint32_t word = 0;
+#pragma unroll
+        for (int i = 0; i < W / 2; ++i) part[i] = 0ull;
+#pragma unroll
+        for (int j = 0; j < kG_StageUnits; ++j) {
+            if (j >= nu) break;
+            int v[W];
+            tc_ld_nowait<W>(t0 + (uint32_t)(j * kPad), v);
+            word = lds32(rec + j * kG_MmaTile);
+            // 2^100; 2^97 times the factor: the exact dot times 2^-49 (times 16 for Q4_0), and what takes the offset 2^19 out again
+            const float m = kGroup ? (float)(word & 0xFFFFu) : 1.0f;
+            const float kr = kGroup ? m * __uint_as_float(kRowScaleBits - (3u << 23)) : __uint_as_float(kRowScaleBits);
+            const float ko = kGroup ? m * __uint_as_float(kOffsetBits - (3u << 23)) : __uint_as_float(kOffsetBits);
+            const uint64_t r2 = pack2f(kr, kr), o2 = pack2f(ko, ko), d2 = pack2(word, word);
+            tc_wait_ld();
+            if (kHandshake && j + 1 == nu) {   // the slot's last values are in registers: the MMAs may overwrite it
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive_n(&sh.tempty[tp.slot], 4 / COLG);
+            }
+#pragma unroll
+            for (int g = 0; g < W / 4; ++g) {
+                uint64_t s[2];
+                lds_2x64(sb + (uint32_t)(j * (kPad * 36)) + 16u * g, s[0], s[1]);
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    const uint64_t t = fma2(pack2((uint32_t)v[4 * g + 2 * i] + (1u << 19), (uint32_t)v[4 * g + 2 * i + 1] + (1u << 19)), r2, o2);
+                    if (kGroup) part[2 * g + i] = fma2(t, s[i], part[2 * g + i]);
+                    else acc[2 * g + i] = fma2(mul2(d2, s[i]), t, acc[2 * g + i]);
+                }
+            }
+        }
+        tp.next();
+        if (!kHandshake) tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_n(&sh.empty1[pos.r], 4 / COLG);   // 4 * COLG warps per stage, 16 arrivals
+        pos.next(true);
+        if (kGroup) {
+            const float d = h2f(word >> 16);
+            const uint64_t d2 = pack2f(d, d);
+#pragma unroll
+            for (int i = 0; i < W / 2; ++i) acc[i] = fma2(d2, part[i], acc[i]);
+        }
+        if (--left == 0 || b0 + kG_StageUnits >= nb) {   // a slice of K is complete
+            left = slice;
+#pragma unroll
+            for (int i = 0; i < W / 2; ++i) { total[i] = add2(total[i], acc[i]); acc[i] = 0ull; }
+        }
+    }
+    return true;
+}
+
 // The binary counter of readback_min: sum completes level after level as long as that level has a pending left half.
 template <int L>
 __device__ __forceinline__ void count_up(int n, uint64_t (&sum)[4], uint64_t (&st)[5][4]) {
@@ -549,10 +644,22 @@ __device__ __forceinline__ bool readback(const Params& p, const GemmWork& w, Gem
     return publish_sums<W>(p.status, sh, xch, q, part, lane, xphase, acc2, ok);
 }
 
+template <class Policy, class Params, int COLG, int W>
+__device__ __forceinline__ bool readback_as_gemv(const Params& p, const GemmWork& w, GemmShared& sh, uint32_t ring1, uint32_t ring2, float* xch, uint32_t tmem, int q,
+                                                 int colg, int lane, RingPos& pos, TmemPos& tp, uint32_t& xphase) {
+    pos.geometry(COLG * W <= 32);
+    const int nb = uniform(w.nb), slice = uniform(Policy::slice(p, w));
+    uint64_t total[W / 2];
+    const bool ok = uniform(Policy::type(p, w)) == CHIMERE_TYPE_Q4_0
+                        ? readback_ordered<CHIMERE_TYPE_Q4_0, COLG, W>(sh, ring1, ring2, tmem, p.status, nb, slice, q, colg, lane, pos, tp, total)
+                        : readback_ordered<CHIMERE_TYPE_IQ3_S, COLG, W>(sh, ring1, ring2, tmem, p.status, nb, slice, q, colg, lane, pos, tp, total);
+    return publish_sums<W>(p.status, sh, xch, q, colg, lane, xphase, total, ok);
+}
+
 // Slim tiles of packed weights: the read-back needs few of its warps and the two expander warps would be what bounds the kernel
 // (1000 of 1490 cycles per stage with 16 columns), so parts 2 and 3 of the read-back warps expand instead, a row tile and
 // two of a stage's four units each: warp x of eight.
-template <class Policy, class Params, int W>
+template <class Policy, int MODE, class Params, int W>
 __device__ __forceinline__ bool expand_slim(const Params& p, const GemmWork& w, GemmShared& sh, uint32_t ring1, uint32_t ring2, int x, int lane, RingPos& pos,
                                             TmemPos& tp, uint32_t& xphase) {
     const int type = uniform(Policy::type(p, w)), nb = uniform(w.nb);
@@ -561,11 +668,10 @@ __device__ __forceinline__ bool expand_slim(const Params& p, const GemmWork& w, 
     const uint32_t t = x & 3, h = x >> 2;
     const uint32_t src = ring1 + t * kRawTile, dst = ring2 + h * (2 * kG_MmaTile) + t * 512 + lane * 16, rec = ring2 + 4096 + h * (2 * kG_MmaTile) + (t * 32 + lane) * 4;
     const int nstages = (nb + kG_StageUnits - 1) / kG_StageUnits;
-    float d3 = 0.0f;        // IQ3_S: this lane's row's scales of the super-block, kept over its two stages
-    uint32_t sc3 = 0u;
+    uint32_t d3 = 0u, sc3 = 0u;   // IQ3_S: this lane's row's scales of the super-block, kept over its two stages
     bool ok = true;
     for (int s = 0; s < nstages && ok; ++s) {
-        const int u0 = stage_unit(type, s);
+        const int u0 = stage_unit<MODE>(type, s);
         if (!mbar_wait(&sh.full1[pos.r], pos.par1()) || !mbar_wait(&sh.empty1[pos.lag()], pos.released(pos.lag()))) { ok = false; break; }
         const uint32_t raw = src + pos.slot1_off(), a = (uint32_t)pos.e * kG_ASlot;
         if (type == CHIMERE_TYPE_Q4_0) {
@@ -578,14 +684,14 @@ __device__ __forceinline__ bool expand_slim(const Params& p, const GemmWork& w, 
         } else {
             const uint4 v0 = lds128(raw + (2 * h) * 512 + lane * 16), v1 = lds128(raw + (2 * h + 1) * 512 + lane * 16);
             if (!(s & 1)) {   // the scales came behind these units
-                d3 = h2f(lds16(raw + 2048 + lane * 2)) * 0.125f;
+                d3 = lds16(raw + 2048 + lane * 2);
                 sc3 = lds32(raw + 2048 + 64 + lane * 4);
             }
             const uint32_t sc = sc3 >> (4 * (u0 & 4) + 8 * h);
             expand_unit<CHIMERE_TYPE_IQ3_S>(v0, dst + a);
             expand_unit<CHIMERE_TYPE_IQ3_S>(v1, dst + a + kG_MmaTile);
-            sts_f32(rec + a, d3 * (float)(1u + 2u * (sc & 15u)));
-            sts_f32(rec + a + kG_MmaTile, d3 * (float)(1u + 2u * ((sc >> 4) & 15u)));
+            sts_u32(rec + a, iq3s_word<MODE>(d3, sc & 15u));
+            sts_u32(rec + a + kG_MmaTile, iq3s_word<MODE>(d3, (sc >> 4) & 15u));
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the MMAs read what ordinary stores wrote
         __syncwarp();
@@ -603,14 +709,14 @@ __device__ __forceinline__ bool expand_slim(const Params& p, const GemmWork& w, 
 }
 
 // Warps 4..7: what happens to a tile's sums, while the read-back warps are at the next tile.
-template <class Policy, bool MIN, class Params>
+template <class Policy, int MODE, class Params>
 __device__ __forceinline__ bool store_tile(const Params& p, const GemmWork& w, GemmShared& sh, const float* xch, int ew, int lane, uint32_t& xphase) {
     const bool ok = mbar_wait(&sh.xfull, xphase & 1u);
     ++xphase;
     if (!ok) { gemm_timeout(sh, p.status, lane); return false; }
-    if (MIN || w.npad == 128) Policy::template store<1, MIN>(p, w, xch, ew, lane);
-    else if (w.npad == 64 || Policy::type(p, w) < kTypeOperand) Policy::template store<2, false>(p, w, xch, ew, lane);
-    else Policy::template store<4, false>(p, w, xch, ew, lane);
+    if (MODE != kPlain || w.npad == 128) Policy::template store<1, MODE>(p, w, xch, ew, lane);
+    else if (w.npad == 64 || Policy::type(p, w) < kTypeOperand) Policy::template store<2, kPlain>(p, w, xch, ew, lane);
+    else Policy::template store<4, kPlain>(p, w, xch, ew, lane);
     __syncwarp();
     if (lane == 0) mbar_arrive_cta(&sh.xempty);
     return true;
@@ -627,8 +733,7 @@ __device__ __forceinline__ int take_tile(GemmShared& sh, int32_t* status, uint32
     return idx;
 }
 
-// MIN: the tiles with minimums (Q4_K / Q5_K shared expert) and no others
-template <class Policy, class Params, bool MIN = false>
+template <class Policy, class Params, int MODE = kPlain>
 __global__ void __launch_bounds__(kG_Threads, 1) gemm_i8_kernel(const Params p, int32_t* tile_counter) {
     extern __shared__ uint8_t smem_raw[];
     __shared__ GemmShared sh;
@@ -671,9 +776,23 @@ __global__ void __launch_bounds__(kG_Threads, 1) gemm_i8_kernel(const Params p, 
         bool ok = true;
         while (ok && (idx = take_tile(sh, p.status, tn, lane)) >= 0) {
             GemmWork w;
-            Policy::template work<MIN>(p, idx, w);
+            Policy::template work<MODE>(p, idx, w);
             const uint32_t r1 = smem_u32(ring1), r2 = smem_u32(ring2);
-            if (MIN) {
+            if (MODE == kOrdered) {
+                switch (uniform(w.npad)) {
+                    case 64: ok = readback_as_gemv<Policy, Params, 4, 16>(p, w, sh, r1, r2, xch, tmem, q, part, lane, pos, tp, xphase); break;
+                    case 32:
+                        if (part < 2) ok = readback_as_gemv<Policy, Params, 2, 16>(p, w, sh, r1, r2, xch, tmem, q, part, lane, pos, tp, xphase);
+                        else ok = expand_slim<Policy, MODE, Params, 32>(p, w, sh, r1, r2, warp - kG_FirstRb - 8, lane, pos, tp, xphase);
+                        break;
+                    default:
+                        if (part < 2) ok = readback_as_gemv<Policy, Params, 2, 8>(p, w, sh, r1, r2, xch, tmem, q, part, lane, pos, tp, xphase);
+                        else ok = expand_slim<Policy, MODE, Params, 16>(p, w, sh, r1, r2, warp - kG_FirstRb - 8, lane, pos, tp, xphase);
+                        break;
+                }
+                continue;
+            }
+            if (MODE == kMin) {
                 const int nb = uniform(w.nb);
                 ok = readback_min(sh, r1, r2, xch, tmem, p.status, nb, Policy::tree_order(p) ? nb >> 5 : nb, q, part, lane, pos, tp, xphase);
                 continue;
@@ -684,12 +803,12 @@ __global__ void __launch_bounds__(kG_Threads, 1) gemm_i8_kernel(const Params p, 
                 case 32:
                     if (uniform(Policy::type(p, w)) >= kTypeOperand) ok = readback<Policy, Params, 1, 4, 32>(p, w, sh, r1, r2, xch, tmem, q, part, lane, pos, tp, xphase);
                     else if (part < 2) ok = readback<Policy, Params, 1, 2, 32>(p, w, sh, r1, r2, xch, tmem, q, part, lane, pos, tp, xphase);
-                    else ok = expand_slim<Policy, Params, 32>(p, w, sh, r1, r2, warp - kG_FirstRb - 8, lane, pos, tp, xphase);
+                    else ok = expand_slim<Policy, MODE, Params, 32>(p, w, sh, r1, r2, warp - kG_FirstRb - 8, lane, pos, tp, xphase);
                     break;
                 default:
                     if (uniform(Policy::type(p, w)) >= kTypeOperand) ok = readback<Policy, Params, 1, 4, 16>(p, w, sh, r1, r2, xch, tmem, q, part, lane, pos, tp, xphase);
                     else if (part < 2) ok = readback<Policy, Params, 1, 2, 16>(p, w, sh, r1, r2, xch, tmem, q, part, lane, pos, tp, xphase);
-                    else ok = expand_slim<Policy, Params, 16>(p, w, sh, r1, r2, warp - kG_FirstRb - 8, lane, pos, tp, xphase);
+                    else ok = expand_slim<Policy, MODE, Params, 16>(p, w, sh, r1, r2, warp - kG_FirstRb - 8, lane, pos, tp, xphase);
                     break;
             }
         }
@@ -706,7 +825,7 @@ __global__ void __launch_bounds__(kG_Threads, 1) gemm_i8_kernel(const Params p, 
                 do {   // a skipped index costs one more atomic
                     if (lane == 0) idx = atomicAdd(tile_counter, 1);
                     idx = __shfl_sync(0xffffffffu, idx, 0);
-                    ws = Policy::template work<MIN>(p, idx, w);
+                    ws = Policy::template work<MODE>(p, idx, w);
                 } while (ws == kWorkSkip);
                 const int slot = (int)(tn % kG_Sched);
                 if (!mbar_wait(&sh.sempty[slot], ((tn / kG_Sched) & 1u) ^ 1u)) { gemm_timeout(sh, p.status, lane); ok = false; break; }
@@ -716,7 +835,7 @@ __global__ void __launch_bounds__(kG_Threads, 1) gemm_i8_kernel(const Params p, 
                 }
                 ++tn;
                 if (ws == kWorkEnd) break;
-                ok = produce_tile<Policy>(p, w, sh, ring1, ring2, pos, lane);
+                ok = produce_tile<Policy, MODE>(p, w, sh, ring1, ring2, pos, lane);
             }
             if (!ok)   // a wait ran out: the copies already asked for have to land before this CTA's memory goes away
                 for (int r = 0; r < pos.slots1(); ++r) mbar_wait(&sh.full1[r], pos.released(r));
@@ -726,21 +845,21 @@ __global__ void __launch_bounds__(kG_Threads, 1) gemm_i8_kernel(const Params p, 
             int idx;
             while (ok && (idx = take_tile(sh, p.status, tn, lane)) >= 0) {
                 GemmWork w;
-                Policy::template work<MIN>(p, idx, w);
+                Policy::template work<MODE>(p, idx, w);
                 const uint32_t r1 = smem_u32(ring1), r2 = smem_u32(ring2);
                 if (warp == 1) {
                     const uint32_t cst = smem_u32(smem);
-                    if (MIN) ok = mma_tile<Policy, 32>(p, w, sh, cst, r1, r2, tmem, pos, tp, lane);
+                    if (MODE == kMin) ok = mma_tile<Policy, MODE, 32>(p, w, sh, cst, r1, r2, tmem, pos, tp, lane);
                     else switch (uniform(w.npad)) {
-                        case 128: ok = mma_tile<Policy, 128>(p, w, sh, cst, r1, r2, tmem, pos, tp, lane); break;
-                        case 64: ok = mma_tile<Policy, 64>(p, w, sh, cst, r1, r2, tmem, pos, tp, lane); break;
-                        case 32: ok = mma_tile<Policy, 32>(p, w, sh, cst, r1, r2, tmem, pos, tp, lane); break;
-                        default: ok = mma_tile<Policy, 16>(p, w, sh, cst, r1, r2, tmem, pos, tp, lane); break;
+                        case 128: if (MODE == kPlain) ok = mma_tile<Policy, MODE, 128>(p, w, sh, cst, r1, r2, tmem, pos, tp, lane); break;
+                        case 64: ok = mma_tile<Policy, MODE, 64>(p, w, sh, cst, r1, r2, tmem, pos, tp, lane); break;
+                        case 32: ok = mma_tile<Policy, MODE, 32>(p, w, sh, cst, r1, r2, tmem, pos, tp, lane); break;
+                        default: ok = mma_tile<Policy, MODE, 16>(p, w, sh, cst, r1, r2, tmem, pos, tp, lane); break;
                     }
                 } else if (warp < kG_FirstEpi) {
-                    ok = expand_tile<Policy>(p, w, sh, r1, r2, pos, warp - 2, lane);
+                    ok = expand_tile<Policy, MODE>(p, w, sh, r1, r2, pos, warp - 2, lane);
                 } else {
-                    ok = store_tile<Policy, MIN>(p, w, sh, xch, warp - kG_FirstEpi, lane, xphase);
+                    ok = store_tile<Policy, MODE>(p, w, sh, xch, warp - kG_FirstEpi, lane, xphase);
                 }
             }
         }
@@ -757,7 +876,7 @@ __global__ void __launch_bounds__(kG_Threads, 1) gemm_i8_kernel(const Params p, 
 // ------------------------------------------------------------------ policies ----
 // plain fp32 tile store: out[(row0 + r) * ldo + col0 + c] = D[r][c]  (the primitive; operands in the mma128 form)
 struct PlainPolicy {
-    template <bool>
+    template <int>
     __device__ static __forceinline__ int work(const GemmParams& p, int idx, GemmWork& w) {
         if (idx >= p.n_items) return kWorkEnd;
         const GemmItem it = p.items[idx];
@@ -768,9 +887,10 @@ struct PlainPolicy {
         return kWorkOk;
     }
     __device__ static __forceinline__ int type(const GemmParams&, const GemmWork&) { return kTypeOperand; }
+    __device__ static __forceinline__ int slice(const GemmParams&, const GemmWork&) { return 1; }
     __device__ static __forceinline__ bool tree_order(const GemmParams&) { return false; }
     __device__ static __forceinline__ RowTiles rows(const GemmParams& p, const GemmWork& w) { return RowTiles{p.a_base + p.items[w.expert].a_offset, nullptr, 0, 0, 0}; }
-    template <int KG, bool MIN>
+    template <int KG, int MODE>
     __device__ static __forceinline__ void store(const GemmParams& p, const GemmWork& w, const float* xch, int ew, int lane) {
         for (int r = ew; r < w.rt; r += kG_EpiWarps)   // (all tiles of the primitive are 128 columns wide: one share)
             for (int c = lane; c < w.n_valid; c += 32) p.out[(size_t)(w.aux0 + r) * p.ldo + w.aux1 + c] = xch[c * 128 + r];
@@ -785,9 +905,9 @@ __device__ __forceinline__ int tile_width(int n) { return n <= 16 ? 16 : n <= 32
 
 // What the gate/up and the down launch share: the tile list and where a row tile's weights are.
 struct MoePolicy {
-    template <bool MIN>
+    template <int MODE>
     __device__ static __forceinline__ int work(const PrefillGemmParams& p, int idx, GemmWork& w) {
-        if (MIN) {   // shared-expert tiles of 32 tokens; word 1 of the list: their first column / 16
+        if (MODE == kMin) {   // shared-expert tiles of 32 tokens; word 1 of the list: their first column / 16
             const PrefillGemmMats& m = p.m[1];
             const int j = idx / m.row_tiles, t0 = j * 32;
             if (t0 >= p.T) return kWorkEnd;
@@ -812,6 +932,7 @@ struct MoePolicy {
         return kWorkOk;
     }
     __device__ static __forceinline__ int type(const PrefillGemmParams& p, const GemmWork& w) { return p.m[w.shared].type; }
+    __device__ static __forceinline__ int slice(const PrefillGemmParams& p, const GemmWork& w) { return p.m[w.shared].slice; }
     __device__ static __forceinline__ bool tree_order(const PrefillGemmParams& p) { return p.shared_sums != 0; }   // (set for the gate/up launch)
     // gated: two 32-row tiles of the gate matrix and the same two of the up matrix; else four of the one matrix
     __device__ static __forceinline__ RowTiles rows(const PrefillGemmParams& p, const GemmWork& w) {
@@ -846,12 +967,12 @@ __device__ __forceinline__ float xch_sum(const float* xch, int npad, int row, in
 // a 32-row block of the intermediate and every second or every column of the tile, two columns at a time so that the
 // divisions of one hide the other's.
 struct GateUpPolicy : MoePolicy {
-    template <int KG, bool MIN>
+    template <int KG, int MODE>
     __device__ static __forceinline__ void store(const PrefillGemmParams& p, const GemmWork& w, const float* xch, int ew, int lane) {
         const int nrb = p.dual ? 2 : 4, rb = ew & (nrb - 1), blk = w.rt * nrb + rb;
         if (blk >= p.m[w.shared].rows32) return;     // (the last row tile may be partly filled)
         const int cstep = kG_EpiWarps / nrb, r = rb * 32 + lane;
-        const bool sums = MIN;   // the down matrix has minimums too: it wants the blocks' sums
+        const bool sums = MODE == kMin;   // the down matrix has minimums too: it wants the blocks' sums
         uint8_t* tile = p.out_tiles + (size_t)w.col16 * p.out_col16_bytes;
         uint8_t* dst = sums ? tile + (size_t)(blk >> 2) * (w.npad * 160) + (blk & 3) * (w.npad * 36) : tile + (size_t)blk * (w.npad * 36);
         float* sdst = reinterpret_cast<float*>(tile + (size_t)(blk >> 2) * (w.npad * 160) + w.npad * 144 + (blk & 3) * (w.npad * 4));
@@ -863,7 +984,7 @@ struct GateUpPolicy : MoePolicy {
             for (int i = 0; i < 2; ++i) {
                 const int ci = min(c + i * cstep, w.n_valid - 1);
                 const float a = xch_sum<KG>(xch, w.npad, r, ci);
-                if (p.dual) { const float u = xch_sum<KG>(xch, w.npad, r + 64, ci); v[i] = MIN ? silu_mul_ref(a, u) : silu_mul_near(a, u); }
+                if (p.dual) { const float u = xch_sum<KG>(xch, w.npad, r + 64, ci); v[i] = MODE != kPlain ? silu_mul_ref(a, u) : silu_mul_near(a, u); }
                 else { const float t = fmaxf(a, 0.0f); v[i] = t * t; }
             }
 #pragma unroll
@@ -898,7 +1019,7 @@ struct GateUpPolicy : MoePolicy {
 // down: rows of H; the tile's columns are pairs, written to pair_out[pair row][H].  A warp stores the 128 rows of every fourth
 // column, four rows per lane (H is a multiple of 32).
 struct DownPolicy : MoePolicy {
-    template <int KG, bool MIN>
+    template <int KG, int MODE>
     __device__ static __forceinline__ void store(const PrefillGemmParams& p, const GemmWork& w, const float* xch, int ew, int lane) {
         const bool rows = w.rt * 128 + lane * 4 < p.H;
         float* out = p.pair_out + w.rt * 128 + lane * 4;
@@ -959,12 +1080,12 @@ static int gemm_grid(int n_items) {
     const int n_sm = sm_count();
     return n_items < n_sm ? n_items : n_sm;
 }
-template <class Policy, bool MIN = false, class Params>
+template <class Policy, int MODE = kPlain, class Params>
 static cudaError_t launch_gemm(const Params& p, int n_items, int32_t* counter, cudaStream_t stream) {
     static bool attr_done[64] = {};
-    cudaError_t e = max_smem_once(gemm_i8_kernel<Policy, Params, MIN>, (int)kG_Smem, attr_done);
+    cudaError_t e = max_smem_once(gemm_i8_kernel<Policy, Params, MODE>, (int)kG_Smem, attr_done);
     if (e != cudaSuccess) return e;
-    return launch_pdl(gemm_i8_kernel<Policy, Params, MIN>, dim3(gemm_grid(n_items)), kG_Threads, kG_Smem, stream, p, counter);
+    return launch_pdl(gemm_i8_kernel<Policy, Params, MODE>, dim3(gemm_grid(n_items)), kG_Threads, kG_Smem, stream, p, counter);
 }
 
 // tile_counter: one int32 of device memory that is zero when the kernel starts (it ends at n_items + the number of CTAs)
@@ -982,9 +1103,10 @@ cudaError_t launch_prefill_gemm(const PrefillGemmParams& p, bool down, int n_til
     int32_t* counter = const_cast<int32_t*>(p.tiles) + (down ? 5 : 4);
     if (p.m[1].type == kTypeOperandMin) {   // (words 6 / 7: these launches' counters)
         const int n_min = (p.T + 31) / 32 * p.m[1].row_tiles;
-        const cudaError_t e = down ? launch_gemm<DownPolicy, true>(p, n_min, counter + 2, stream) : launch_gemm<GateUpPolicy, true>(p, n_min, counter + 2, stream);
+        const cudaError_t e = down ? launch_gemm<DownPolicy, kMin>(p, n_min, counter + 2, stream) : launch_gemm<GateUpPolicy, kMin>(p, n_min, counter + 2, stream);
         if (e != cudaSuccess) return e;
     }
+    if (p.as_gemv) return down ? launch_gemm<DownPolicy, kOrdered>(p, n_items, counter, stream) : launch_gemm<GateUpPolicy, kOrdered>(p, n_items, counter, stream);
     return down ? launch_gemm<DownPolicy>(p, n_items, counter, stream) : launch_gemm<GateUpPolicy>(p, n_items, counter, stream);
 }
 
@@ -1096,7 +1218,7 @@ cudaError_t launch_pack_mma128_q8_0(const void* raw, void* out, int n_mats, int 
 // are equally wide.
 __device__ __forceinline__ uint64_t width_bit(int n, uint64_t count) { return n > 64 ? count : n > 32 ? count << 16 : n > 16 ? count << 32 : count << 48; }
 __global__ void __launch_bounds__(256) build_tiles_kernel(const int32_t* offsets, const int32_t* perm, int32_t* tiles, int32_t* list, int E, int T,
-                                                          int has_shared, int gemm_min, int shared_32) {
+                                                          int has_shared, int gemm_min, int shared_32, int widest) {
     __shared__ uint64_t scan[8];
     __shared__ int scan_n[8];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -1119,8 +1241,9 @@ __global__ void __launch_bounds__(256) build_tiles_kernel(const int32_t* offsets
         }
         if (tid == 0) { list[0] = total; list[1] = total; list[2] = 0; list[3] = 0; }
     }
-    const int nf = cnt >> 7, rem = cnt & 127;
-    const uint64_t own = (uint64_t)nf + (rem ? width_bit(rem, 1) : 0ull);
+    const int full = widest, fshift = widest == 128 ? 7 : 6, kf = 7 - fshift;   // columns of a full tile, their width's place in the list
+    const int nf = cnt >> fshift, rem = cnt & (full - 1);
+    const uint64_t own = width_bit(full, (uint64_t)nf) + (rem ? width_bit(rem, 1) : 0ull);
     uint64_t incl = own;
 #pragma unroll
     for (int s = 1; s < 32; s <<= 1) {
@@ -1133,8 +1256,8 @@ __global__ void __launch_bounds__(256) build_tiles_kernel(const int32_t* offsets
     for (int w = 0; w < 8; ++w) { if (w < warp) before += scan[w]; total += scan[w]; }
     // the shared expert's tiles: 128 columns and a rest, or (shared_32) tiles of 32 that are not on the list, their columns behind all
     // others'
-    const int sh_full = has_shared && !shared_32 ? T >> 7 : 0, sh_rem = has_shared && !shared_32 ? T & 127 : 0;
-    const uint64_t shared = (uint64_t)sh_full + (sh_rem ? width_bit(sh_rem, 1) : 0ull);
+    const int sh_full = has_shared && !shared_32 ? T >> fshift : 0, sh_rem = has_shared && !shared_32 ? T & (full - 1) : 0;
+    const uint64_t shared = width_bit(full, (uint64_t)sh_full) + (sh_rem ? width_bit(sh_rem, 1) : 0ull);
     total += shared;
     before += shared;   // the shared expert's tiles lead every width
     int first[5], col16[5];   // first tile and first column / 16 of each width
@@ -1148,13 +1271,13 @@ __global__ void __launch_bounds__(256) build_tiles_kernel(const int32_t* offsets
     int4* tv = reinterpret_cast<int4*>(tiles + kTileHeader);
     auto put = [&](int k, int i, int expert, int start, int n) { tv[first[k] + i] = make_int4(expert, start, n, col16[k] + i * (8 >> k)); };
     auto width_of = [](int n) { return n > 64 ? 0 : n > 32 ? 1 : n > 16 ? 2 : 3; };
-    for (int i = tid; i < sh_full; i += 256) put(0, i, -1, i * 128, 128);
-    if (tid == 0 && sh_rem) put(width_of(sh_rem), sh_rem > 64 ? sh_full : 0, -1, sh_full * 128, sh_rem);
-    const int f0 = (int)(before & 0xFFFFu);
-    for (int i = 0; i < nf; ++i) put(0, f0 + i, tid, off + i * 128, 128);
+    for (int i = tid; i < sh_full; i += 256) put(kf, i, -1, i * full, full);
+    if (tid == 0 && sh_rem) put(width_of(sh_rem), width_of(sh_rem) == kf ? sh_full : 0, -1, sh_full * full, sh_rem);
+    const int f0 = (int)((before >> (16 * kf)) & 0xFFFFu);
+    for (int i = 0; i < nf; ++i) put(kf, f0 + i, tid, off + i * full, full);
     if (rem) {
         const int k = width_of(rem);
-        put(k, (int)((before >> (16 * k)) & 0xFFFFu) + (k == 0 ? nf : 0), tid, off + nf * 128, rem);
+        put(k, (int)((before >> (16 * k)) & 0xFFFFu) + (k == kf ? nf : 0), tid, off + nf * full, rem);
     }
     if (tid == 0) {
         tiles[0] = first[4]; tiles[1] = col16[4]; tiles[2] = 0; tiles[3] = 0;
@@ -1204,8 +1327,8 @@ __global__ void __launch_bounds__(256) gather_tiles_kernel(const int32_t* tiles,
 }
 
 cudaError_t launch_build_tiles(const int32_t* offsets, const int32_t* perm, int32_t* tiles, int32_t* list, int E, int T, int has_shared, int gemm_min,
-                               int shared_32, cudaStream_t stream) {
-    return launch_pdl(build_tiles_kernel, dim3(1), 256, 0, stream, offsets, perm, tiles, list, E, T, has_shared, gemm_min, shared_32);
+                               int shared_32, int widest, cudaStream_t stream) {
+    return launch_pdl(build_tiles_kernel, dim3(1), 256, 0, stream, offsets, perm, tiles, list, E, T, has_shared, gemm_min, shared_32, widest);
 }
 
 cudaError_t launch_gather_tiles(const int32_t* tiles, const int32_t* perm, const int8_t* x_q, int64_t x_q_stride, const float* x_d,

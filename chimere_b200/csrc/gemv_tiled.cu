@@ -713,6 +713,16 @@ static cudaError_t dispatch_tile(int type, const GemvParams& p, int max_entries,
 #undef CHIMERE_LAUNCH
 }
 
+int tiled_slice_units(int type, int ncols, int wk) {
+    const int chunk = type == CHIMERE_TYPE_IQ3_S ? Tiled<CHIMERE_TYPE_IQ3_S>::kChunkUnits : Tiled<CHIMERE_TYPE_Q4_0>::kChunkUnits;   // (Q8_0: as Q4_0)
+    return ((ncols / 32 + wk - 1) / wk + chunk - 1) / chunk * chunk;
+}
+bool tiled_bulk_runs(const GemvParams& gate_up, const GemvParams& down) {
+    const TiledGeomHost g = tiled_gate_up_geom(gate_up.type_routed, gate_up.type_shared, gate_up.H, gate_up.nrows_shared > 0);
+    const TiledGeomHost d = tiled_down_geom(down.type_routed, down.ncols_routed, down.type_shared, down.nrows_shared > 0 ? down.ncols_shared : 0, down.T);
+    return plan_bulk(gate_up, kStageGateUp, gate_up.act == CHIMERE_ACT_SWIGLU, g.wk, g.wr).ok && plan_bulk(down, kStageDown, false, d.wk, d.wr).ok;
+}
+
 cudaError_t launch_gate_up_tiled(const GemvParams& p, int max_entries, cudaStream_t stream) {
     const TiledGeomHost g = tiled_gate_up_geom(p.type_routed, p.type_shared, p.H, p.nrows_shared > 0);
     cudaError_t e = dispatch_tile<kStageGateUp>(p.type_routed, p, max_entries, g.wk, g.wr, stream);
@@ -723,7 +733,7 @@ cudaError_t launch_gate_up_tiled(const GemvParams& p, int max_entries, cudaStrea
 
 // p.n_row_tiles must be ceil(H / (32 * wr)) with the geometry of tiled_down_geom
 cudaError_t launch_down_tiled(const GemvParams& p, int max_entries, cudaStream_t stream) {
-    const TiledGeomHost g = tiled_down_geom(p.type_routed, p.ncols_routed, p.type_shared, p.nrows_shared > 0 ? p.ncols_shared : 0, p.T);
+    const TiledGeomHost g = tiled_down_geom(p.type_routed, p.ncols_routed, p.type_shared, p.nrows_shared > 0 ? p.ncols_shared : p.split_cols_shared, p.T);
     cudaError_t e = dispatch_tile<kStageDown>(p.type_routed, p, max_entries, g.wk, g.wr, stream);
     if (e == cudaSuccess && p.nrows_shared > 0 && p.type_shared != p.type_routed)
         e = dispatch_tile<kStageDown>(p.type_shared, p, max_entries, g.wk, g.wr, stream);

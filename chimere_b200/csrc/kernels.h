@@ -79,6 +79,7 @@ struct GemvParams {
     float* out_soa_d; int64_t out_soa_d_stride;
     int32_t* status;
     int no_combine;              // down stage: only write the per-pair rows (the caller combines)
+    int split_cols_shared;       // down stage without the shared expert: its row width, which still has a say in how K is split
     int few_tokens;              // T counts row slots that are mostly empty (fixed-size expert-parallel exchange): size the
                                  // kernels as for a decode batch whatever T says
 };
@@ -150,6 +151,7 @@ struct PrefillGemmMats {
     int64_t tile_bytes;                        // bytes of a 32-row tile
     int type, ncols;                           // weight type, K
     int rows32, row_tiles;                     // 32-row tiles of a matrix; output tiles per token tile
+    int slice;                                 // as_gemv: stages of four 32-wide blocks per K slice of the GEMV kernels
 };
 struct PrefillGemmParams {
     const int32_t* tiles;            // tile list (word 0 = count, words 4 / 5 = tile counters of the gate/up / down launch, tiles from word 8)
@@ -162,11 +164,12 @@ struct PrefillGemmParams {
     int dual, T, top_k, H;
     uint8_t* inter_q8; int64_t inter_stride;   // gate/up: Q8_1 rows of the intermediates as the GEMV kernels leave them (null = not wanted)
     int shared_sums;                 // gate/up: the shared expert's token tiles of the down GEMM carry block sums (kTypeOperandMin)
+    int as_gemv;                     // sums bit for bit as the GEMV kernels form them (packed weights, token tiles of up to 64 columns)
     int32_t* status;
 };
 cudaError_t launch_prefill_gemm(const PrefillGemmParams& p, bool down, int n_tiles_max, cudaStream_t stream);
 cudaError_t launch_build_tiles(const int32_t* offsets, const int32_t* perm, int32_t* tiles, int32_t* list, int E, int T, int has_shared, int gemm_min,
-                               int shared_32, cudaStream_t stream);
+                               int shared_32, int widest, cudaStream_t stream);   // widest: columns of a full token tile, 128 or 64
 cudaError_t launch_gather_tiles(const int32_t* tiles, const int32_t* perm, const int8_t* x_q, int64_t x_q_stride, const float* x_d,
                                 int x_d_stride, const uint8_t* x_q8, uint8_t* b_tiles, int64_t b_col16_bytes, int H, int top_k, int n_tiles_max,
                                 bool shared_sums, int T, cudaStream_t stream);
@@ -191,6 +194,10 @@ TiledGeomHost tiled_gate_up_geom(int type_routed, int type_shared, int H, bool h
 TiledGeomHost tiled_down_geom(int type_routed, int F, int type_shared, int F_s, int T);
 cudaError_t launch_pack(int type, const void* raw, void* out, int n_mats, int nrows, int ncols, int64_t raw_stride,
                         int64_t out_stride, cudaStream_t stream);
+// Units of a row that one K slice of the bulk-copy kernel holds, and whether that kernel runs at all for these parameters (the
+// fallback adds in another order): what the grouped GEMM needs to form the same sums.
+int tiled_slice_units(int type, int ncols, int wk);
+bool tiled_bulk_runs(const GemvParams& gate_up, const GemvParams& down);
 cudaError_t launch_gate_up_tiled(const GemvParams& p, int max_entries, cudaStream_t stream);
 cudaError_t launch_down_tiled(const GemvParams& p, int max_entries, cudaStream_t stream);
 cudaError_t launch_block_sumi_tiled(int type, const void* packed, const void* xq8, int32_t* sumi, int ncols, int nrows,

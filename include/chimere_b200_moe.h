@@ -133,7 +133,8 @@ int chimere_b200_pack_matrix(int wtype, const void* d_raw, void* d_out, int nrow
                              cudaStream_t stream);
 
 /* y[T][H] = MoE(x[T][H]).  Replaces moe_ffn.rs:1094-1766 for T tokens.  x, y: device f32.
- * Capturable in a CUDA graph: no allocation, no host synchronisation, no device-to-host copy. */
+ * Capturable in a CUDA graph: no allocation, no host synchronisation, no device-to-host copy.
+ * A token's row is the same bits whatever the other tokens of the call are. */
 int chimere_b200_moe_forward(const chimere_moe_layer* w, const float* d_x, float* d_y, int T,
                              chimere_moe_workspace* ws, cudaStream_t stream);
 

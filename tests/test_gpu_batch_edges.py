@@ -70,3 +70,22 @@ def test_decode_entry_steps(cfg, T):
 @pytest.mark.parametrize("T", [129, 160, 545])
 def test_tiled_router(H, T):
     _check(configs.scaled(Q4, E=256, H=H, F=64, F_s=64), T, prefill=False)
+
+
+# The decode entry sends popular experts to the GEMM and the others to the GEMV kernels; a token's row is the same bits either way,
+# whatever the batch: odd numbers of K slices and units, IQ3_S in both places, a shared expert narrower than the routed ones.
+@pytest.mark.parametrize("cfg", [configs.scaled(Q4, E=16, F=256, F_s=512, H=2048, name="q4"),
+                                 configs.scaled(IQ3, E=16, F=512, F_s=256, H=1024, type_down=configs.IQ3_S, name="iq3"),
+                                 configs.scaled(IQ3, E=8, top_k=4, F=320, F_s=0, H=2560, name="iq3 gate, q4 down"),
+                                 configs.scaled(configs.NEMOTRON_Q4_0, E=8, H=2688, F=800, F_s=96, name="relu"),
+                                 configs.scaled(IQ3, E=16, F=256, F_s=512, H=1024, type_sh_gate_up=formats.TYPE_Q5_K, type_sh_down=formats.TYPE_Q5_K, name="q5k")],
+                         ids=lambda c: c.name)
+@pytest.mark.parametrize("T", [17, 41, 64, 150])
+def test_decode_rows_do_not_depend_on_the_batch(cfg, T):
+    tiled = MoeWeightsTiled(configs.make_layer(cfg, device="cuda"))
+    x = configs.make_input(cfg, T, device="cuda")
+    sc, one = MoeScratch(tiled, T), MoeScratch(tiled, 1)
+    y = forward_moe(tiled, sc, x)
+    single = torch.cat([forward_moe(tiled, one, x[t:t + 1].contiguous()) for t in range(T)])
+    assert sc.status() == 0 and one.status() == 0
+    assert torch.equal(y, single)
