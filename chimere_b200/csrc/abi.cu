@@ -132,10 +132,18 @@ struct Layout {
     size_t gemm, gemm_bytes;   // the decode entry's token tiles (gemm_bytes = 0: never on the GEMM)
 };
 
-int max_entries_for(const chimere_moe_layer* w, int T) {
-    const int P = T * w->top_k, g = group_tokens(T, (int64_t)w->F * w->H);
-    const int routed = (w->E < P ? w->E : P) + P / g;
+int entries_for(const chimere_moe_layer* w, int T, int group) {
+    const int P = T * w->top_k, routed = (w->E < P ? w->E : P) + P / group;
     return (routed < P ? routed : P) + (w->F_s > 0 ? (T + shared_group_tokens(T) - 1) / shared_group_tokens(T) : 0);
+}
+int max_entries_for(const chimere_moe_layer* w, int T) { return entries_for(w, T, group_tokens(T, (int64_t)w->F * w->H)); }
+// Entries that any batch of up to T tokens may need: between two steps of the entries' size their number grows with the batch, so the
+// last batch before each step and T itself decide.  (Matrices of any width: layers of different widths may share a workspace.)
+int list_capacity(const chimere_moe_layer* w, int T) {
+    int most = entries_for(w, T, group_tokens(T, 0));
+    for (int t : kEntrySteps)
+        if (t < T && entries_for(w, t, group_tokens(t, 0)) > most) most = entries_for(w, t, group_tokens(t, 0));
+    return most;
 }
 
 // extra_rows: per-pair output rows beyond the routed pairs' and the shared expert's own (a K-quant shared expert's rows on the
@@ -146,9 +154,7 @@ Layout make_layout(const chimere_moe_layer* w, int T, int extra_rows = 0) {
     const int k = w->top_k, H = w->H, E = w->E;
     const int Fmax = w->F > w->F_s ? w->F : w->F_s;
     const size_t pairs = (size_t)T * k + (w->F_s > 0 ? T : 0);
-    L.max_entries = max_entries_for(w, T);   // T = the workspace's capacity; a smaller batch may need a few more entries
-    for (int t : {8, kFewTokens})   // (smaller entries up to these batch sizes)
-        if (T > t && max_entries_for(w, t) > L.max_entries) L.max_entries = max_entries_for(w, t);
+    L.max_entries = list_capacity(w, T);
     L.tile_rows = down_tile_rows(w->type_down, w->F, w->type_sh_down, w->F_s);
     L.n_row_tiles = (H + L.tile_rows - 1) / L.tile_rows;
     L.n_row_tiles_tiled = (H + 31) / 32;   // counters for the finest row tiling any batch size may choose
@@ -247,6 +253,7 @@ static RouteParams route_params(const chimere_moe_layer* w, const float* d_x, in
     // the dispatch of a large batch counts in the memory of the down stage's combine counters (zero between the stages'
     // uses, and large enough from a few dozen tokens on)
     const Layout L = make_layout(w, ws->max_T);
+    p.list_capacity = L.max_entries;
     const size_t combine_ints = (size_t)L.n_counters - kCtrRouteTile - (ws->max_T + 7) / 8;
     const size_t need = (size_t)((T * w->top_k + 127) / 128) * 256 + 260;
     // the router of a large batch rewrites its rows into the per-pair output area, which the down stage fills only later; its

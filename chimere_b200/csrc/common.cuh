@@ -17,13 +17,19 @@ constexpr int kMaxGroupTokens = 8;   // tokens one GEMV work entry carries
 constexpr int kSharedGroupTokens = 2;  // ... for the shared expert (every token uses it): smaller entries balance the grid
 // Decode-size batches give every token its own shared-expert entry: the kernels stage one token per pass there, and
 // a second pass in the same CTA is a longer chain than a second CTA reading the shared matrices from L2.
-__host__ __device__ inline int shared_group_tokens(int T) { return T <= 8 ? 1 : kSharedGroupTokens; }
+constexpr int kSingleSharedTokens = 8;
+__host__ __device__ inline int shared_group_tokens(int T) { return T <= kSingleSharedTokens ? 1 : kSharedGroupTokens; }
 // Tokens per routed entry.  In a decode-size batch every pair is an entry of its own: a popular expert's pairs are spread over
 // the SMs (its matrices then come from L2 again) instead of being a chain of passes in one CTA -- 8 skewed tokens through 256
 // experts of 512 x 2048 65 -> 37 us, 8 uniform ones 43 -> 38.  Matrices of more than 2M weights (1856 x 2688) cost more to fetch
 // twice than a second pass: two pairs per entry.
 constexpr int kFewTokens = 40;   // the largest batch for which the GEMV kernels are sized for one or two pairs per expert
-__host__ __device__ inline int group_tokens(int T, int64_t weights) { return T > kFewTokens ? kMaxGroupTokens : weights > (1 << 21) || T > 24 ? 2 : 1; }
+constexpr int kSinglePairTokens = 24;   // ... and for one
+__host__ __device__ inline int group_tokens(int T, int64_t weights) {
+    return T > kFewTokens ? kMaxGroupTokens : weights > (1 << 21) || T > kSinglePairTokens ? 2 : 1;
+}
+// Behind each of these batch sizes the entries get longer and their number can fall: a work list is sized for every one below its capacity.
+constexpr int kEntrySteps[] = {kSingleSharedTokens, kSinglePairTokens, kFewTokens};
 constexpr int kMaxTopK = 8;
 constexpr int kMaxExperts = 256;
 
@@ -38,6 +44,7 @@ constexpr int kListEntry = 12;
 
 // status bits a kernel may raise in the workspace status word
 constexpr int kStatusWaitTimeout = 1;
+constexpr int kStatusListFull = 2;
 
 __device__ __forceinline__ float h2f(uint32_t bits) { return __half2float(__ushort_as_half((unsigned short)bits)); }
 __device__ __forceinline__ uint32_t ld_u16(const uint8_t* p) { return *reinterpret_cast<const uint16_t*>(p); }

@@ -17,6 +17,7 @@ struct RouteParams {
     int list_mode;              // 0: work list for routed + shared entries; 1: shared-expert entries only (expert-parallel home
                                 // rank); 2: an empty list (the prefill path builds its own from offsets and perm)
     int group;                  // pairs per routed work entry (0 = kMaxGroupTokens)
+    int list_capacity;          // entries the work list has room for (more raise kStatusListFull and are left out)
     float route_scale;
     const float* x;             // [T][H]
     const float* router_w;      // [E][H]

@@ -261,6 +261,10 @@ __device__ void build_dispatch(const RouteParams& p, int* smem_i, const int* s_i
     const int sgt = shared_group_tokens(p.T);
     const int nsh = p.has_shared ? (p.T + sgt - 1) / sgt : 0;
     if (p.list_mode != 0) total_routed = 0;
+    if (nsh + total_routed > p.list_capacity) {   // (never, if the workspace was made for this layer and batch)
+        total_routed = max(0, p.list_capacity - nsh);
+        if (tid == 0 && p.status) atomicOr(p.status, kStatusListFull);
+    }
     for (int i = tid; i < (p.list_mode == 2 ? 0 : nsh); i += 256) {
         int* ent = p.group_list + kListHeader + kListEntry * i;
         const int t0 = i * sgt, mm = min(sgt, p.T - t0);
@@ -735,7 +739,11 @@ __global__ void __launch_bounds__(kDispatchChunk) dispatch_place_kernel(const Ro
     __syncthreads();
     const int sgt = shared_group_tokens(p.T);
     const int nsh = (p.has_shared && p.list_mode != 2) ? (p.T + sgt - 1) / sgt : 0;
-    const int total_routed = p.list_mode == 0 ? s_ent[256] : 0;
+    int total_routed = p.list_mode == 0 ? s_ent[256] : 0;
+    if (nsh + total_routed > p.list_capacity) {
+        total_routed = max(0, p.list_capacity - nsh);
+        if (tid == 0 && p.status) atomicOr(p.status, kStatusListFull);
+    }
     for (int i = tid; i < nsh; i += kDispatchChunk) {
         int* ent = p.group_list + kListHeader + kListEntry * i;
         const int t0 = i * sgt, mm = min(sgt, p.T - t0);
@@ -1191,7 +1199,8 @@ constexpr size_t kNoAllocXd = kNoAllocXq + (size_t)kNoAllocMaxT * kNoAllocMaxH; 
 constexpr size_t kNoAllocPerm = kNoAllocXd + (size_t)kNoAllocMaxT * (kNoAllocMaxH / 32) * 4;  // [T*8] i32
 constexpr size_t kNoAllocOffsets = kNoAllocPerm + (size_t)kNoAllocMaxT * kMaxTopK * 4;        // [257] i32
 constexpr size_t kNoAllocList = kNoAllocOffsets + 1280;                                       // work list
-constexpr size_t kNoAllocBytes = kNoAllocList + (size_t)(kListHeader + kListEntry * (kMaxExperts + kNoAllocMaxT * kMaxTopK + kNoAllocMaxT)) * 4 + 256;
+constexpr int kNoAllocEntries = kMaxExperts + kNoAllocMaxT * kMaxTopK + kNoAllocMaxT;
+constexpr size_t kNoAllocBytes = kNoAllocList + (size_t)(kListHeader + kListEntry * kNoAllocEntries) * 4 + 256;
 
 static __device__ __align__(256) unsigned char g_route_scratch[kNoAllocBytes];   // ~680 KiB per GPU
 
@@ -1243,6 +1252,7 @@ extern "C" int chimere_b200_moe_route_noalloc(const chimere_moe_layer* w, const 
     p.perm = (int32_t*)(base + kNoAllocPerm);
     p.offsets = (int32_t*)(base + kNoAllocOffsets);
     p.group_list = (int32_t*)(base + kNoAllocList);
+    p.list_capacity = kNoAllocEntries;
     p.topk_idx = d_topk_idx;   // results go straight to the caller's buffers
     p.topk_w = d_topk_w;
     e = launch_route(p, stream);

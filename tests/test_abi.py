@@ -1,10 +1,12 @@
 """The C-ABI library builds, loads, exports every symbol the header declares, and rejects bad
 arguments on the host (no GPU needed: argument errors are found before anything is launched)."""
 import ctypes as C
+import itertools
 import os
 import re
 
 import pytest
+import torch
 
 from chimere_b200 import abi, build
 
@@ -83,3 +85,27 @@ def test_missing_library_fails_loudly(monkeypatch, tmp_path):
     monkeypatch.setattr(abi, "LIB_PATH", str(tmp_path / "nope.so"))
     with pytest.raises(RuntimeError, match="no CPU or PyTorch fallback"):
         abi.load()
+
+
+def _most_entries(E, k, shared, t):
+    """Work entries that a batch of t tokens can need, at the rule's smallest entries: one pair up to 24 tokens, two up to 40, else
+    eight; the shared expert one token per entry up to 8 tokens, else two."""
+    P, group = t * k, 1 if t <= 24 else 2 if t <= 40 else 8
+    return min(P, min(E, P) + P // group) + ((t if t <= 8 else (t + 1) // 2) if shared else 0)
+
+
+@pytest.mark.parametrize("max_T", [1, 7, 8, 9, 16, 24, 25, 28, 32, 40, 41, 64, 65, 128, 200])
+def test_work_list_has_room_for_every_smaller_batch(lib, max_T):
+    """The list lies in front of the counters in the workspace: what a call writes past its room would land on them."""
+    dev = "cuda" if torch.cuda.is_available() else "cpu"
+    for E, k, F_s, F in itertools.product([1, 4, 8, 16, 32, 64, 128, 256], [1, 2, 6, 8], [0, 256], [256, 8448]):
+        if k > E:
+            continue
+        w = _layer(E=E, top_k=k, H=256, F=F, F_s=F_s)
+        n = lib.chimere_b200_moe_workspace_bytes(C.byref(w), max_T)
+        arena = torch.empty(n + 256, dtype=torch.uint8, device=dev)
+        ws = abi.MoeWorkspace()
+        rc = lib.chimere_b200_moe_workspace_init(C.byref(ws), (arena.data_ptr() + 255) & ~255, n, C.byref(w), max_T, None)
+        assert rc == 0 or (dev == "cpu" and rc <= -100)   # (the pointers are laid out before the device is asked to clear anything)
+        need = max(_most_entries(E, k, F_s > 0, t) for t in range(1, max_T + 1))
+        assert ws.counters - ws.group_list >= 4 * (4 + 12 * need), (E, k, F_s, F)

@@ -89,3 +89,22 @@ def test_decode_rows_do_not_depend_on_the_batch(cfg, T):
     single = torch.cat([forward_moe(tiled, one, x[t:t + 1].contiguous()) for t in range(T)])
     assert sc.status() == 0 and one.status() == 0
     assert torch.equal(y, single)
+
+
+# a workspace for more tokens than the call has: the smaller batch may cut its pairs into more entries than the full one
+@pytest.mark.parametrize("kw", [dict(E=8), dict(E=16), dict(E=64), dict(E=4, top_k=2, F_s=0)], ids=str)
+@pytest.mark.parametrize("max_T", [25, 32, 40, 64])
+def test_smaller_batches_in_a_larger_workspace(kw, max_T):
+    cfg = configs.scaled(Q4, **{**dict(H=512, F=128, F_s=128), **kw})
+    raw = configs.make_layer(cfg, device="cuda")
+    tiled = MoeWeightsTiled(raw)
+    sc = MoeScratch(tiled, max_T)
+    for T in (24, 24, 8, 25, 24):
+        x = configs.make_input(cfg, T, device="cuda")
+        y = forward_moe(tiled, sc, x)
+        torch.cuda.synchronize()
+        assert sc.status() == 0
+        idx = sc.topk_indices(T).cpu().numpy()
+        check_rows(y.cpu().numpy(), oracle_on_gpu_routing(raw.to("cpu"), x.cpu().numpy(), idx)["y"])
+        perm, offs = oracle.permute(idx, cfg.E)
+        assert np.array_equal(sc.perm(T).cpu().numpy(), perm) and np.array_equal(sc.offsets().cpu().numpy(), offs)
