@@ -136,13 +136,17 @@ int entries_for(const chimere_moe_layer* w, int T, int group) {
     const int P = T * w->top_k, routed = (w->E < P ? w->E : P) + P / group;
     return (routed < P ? routed : P) + (w->F_s > 0 ? (T + shared_group_tokens(T) - 1) / shared_group_tokens(T) : 0);
 }
-int max_entries_for(const chimere_moe_layer* w, int T) { return entries_for(w, T, group_tokens(T, (int64_t)w->F * w->H)); }
+bool wide_weights(const chimere_moe_layer* w) {
+    return w->layout == CHIMERE_LAYOUT_GGML || w->type_up == CHIMERE_TYPE_Q8_0 || w->type_down == CHIMERE_TYPE_Q8_0;
+}
+int layer_group(const chimere_moe_layer* w, int T) { return group_tokens(T, (int64_t)w->F * w->H, wide_weights(w)); }
+int max_entries_for(const chimere_moe_layer* w, int T) { return entries_for(w, T, layer_group(w, T)); }
 // Entries that any batch of up to T tokens may need: between two steps of the entries' size their number grows with the batch, so the
-// last batch before each step and T itself decide.  (Matrices of any width: layers of different widths may share a workspace.)
+// last batch before each step and T itself decide.  (The shortest entries: layers of different widths and types may share a workspace.)
 int list_capacity(const chimere_moe_layer* w, int T) {
-    int most = entries_for(w, T, group_tokens(T, 0));
+    int most = entries_for(w, T, group_tokens(T, 0, false));
     for (int t : kEntrySteps)
-        if (t < T && entries_for(w, t, group_tokens(t, 0)) > most) most = entries_for(w, t, group_tokens(t, 0));
+        if (t < T && entries_for(w, t, group_tokens(t, 0, false)) > most) most = entries_for(w, t, group_tokens(t, 0, false));
     return most;
 }
 
@@ -242,7 +246,7 @@ static RouteParams route_params(const chimere_moe_layer* w, const float* d_x, in
     p.T = T; p.H = w->H; p.E = w->E; p.top_k = w->top_k; p.route_mode = w->route_mode;
     p.has_shared = w->F_s > 0;
     p.route_scale = w->route_scale;
-    p.group = group_tokens(T, (int64_t)w->F * w->H);
+    p.group = layer_group(w, T);
     p.x = d_x; p.router_w = w->router_w; p.router_bias = w->router_bias;
     p.shexp_gate_w = (w->F_s > 0 || keep_gate_vector) ? w->shexp_gate_w : nullptr;
     p.router_logits = ws->router_logits; p.sh_gate_logit = ws->sh_gate_logit;
@@ -441,6 +445,7 @@ static GemvParams gate_up_params(const chimere_moe_layer* w, int T, chimere_moe_
     GemvParams g{};
     g.T = T; g.top_k = w->top_k; g.H = w->H;
     g.act = w->act;
+    g.few_limit = wide_weights(w) ? kFewTokensWide : kFewTokens;
     g.group_list = ws->group_list; g.perm = ws->perm;
     g.status = ws->status;
     g.ncols_routed = w->H; g.ncols_shared = w->H;
@@ -460,6 +465,7 @@ static GemvParams down_params(const chimere_moe_layer* w, float* d_y, int T, chi
     GemvParams g{};
     g.T = T; g.top_k = w->top_k; g.H = w->H;
     g.act = w->act;
+    g.few_limit = wide_weights(w) ? kFewTokensWide : kFewTokens;
     g.group_list = ws->group_list; g.perm = ws->perm;
     g.status = ws->status;
     g.ncols_routed = w->F; g.ncols_shared = w->F_s;

@@ -21,12 +21,15 @@ constexpr int kSingleSharedTokens = 8;
 __host__ __device__ inline int shared_group_tokens(int T) { return T <= kSingleSharedTokens ? 1 : kSharedGroupTokens; }
 // Tokens per routed entry.  In a decode-size batch every pair is an entry of its own: a popular expert's pairs are spread over
 // the SMs (its matrices then come from L2 again) instead of being a chain of passes in one CTA -- 8 skewed tokens through 256
-// experts of 512 x 2048 65 -> 37 us, 8 uniform ones 43 -> 38.  Matrices of more than 2M weights (1856 x 2688) cost more to fetch
-// twice than a second pass: two pairs per entry.
+// Q4_0 experts of 512 x 2048 63 -> 35 us, 8 uniform ones 58 -> 38.  Matrices of more than 2M weights (1856 x 2688) cost more to fetch
+// twice than a second pass: two pairs per entry.  `wide`: Q8_0 matrices (139 KB of gate and up rows in a CTA, one CTA per SM) do
+// so at any size -- 8 skewed tokens take 78 us in entries of up to eight pairs and 117 in entries of one, 24 tokens 124 and 295 -- and
+// so do the kernels on raw ggml blocks, which unpack a row once per entry (Q4_0, 8 / 24 skewed tokens 81 / 134 us and 91 / 227).
 constexpr int kFewTokens = 40;   // the largest batch for which the GEMV kernels are sized for one or two pairs per expert
 constexpr int kSinglePairTokens = 24;   // ... and for one
-__host__ __device__ inline int group_tokens(int T, int64_t weights) {
-    return T > kFewTokens ? kMaxGroupTokens : weights > (1 << 21) || T > kSinglePairTokens ? 2 : 1;
+constexpr int kFewTokensWide = 16;      // Q8_0: the largest batch for which they are sized for as many CTAs as one token per pass allows
+__host__ __device__ inline int group_tokens(int T, int64_t weights, bool wide) {
+    return wide || T > kFewTokens ? kMaxGroupTokens : weights > (1 << 21) || T > kSinglePairTokens ? 2 : 1;
 }
 // Behind each of these batch sizes the entries get longer and their number can fall: a work list is sized for every one below its capacity.
 constexpr int kEntrySteps[] = {kSingleSharedTokens, kSinglePairTokens, kFewTokens};

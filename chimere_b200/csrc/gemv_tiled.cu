@@ -655,7 +655,7 @@ static BulkPlan plan_bulk(const GemvParams& p, int stage, bool dual, int wk, int
     const int max_ctas = min(8, 1536 / threads);
     // decode-size batches: as many CTAs per SM as fit one token per pass, then as many tokens as still fit;
     // larger batches: at least four tokens per pass if that fits at all
-    const int mt_floor = (p.T > kFewTokens && !p.few_tokens) ? 4 : 1;
+    const int mt_floor = (p.T > p.few_limit && !p.few_tokens) ? 4 : 1;
     for (int floor_mt = mt_floor; floor_mt >= 1 && !b.ok; floor_mt = (floor_mt == 1 ? 0 : 1)) {
         auto bytes = [&](int mt, bool overlay) { return (int64_t)bulk_smem((uint32_t)tb, ncols_max, wr, wk, nmat, mt, need_red, overlay).total; };
         auto ctas_of = [&](int mt, bool overlay) {

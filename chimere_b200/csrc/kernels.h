@@ -81,6 +81,7 @@ struct GemvParams {
     int32_t* status;
     int no_combine;              // down stage: only write the per-pair rows (the caller combines)
     int split_cols_shared;       // down stage without the shared expert: its row width, which still has a say in how K is split
+    int few_limit;               // batches of up to so many tokens are decode-size (one token per pass decides how many CTAs share an SM)
     int few_tokens;              // T counts row slots that are mostly empty (fixed-size expert-parallel exchange): size the
                                  // kernels as for a decode batch whatever T says
 };

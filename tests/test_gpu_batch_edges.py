@@ -7,7 +7,7 @@ import torch
 
 import oracle
 from chimere_b200 import configs, formats
-from chimere_b200.layer import MoeScratch, MoeWeightsPrefill, MoeWeightsTiled, forward_moe, forward_moe_prefill
+from chimere_b200.layer import MoeScratch, MoeWeightsPrefill, MoeWeightsTiled, forward_moe, forward_moe_prefill, route_only
 from parity_util import check_rows, oracle_on_gpu_routing
 
 pytestmark = pytest.mark.gpu
@@ -108,3 +108,14 @@ def test_smaller_batches_in_a_larger_workspace(kw, max_T):
         check_rows(y.cpu().numpy(), oracle_on_gpu_routing(raw.to("cpu"), x.cpu().numpy(), idx)["y"])
         perm, offs = oracle.permute(idx, cfg.E)
         assert np.array_equal(sc.perm(T).cpu().numpy(), perm) and np.array_equal(sc.offsets().cpu().numpy(), offs)
+
+
+# Eight tokens of one expert: an entry each where several CTAs share an SM, one entry for all where a CTA's weights fill it (Q8_0) and on
+# raw blocks, which a kernel unpacks once per entry.
+@pytest.mark.parametrize("cfg,packed,entries", [(Q4, True, 8), (IQ3, True, 8), (Q8, True, 1), (Q4, False, 1)], ids=lambda v: getattr(v, "name", str(v)))
+def test_pairs_per_entry(cfg, packed, entries):
+    raw = configs.make_layer(configs.scaled(cfg, E=1, top_k=1, H=512, F=256, F_s=0, zipf_bias=False), device="cuda")
+    w = MoeWeightsTiled(raw) if packed else raw
+    sc = MoeScratch(w, 64)
+    route_only(w, sc, configs.make_input(configs.scaled(cfg, H=512), 8, device="cuda"))
+    assert sc._view(sc.ws.group_list, 16).view(torch.int32).tolist() == [entries, entries, 0, 0]
