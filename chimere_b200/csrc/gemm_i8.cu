@@ -294,11 +294,12 @@ __device__ __forceinline__ bool expand_tile(const Params& p, const GemmWork& w, 
     const bool slim = uniform(w.npad) <= 32;
     pos.geometry(slim);
     const int nstages = (nb + kG_StageUnits - 1) / kG_StageUnits;
-    if ((MODE != kOrdered && type >= kTypeOperand) || slim) {   // nothing to do (slim tiles: half of the read-back warps expand) but keep step
-        for (int s = 0; s + 1 < nstages; ++s) pos.next(MODE == kOrdered || type < kTypeOperand);
-        // (parity tells a barrier's phases apart only within a round: see the tile's last bytes arrive before going on)
-        if (!mbar_wait(&sh.full1[pos.r], pos.par1())) { gemm_timeout(sh, p.status, lane); return false; }
-        pos.next(MODE == kOrdered || type < kTypeOperand);
+    if ((MODE != kOrdered && type >= kTypeOperand) || slim) {   // nothing to do (slim tiles: half of the read-back warps expand) but keep step:
+        // parity tells a barrier's phases apart only while nobody is two behind, so every stage is seen to arrive
+        for (int s = 0; s < nstages; ++s) {
+            if (!mbar_wait(&sh.full1[pos.r], pos.par1())) { gemm_timeout(sh, p.status, lane); return false; }
+            pos.next(MODE == kOrdered || type < kTypeOperand);
+        }
         return true;
     }
     uint32_t d3[2] = {0u, 0u}, sc3[2] = {0u, 0u};   // IQ3_S: this lane's rows' scales of the super-block, kept over its two stages

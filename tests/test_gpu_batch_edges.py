@@ -58,6 +58,19 @@ def test_mixed_operand_forms(T):
     _check(configs.scaled(Q4, E=4, top_k=2, H=512, F=256, F_s=256, type_sh_gate_up=configs.Q8_0, type_sh_down=configs.Q8_0), T, prefill=True)
 
 
+# ... enough wide tiles of both that every CTA goes from one form to the other, with more stages per tile than the rings have slots
+def test_mixed_operand_forms_tile_after_tile():
+    cfg = configs.scaled(Q4, E=4, top_k=2, H=2048, F=512, F_s=1024, type_sh_gate_up=configs.Q8_0, type_sh_down=configs.Q8_0)
+    raw, T = configs.make_layer(cfg, device="cuda"), 2100
+    tiled = MoeWeightsTiled(raw)
+    x, sc = configs.make_input(cfg, T, device="cuda"), MoeScratch(tiled, T)
+    want = forward_moe(tiled, sc, x).clone()      # (a Q8_0 shared expert keeps the decode entry on the GEMV kernels)
+    pw = MoeWeightsPrefill(raw)
+    for _ in range(5):
+        check_rows(forward_moe_prefill(tiled, pw, sc, x).cpu().numpy(), want.cpu().numpy())
+    assert sc.status() == 0
+
+
 @pytest.mark.parametrize("cfg,T", [(configs.scaled(Q4, E=16, F=128, F_s=128, H=512), t) for t in (16, 17, 24, 25, 40, 41, 64)] +
                                   [(configs.scaled(configs.NEMOTRON_Q4_0, E=8, H=2688, F=800, F_s=1600, name="wide experts"), t) for t in (8, 16, 17, 33)],
                          ids=lambda v: getattr(v, "name", str(v)))
