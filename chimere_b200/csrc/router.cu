@@ -812,7 +812,14 @@ __global__ void __launch_bounds__(256) permute_kernel(const RouteParams p) {
 // rows of every token in slot order (weighted_combine_kernel, chimere_kernels.cu:1551-1565) plus the
 // sigmoid-gated shared expert (sigmoid_gate_add_kernel, scratch_pool.rs:266-277).
 // HBM-bound: T * (k + 1) rows in, T out.  Four elements per thread and every row's load issued before the first is used
-// (k <= kMaxTopK): 161 us with one element and one load at a time at T = 8192, k = 8, H = 2048.
+// (k <= kMaxTopK): 161 us with one element and one load at a time at T = 8192, k = 8, H = 2048.  ALIGNED: rows, shared rows and y
+// lie on 16-byte boundaries and go as one access of four elements; a caller's y or rows may lie on any float.
+template <bool ALIGNED>
+__device__ __forceinline__ float4 ld_row4(const float* p) {
+    if (ALIGNED) return __ldcs(reinterpret_cast<const float4*>(p));
+    return make_float4(__ldcs(p), __ldcs(p + 1), __ldcs(p + 2), __ldcs(p + 3));
+}
+template <bool ALIGNED>
 __global__ void __launch_bounds__(256) ep_finish_kernel(const float* __restrict__ rows, const int32_t* __restrict__ slot, const float* __restrict__ topk_w,
                                                         const float* __restrict__ shared_rows, const float* __restrict__ sh_logit, float* __restrict__ y,
                                                         int T, int H, int k) {
@@ -828,10 +835,10 @@ __global__ void __launch_bounds__(256) ep_finish_kernel(const float* __restrict_
     for (int j = 0; j < kMaxTopK; ++j)
         if (j < k) {
             const size_t r = slot ? (size_t)slot[t * k + j] : (size_t)t * k + j;   // where pair (t, j) came back
-            v[j] = __ldcs(reinterpret_cast<const float4*>(rows + r * H + h));
+            v[j] = ld_row4<ALIGNED>(rows + r * H + h);
             w[j] = topk_w[(size_t)t * k + j];
         }
-    if (shared_rows) sh = __ldcs(reinterpret_cast<const float4*>(shared_rows + (size_t)t * H + h));
+    if (shared_rows) sh = ld_row4<ALIGNED>(shared_rows + (size_t)t * H + h);
     float4 sum = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 #pragma unroll
     for (int j = 0; j < kMaxTopK; ++j)
@@ -842,7 +849,9 @@ __global__ void __launch_bounds__(256) ep_finish_kernel(const float* __restrict_
             sum.x = fmaf(sh.x, g, sum.x); sum.y = fmaf(sh.y, g, sum.y); sum.z = fmaf(sh.z, g, sum.z); sum.w = fmaf(sh.w, g, sum.w);
         } else { sum.x += sh.x; sum.y += sh.y; sum.z += sh.z; sum.w += sh.w; }
     }
-    *reinterpret_cast<float4*>(y + (size_t)t * H + h) = sum;
+    float* out = y + (size_t)t * H + h;
+    if (ALIGNED) *reinterpret_cast<float4*>(out) = sum;
+    else { out[0] = sum.x; out[1] = sum.y; out[2] = sum.z; out[3] = sum.w; }
 }
 
 // Fixed-size dispatch of an expert-parallel layer.  Slot s = (destination rank d, position i) of the send
@@ -1091,7 +1100,9 @@ cudaError_t launch_ep_finish(const float* rows, const int32_t* slot, const float
                              float* y, int T, int H, int k, cudaStream_t stream) {
     const int64_t n = (int64_t)T * (H / 4);   // (H is a multiple of 32)
     if (n <= 0) return cudaSuccess;
-    return launch_pdl(ep_finish_kernel, dim3((unsigned)((n + 255) / 256)), 256, 0, stream, rows, slot, topk_w, shared_rows, sh_logit, y, T, H, k);
+    const bool aligned = (((uintptr_t)rows | (uintptr_t)shared_rows | (uintptr_t)y) & 15) == 0;   // (H is a multiple of four: so is every row then)
+    return launch_pdl(aligned ? ep_finish_kernel<true> : ep_finish_kernel<false>, dim3((unsigned)((n + 255) / 256)), 256, 0, stream, rows, slot, topk_w,
+                      shared_rows, sh_logit, y, T, H, k);
 }
 
 // Exact-size dispatch (prefill-size batches): the routing kernel's dispatch has already sorted the pairs by expert, and the

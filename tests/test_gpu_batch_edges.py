@@ -7,7 +7,7 @@ import torch
 
 import oracle
 from chimere_b200 import configs, formats
-from chimere_b200.layer import MoeScratch, MoeWeightsPrefill, MoeWeightsTiled, forward_moe, forward_moe_prefill, route_only
+from chimere_b200.layer import MoeScratch, MoeWeightsPrefill, MoeWeightsTiled, forward_moe, forward_moe_host, forward_moe_prefill, route_only
 from parity_util import check_rows, oracle_on_gpu_routing
 
 pytestmark = pytest.mark.gpu
@@ -132,3 +132,29 @@ def test_pairs_per_entry(cfg, packed, entries):
     sc = MoeScratch(w, 64)
     route_only(w, sc, configs.make_input(configs.scaled(cfg, H=512), 8, device="cuda"))
     assert sc._view(sc.ws.group_list, 16).view(torch.int32).tolist() == [entries, entries, 0, 0]
+
+
+# An output is a float pointer and may start on any float (a view into a larger buffer), also where the combine stores four at a time.
+@pytest.mark.parametrize("T", [8, 64, 200])
+@pytest.mark.parametrize("entry", ["decode", "host", "prefill"])
+def test_outputs_on_any_float_boundary(entry, T):
+    cfg = configs.scaled(Q4, E=16, F=128, F_s=128, H=512)
+    raw = configs.make_layer(cfg, device="cuda")
+    tiled = MoeWeightsTiled(raw)
+    x, sc = configs.make_input(cfg, T, device="cuda"), MoeScratch(tiled, T)
+    pw = MoeWeightsPrefill(raw)
+    results = []
+    for shift in range(4):
+        room = torch.zeros(T * cfg.H + 4, pin_memory=entry == "host") if entry == "host" else torch.zeros(T * cfg.H + 4, device="cuda")
+        y = room[shift:shift + T * cfg.H].reshape(T, cfg.H)
+        if entry == "decode":
+            forward_moe(tiled, sc, x, y)
+        elif entry == "host":
+            forward_moe_host(tiled, sc, x.cpu().pin_memory(), y)
+        else:
+            forward_moe_prefill(tiled, pw, sc, x, y)
+        torch.cuda.synchronize()
+        rest = room.cpu()
+        assert sc.status() == 0 and rest[:shift].abs().sum() == 0 and rest[shift + T * cfg.H:].abs().sum() == 0
+        results.append(y.cpu().clone())
+    assert all(torch.equal(r, results[0]) for r in results)
