@@ -985,7 +985,7 @@ struct GateUpPolicy : MoePolicy {
             for (int i = 0; i < 2; ++i) {
                 const int ci = min(c + i * cstep, w.n_valid - 1);
                 const float a = xch_sum<KG>(xch, w.npad, r, ci);
-                if (p.dual) { const float u = xch_sum<KG>(xch, w.npad, r + 64, ci); v[i] = MODE != kPlain ? silu_mul_ref(a, u) : silu_mul_near(a, u); }
+                if (p.dual) { const float u = xch_sum<KG>(xch, w.npad, r + 64, ci); v[i] = MODE != kPlain ? silu_mul_ref(a, u) : silu_mul_fast(a, u); }
                 else { const float t = fmaxf(a, 0.0f); v[i] = t * t; }
             }
 #pragma unroll
