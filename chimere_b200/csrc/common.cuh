@@ -223,22 +223,26 @@ __device__ __forceinline__ float silu_mul_fast(float g, float u) {
 __device__ __forceinline__ int round_int(float x) { return __float2int_rz(__fadd_rz(x, copysignf(0.5f, x))); }
 
 // One 32-value block of Q8_1 by one warp, lane = value: d = amax / 127 and q = roundf(v / d), both quotients correctly rounded as
-// the compiler's division gives them, in a third of its instructions: with the correctly rounded reciprocal r of b, the last of
+// the division operator's are: with the correctly rounded reciprocal r of b, the last of
 //   q0 = a * r,  q1 = q0 + r * (a - b * q0),  q2 = q1 + r * (a - b * q1)
-// is the correctly rounded a / b (Markstein 1990, theorem on division by a correctly rounded reciprocal) as long as nothing
-// underflows or overflows; blocks outside a wide range of magnitudes take the plain division.
+// is the correctly rounded a / b (P. Markstein, "Computation of elementary functions on the IBM RISC System/6000 processor", 1990,
+// theorem on division by a correctly rounded reciprocal) as long as nothing underflows or overflows.  Blocks outside a wide
+// range of magnitudes, and blocks with a NaN, which the maximum leaves out, take the plain operations.
 __device__ __forceinline__ float div_by_recip(float a, float b, float r) {
     float q = a * r;
     q = fmaf(fmaf(-q, b, a), r, q);
     return fmaf(fmaf(-q, b, a), r, q);
 }
 __device__ __forceinline__ int8_t q8_1_warp(float v, float& d) {
-    // largest magnitude: bit patterns of non-negative floats order like the values
-    const float amax = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(fabsf(v))));
+    // largest magnitude: bit patterns of non-negative floats order like the values, with the NaNs above infinity
+    float amax = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(fabsf(v))));
     if (amax > 1e-25f && amax < 1e25f) {
         d = div_by_recip(amax, 127.0f, 1.0f / 127.0f);
         return (int8_t)round_int(div_by_recip(v, d, __frcp_rn(d)));
     }
+    amax = fabsf(v);
+#pragma unroll
+    for (int s = 16; s > 0; s >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, s));
     d = amax / 127.0f;
     return amax == 0.0f ? (int8_t)0 : (int8_t)roundf(v / d);
 }

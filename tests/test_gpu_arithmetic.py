@@ -22,6 +22,41 @@ __global__ void silu_kernel(unsigned long long* bad) {
         if (!same(w, v) && !zero && !(tail && v <= 0.0f && v >= -2.5e-36f)) atomicAdd(bad, 1ull);
     }
 }
+// one block of 32 values per warp: Q8_1 with the division operator, fmaxf over the block (NaN left out) and roundf
+__device__ unsigned mix(unsigned long long x) {
+    x ^= x >> 33; x *= 0xff51afd7ed558ccdull; x ^= x >> 33; x *= 0xc4ceb9fe1a85ec53ull; x ^= x >> 33;
+    return (unsigned)x;
+}
+__global__ void q8_kernel(unsigned long long* bad) {
+    const int lane = threadIdx.x & 31;
+    for (unsigned long long blk = blockIdx.x * 8ull + (threadIdx.x >> 5); blk < (1ull << 24); blk += gridDim.x * 8ull) {
+        const unsigned hb = mix(2 * blk + 1), h = mix((blk * 32 + lane) * 2);
+        // the block's magnitude: all of the floats', with the limits of the fast form among them; its values: uniform, around the
+        // half-way points, far smaller, zeros, infinities, NaN
+        float top = __uint_as_float((hb >> 1) & 0x7FFFFFFFu);
+        if ((hb & 7) == 1) top = 1e-25f * (1.0f + (float)(hb >> 20) * 1e-6f);
+        if ((hb & 7) == 2) top = 1e25f * (1.0f - (float)(hb >> 20) * 1e-6f);
+        if ((hb & 7) > 3) top = (float)(hb >> 8) * 1e-5f;
+        const float step = top / 127.0f;
+        float v = top * ((float)(h >> 8) / 16777216.0f);
+        if ((hb & 24) == 8) v = step * ((float)(h % 127) + 0.5f) * (1.0f + (float)((int)(h >> 16) % 5 - 2) * 5.9e-8f);
+        if ((hb & 24) == 16 && lane > 3) v *= 1e-30f;
+        if ((hb & 96) == 32 && (h & 31) == 0) v = __uint_as_float(0x7FC00000u);
+        if ((hb & 480) == 64 && lane == (hb >> 27)) v = __uint_as_float(0x7F800000u);
+        if ((hb & 0xF00) == 0 && (h & 3)) v = 0.0f;
+        if ((hb & 0xFFF000) == 0) v = (hb >> 24) & 1 ? 0.0f : __uint_as_float(0x7FC00000u);
+        if (lane == 5 && !((hb >> 11) & 1)) v = top;
+        if (h & 0x800000u) v = -v;
+        float d;
+        const int8_t q = q8_1_warp(v, d);
+        float amax = fabsf(v);
+        for (int m = 16; m > 0; m >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, m));
+        const float dp = amax / 127.0f;
+        const int8_t qp = amax == 0.0f ? (int8_t)0 : (int8_t)roundf(v / dp);
+        if (q != qp || !same(d, dp)) atomicAdd(bad, 1ull);
+    }
+}
+extern "C" int q8_check(unsigned long long* bad) { q8_kernel<<<1184, 256>>>(bad); return (int)cudaDeviceSynchronize(); }
 extern "C" int silu_check(unsigned long long* bad) { silu_kernel<<<1184, 256>>>(bad); return (int)cudaDeviceSynchronize(); }
 """
 
@@ -46,3 +81,26 @@ def _mismatches(check):
 
 def test_silu_is_the_reference_quotient_for_every_float(lib):
     assert _mismatches(lib.silu_check) == 0
+
+
+def test_q8_1_blocks_are_those_of_the_plain_operations(lib):
+    assert _mismatches(lib.q8_check) == 0
+
+
+@pytest.mark.parametrize("T", [3, 40, 200])
+def test_routers_and_operator_quantise_alike(T):
+    """The Q8_1 rows that the routers leave and those of the operator entry are the same bytes, NaN, infinities and extremes included."""
+    from chimere_b200 import abi, configs
+    from chimere_b200.layer import MoeScratch, MoeWeightsTiled, route_only
+    cfg = configs.scaled(configs.QWEN_Q4_0, E=256, H=512, F=64, F_s=0)
+    tiled = MoeWeightsTiled(configs.make_layer(cfg, device="cuda"))
+    x = configs.make_input(cfg, T, device="cuda")
+    x[0, 3], x[0, 40], x[0, 41], x[1, 70] = float("nan"), float("inf"), float("-inf"), 1e30
+    x[1, 96:128], x[1, 128:160], x[2, :32] = float("nan"), 0.0, torch.arange(32, device="cuda") * 1e-28
+    x[2, 64:96] = torch.arange(32, device="cuda") + 0.5
+    x[2, 64] = 127.0
+    sc = MoeScratch(tiled, T)
+    route_only(tiled, sc, x)
+    want = torch.zeros(T, 512 // 32 * 36, dtype=torch.uint8, device="cuda")
+    abi.load().chimere_quantize_q8_1_batched(x.data_ptr(), want.data_ptr(), 512, 512, T, torch.cuda.current_stream().cuda_stream)
+    assert torch.equal(sc.x_q8(T), want)
