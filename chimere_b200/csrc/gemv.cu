@@ -415,24 +415,24 @@ __global__ void rmsnorm_kernel(const float* x, float* y, int H, float eps) {
 // registers, longer ones are read again), and every warp sums the 256 partial sums itself instead of meeting eight times (10.5 us
 // -> 3.5 at 2 rows of 2048, cold).
 constexpr int kNormRegs = 16;
-__global__ void __launch_bounds__(256) add_residual_rmsnorm_kernel(const float* __restrict__ hidden, float* __restrict__ residual,
-                                                                   const float* __restrict__ weight, float* __restrict__ normed, int H, float eps) {
+// (No __restrict__, here or in the other kernels launched programmatically: the kernel before may write what these pointers name, and
+// reads of memory that the compiler may take for constant are not held back by griddep_wait().)
+__global__ void __launch_bounds__(256) add_residual_rmsnorm_kernel(const float* hidden, float* residual, const float* weight, float* normed, int H,
+                                                                   float eps) {
     __shared__ float s_sum[256];
     const int tid = threadIdx.x, lane = tid & 31;
-    float w[kNormRegs];
-#pragma unroll
-    for (int j = 0; j < kNormRegs; ++j) w[j] = j * 256 + tid < H ? weight[j * 256 + tid] : 0.0f;   // (a constant of the layer)
-    griddep_wait();                       // the rows may come from the previous kernel of the stream
+    griddep_wait();                       // the rows and the weight may come from the previous kernel of the stream
     if (tid == 0) griddep_launch();
     const float* h = hidden + (size_t)blockIdx.x * H;
     float* r = residual + (size_t)blockIdx.x * H;
     float* out = normed + (size_t)blockIdx.x * H;
-    float v[kNormRegs], hv[kNormRegs];
+    float v[kNormRegs], hv[kNormRegs], w[kNormRegs];
 #pragma unroll
     for (int j = 0; j < kNormRegs; ++j) {
         const int i = j * 256 + tid;
         hv[j] = i < H ? h[i] : 0.0f;
         v[j] = i < H ? r[i] : 0.0f;
+        w[j] = i < H ? weight[i] : 0.0f;
     }
     float sum_sq = 0.0f;
 #pragma unroll

@@ -94,10 +94,9 @@ __device__ __forceinline__ float dot_sub(const SubBlock& s, const uint8_t* xb) {
 // to the routed sum, scratch_pool.rs:266-277).  blockIdx.z = 1 takes the second matrix / output (gate beside up).
 constexpr int kTokensPerCta = 8;
 template <int TYPE>
-__global__ void __launch_bounds__(32 * kRowsPerCta) kquant_mmvq_kernel(const uint8_t* __restrict__ w, const uint8_t* __restrict__ w2,
-                                                                      const uint8_t* __restrict__ xq8, int64_t x_stride, float* __restrict__ y,
-                                                                      float* __restrict__ y2, int64_t y_stride, int n_inputs, int tpc, int ncols,
-                                                                      int nrows, int mode, const float* __restrict__ logit) {
+__global__ void __launch_bounds__(32 * kRowsPerCta) kquant_mmvq_kernel(const uint8_t* w, const uint8_t* w2, const uint8_t* xq8, int64_t x_stride, float* y,
+                                                                      float* y2, int64_t y_stride, int n_inputs, int tpc, int ncols, int nrows, int mode,
+                                                                      const float* logit) {
     const int lane = threadIdx.x & 31, row = blockIdx.x * kRowsPerCta + (threadIdx.x >> 5);
     const int t0 = blockIdx.y * tpc, nt = min(tpc, n_inputs - t0);   // tpc <= kTokensPerCta input rows per CTA
     griddep_wait();   // (a no-op unless launched programmatically behind the kernel that writes the inputs)
@@ -135,8 +134,7 @@ __global__ void __launch_bounds__(32 * kRowsPerCta) kquant_mmvq_kernel(const uin
 
 // One warp per (row t, block b of 32): v = silu(g) * u (or relu(u)^2 without a gate row) -> one Q8_1 block, as the gate/up
 // kernels write their intermediates (d = amax / 127 in f16, s = the sum of the 32 values).
-__global__ void __launch_bounds__(256) act_q8_1_kernel(const float* __restrict__ g, const float* __restrict__ u, int64_t in_stride,
-                                                       uint8_t* __restrict__ out, int64_t out_stride, int T, int F) {
+__global__ void __launch_bounds__(256) act_q8_1_kernel(const float* g, const float* u, int64_t in_stride, uint8_t* out, int64_t out_stride, int T, int F) {
     const int lane = threadIdx.x & 31, nb = F >> 5;
     const int64_t wid = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
     griddep_wait();

@@ -455,11 +455,10 @@ __global__ void __launch_bounds__(256) route_prep_kernel(const RouteParams p) {
     const int row = token ? blockIdx.x : blockIdx.x - p.T, rows = token ? p.T : p.E;
     const float* src = token ? p.x + (size_t)row * H : p.router_w + (size_t)row * H;
     float v[4 * NQ];
-    if (token) griddep_wait();
+    griddep_wait();
+    if (tid == 0) griddep_launch();
 #pragma unroll
     for (int i = 0; i < 4 * NQ; ++i) v[i] = i * 256 + tid < H ? src[i * 256 + tid] : 0.0f;
-    if (!token) griddep_wait();   // (the router's rows are constants; the scratch may still be in use)
-    if (tid == 0) griddep_launch();
     const int n = (int)(__brev((unsigned)tid) >> 24);
     float* dst = p.scratch + (token ? 0 : (size_t)p.T * kRouteChunks * kPitch);
     dst += ((size_t)(n / kRoutePartials) * rows + row) * kPitch + (n % kRoutePartials) * (4 * NQ);
@@ -470,7 +469,7 @@ __global__ void __launch_bounds__(256) route_prep_kernel(const RouteParams p) {
         float acc = 0.0f;
 #pragma unroll
         for (int i = 0; i < 4 * NQ; ++i)
-            if (i * 256 + tid < H) acc = fmaf(__ldg(p.shexp_gate_w + i * 256 + tid), v[i], acc);
+            if (i * 256 + tid < H) acc = fmaf(p.shexp_gate_w[i * 256 + tid], v[i], acc);
         red[tid] = acc;
     }
     const int nbH = H >> 5;
@@ -820,9 +819,8 @@ __device__ __forceinline__ float4 ld_row4(const float* p) {
     return make_float4(__ldcs(p), __ldcs(p + 1), __ldcs(p + 2), __ldcs(p + 3));
 }
 template <bool ALIGNED>
-__global__ void __launch_bounds__(256) ep_finish_kernel(const float* __restrict__ rows, const int32_t* __restrict__ slot, const float* __restrict__ topk_w,
-                                                        const float* __restrict__ shared_rows, const float* __restrict__ sh_logit, float* __restrict__ y,
-                                                        int T, int H, int k) {
+__global__ void __launch_bounds__(256) ep_finish_kernel(const float* rows, const int32_t* slot, const float* topk_w, const float* shared_rows, const float* sh_logit,
+                                                        float* y, int T, int H, int k) {
     griddep_wait();
     if (threadIdx.x == 0) griddep_launch();
     const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;

@@ -5,7 +5,7 @@ import pytest
 import torch
 
 from chimere_b200 import configs, formats
-from chimere_b200.layer import MoeScratch, MoeWeightsPrefill, MoeWeightsTiled, forward_moe, forward_moe_prefill
+from chimere_b200.layer import MoeScratch, MoeWeightsPrefill, MoeWeightsTiled, forward_moe, forward_moe_prefill, forward_moe_residual_norm
 
 pytestmark = pytest.mark.gpu
 
@@ -51,3 +51,35 @@ def test_layer_call_replays_from_a_graph(kind, cfg, T):
         torch.cuda.synchronize()
         assert torch.equal(y, want)
     assert sc.status() == 0
+
+
+def test_norm_weight_and_router_rows_from_the_call_before():
+    """A call may read what the kernel directly in front of it in the stream has written, although it is launched programmatically:
+    here the norm weight, and the router's rows of a batch that takes the tiled router."""
+    cfg = configs.scaled(configs.QWEN_IQ3S, E=256, F=256, F_s=0, H=2048)
+    raw = configs.make_layer(cfg, device="cuda")
+    tiled, T = MoeWeightsTiled(raw), 160
+    first, second = MoeScratch(tiled, 1), MoeScratch(tiled, T)
+    x1, hidden = configs.make_input(cfg, 1, device="cuda", seed=1), configs.make_input(cfg, T, device="cuda", seed=2)
+    weight, residual, y = torch.empty(1, cfg.H, device="cuda"), torch.empty(T, cfg.H, device="cuda"), torch.empty(T, cfg.H, device="cuda")
+    results = []
+    for wait in (True, False, False, False):
+        weight.fill_(1.0)
+        residual.fill_(0.25)
+        torch.cuda.synchronize()
+        forward_moe(tiled, first, x1, weight)
+        if wait:
+            torch.cuda.synchronize()
+        forward_moe_residual_norm(tiled, second, hidden, residual, weight, 1e-6, y)
+        results.append(y.clone())
+    assert all(torch.equal(r, results[0]) for r in results)
+    results = []
+    for wait in (True, False, False, False):
+        raw.router_weight[0].fill_(0.0)
+        torch.cuda.synchronize()
+        forward_moe(tiled, first, x1, raw.router_weight[:1])
+        if wait:
+            torch.cuda.synchronize()
+        forward_moe(tiled, second, hidden, y)
+        results.append(y.clone())
+    assert all(torch.equal(r, results[0]) for r in results)
