@@ -395,8 +395,23 @@ __device__ __forceinline__ bool mma_tile(const Params& p, const GemmWork& w, Gem
 
 // W accumulator columns of this thread's row: acc[c] += (dot * sa) * sb[c] with dot * sa = fma(reading, sa, offset * sa),
 // rounded once like a plain product.  sb: shared address of the first column's token scale.
-template <int W, uint32_t kBias>
+// ANY_SCALE: scales may be any f32 (2^100 times one above 2^28 is infinite), so the exact dot comes first, without a power of two.
+template <int W, uint32_t kBias, bool ANY_SCALE>
 __device__ __forceinline__ void block_values(const int (&v)[W], float sa, uint32_t sb, uint64_t* acc2) {
+    if (ANY_SCALE) {
+        const uint64_t r2 = pack2(kRowScaleBits, kRowScaleBits), o2 = pack2(kOffsetBits, kOffsetBits), p2 = pack2(kSumScaleBits, kSumScaleBits), a2 = pack2f(sa, sa);
+#pragma unroll
+        for (int g = 0; g < W / 4; ++g) {
+            uint64_t s[2];
+            lds_2x64(sb + 16u * g, s[0], s[1]);
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                const uint64_t t = mul2(fma2(pack2((uint32_t)v[4 * g + 2 * i] + kBias, (uint32_t)v[4 * g + 2 * i + 1] + kBias), r2, o2), p2);
+                acc2[2 * g + i] = fma2(mul2(t, a2), s[i], acc2[2 * g + i]);
+            }
+        }
+        return;
+    }
     const float sr = sa * __uint_as_float(kRowScaleBits), c = sa * __uint_as_float(kOffsetBits);
     const uint64_t sa2 = pack2f(sr, sr);
     const uint64_t c2 = pack2f(c, c);
@@ -414,7 +429,7 @@ __device__ __forceinline__ void block_values(const int (&v)[W], float sa, uint32
 // The read-back of one tile by one warp: column group colg of W columns; in tiles of up to 64 columns the warps of a column
 // group also share the stages among them (KG shares, stage s to share s % KG), so that a warp has that much longer for the
 // latency of one stage (barrier, TMEM load, scales: about a thousand cycles).
-template <int COLG, int KG, int W>
+template <int COLG, int KG, int W, bool ANY_SCALE>
 __device__ __forceinline__ bool readback_tile(GemmShared& sh, uint32_t ring1, uint32_t ring2, uint32_t tmem, int32_t* status, int nb, bool expanded, int q,
                                               int part, int lane, RingPos& pos, TmemPos& tp, uint64_t* acc2) {
     constexpr int kPad = COLG * W, kBps = blocks_per_slot(kPad);
@@ -453,7 +468,7 @@ __device__ __forceinline__ bool readback_tile(GemmShared& sh, uint32_t ring1, ui
                             __syncwarp();
                             if (lane == 0) mbar_arrive_n(&sh.tempty[tp.slot], 4 / COLG);
                         }
-                        block_values<W, kPad == 128 ? 0u : 1u << 19>(v, sa, sb + (uint32_t)((j0 + i) * (kPad * 36)), acc2);
+                        block_values<W, kPad == 128 ? 0u : 1u << 19, ANY_SCALE>(v, sa, sb + (uint32_t)((j0 + i) * (kPad * 36)), acc2);
                     }
                 }
                 tp.next();
@@ -561,14 +576,14 @@ __device__ __forceinline__ void count_up(int n, uint64_t (&sum)[4], uint64_t (&s
 }
 
 // A warp's sums of a tile into the exchange buffer (part = share * column groups + column group).
-template <int W>
+template <int W, bool UNSCALED = false>
 __device__ __forceinline__ bool publish_sums(int32_t* status, GemmShared& sh, float* xch, int q, int part, int lane, uint32_t& xphase, const uint64_t* acc2, bool ok) {
     if (!mbar_wait(&sh.xempty, (xphase & 1u) ^ 1u)) { gemm_timeout(sh, status, lane); ok = false; }   // the tile before has been stored
     ++xphase;
     float* mine = xch + part * (W * 128) + q * 32 + lane;
     const uint64_t sc2 = pack2(kSumScaleBits, kSumScaleBits);
 #pragma unroll
-    for (int i = 0; i < W / 2; ++i) unpack2(mul2(acc2[i], sc2), mine[(2 * i) * 128], mine[(2 * i + 1) * 128]);
+    for (int i = 0; i < W / 2; ++i) unpack2(UNSCALED ? acc2[i] : mul2(acc2[i], sc2), mine[(2 * i) * 128], mine[(2 * i + 1) * 128]);
     __syncwarp();
     if (lane == 0) mbar_arrive_cta(&sh.xfull);
     return ok;
@@ -641,8 +656,8 @@ __device__ __forceinline__ bool readback(const Params& p, const GemmWork& w, Gem
     uint64_t acc2[W / 2];
 #pragma unroll
     for (int i = 0; i < W / 2; ++i) acc2[i] = 0ull;
-    bool ok = readback_tile<COLG, KG, W>(sh, ring1, ring2, tmem, p.status, uniform(w.nb), uniform(Policy::type(p, w)) < kTypeOperand, q, part, lane, pos, tp, acc2);
-    return publish_sums<W>(p.status, sh, xch, q, part, lane, xphase, acc2, ok);
+    const bool ok = readback_tile<COLG, KG, W, Policy::kAnyScale>(sh, ring1, ring2, tmem, p.status, uniform(w.nb), uniform(Policy::type(p, w)) < kTypeOperand, q, part, lane, pos, tp, acc2);
+    return publish_sums<W, Policy::kAnyScale>(p.status, sh, xch, q, part, lane, xphase, acc2, ok);
 }
 
 template <class Policy, class Params, int COLG, int W>
@@ -877,6 +892,7 @@ __global__ void __launch_bounds__(kG_Threads, 1) gemm_i8_kernel(const Params p, 
 // ------------------------------------------------------------------ policies ----
 // plain fp32 tile store: out[(row0 + r) * ldo + col0 + c] = D[r][c]  (the primitive; operands in the mma128 form)
 struct PlainPolicy {
+    static constexpr bool kAnyScale = true;
     template <int>
     __device__ static __forceinline__ int work(const GemmParams& p, int idx, GemmWork& w) {
         if (idx >= p.n_items) return kWorkEnd;
@@ -906,6 +922,7 @@ __device__ __forceinline__ int tile_width(int n) { return n <= 16 ? 16 : n <= 32
 
 // What the gate/up and the down launch share: the tile list and where a row tile's weights are.
 struct MoePolicy {
+    static constexpr bool kAnyScale = false;   // (ggml's scales are f16)
     template <int MODE>
     __device__ static __forceinline__ int work(const PrefillGemmParams& p, int idx, GemmWork& w) {
         if (MODE == kMin) {   // shared-expert tiles of 32 tokens; word 1 of the list: their first column / 16

@@ -15,7 +15,7 @@ def _pack(lib, q, sc):
     return out
 
 
-def _run(rows, tokens, cols, unit_scales):
+def _run(rows, tokens, cols, unit_scales, sa_times=1.0, sb_times=1.0):
     lib = abi.load()
     g = torch.Generator(device="cuda").manual_seed(rows * 7 + tokens)
     A = torch.randint(-127, 128, (rows, cols), generator=g, device="cuda", dtype=torch.int32).to(torch.int8)
@@ -27,6 +27,7 @@ def _run(rows, tokens, cols, unit_scales):
         # weight-side scales as ggml has them: an f16 value (times a small odd factor, as IQ3_S sub-blocks do)
         sa = (torch.rand(rows, nb, generator=g, device="cuda") * 0.01 + 0.001).half().float() * (1 + 2 * torch.randint(0, 16, (rows, nb), generator=g, device="cuda"))
         sb = torch.rand(tokens, nb, generator=g, device="cuda") * 0.05 + 0.001
+        sa, sb = sa * sa_times, sb * sb_times
     pa, pb = _pack(lib, A, sa), _pack(lib, B, sb)
     out = torch.full((rows, tokens), float("nan"), device="cuda")
     items = torch.zeros(((rows + 127) // 128) * ((tokens + 127) // 128) * 32 + 256, dtype=torch.uint8, device="cuda")
@@ -51,6 +52,14 @@ def test_integer_dots_exact_with_unit_scales(rows, tokens, cols):
 @pytest.mark.parametrize("rows,tokens,cols", [(256, 200, 512), (512, 128, 2048), (256, 60, 1024), (256, 9, 160)])
 def test_block_scaled_result(rows, tokens, cols):
     out, ref = _run(rows, tokens, cols, unit_scales=False)
+    rel = (out.double() - ref).abs().max() / ref.abs().max()
+    assert rel < 1e-5, float(rel)
+
+
+# the primitive takes any f32 scales, not only f16 ones
+@pytest.mark.parametrize("sa_times,sb_times", [(1e12, 1.0), (1e30, 1e-12), (1e-30, 1e12), (1e-20, 1e-10)])
+def test_scales_of_any_size(sa_times, sb_times):
+    out, ref = _run(256, 150, 512, unit_scales=False, sa_times=sa_times, sb_times=sb_times)
     rel = (out.double() - ref).abs().max() / ref.abs().max()
     assert rel < 1e-5, float(rel)
 
