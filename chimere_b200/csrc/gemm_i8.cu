@@ -1232,9 +1232,11 @@ cudaError_t launch_pack_mma128_q8_0(const void* raw, void* out, int n_mats, int 
 // GEMV work list of the others (gemm_min <= kMaxGroupTokens + 1).  One CTA of 256 threads,
 // thread e = expert e.  Wide tiles come first and the narrow ones last, so that the persistent GEMM CTAs, which take tiles
 // in order, end on cheap ones; within a width the shared expert's tile leads.  Tiles per width are counted with one scan
-// (four 16-bit counters in a 64-bit word), and a tile's first column follows from its place, because all tiles of a width
+// (a 64-bit word of counters, 28 bits for the full tiles' width and 12 for each narrower one, of which an expert has at most one tile), and a tile's first column follows from its place, because all tiles of a width
 // are equally wide.
-__device__ __forceinline__ uint64_t width_bit(int n, uint64_t count) { return n > 64 ? count : n > 32 ? count << 16 : n > 16 ? count << 32 : count << 48; }
+__device__ __forceinline__ int width_class(int n) { return n > 64 ? 0 : n > 32 ? 1 : n > 16 ? 2 : 3; }
+__device__ __forceinline__ int width_shift(int k) { return k <= 0 ? 0 : 16 + 12 * k; }    // k: classes below the full tiles'
+__device__ __forceinline__ int width_count(uint64_t counts, int k) { return (int)(counts >> width_shift(k)) & (k <= 0 ? (1 << 28) - 1 : 0xFFF); }
 __global__ void __launch_bounds__(256) build_tiles_kernel(const int32_t* offsets, const int32_t* perm, int32_t* tiles, int32_t* list, int E, int T,
                                                           int has_shared, int gemm_min, int shared_32, int widest) {
     __shared__ uint64_t scan[8];
@@ -1261,7 +1263,8 @@ __global__ void __launch_bounds__(256) build_tiles_kernel(const int32_t* offsets
     }
     const int full = widest, fshift = widest == 128 ? 7 : 6, kf = 7 - fshift;   // columns of a full tile, their width's place in the list
     const int nf = cnt >> fshift, rem = cnt & (full - 1);
-    const uint64_t own = width_bit(full, (uint64_t)nf) + (rem ? width_bit(rem, 1) : 0ull);
+    auto one = [&](int n) { return 1ull << width_shift(width_class(n) - kf); };
+    const uint64_t own = (uint64_t)nf + (rem ? one(rem) : 0ull);
     uint64_t incl = own;
 #pragma unroll
     for (int s = 1; s < 32; s <<= 1) {
@@ -1275,27 +1278,26 @@ __global__ void __launch_bounds__(256) build_tiles_kernel(const int32_t* offsets
     // the shared expert's tiles: 128 columns and a rest, or (shared_32) tiles of 32 that are not on the list, their columns behind all
     // others'
     const int sh_full = has_shared && !shared_32 ? T >> fshift : 0, sh_rem = has_shared && !shared_32 ? T & (full - 1) : 0;
-    const uint64_t shared = width_bit(full, (uint64_t)sh_full) + (sh_rem ? width_bit(sh_rem, 1) : 0ull);
+    const uint64_t shared = (uint64_t)sh_full + (sh_rem ? one(sh_rem) : 0ull);
     total += shared;
     before += shared;   // the shared expert's tiles lead every width
     int first[5], col16[5];   // first tile and first column / 16 of each width
     first[0] = 0; col16[0] = 0;
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-        const int n = (int)((total >> (16 * k)) & 0xFFFFu);
+        const int n = k < kf ? 0 : width_count(total, k - kf);
         first[k + 1] = first[k] + n;
         col16[k + 1] = col16[k] + n * (8 >> k);
     }
     int4* tv = reinterpret_cast<int4*>(tiles + kTileHeader);
     auto put = [&](int k, int i, int expert, int start, int n) { tv[first[k] + i] = make_int4(expert, start, n, col16[k] + i * (8 >> k)); };
-    auto width_of = [](int n) { return n > 64 ? 0 : n > 32 ? 1 : n > 16 ? 2 : 3; };
     for (int i = tid; i < sh_full; i += 256) put(kf, i, -1, i * full, full);
-    if (tid == 0 && sh_rem) put(width_of(sh_rem), width_of(sh_rem) == kf ? sh_full : 0, -1, sh_full * full, sh_rem);
-    const int f0 = (int)((before >> (16 * kf)) & 0xFFFFu);
+    if (tid == 0 && sh_rem) put(width_class(sh_rem), width_class(sh_rem) == kf ? sh_full : 0, -1, sh_full * full, sh_rem);
+    const int f0 = width_count(before, 0);
     for (int i = 0; i < nf; ++i) put(kf, f0 + i, tid, off + i * full, full);
     if (rem) {
-        const int k = width_of(rem);
-        put(k, (int)((before >> (16 * k)) & 0xFFFFu) + (k == kf ? nf : 0), tid, off + nf * full, rem);
+        const int k = width_class(rem);
+        put(k, width_count(before, k - kf) + (k == kf ? nf : 0), tid, off + nf * full, rem);
     }
     if (tid == 0) {
         tiles[0] = first[4]; tiles[1] = col16[4]; tiles[2] = 0; tiles[3] = 0;

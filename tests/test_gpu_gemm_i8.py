@@ -98,3 +98,18 @@ def test_prefill_forward_matches_oracle_and_gemv_path(cfg, T):
         assert rel.max() <= 1e-2 and cos.min() >= 0.9999, (name, rel.max(), cos.min())
     # the two GPU paths compute the same integer block dots; only fp32 summation order differs
     assert (y - y_gemv).abs().max() <= 2e-3 * y_gemv.abs().max()
+
+
+def test_more_token_tiles_than_sixteen_bits_count():
+    """A batch of 66 thousand full token tiles: its first and last rows are those of a small batch of the same tokens."""
+    cfg = configs.scaled(configs.QWEN_Q4_0, E=8, H=256, F=64, F_s=64)
+    raw, T, n = configs.make_layer(cfg, device="cuda"), 940_000, 256
+    tiled, pw = MoeWeightsTiled(raw), MoeWeightsPrefill(raw)
+    x = configs.make_input(cfg, T, device="cuda")
+    sc, small = MoeScratch(tiled, T), MoeScratch(tiled, n)
+    y = forward_moe_prefill(tiled, pw, sc, x)
+    assert sc.status() == 0
+    for part in (slice(0, n), slice(T // 2, T // 2 + n), slice(T - n, T)):
+        want = forward_moe_prefill(tiled, pw, small, x[part].contiguous())
+        # (narrower tiles add in another order: single 8-bit steps of the intermediates)
+        assert (y[part] - want).abs().max() <= 1e-2 * want.abs().max()
