@@ -316,16 +316,18 @@ __device__ void build_dispatch(const RouteParams& p, int* smem_i, const int* s_i
     }
 }
 
-// grid = (row tiles, token tiles), 256 threads.  Thread p owns partial sum p of every output of
-// the tile: elements p, p+256, ... in ascending order, one fused multiply-add each.
-template <int TT, int TE>
+// grid = (row tiles, token tiles), 256 threads; TOKENS_X: (token tiles, row tiles), for more than the 65535 token tiles that the
+// second dimension holds.  Thread p owns partial sum p of every output of the tile: elements p, p+256, ... in ascending order, one
+// fused multiply-add each.
+template <int TT, int TE, bool TOKENS_X = false>
 __global__ void __launch_bounds__(256) route_kernel(const RouteParams p) {
     extern __shared__ __align__(16) float smem_f[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int H = p.H, E = p.E;
     const int nrows = E + (p.shexp_gate_w ? 1 : 0);
-    const int t0 = blockIdx.y * TT, r0 = blockIdx.x * TE;
-    const int n_rtiles = gridDim.x;
+    const int ttile = TOKENS_X ? blockIdx.x : blockIdx.y, rtile = TOKENS_X ? blockIdx.y : blockIdx.x;
+    const int t0 = ttile * TT, r0 = rtile * TE;
+    const int n_ttiles = TOKENS_X ? gridDim.x : gridDim.y, n_rtiles = TOKENS_X ? gridDim.y : gridDim.x;
 
     // ---- partial dot products; the router rows come from DRAM, so their loads go out first and the Q8_1 of
     //      this token tile's input rows (blocks dealt round-robin to the row tiles) runs while they are in flight ----
@@ -357,7 +359,7 @@ __global__ void __launch_bounds__(256) route_kernel(const RouteParams p) {
             if (tid == 0) griddep_launch();   // the grouped GEMV that follows may bring its CTAs in; it waits for this grid itself
             const int nbH = H >> 5;
             const int nt = min(TT, p.T - t0);
-            for (int q = blockIdx.x * 8 + warp; q < nt * nbH; q += n_rtiles * 8) {
+            for (int q = rtile * 8 + warp; q < nt * nbH; q += n_rtiles * 8) {
                 const int tt = q / nbH, b = q - tt * nbH;
                 const float xi = p.x[(size_t)(t0 + tt) * H + b * 32 + lane];
                 quantize_block_q8_1(xi, p.x_q8 + ((size_t)(t0 + tt) * nbH + b) * kQ81Bytes, lane,
@@ -401,24 +403,24 @@ __global__ void __launch_bounds__(256) route_kernel(const RouteParams p) {
     __shared__ int s_flag;
     __shared__ int s_ids[TT * kMaxTopK];
     __syncthreads();   // every thread's writes are ordered before thread 0's counter increment, which releases them
-    if (tid == 0) s_flag = (atom_add_acq_rel_gpu(&p.counters[kCtrRouteTile + blockIdx.y], 1) == n_rtiles - 1);   // ... and acquires the other CTAs'
+    if (tid == 0) s_flag = (atom_add_acq_rel_gpu(&p.counters[kCtrRouteTile + ttile], 1) == n_rtiles - 1);   // ... and acquires the other CTAs'
     __syncthreads();
     if (!s_flag) return;
-    if (tid == 0) p.counters[kCtrRouteTile + blockIdx.y] = 0;
+    if (tid == 0) p.counters[kCtrRouteTile + ttile] = 0;
     for (int a = warp; a < TT; a += 8) {
         const int t = t0 + a;
         if (t < p.T) topk_warp(p, p.router_logits + (size_t)t * E, t, lane, red + warp * 256, s_ids + a * p.top_k);
     }
 
     // ---- last token tile overall: dispatch permutation and work list ----
-    if (gridDim.y == 1) {
+    if (n_ttiles == 1) {
         // the only token tile: its ids are all in shared memory
         __syncthreads();
         build_dispatch(p, reinterpret_cast<int*>(smem_f), s_ids, 0);
         return;
     }
     __syncthreads();   // every thread's writes are ordered before thread 0's counter increment, which releases them
-    if (tid == 0) s_flag = (atom_add_acq_rel_gpu(&p.counters[kCtrRouteAll], 1) == (int)gridDim.y - 1);   // ... and acquires the other CTAs'
+    if (tid == 0) s_flag = (atom_add_acq_rel_gpu(&p.counters[kCtrRouteAll], 1) == n_ttiles - 1);   // ... and acquires the other CTAs'
     __syncthreads();
     if (!s_flag) return;
     if (tid == 0) p.counters[kCtrRouteAll] = 0;
@@ -1169,11 +1171,17 @@ cudaError_t launch_route(const RouteParams& p, cudaStream_t stream) {
         }
     } else {
         constexpr int TT = 8, TE = 8;
-        static bool attr_done[64] = {};
+        const unsigned rtiles = (nrows + TE - 1) / TE, ttiles = (p.T + TT - 1) / TT;
+        static bool attr_done[64] = {}, attr_done_x[64] = {};
+        if (ttiles > 65535) {
+            cudaError_t e = max_smem_once(route_kernel<TT, TE, true>, (int)route_smem(TT, TE), attr_done_x);
+            if (e != cudaSuccess) return e;
+            route_kernel<TT, TE, true><<<dim3(ttiles, rtiles), 256, route_smem(TT, TE), stream>>>(p);
+            return cudaGetLastError();
+        }
         cudaError_t e = max_smem_once(route_kernel<TT, TE>, (int)route_smem(TT, TE), attr_done);
         if (e != cudaSuccess) return e;
-        dim3 grid((nrows + TE - 1) / TE, (p.T + TT - 1) / TT);
-        route_kernel<TT, TE><<<grid, 256, route_smem(TT, TE), stream>>>(p);
+        route_kernel<TT, TE><<<dim3(rtiles, ttiles), 256, route_smem(TT, TE), stream>>>(p);
     }
     return cudaGetLastError();
 }

@@ -158,3 +158,18 @@ def test_outputs_on_any_float_boundary(entry, T):
         assert sc.status() == 0 and rest[:shift].abs().sum() == 0 and rest[shift + T * cfg.H:].abs().sum() == 0
         results.append(y.cpu().clone())
     assert all(torch.equal(r, results[0]) for r in results)
+
+
+# more token tiles than a grid's second dimension holds, on the simple router (one routed expert per token leaves the tiled one no scratch)
+def test_router_of_many_tokens():
+    cfg = configs.scaled(Q4, E=4, top_k=1, H=128, F=32, F_s=0)
+    tiled, T, n = MoeWeightsTiled(configs.make_layer(cfg, device="cuda")), 8 * 65535 + 13, 64
+    x = configs.make_input(cfg, T, device="cuda")
+    sc, small = MoeScratch(tiled, T), MoeScratch(tiled, n)
+    route_only(tiled, sc, x)
+    ids = sc.topk_indices(T).flatten()
+    assert sc.status() == 0
+    for part in (slice(0, n), slice(T - n, T)):
+        route_only(tiled, small, x[part].contiguous())
+        assert torch.equal(sc.router_logits(T)[part], small.router_logits(n)) and torch.equal(ids[part], small.topk_indices(n).flatten())
+    assert torch.equal(sc.perm(T).long(), torch.argsort(ids, stable=True))
