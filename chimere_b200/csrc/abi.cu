@@ -35,10 +35,11 @@ inline chimere_moe_layer routed_only(const chimere_moe_layer* w) {
 }
 
 // ... and whether that shared expert can go through the grouped GEMM (prefill-size batches): all three matrices Q4_K or Q5_K
-// (Q6_K has a scale per 16 weights, the MMA's blocks are 32 wide), rows of whole rounds of 32 blocks, gated.
+// (Q6_K has a scale per 16 weights, the MMA's blocks are 32 wide), rows of whole rounds of 32 blocks, gated, read by words.
 inline bool kshared_gemm(const chimere_moe_layer* w) {
     auto ok = [](int t) { return t == CHIMERE_TYPE_Q4_K || t == CHIMERE_TYPE_Q5_K; };
-    return kshared(w) && w->H % 1024 == 0 && w->act == CHIMERE_ACT_SWIGLU && ok(w->type_sh_gate) && ok(w->type_sh_up) && ok(w->type_sh_down);
+    return kshared(w) && w->H % 1024 == 0 && w->act == CHIMERE_ACT_SWIGLU && ok(w->type_sh_gate) && ok(w->type_sh_up) && ok(w->type_sh_down) &&
+           (((uintptr_t)w->sh_gate | (uintptr_t)w->sh_up | (uintptr_t)w->sh_down) & 3) == 0;
 }
 
 int validate_layer(const chimere_moe_layer* w) {
@@ -99,7 +100,7 @@ int prefill_dims_ok(const chimere_moe_layer* w) {
     if (w->H % 128 || w->F % rpt || w->F_s % rpt) return 0;
     return 1;
 }
-struct PrefillArena { size_t tiles, bx, b2, total; int64_t bx_col16, b2_col16; };
+struct PrefillArena { size_t tiles, bx, b2, sh_rows, total; int64_t bx_col16, b2_col16; };
 PrefillArena prefill_arena(const chimere_moe_layer* w, int T) {
     PrefillArena A{};
     const int Fmax = w->F > w->F_s ? w->F : w->F_s;
@@ -111,6 +112,9 @@ PrefillArena prefill_arena(const chimere_moe_layer* w, int T) {
     A.tiles = o; o += up256((size_t)(8 + 4 * n_tiles_max_for(w, T, kForwardTileColumns)) * 4);
     A.bx = o; o += up256((size_t)(cols * A.bx_col16));
     A.b2 = o; o += up256((size_t)(cols * A.b2_col16));
+    // a K-quant shared expert's output rows: the workspace's per-pair rows have no room for them (its layout is that of the
+    // routed experts alone, so that layers with other shared experts can use the same workspace)
+    A.sh_rows = o; o += kshared_gemm(w) ? up256((size_t)T * w->H * 4) : 0;
     A.total = o;
     return A;
 }
@@ -150,10 +154,8 @@ int list_capacity(const chimere_moe_layer* w, int T) {
     return most;
 }
 
-// extra_rows: per-pair output rows beyond the routed pairs' and the shared expert's own (a K-quant shared expert's rows on the
-// grouped GEMM; they come last, so that the rest of the layout does not depend on them)
-Layout make_layout(const chimere_moe_layer* w, int T, int extra_rows = 0) {
-    if (kshared(w)) { const chimere_moe_layer r = routed_only(w); return make_layout(&r, T, kshared_gemm(w) ? T : 0); }
+Layout make_layout(const chimere_moe_layer* w, int T) {
+    if (kshared(w)) { const chimere_moe_layer r = routed_only(w); return make_layout(&r, T); }
     Layout L{};
     const int k = w->top_k, H = w->H, E = w->E;
     const int Fmax = w->F > w->F_s ? w->F : w->F_s;
@@ -184,7 +186,7 @@ Layout make_layout(const chimere_moe_layer* w, int T, int extra_rows = 0) {
     L.inter_q = o; o += up256(pairs * Fmax);
     L.inter_d = o; o += up256(pairs * L.inter_d_stride * 4);
     L.status = o; o += 256;
-    L.pair_out = o; o += up256((pairs + extra_rows) * H * 4);
+    L.pair_out = o; o += up256(pairs * H * 4);
     L.gemm = o;
     L.gemm_bytes = forward_gemm(w, T) ? prefill_arena(w, T).total : 0;
     o += up256(L.gemm_bytes);
@@ -289,6 +291,7 @@ static int kshared_chain(const chimere_moe_layer* w, int T, float* d_y, chimere_
 static int gemm_experts(const chimere_moe_layer* w, const chimere_moe_prefill_weights* pw, int E, int T, chimere_moe_workspace* ws, cudaStream_t stream,
                         const void* d_packed = nullptr, int row_bytes = 0, bool mixed = false);
 static cudaError_t finish_tokens(const chimere_moe_layer* w, float* d_y, int T, chimere_moe_workspace* ws, cudaStream_t stream);
+static float* gemm_shared_rows(const chimere_moe_layer* w, int T, const chimere_moe_workspace* ws);
 static GemvParams gate_up_params(const chimere_moe_layer* w, int T, chimere_moe_workspace* ws, const Layout& L);
 static GemvParams down_params(const chimere_moe_layer* w, float* d_y, int T, chimere_moe_workspace* ws, const Layout& L);
 
@@ -891,6 +894,7 @@ static int gemm_experts(const chimere_moe_layer* w, const chimere_moe_prefill_we
         g.b_tiles = base + (down ? A.b2 : A.bx); g.b_col16_bytes = down ? A.b2_col16 : A.bx_col16;
         g.out_tiles = base + A.b2; g.out_col16_bytes = A.b2_col16;
         g.pair_out = ws->pair_out;
+        g.shared_out = gemm_shared_rows(w, T, ws);
         if (mixed) {   // sums as the GEMV kernels form them: a token's result does not depend on its batch
             g.inter_q8 = ws->inter_q8; g.inter_stride = (int64_t)L.inter_stride;
             g.as_gemv = 1;
@@ -903,9 +907,15 @@ static int gemm_experts(const chimere_moe_layer* w, const chimere_moe_prefill_we
     return cuda_rc(e);
 }
 
+// where the GEMM leaves the shared expert's rows
+static float* gemm_shared_rows(const chimere_moe_layer* w, int T, const chimere_moe_workspace* ws) {
+    if (kshared(w)) return (float*)((uint8_t*)ws->prefill_arena + prefill_arena(w, ws->max_T).sh_rows);
+    return ws->pair_out + (size_t)T * w->top_k * w->H;
+}
+
 // routing-weighted sum of every token's pair rows in slot order + the sigmoid-gated shared expert
 static cudaError_t finish_tokens(const chimere_moe_layer* w, float* d_y, int T, chimere_moe_workspace* ws, cudaStream_t stream) {
-    const float* shared_rows = w->F_s > 0 ? ws->pair_out + (size_t)T * w->top_k * w->H : nullptr;
+    const float* shared_rows = w->F_s > 0 ? gemm_shared_rows(w, T, ws) : nullptr;
     const float* logit = (w->F_s > 0 && w->shexp_gate_w) ? ws->sh_gate_logit : nullptr;
     return launch_ep_finish(ws->pair_out, nullptr, ws->topk_w, shared_rows, logit, d_y, T, w->H, w->top_k, stream);
 }
@@ -915,8 +925,9 @@ int chimere_b200_moe_forward_prefill(const chimere_moe_layer* w, const chimere_m
     int rc = check_call(w, d_x, d_y, T, ws, true);
     if (rc) return rc;
     if (!pw || !ws->prefill_arena) return -1;
-    // A K-quant shared expert goes through the GEMM with the routed ones where it can, else it follows as GEMVs per token.
-    const bool ks = kshared(w), gemm = ks && kshared_gemm(w) && pw->sh_gu && pw->sh_down;
+    // A K-quant shared expert goes through the GEMM with the routed ones where it can (and where the scratch was made for that: its
+    // token tiles are larger), else it follows as GEMVs per token.
+    const bool ks = kshared(w), gemm = ks && kshared_gemm(w) && pw->sh_gu && pw->sh_down && ws->prefill_bytes >= prefill_arena(w, ws->max_T).total;
     const chimere_moe_layer wr_ = ks && !gemm ? routed_only(w) : *w;
     const chimere_moe_layer* wr = &wr_;
     if (wr->layout != CHIMERE_LAYOUT_TILED32 || !prefill_dims_ok(wr)) return -2;

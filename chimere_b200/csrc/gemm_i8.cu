@@ -1035,18 +1035,18 @@ struct GateUpPolicy : MoePolicy {
 };
 
 // down: rows of H; the tile's columns are pairs, written to pair_out[pair row][H].  A warp stores the 128 rows of every fourth
-// column, four rows per lane (H is a multiple of 32).
+// column, four rows per lane (H is a multiple of 32).  The shared expert's rows have a place of their own.
 struct DownPolicy : MoePolicy {
     template <int KG, int MODE>
     __device__ static __forceinline__ void store(const PrefillGemmParams& p, const GemmWork& w, const float* xch, int ew, int lane) {
         const bool rows = w.rt * 128 + lane * 4 < p.H;
-        float* out = p.pair_out + w.rt * 128 + lane * 4;
+        float* out = (w.shared ? p.shared_out : p.pair_out) + w.rt * 128 + lane * 4;
         const float* x = xch + lane * 4;
         for (int c0 = 0; c0 < w.n_valid; c0 += 128) {
             // this lane's pair rows: of columns ew + 4 * lane
             const int cl = c0 + ew + 4 * lane;
             int prow = 0;
-            if (cl < w.n_valid) prow = w.shared ? p.T * p.top_k + w.start + cl : __ldcg(p.perm + w.start + cl);
+            if (cl < w.n_valid) prow = w.shared ? w.start + cl : __ldcg(p.perm + w.start + cl);
             const int n = min(32, (w.n_valid - c0 - ew + 3) >> 2);
 #pragma unroll 4
             for (int i = 0; i < n; ++i) {

@@ -162,6 +162,7 @@ struct PrefillGemmParams {
     const uint8_t* b_tiles; int64_t b_col16_bytes;   // token tiles (input); bytes of 16 columns over all of K
     uint8_t* out_tiles; int64_t out_col16_bytes;     // gate/up: token tiles of the down GEMM (output)
     float* pair_out;                                 // down: per-pair rows [pairs][H]
+    float* shared_out;                               // ... and the shared expert's [T][H]
     int row_tiles_max;
     int dual, T, top_k, H;
     uint8_t* inter_q8; int64_t inter_stride;   // gate/up: Q8_1 rows of the intermediates as the GEMV kernels leave them (null = not wanted)

@@ -113,3 +113,23 @@ def test_more_token_tiles_than_sixteen_bits_count():
         want = forward_moe_prefill(tiled, pw, small, x[part].contiguous())
         # (narrower tiles add in another order: single 8-bit steps of the intermediates)
         assert (y[part] - want).abs().max() <= 1e-2 * want.abs().max()
+
+
+def test_layers_with_different_shared_experts_share_a_workspace():
+    """Scratch made for a layer whose K-quant shared expert stays on the GEMV kernels serves one whose shared expert could go through
+    the GEMM, and the other way round; in the first case the GEMM's larger token tiles do not fit and the GEMVs are taken."""
+    from chimere_b200 import formats
+    base = configs.scaled(configs.QWEN_IQ3S, E=8, top_k=2, H=1024, F=256, F_s=512)
+    layers = [configs.scaled(base, type_sh_gate_up=formats.TYPE_Q5_K, type_sh_down=t, seed=s) for s, t in enumerate((formats.TYPE_Q6_K, formats.TYPE_Q5_K))]
+    T = 96
+    raws = [configs.make_layer(c, device="cuda") for c in layers]
+    tiled, pws = [MoeWeightsTiled(r) for r in raws], [MoeWeightsPrefill(r) for r in raws]
+    x = configs.make_input(base, T, device="cuda")
+    want = [oracle.moe_forward(r.to("cpu"), x.cpu().numpy(), taps=False)["y"] for r in raws]
+    for made_for in (0, 1):
+        sc = MoeScratch(tiled[made_for], T)
+        sc.enable_prefill()
+        for i in (0, 1, 0):
+            y = forward_moe_prefill(tiled[i], pws[i], sc, x).cpu().numpy()
+            assert sc.status() == 0
+            assert np.abs(y - want[i]).max() <= 1e-2 * np.abs(want[i]).max()
