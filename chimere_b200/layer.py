@@ -177,6 +177,9 @@ class MoeScratch:
         n = lib.chimere_b200_moe_prefill_bytes(C.byref(self.w.as_struct()), self.max_T)
         if n == 0:
             raise RuntimeError("chimere_b200_moe_prefill_bytes rejected the layer")
+        if self.ws.prefill_arena and self.ws.prefill_bytes >= n:   # the workspace holds such scratch already (4-bit layers, more than a few dozen tokens)
+            self.prefill = self._view(self.ws.prefill_arena, n)
+            return
         self.prefill = torch.zeros(n, dtype=torch.uint8, device=self.device)
         self.ws.prefill_arena, self.ws.prefill_bytes = self.prefill.data_ptr(), n
 

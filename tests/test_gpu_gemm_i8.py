@@ -133,3 +133,11 @@ def test_layers_with_different_shared_experts_share_a_workspace():
             y = forward_moe_prefill(tiled[i], pws[i], sc, x).cpu().numpy()
             assert sc.status() == 0
             assert np.abs(y - want[i]).max() <= 1e-2 * np.abs(want[i]).max()
+
+
+def test_prefill_scratch_is_the_workspaces_own_where_it_has_some():
+    cfg = configs.scaled(configs.QWEN_Q4_0, E=8, top_k=2, H=512, F=256, F_s=256)
+    sc = MoeScratch(MoeWeightsTiled(configs.make_layer(cfg, device="cuda")), 64)
+    before = torch.cuda.memory_allocated()
+    sc.enable_prefill()
+    assert torch.cuda.memory_allocated() == before and sc.prefill.data_ptr() == sc.ws.prefill_arena
