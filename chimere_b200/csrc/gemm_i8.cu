@@ -124,7 +124,8 @@ constexpr uint32_t kSumScaleBits = 0x58000000u;      // 2^49
 
 struct GemmShared {
     uint64_t full1[kG_RingSlotsSlim];                // ring 1: a stage's bytes have landed (kTypeOperand: those of ring 2 as well)
-    uint64_t empty1[kG_RingSlotsSlim];               // ... the stage has been read back, and both its slots are free
+    uint64_t empty1[kG_RingSlotsSlim];               // ... the stage has been read back, and both its slots are free: one arrival of every
+                                                     // read-back warp, whatever its part in the tile
     uint64_t xfull2[kG_ASlots];                      // ring 2: operand and scales expanded
     uint64_t tfull[kG_TmemSlots], tempty[kG_TmemSlots];   // accumulators of a slot complete / read back (tempty: wide tiles only)
     uint64_t sfull[kG_Sched], sempty[kG_Sched];      // a tile index has been published / taken by every other warp
@@ -168,6 +169,9 @@ struct RingPos {
         e = e + 1 == kG_ASlots ? 0 : e + 1;
     }
 };
+// (All waits are on parities.  Who waits on a barrier has to be someone without whom it cannot go two phases on: a stage is released by
+// all 16 read-back warps, each of which has seen its accumulators complete or has expanded it; MMA and expander warps are held by what they
+// feed; warps 2..3, which sit out some tiles, come back to drained rings.)
 // TMEM slots of a tile of npad columns (512 columns in all): two blocks per slot in a 128-column tile, else a whole stage.
 struct TmemPos {
     int slot = 0, npad = 0, nslots = 0;
@@ -287,6 +291,10 @@ __device__ __forceinline__ uint32_t iq3s_word(uint32_t d16, uint32_t sub) {
 }
 __device__ __forceinline__ void sts_u32(uint32_t a, uint32_t v) { asm volatile("st.shared.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory"); }
 
+// Whether warps 2..3 expand a tile's weights: not those in operand order, and in slim tiles half of the read-back warps do it.
+template <int MODE>
+__device__ __forceinline__ bool warps23_expand(int type, bool slim) { return (MODE == kOrdered || type < kTypeOperand) && !slim; }
+
 // Warps 2..3: warp x takes row tiles x and x + 2 of every stage.
 template <class Policy, int MODE, class Params>
 __device__ __forceinline__ bool expand_tile(const Params& p, const GemmWork& w, GemmShared& sh, uint32_t ring1, uint32_t ring2, RingPos& pos, int x, int lane) {
@@ -294,12 +302,8 @@ __device__ __forceinline__ bool expand_tile(const Params& p, const GemmWork& w, 
     const bool slim = uniform(w.npad) <= 32;
     pos.geometry(slim);
     const int nstages = (nb + kG_StageUnits - 1) / kG_StageUnits;
-    if ((MODE != kOrdered && type >= kTypeOperand) || slim) {   // nothing to do (slim tiles: half of the read-back warps expand) but keep step:
-        // parity tells a barrier's phases apart only while nobody is two behind, so every stage is seen to arrive
-        for (int s = 0; s < nstages; ++s) {
-            if (!mbar_wait(&sh.full1[pos.r], pos.par1())) { gemm_timeout(sh, p.status, lane); return false; }
-            pos.next(MODE == kOrdered || type < kTypeOperand);
-        }
+    if (!warps23_expand<MODE>(type, slim)) {   // nothing to do but keep step; no waits: nothing holds the rings back for these warps here
+        for (int s = 0; s < nstages; ++s) pos.next(MODE == kOrdered || type < kTypeOperand);
         return true;
     }
     uint32_t d3[2] = {0u, 0u}, sc3[2] = {0u, 0u};   // IQ3_S: this lane's rows' scales of the super-block, kept over its two stages
@@ -442,10 +446,9 @@ __device__ __forceinline__ bool readback_tile(GemmShared& sh, uint32_t ring1, ui
     int share = 0;
     for (int b0 = 0; b0 < nb; b0 += kG_StageUnits) {
         const int nu = min(kG_StageUnits, nb - b0);
-        if (KG > 1 && share != kg) {   // another share's stage: keep step
-            // a barrier's phases are told apart by parity, so nobody may be a whole round of slots ahead: everyone waits for
-            // a tile's last stage (the stages between are never further behind than a warp's own last one)
-            if (nu == nb - b0 && !mbar_wait(&sh.tfull[tp.slot], tp.par())) { gemm_timeout(sh, status, lane); return false; }
+        if (KG > 1 && share != kg) {   // another share's stage: seen and released like its own, so that no warp is ever two phases behind a barrier
+            if (!mbar_wait(&sh.tfull[tp.slot], tp.par())) { gemm_timeout(sh, status, lane); return false; }
+            if (kHandshake && lane == 0) mbar_arrive_cta(&sh.tempty[tp.slot]);
             tp.next();
         } else {
             const uint32_t rec = rec0 + (uint32_t)pos.e * kG_ASlot, sb = sb0 + pos.slot1_off();
@@ -466,7 +469,7 @@ __device__ __forceinline__ bool readback_tile(GemmShared& sh, uint32_t ring1, ui
                         if (kHandshake && i + 1 == cnt) {   // the slot's last values are in registers: the MMAs may overwrite it
                             tc_fence_before();
                             __syncwarp();
-                            if (lane == 0) mbar_arrive_n(&sh.tempty[tp.slot], 4 / COLG);
+                            if (lane == 0) mbar_arrive_cta(&sh.tempty[tp.slot]);
                         }
                         block_values<W, kPad == 128 ? 0u : 1u << 19, ANY_SCALE>(v, sa, sb + (uint32_t)((j0 + i) * (kPad * 36)), acc2);
                     }
@@ -475,8 +478,8 @@ __device__ __forceinline__ bool readback_tile(GemmShared& sh, uint32_t ring1, ui
             }
             if (!kHandshake) tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive_n(&sh.empty1[pos.r], 4 / COLG);   // 4 * COLG warps per stage, 16 arrivals
         }
+        if (lane == 0) mbar_arrive_cta(&sh.empty1[pos.r]);
         if (KG > 1) share = share + 1 == KG ? 0 : share + 1;
         pos.next(expanded);
     }
@@ -526,7 +529,7 @@ __device__ __forceinline__ bool readback_ordered(GemmShared& sh, uint32_t ring1,
             if (kHandshake && j + 1 == nu) {   // the slot's last values are in registers: the MMAs may overwrite it
                 tc_fence_before();
                 __syncwarp();
-                if (lane == 0) mbar_arrive_n(&sh.tempty[tp.slot], 4 / COLG);
+                if (lane == 0) mbar_arrive_cta(&sh.tempty[tp.slot]);
             }
 #pragma unroll
             for (int g = 0; g < W / 4; ++g) {
@@ -543,7 +546,7 @@ __device__ __forceinline__ bool readback_ordered(GemmShared& sh, uint32_t ring1,
         tp.next();
         if (!kHandshake) tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive_n(&sh.empty1[pos.r], 4 / COLG);   // 4 * COLG warps per stage, 16 arrivals
+        if (lane == 0) mbar_arrive_cta(&sh.empty1[pos.r]);
         pos.next(true);
         if (kGroup) {
             const float d = h2f(word >> 16);
@@ -712,8 +715,10 @@ __device__ __forceinline__ bool expand_slim(const Params& p, const GemmWork& w, 
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the MMAs read what ordinary stores wrote
         __syncwarp();
         if (lane == 0) mbar_arrive_cta(&sh.xfull2[pos.e]);
-        // (as in readback_tile: see the tile's last stage complete before going on)
-        if (s + 1 == nstages && !mbar_wait(&sh.tfull[tp.slot], tp.par())) ok = false;
+        // a stage is released by all of the read-back warps, and a tile's last one only when these have seen its accumulators complete: the
+        // next tile may use the TMEM slots without them
+        if (s + 1 == nstages && !mbar_wait(&sh.tfull[tp.slot], tp.par())) { ok = false; break; }
+        if (lane == 0) mbar_arrive_cta(&sh.empty1[pos.r]);
         tp.next();
         pos.next(true);
     }
@@ -835,6 +840,7 @@ __global__ void __launch_bounds__(kG_Threads, 1) gemm_i8_kernel(const Params p, 
         bool ok = true;
         if (warp == 0) {
             // ------------------------------ tile scheduler + operand producer ------------------------------
+            bool skipped = false;   // warps 2..3 sat out the tile before
             while (ok) {
                 GemmWork w;
                 int idx = 0, ws;
@@ -843,6 +849,16 @@ __global__ void __launch_bounds__(kG_Threads, 1) gemm_i8_kernel(const Params p, 
                     idx = __shfl_sync(0xffffffffu, idx, 0);
                     ws = Policy::template work<MODE>(p, idx, w);
                 } while (ws == kWorkSkip);
+                if (ws == kWorkOk) {
+                    // Parity tells a barrier's phases apart only for those who are at most one behind, and warps 2..3 saw nothing of the tiles
+                    // that they sat out: they learn of a tile of theirs when every stage before it has been read back.
+                    const bool expand = warps23_expand<MODE>(uniform(Policy::type(p, w)), uniform(w.npad) <= 32);
+                    if (expand && skipped)
+                        for (int r = 0; r < pos.slots1() && ok; ++r)
+                            if (!mbar_wait(&sh.empty1[r], pos.released(r))) { gemm_timeout(sh, p.status, lane); ok = false; }
+                    if (!ok) break;
+                    skipped = !expand;
+                }
                 const int slot = (int)(tn % kG_Sched);
                 if (!mbar_wait(&sh.sempty[slot], ((tn / kG_Sched) & 1u) ^ 1u)) { gemm_timeout(sh, p.status, lane); ok = false; break; }
                 if (lane == 0) {

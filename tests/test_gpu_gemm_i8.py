@@ -141,3 +141,20 @@ def test_prefill_scratch_is_the_workspaces_own_where_it_has_some():
     before = torch.cuda.memory_allocated()
     sc.enable_prefill()
     assert torch.cuda.memory_allocated() == before and sc.prefill.data_ptr() == sc.ws.prefill_arena
+
+
+@pytest.mark.parametrize("cfg,T", [(configs.scaled(configs.QWEN_Q4_0, E=8, top_k=2, H=4096, F=1536, F_s=0), 8),      # tiles of 16 columns, 32 / 12 stages
+                                   (configs.scaled(configs.QWEN_Q4_0, E=64, H=128, F=128, F_s=128), 64),              # tiles of one stage
+                                   (configs.scaled(configs.QWEN_Q8_0, E=32, H=256, F=256, F_s=256, zipf_bias=False), 250),   # 64 columns in operand order
+                                   (configs.scaled(configs.QWEN_Q4_0, E=8, top_k=2, H=512, F=512, F_s=512, type_sh_gate_up=configs.Q8_0, type_sh_down=configs.Q8_0), 700)],
+                         ids=["narrow", "one stage", "operand order", "both forms"])
+def test_call_after_call(cfg, T):
+    """The GEMM's warps take different parts in tiles of different forms and widths; many short calls, every one the same bits."""
+    raw = configs.make_layer(cfg, device="cuda")
+    tiled, pw = MoeWeightsTiled(raw), MoeWeightsPrefill(raw)
+    x, sc = configs.make_input(cfg, T, device="cuda"), MoeScratch(tiled, T)
+    first = forward_moe_prefill(tiled, pw, sc, x).clone()
+    y, different = torch.empty_like(first), torch.zeros((), dtype=torch.int64, device="cuda")
+    for _ in range(300):
+        different += (forward_moe_prefill(tiled, pw, sc, x, y) != first).sum()
+    assert sc.status() == 0 and int(different) == 0
