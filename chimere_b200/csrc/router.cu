@@ -1155,7 +1155,10 @@ static cudaError_t launch_route_tiles(const RouteParams& p, cudaStream_t stream)
 
 cudaError_t launch_route(const RouteParams& p, cudaStream_t stream) {
     const int nrows = p.E + (p.shexp_gate_w ? 1 : 0);
-    if (p.T <= 32 && nrows <= sm_count()) {   // few experts: a row per CTA, up to 3072 columns in flight at once
+    const int ttiles8 = (p.T + 7) / 8;
+    // few experts: a row per CTA, up to 3072 columns in flight at once, as long as that is one CTA per SM (64 experts of H = 2048, 8 tokens
+    // 9.6 -> 9.1 us, but 24 tokens 10.9 -> 11.7); a single row of 2048 is faster in pairs of outputs (6.9 against 7.3)
+    if (p.T <= 32 && nrows * ttiles8 <= sm_count() && (p.T > 1 || p.H > 2048)) {
         constexpr int TT = 8, TE = 1;
         return launch_pdl(route_kernel<TT, TE>, dim3(nrows, (p.T + TT - 1) / TT), 256, route_smem(TT, TE), stream, p);
     } else if (p.T <= 32) {

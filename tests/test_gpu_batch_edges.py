@@ -160,6 +160,13 @@ def test_outputs_on_any_float_boundary(entry, T):
     assert all(torch.equal(r, results[0]) for r in results)
 
 
+# one or two router rows per CTA: around one CTA per SM, around the row width that takes one row of inputs in pairs
+@pytest.mark.parametrize("E,T", [(73, 9), (74, 9), (147, 8), (148, 8), (36, 32), (37, 32), (8, 1)])
+@pytest.mark.parametrize("H", [2048, 2176])
+def test_small_router(E, T, H):
+    _check(configs.scaled(Q4, E=E, H=H, F=64, F_s=64), T, prefill=False)
+
+
 # more token tiles than a grid's second dimension holds, on the simple router (one routed expert per token leaves the tiled one no scratch)
 def test_router_of_many_tokens():
     cfg = configs.scaled(Q4, E=4, top_k=1, H=128, F=32, F_s=0)
