@@ -120,11 +120,17 @@ PrefillArena prefill_arena(const chimere_moe_layer* w, int T) {
 }
 // Whether the decode entry may take the grouped GEMM for T tokens of a layer (w without a K-quant shared expert): weights it
 // reads in the tiled32 form, and enough tokens.
-bool forward_gemm(const chimere_moe_layer* w, int T) {
-    if (T < forward_gemm_tokens(w) || w->layout != CHIMERE_LAYOUT_TILED32 || !prefill_dims_ok(w)) return false;
+bool packed_types(const chimere_moe_layer* w) {
     auto ok = [](int t) { return t == CHIMERE_TYPE_Q4_0 || t == CHIMERE_TYPE_IQ3_S; };
     return ok(w->type_up) && ok(w->type_down) && (w->F_s == 0 || (ok(w->type_sh_up) && ok(w->type_sh_down)));
 }
+bool forward_gemm(const chimere_moe_layer* w, int T) {
+    return T >= forward_gemm_tokens(w) && w->layout == CHIMERE_LAYOUT_TILED32 && prefill_dims_ok(w) && packed_types(w);
+}
+// Whether a batch is too small for the prefill entry's GEMM: tiles of mostly one pair.  256 IQ3_S experts of 512 x 2048, 16 tokens: uniform
+// routing 115 us on the GEMM, 57 as decode (103 when the prefill entry left experts of fewer than eight pairs to the GEMV kernels), skewed
+// routing 47 and 53; eight experts, one token 43 and 26.  Q8_0 weights, whose GEMV entries fill an SM each, are the faster on the GEMM at one token.
+bool prefill_as_decode(const chimere_moe_layer* w, int T) { return 2 * (int64_t)T * w->top_k <= w->E && packed_types(w); }
 
 struct Layout {
     size_t topk_idx, topk_w, logits, sh_logit, x_q8, perm, offsets, group_list, counters, inter_q8, pair_out, status, total;
@@ -932,6 +938,8 @@ int chimere_b200_moe_forward_prefill(const chimere_moe_layer* w, const chimere_m
     const chimere_moe_layer* wr = &wr_;
     if (wr->layout != CHIMERE_LAYOUT_TILED32 || !prefill_dims_ok(wr)) return -2;
     const chimere_moe_layer route_ = ks ? routed_only(w) : *w;
+    if (ws->prefill_bytes < prefill_arena(wr, ws->max_T).total || ((uintptr_t)ws->prefill_arena & 255)) return -4;
+    if (prefill_as_decode(&route_, T)) return chimere_b200_moe_forward(w, d_x, d_y, T, ws, stream);
     RouteParams rp = route_params(&route_, d_x, T, ws, ks);
     rp.list_mode = 2;   // no work entries: the tile builder makes its own list
     cudaError_t e = launch_route(rp, stream);

@@ -160,6 +160,15 @@ def test_outputs_on_any_float_boundary(entry, T):
     assert all(torch.equal(r, results[0]) for r in results)
 
 
+# the prefill entry with fewer pairs than half the experts, and with one token more
+@pytest.mark.parametrize("cfg", [configs.scaled(IQ3, E=32, H=512, F=256, F_s=256), configs.scaled(Q8, E=32, H=512, F=64, F_s=64),
+                                 configs.scaled(IQ3, E=32, H=1024, F=256, F_s=512, type_sh_gate_up=formats.TYPE_Q5_K, type_sh_down=formats.TYPE_Q5_K, name="q5k")],
+                         ids=lambda c: c.name)
+@pytest.mark.parametrize("T", [1, 2, 3])
+def test_prefill_entry_of_a_few_tokens(cfg, T):
+    _check(cfg, T, prefill=True)
+
+
 # one or two router rows per CTA: around one CTA per SM, around the row width that takes one row of inputs in pairs
 @pytest.mark.parametrize("E,T", [(73, 9), (74, 9), (147, 8), (148, 8), (36, 32), (37, 32), (8, 1)])
 @pytest.mark.parametrize("H", [2048, 2176])
