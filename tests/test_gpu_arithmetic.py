@@ -1,9 +1,10 @@
-"""The device helpers that stand in for division, against the division operator and roundf on the same GPU, bit for bit.  The
-helpers are compiled from the library's own header."""
+"""Device helpers of the library's own header, compiled into kernels of their own: those that stand in for division against the division
+operator and roundf on the same GPU, bit for bit, and the bounded wait."""
 import ctypes as C
 import os
 import shutil
 import subprocess
+import time
 
 import pytest
 import torch
@@ -57,6 +58,14 @@ __global__ void q8_kernel(unsigned long long* bad) {
     }
 }
 extern "C" int q8_check(unsigned long long* bad) { q8_kernel<<<1184, 256>>>(bad); return (int)cudaDeviceSynchronize(); }
+// a wait on a barrier that nobody arrives at: comes back with false
+__global__ void wait_kernel(unsigned long long* bad) {
+    __shared__ __align__(8) uint64_t bar;
+    if (threadIdx.x == 0) { mbar_init(&bar, 1); mbar_fence_init(); }
+    __syncthreads();
+    if (mbar_wait(&bar, 0)) atomicAdd(bad, 1ull);
+}
+extern "C" int wait_check(unsigned long long* bad) { wait_kernel<<<1, 32>>>(bad); return (int)cudaDeviceSynchronize(); }
 extern "C" int silu_check(unsigned long long* bad) { silu_kernel<<<1184, 256>>>(bad); return (int)cudaDeviceSynchronize(); }
 """
 
@@ -104,3 +113,10 @@ def test_routers_and_operator_quantise_alike(T):
     want = torch.zeros(T, 512 // 32 * 36, dtype=torch.uint8, device="cuda")
     abi.load().chimere_quantize_q8_1_batched(x.data_ptr(), want.data_ptr(), 512, 512, T, torch.cuda.current_stream().cuda_stream)
     assert torch.equal(sc.x_q8(T), want)
+
+
+def test_a_wait_that_nobody_ends_gives_up_within_seconds(lib):
+    torch.cuda.synchronize()
+    start = time.monotonic()
+    assert _mismatches(lib.wait_check) == 0
+    assert time.monotonic() - start < 5.0
