@@ -185,10 +185,8 @@ __host__ __device__ constexpr int blocks_per_slot(int npad) { return npad == 128
 __device__ __forceinline__ void mbar_arrive_n(uint64_t* bar, uint32_t n) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(n) : "memory");
 }
-__device__ __forceinline__ void gemm_timeout(GemmShared& sh, int32_t* status, int lane) {
-    if (lane == 0 && status) atomicOr(status, kStatusWaitTimeout);
-    sh.failed = 1;
-}
+// A wait ran out: noted here, reported by the CTA's last step.
+__device__ __forceinline__ void gemm_timeout(GemmShared& sh) { sh.failed = 1; }
 
 // ------------------------------------------------------------------ roles ----
 // First unit of stage s.  IQ3_S tiles keep a super-block's scales behind its eight units, so its second half is taken first
@@ -205,7 +203,7 @@ __device__ __forceinline__ bool produce_tile(const Params& p, const GemmWork& w,
     const int slim = npad <= 32;
     if (slim != pos.slim) {   // the other slot geometry: every slot of the old one has to be empty first
         for (int r = 0; r < pos.slots1(); ++r)
-            if (!mbar_wait(&sh.empty1[r], pos.released(r))) { gemm_timeout(sh, p.status, lane); return false; }
+            if (!mbar_wait(&sh.empty1[r], pos.released(r))) { gemm_timeout(sh); return false; }
         pos.geometry(slim);
     }
     // four row tiles: two at src0, two at src1 (neighbours tile_bytes apart), n0 and n1 of them there
@@ -220,7 +218,7 @@ __device__ __forceinline__ bool produce_tile(const Params& p, const GemmWork& w,
         uint64_t* bar = &sh.full1[pos.r];
         bool ok = mbar_wait(&sh.empty1[pos.r], pos.released(pos.r));
         if (ok && operand) ok = mbar_wait(&sh.empty1[pos.lag()], pos.released(pos.lag()));
-        if (!ok) { gemm_timeout(sh, p.status, lane); return false; }
+        if (!ok) { gemm_timeout(sh); return false; }
         uint8_t* raw = ring1 + pos.slot1_off();
         // a token block: 32 values and a scale per column, beside weights with minimums the column's sum as well (by stages)
         const uint32_t bcol = type == kTypeOperandMin ? 40u : 36u, bbytes = (uint32_t)(nu * npad) * bcol;
@@ -309,7 +307,7 @@ __device__ __forceinline__ bool expand_tile(const Params& p, const GemmWork& w, 
     uint32_t d3[2] = {0u, 0u}, sc3[2] = {0u, 0u};   // IQ3_S: this lane's rows' scales of the super-block, kept over its two stages
     for (int s = 0; s < nstages; ++s) {
         const int u0 = stage_unit<MODE>(type, s);
-        if (!mbar_wait(&sh.full1[pos.r], pos.par1()) || !mbar_wait(&sh.empty1[pos.lag()], pos.released(pos.lag()))) { gemm_timeout(sh, p.status, lane); return false; }
+        if (!mbar_wait(&sh.full1[pos.r], pos.par1()) || !mbar_wait(&sh.empty1[pos.lag()], pos.released(pos.lag()))) { gemm_timeout(sh); return false; }
         const uint32_t raw = ring1 + pos.slot1_off(), a = ring2 + (uint32_t)pos.e * kG_ASlot;
         const uint32_t rec = a + 4096 + (x * 32 + lane) * 4;   // [unit] kG_MmaTile apart, row tile x + 2: 256 bytes further
         if (type == CHIMERE_TYPE_Q4_0) {
@@ -356,7 +354,7 @@ __device__ __forceinline__ bool mma_tile(const Params& p, const GemmWork& w, Gem
     const int nb = uniform(w.nb);
     if (NPAD != tp.npad) {   // another width lays the accumulators out differently: everything has to be read back first
         for (int r = 0; r < pos.slots1(); ++r)
-            if (!mbar_wait(&sh.empty1[r], pos.released(r))) { gemm_timeout(sh, p.status, lane); return false; }
+            if (!mbar_wait(&sh.empty1[r], pos.released(r))) { gemm_timeout(sh); return false; }
         tp.npad = NPAD; tp.slot = 0; tp.nslots = kG_TmemCols / (kBps * NPAD);
     }
     pos.geometry(NPAD <= 32);
@@ -369,13 +367,13 @@ __device__ __forceinline__ bool mma_tile(const Params& p, const GemmWork& w, Gem
     };
     for (int b0 = 0; b0 < nb; b0 += kG_StageUnits) {
         const int nu = min(kG_StageUnits, nb - b0);
-        if (!(expanded ? mbar_wait(&sh.xfull2[pos.e], pos.par2()) : mbar_wait(&sh.full1[pos.r], pos.par1()))) { gemm_timeout(sh, p.status, lane); return false; }
+        if (!(expanded ? mbar_wait(&sh.xfull2[pos.e], pos.par2()) : mbar_wait(&sh.full1[pos.r], pos.par1()))) { gemm_timeout(sh); return false; }
         const uint64_t a = a_base + (uint32_t)pos.e * (kG_ASlot >> 4), b = b_base + (pos.slot1_off() >> 4);
 #pragma unroll
         for (int j0 = 0; j0 < kG_StageUnits; j0 += kBps) {
             if (j0 >= nu) break;
             if (kHandshake) {
-                if (!mbar_wait(&sh.tempty[tp.slot], ((tp.ph_empty >> tp.slot) & 1u) ^ 1u)) { gemm_timeout(sh, p.status, lane); return false; }
+                if (!mbar_wait(&sh.tempty[tp.slot], ((tp.ph_empty >> tp.slot) & 1u) ^ 1u)) { gemm_timeout(sh); return false; }
                 tp.ph_empty ^= 1u << tp.slot;
             }
             tc_fence_after();
@@ -447,7 +445,7 @@ __device__ __forceinline__ bool readback_tile(GemmShared& sh, uint32_t ring1, ui
     for (int b0 = 0; b0 < nb; b0 += kG_StageUnits) {
         const int nu = min(kG_StageUnits, nb - b0);
         if (KG > 1 && share != kg) {   // another share's stage: seen and released like its own, so that no warp is ever two phases behind a barrier
-            if (!mbar_wait(&sh.tfull[tp.slot], tp.par())) { gemm_timeout(sh, status, lane); return false; }
+            if (!mbar_wait(&sh.tfull[tp.slot], tp.par())) { gemm_timeout(sh); return false; }
             if (kHandshake && lane == 0) mbar_arrive_cta(&sh.tempty[tp.slot]);
             tp.next();
         } else {
@@ -455,7 +453,7 @@ __device__ __forceinline__ bool readback_tile(GemmShared& sh, uint32_t ring1, ui
 #pragma unroll
             for (int j0 = 0; j0 < kG_StageUnits; j0 += kBps) {
                 if (j0 >= nu) break;
-                if (!mbar_wait(&sh.tfull[tp.slot], tp.par())) { gemm_timeout(sh, status, lane); return false; }
+                if (!mbar_wait(&sh.tfull[tp.slot], tp.par())) { gemm_timeout(sh); return false; }
                 tc_fence_after();
                 const uint32_t t0 = trow + (uint32_t)(tp.slot * (kBps * kPad));
                 const int cnt = min(kBps, nu - j0);
@@ -507,7 +505,7 @@ __device__ __forceinline__ bool readback_ordered(GemmShared& sh, uint32_t ring1,
     for (int b0 = 0; b0 < nb; b0 += kG_StageUnits) {
         const int nu = min(kG_StageUnits, nb - b0);
         const uint32_t rec = rec0 + (uint32_t)pos.e * kG_ASlot, sb = sb0 + pos.slot1_off();
-        if (!mbar_wait(&sh.tfull[tp.slot], tp.par())) { gemm_timeout(sh, status, lane); return false; }
+        if (!mbar_wait(&sh.tfull[tp.slot], tp.par())) { gemm_timeout(sh); return false; }
         tc_fence_after();
         const uint32_t t0 = trow + (uint32_t)(tp.slot * (kG_StageUnits * kPad));
         uint64_t part[W / 2];
@@ -581,7 +579,7 @@ __device__ __forceinline__ void count_up(int n, uint64_t (&sum)[4], uint64_t (&s
 // A warp's sums of a tile into the exchange buffer (part = share * column groups + column group).
 template <int W, bool UNSCALED = false>
 __device__ __forceinline__ bool publish_sums(int32_t* status, GemmShared& sh, float* xch, int q, int part, int lane, uint32_t& xphase, const uint64_t* acc2, bool ok) {
-    if (!mbar_wait(&sh.xempty, (xphase & 1u) ^ 1u)) { gemm_timeout(sh, status, lane); ok = false; }   // the tile before has been stored
+    if (!mbar_wait(&sh.xempty, (xphase & 1u) ^ 1u)) { gemm_timeout(sh); ok = false; }   // the tile before has been stored
     ++xphase;
     float* mine = xch + part * (W * 128) + q * 32 + lane;
     const uint64_t sc2 = pack2(kSumScaleBits, kSumScaleBits);
@@ -647,7 +645,7 @@ __device__ __forceinline__ bool readback_min(GemmShared& sh, uint32_t ring1, uin
         if (lane == 0) mbar_arrive_cta(&sh.empty1[pos.r]);
         pos.next(false);
     }
-    if (!ok) gemm_timeout(sh, status, lane);
+    if (!ok) gemm_timeout(sh);
     return publish_sums<W>(status, sh, xch, q, part, lane, xphase, sum, ok);
 }
 
@@ -724,7 +722,7 @@ __device__ __forceinline__ bool expand_slim(const Params& p, const GemmWork& w, 
     }
     if (ok && !mbar_wait(&sh.xempty, (xphase & 1u) ^ 1u)) ok = false;
     ++xphase;
-    if (!ok) gemm_timeout(sh, p.status, lane);
+    if (!ok) gemm_timeout(sh);
     if (lane == 0) mbar_arrive_cta(&sh.xfull);   // nothing of this warp's to store
     return ok;
 }
@@ -734,7 +732,7 @@ template <class Policy, int MODE, class Params>
 __device__ __forceinline__ bool store_tile(const Params& p, const GemmWork& w, GemmShared& sh, const float* xch, int ew, int lane, uint32_t& xphase) {
     const bool ok = mbar_wait(&sh.xfull, xphase & 1u);
     ++xphase;
-    if (!ok) { gemm_timeout(sh, p.status, lane); return false; }
+    if (!ok) { gemm_timeout(sh); return false; }
     if (MODE != kPlain || w.npad == 128) Policy::template store<1, MODE>(p, w, xch, ew, lane);
     else if (w.npad == 64 || Policy::type(p, w) < kTypeOperand) Policy::template store<2, kPlain>(p, w, xch, ew, lane);
     else Policy::template store<4, kPlain>(p, w, xch, ew, lane);
@@ -746,7 +744,7 @@ __device__ __forceinline__ bool store_tile(const Params& p, const GemmWork& w, G
 // The next tile of the schedule ring, for every warp but the scheduler's own; negative: no more (or a wait ran out).
 __device__ __forceinline__ int take_tile(GemmShared& sh, int32_t* status, uint32_t& tn, int lane) {
     const int slot = (int)(tn % kG_Sched);
-    if (!mbar_wait(&sh.sfull[slot], (tn / kG_Sched) & 1u)) { gemm_timeout(sh, status, lane); return -1; }
+    if (!mbar_wait(&sh.sfull[slot], (tn / kG_Sched) & 1u)) { gemm_timeout(sh); return -1; }
     const int idx = *reinterpret_cast<volatile int*>(&sh.sched[slot]);
     __syncwarp();
     if (lane == 0) mbar_arrive_cta(&sh.sempty[slot]);
@@ -855,12 +853,12 @@ __global__ void __launch_bounds__(kG_Threads, 1) gemm_i8_kernel(const Params p, 
                     const bool expand = warps23_expand<MODE>(uniform(Policy::type(p, w)), uniform(w.npad) <= 32);
                     if (expand && skipped)
                         for (int r = 0; r < pos.slots1() && ok; ++r)
-                            if (!mbar_wait(&sh.empty1[r], pos.released(r))) { gemm_timeout(sh, p.status, lane); ok = false; }
+                            if (!mbar_wait(&sh.empty1[r], pos.released(r))) { gemm_timeout(sh); ok = false; }
                     if (!ok) break;
                     skipped = !expand;
                 }
                 const int slot = (int)(tn % kG_Sched);
-                if (!mbar_wait(&sh.sempty[slot], ((tn / kG_Sched) & 1u) ^ 1u)) { gemm_timeout(sh, p.status, lane); ok = false; break; }
+                if (!mbar_wait(&sh.sempty[slot], ((tn / kG_Sched) & 1u) ^ 1u)) { gemm_timeout(sh); ok = false; break; }
                 if (lane == 0) {
                     sh.sched[slot] = ws == kWorkEnd ? -1 : idx;
                     mbar_arrive_cta(&sh.sfull[slot]);   // (release: the index is visible to whoever sees the arrival)
@@ -903,6 +901,7 @@ __global__ void __launch_bounds__(kG_Threads, 1) gemm_i8_kernel(const Params p, 
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kG_TmemCols) : "memory");
     }
+    if (tid == 0 && sh.failed && p.status) atomicOr(p.status, kStatusWaitTimeout);
 }
 
 // ------------------------------------------------------------------ policies ----
