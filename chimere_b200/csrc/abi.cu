@@ -903,6 +903,7 @@ static int gemm_experts(const chimere_moe_layer* w, const chimere_moe_prefill_we
         g.shared_out = gemm_shared_rows(w, T, ws);
         if (mixed) {   // sums as the GEMV kernels form them: a token's result does not depend on its batch
             g.inter_q8 = ws->inter_q8; g.inter_stride = (int64_t)L.inter_stride;
+            g.inter_q = ws->inter_q; g.inter_q_stride = L.Fmax; g.inter_d = ws->inter_d; g.inter_d_stride = L.inter_d_stride;
             g.as_gemv = 1;
             const int wk = down ? tiled_down_geom(w->type_down, w->F, w->type_sh_down, w->F_s, T).wk
                                 : tiled_gate_up_geom(w->type_up, w->type_sh_up, w->H, w->F_s > 0).wk;

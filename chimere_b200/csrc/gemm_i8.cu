@@ -1039,7 +1039,11 @@ struct GateUpPolicy : MoePolicy {
                         const int row = w.shared ? p.T * p.top_k + w.start + ci : __ldcg(p.perm + w.start + ci);
                         uint8_t* tap = p.inter_q8 + (size_t)row * p.inter_stride + (size_t)blk * kQ81Bytes;
                         reinterpret_cast<int8_t*>(tap)[4 + lane] = qv;
-                        if (lane == 0) *reinterpret_cast<__half2*>(tap) = __halves2half2(__float2half(d), sh);
+                        p.inter_q[(size_t)row * p.inter_q_stride + blk * 32 + lane] = qv;
+                        if (lane == 0) {
+                            *reinterpret_cast<__half2*>(tap) = __halves2half2(__float2half(d), sh);
+                            p.inter_d[(size_t)row * p.inter_d_stride + blk] = __half2float(__float2half(d));
+                        }
                     }
                 }
             }

@@ -166,6 +166,7 @@ struct PrefillGemmParams {
     int row_tiles_max;
     int dual, T, top_k, H;
     uint8_t* inter_q8; int64_t inter_stride;   // gate/up: Q8_1 rows of the intermediates as the GEMV kernels leave them (null = not wanted)
+    int8_t* inter_q; int64_t inter_q_stride; float* inter_d; int64_t inter_d_stride;   // ... and the same as planes
     int shared_sums;                 // gate/up: the shared expert's token tiles of the down GEMM carry block sums (kTypeOperandMin)
     int as_gemv;                     // sums bit for bit as the GEMV kernels form them (packed weights, token tiles of up to 64 columns)
     int32_t* status;

@@ -160,6 +160,24 @@ def test_outputs_on_any_float_boundary(entry, T):
     assert all(torch.equal(r, results[0]) for r in results)
 
 
+# the taps of the intermediates after a decode call: the planes hold what the Q8_1 rows hold, for every pair and the shared expert
+@pytest.mark.parametrize("cfg", [configs.scaled(IQ3, E=8, top_k=4, H=512, F=256, F_s=512), configs.scaled(configs.NEMOTRON_Q4_0, E=8, top_k=2, H=384, F=160, F_s=96)],
+                         ids=lambda c: c.name)
+@pytest.mark.parametrize("T", [8, 64])
+def test_intermediates_as_planes(cfg, T):
+    tiled = MoeWeightsTiled(configs.make_layer(cfg, device="cuda"))
+    sc = MoeScratch(tiled, T)
+    forward_moe(tiled, sc, configs.make_input(cfg, T, device="cuda"))
+    pairs, wide = T * cfg.top_k, max(cfg.F, cfg.F_s)
+    rows, stride = sc.inter_q8(T), (wide // 32 + 3) & ~3
+    q = sc._view(sc.ws.inter_q, (pairs + T) * wide).reshape(pairs + T, wide)
+    d = sc._view(sc.ws.inter_d, (pairs + T) * stride * 4).view(torch.float32).reshape(pairs + T, stride)
+    for part, width in ((slice(0, pairs), cfg.F), (slice(pairs, pairs + T), cfg.F_s)):
+        blocks = rows[part, :width // 32 * 36].reshape(-1, width // 32, 36)
+        assert torch.equal(q[part, :width].reshape(-1, width // 32, 32), blocks[..., 4:])
+        assert torch.equal(d[part, :width // 32], blocks[..., :2].contiguous().view(torch.float16)[..., 0].float())
+
+
 # the prefill entry with fewer pairs than half the experts, and with one token more
 @pytest.mark.parametrize("cfg", [configs.scaled(IQ3, E=32, H=512, F=256, F_s=256), configs.scaled(Q8, E=32, H=512, F=64, F_s=64),
                                  configs.scaled(IQ3, E=32, H=1024, F=256, F_s=512, type_sh_gate_up=formats.TYPE_Q5_K, type_sh_down=formats.TYPE_Q5_K, name="q5k")],
