@@ -3,8 +3,8 @@
 // The layer-level entries are the C++ counterpart of the reference's Rust orchestration
 // (forward_moe_cudarc_with_cache, chimere-server/src/qwen35_model/moe_ffn.rs:1081-1768, and its
 // scratch owner GgmlGpuBuffers, src/kernels/ggml_gpu.rs:292-407): they validate, lay the
-// caller's arena out, and enqueue three kernels per call.  Nothing here allocates device
-// memory or synchronises, except chimere_b200_moe_forward_host which waits for its stream.
+// caller's arena out, and enqueue three kernels per decode call (eight where the grouped GEMM takes
+// part, up to eleven in prefill).  Nothing here allocates device memory or synchronises, except chimere_b200_moe_forward_host which waits for its stream.
 #include <cstdio>
 #include <cstring>
 #include <vector>
@@ -77,8 +77,12 @@ int validate_layer(const chimere_moe_layer* w) {
 
 // From forward_gemm_tokens() tokens on the decode entry sends experts with at least kForwardGemmPairs pairs, and the shared expert,
 // to the grouped GEMM and the others to the GEMV kernels: a GEMM tile costs the same with 1 pair as with 16, a GEMV entry grows
-// with every pair.  Uniform routing over 256 experts of 512 x 2048 breaks even near 40 tokens, 128 experts of 1856 x 2688 at 17 (there
-// the GEMV kernels have no room for a third CTA per SM); skewed routing gains earlier, but the host does not know the routing.
+// with every pair.  Q4_0, us per layer, GEMV kernels alone / with the GEMM, uniform and (skewed) routing:
+//   256 experts of  512 x 2048: 32 tokens  95 / 127 (86 / 85),   40: 114 / 148 (103 / 99),  41: 168 / 151 (120 / 99)
+//   128 of 768 x 2048:          40 tokens 158 / 175,  41: 200 / 177;     128 of 1024 x 2048: 24: 152 / 149 (148 / 91),  40: 208 / 204 (194 / 116)
+//   64 of 1408 x 2048:          17 tokens 132 / 142,  24: 168 / 169;     128 of 1856 x 2688:  9: 111 / 118 (97 / 93),   17: 180 / 170 (164 / 122)
+// (From 41 tokens on the GEMV entries carry up to eight pairs.)  The best line depends on the routing, which the host does not know: at 17
+// and 41 uniform routing loses 8 % at most and skewed routing gains.  Between 1024 and 1408 columns nothing was measured.
 constexpr int kForwardGemmPairs = 3;
 int forward_gemm_tokens(const chimere_moe_layer* w) { return (int64_t)w->F * w->H > (1 << 21) ? 17 : 41; }
 static_assert(kForwardGemmPairs <= kMaxGroupTokens + 1, "a small expert must fit one work entry");
@@ -718,7 +722,6 @@ int chimere_b200_mma_i8_probe(int n_mma, int n_cols, int n_acc, int32_t* d_statu
     return launch_mma_i8_probe(n_mma, n_cols, n_acc, d_status, stream);
 }
 
-
 // The GEMM reads 4-bit weights in the tiled32 form; Q8_0 matrices, and a shared expert in Q4_K / Q5_K super-blocks, get a copy
 // in the MMA's own order (mma128 tiles; gate and up rows interleaved per 64, so that one output tile holds both).
 namespace {
@@ -952,7 +955,7 @@ int chimere_b200_moe_forward_prefill(const chimere_moe_layer* w, const chimere_m
     return kshared_chain(w, T, d_y, ws, stream);
 }
 
-// Expert-parallel owner rank, prefill-size: as chimere_b200_moe_experts, with the large local experts on the grouped GEMM.
+// Expert-parallel owner rank, prefill-size: as chimere_b200_moe_experts, with the local experts on the grouped GEMM.
 int chimere_b200_moe_experts_prefill(const chimere_moe_layer* w_local, const chimere_moe_prefill_weights* pw_local, int n_rows,
                                      chimere_moe_workspace* ws, cudaStream_t stream) {
     if (n_rows == 0) return 0;

@@ -316,9 +316,12 @@ __global__ void __launch_bounds__(kThreads) down_kernel(const GemvParams p, int 
 
 // ------------------------------------------------------------------ plain GEMV -------------
 // The legacy operator entries: y[slot][row] = W[ids[slot]][row] . xq8[slot] on raw blocks.  A group of 2^lanes_shift lanes owns a
-// row, lane l takes the 32-weight units l, l + lanes, ...; the lanes' sums meet in a butterfly.  A launch reads a few MB, so what
-// bounds it is the latency of one chain: weights are read straight into registers by as many warps as there are rows (staging
-// 64-row tiles in shared memory with 8 lanes per row and up to 8 units each in sequence took 8.5 us for 8 x 512 x 2048 IQ3_S).
+// row, lane l takes the 32-weight units l, l + lanes, ...; the lanes' sums meet in a butterfly.  A launch mostly reads a
+// few MB, so what bounds it is the latency of one chain: weights are read straight into registers by as many warps as there are rows
+// (staging 64-row tiles in shared memory with 8 lanes per row and up to 8 units each in sequence took 8.5 us for 8 x 512 x 2048
+// IQ3_S).  One matrix, us, staged / straight, weights from device memory: 512 x 2048 Q4_0 4.9 / 1.8, Q8_0 4.1 / 2.4, IQ3_S 4.8 / 2.3;
+// 4096 x 4096 8.4 / 5.9, 14.2 / 8.5, 7.2 / 7.0; 12288 x 4096 21.7 / 12.8, 25.0 / 20.0, 16.3 / 14.7; 248320 x 2048 133 / 104, 164 / 166,
+// 119 / 124 (IQ3_S: the codebook in shared memory, several rows per CTA, 121).
 struct PlainParams {
     const uint8_t* w; const uint8_t* xq8; float* y; const int* ids;
     int ncols, nrows; int64_t expert_stride, input_stride;
@@ -413,7 +416,7 @@ __global__ void rmsnorm_kernel(const float* x, float* y, int H, float eps) {
 // of strides 128 .. 1, and every element is scaled as (residual * inv_rms) * weight.
 // Latency-bound at a few rows: a thread's loads all go out before its first store (rows of up to 256 * 16 elements stay in
 // registers, longer ones are read again), and every warp sums the 256 partial sums itself instead of meeting eight times (10.5 us
-// -> 3.5 at 2 rows of 2048, cold).
+// -> 5.8 at 2 rows of 2048, cold).
 constexpr int kNormRegs = 16;
 // (No __restrict__, here or in the other kernels launched programmatically: the kernel before may write what these pointers name, and
 // reads of memory that the compiler may take for constant are not held back by griddep_wait().)

@@ -652,7 +652,7 @@ static BulkPlan plan_bulk(const GemvParams& p, int stage, bool dual, int wk, int
     const int ncols_max = max(p.ncols_routed, p.ncols_shared);
     const int threads = 32 * wk * wr;
     const int sm_bytes = 228 * 1024, per_cta = 1024 + 192;   // an SM's shared memory; per CTA the system's reserve and the kernel's static variables
-    const int max_ctas = min(8, 1536 / threads);
+    const int max_ctas = min(8, 1536 / threads);   // (by threads; the 77-80 registers of a 256-thread CTA allow three)
     // decode-size batches: as many CTAs per SM as fit one token per pass, then as many tokens as still fit;
     // larger batches: at least four tokens per pass if that fits at all
     const int mt_floor = (p.T > p.few_limit && !p.few_tokens) ? 4 : 1;

@@ -108,8 +108,14 @@ typedef struct chimere_moe_workspace {
 } chimere_moe_workspace;
 
 /* ---------------------------------------------------------------- layer-level entries ---- */
+/* The kernels of a call are launched programmatically behind one another and behind the previous kernel of the stream, and may read the
+ * layer's constants (weights, router rows, gate vector) while that kernel is still running: it must not be the one that writes them.
+ * Inputs, residual and norm weight may come from it. */
 
-/* Bytes of device memory a workspace for up to max_T tokens needs. */
+/* Bytes of device memory a workspace for up to max_T tokens needs.  A 4-bit layer in the TILED32 layout gets, from the batch size on at
+ * which chimere_b200_moe_forward uses the grouped GEMM (41 tokens, 17 where a matrix has more than 2M weights), the GEMM's
+ * scratch as well (prefill_arena / prefill_bytes below): for 256 experts of 512 x 2048 21 MB instead of 6 at 64 tokens, 1.2 GB
+ * instead of 0.7 at 8192.  It serves the prefill entry too where chimere_b200_moe_prefill_bytes is not larger. */
 size_t chimere_b200_moe_workspace_bytes(const chimere_moe_layer* w, int max_T);
 
 /* Carve `ws` out of the caller's device arena (`bytes` >= workspace_bytes, 256-byte aligned)
@@ -305,7 +311,8 @@ int chimere_b200_moe_pack_prefill(const chimere_moe_layer* raw, void* d_arena, s
                                   chimere_moe_prefill_weights* out, cudaStream_t stream);
 /* Extra scratch the prefill path needs for up to max_T tokens; pass it with ws->prefill_arena / prefill_bytes. */
 size_t chimere_b200_moe_prefill_bytes(const chimere_moe_layer* w, int max_T);
-/* y = MoE(x) like chimere_b200_moe_forward; `w` TILED32, `pw` what chimere_b200_moe_pack_prefill made of the same layer. */
+/* y = MoE(x) like chimere_b200_moe_forward; `w` TILED32, `pw` what chimere_b200_moe_pack_prefill made of the same layer.  4-bit experts
+ * with fewer pairs than half of them run as in chimere_b200_moe_forward. */
 int chimere_b200_moe_forward_prefill(const chimere_moe_layer* w, const chimere_moe_prefill_weights* pw,
                                      const float* d_x, float* d_y, int T, chimere_moe_workspace* ws,
                                      cudaStream_t stream);
@@ -334,7 +341,7 @@ int chimere_b200_moe_routing_trace(const chimere_moe_layer* w, int T, const chim
 int chimere_b200_moe_experts_prefill(const chimere_moe_layer* w_local, const chimere_moe_prefill_weights* pw_local, int n_rows,
                                      chimere_moe_workspace* ws, cudaStream_t stream);
 /* Expert-parallel home rank, prefill-size batches: chimere_b200_moe_shared_expert on the grouped GEMM.  pw: a GEMM copy that
- * holds the shared expert's matrices; ws needs the prefill arena.  Overwrites the work list of the routing call. */
+ * holds the shared expert's matrices; ws needs the prefill arena. */
 int chimere_b200_moe_shared_expert_prefill(const chimere_moe_layer* w, const chimere_moe_prefill_weights* pw, int T,
                                            chimere_moe_workspace* ws, cudaStream_t stream);
 /* The same on rows that lie where an exchange left them (the row format of chimere_b200_moe_ep_pack). */

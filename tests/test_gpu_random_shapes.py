@@ -1,7 +1,7 @@
 """Seeded random layer shapes, weight types, routing variants and batch sizes through both whole-layer entries: router
 logits, dispatch permutation and offsets bit for bit, output rows within the benchmark's tolerance of the CPU oracle.
 Complements the fixed configurations: odd expert counts, top-k from 1 to 8, layers without a shared expert, K-quant
-shared experts, batches on both sides of every kernel-selection threshold (4, 8, 32 tokens; the GEMM's 8 rows per expert)."""
+shared experts, batch sizes from 1 to 200 (the steps of the kernel selection themselves: test_gpu_batch_edges.py)."""
 import random
 
 import numpy as np
