@@ -75,6 +75,14 @@ int validate_layer(const chimere_moe_layer* w) {
     return 0;
 }
 
+// Decode batches whose every (token, expert) pair is an item of its own (pairs.cu).  us per layer against the work list's entries of one or
+// two pairs: 256 experts of 512 x 2048, top 8: 8 tokens 31 / 38, 24: 65 / 78, 40 tokens 101 / 115 (skewed 90 / 104); 128 of
+// 1856 x 2688, top 6: 1 token 24 / 28, 8: 88 / 101, 12: 121 / 136, 16: 159 / 172.
+bool pair_batch(const chimere_moe_layer* w, int T) {
+    const int64_t P = (int64_t)T * w->top_k;
+    return T <= 4 || (T <= 40 && ((int64_t)w->F * w->H > (1 << 21) ? 16 * P <= 9 * w->E : 4 * P <= 5 * w->E));
+}
+
 // From forward_gemm_tokens() tokens on the decode entry sends experts with at least kForwardGemmPairs pairs, and the shared expert,
 // to the grouped GEMM and the others to the GEMV kernels: a GEMM tile costs the same with 1 pair as with 16, a GEMV entry grows
 // with every pair.  Q4_0, us per layer, GEMV kernels alone / with the GEMM, uniform and (skewed) routing:
@@ -612,6 +620,41 @@ int chimere_b200_moe_down_combine(const chimere_moe_layer* w, float* d_y, int T,
     return cuda_rc(run_down(w, down_params(w, d_y, T, ws, L), max_entries_for(w, T), stream));
 }
 
+// Decode batches up to pair_batch()'s line run without a work list where the pair kernels take the layer: the router's logits, then
+// two launches that select their experts themselves.  A K-quant shared expert rides along or follows as kshared_chain.
+static PairExtras pair_extras(const chimere_moe_layer* w, chimere_moe_workspace* ws) {
+    PairExtras x{};
+    if (!kshared(w) || !pairs_take_kquant(*w)) return x;
+    x.type = w->type_sh_up; x.type_down = w->type_sh_down; x.F_s = w->F_s;
+    x.gate = (const uint8_t*)w->sh_gate; x.up = (const uint8_t*)w->sh_up; x.down = (const uint8_t*)w->sh_down;
+    x.rows = ws->pair_out;
+    x.logit = w->shexp_gate_w ? ws->sh_gate_logit : nullptr;
+    return x;
+}
+static bool pairs_forward(const chimere_moe_layer* w, int T, chimere_moe_workspace* ws) {
+    if (!pair_batch(w, T) || w->layout != CHIMERE_LAYOUT_TILED32) return false;
+    const chimere_moe_layer wr = kshared(w) ? routed_only(w) : *w;
+    const Layout L = make_layout(&wr, ws->max_T);
+    return pairs_run(gate_up_params(&wr, T, ws, L), down_params(&wr, nullptr, T, ws, L), pair_extras(w, ws));
+}
+static int run_pairs(const chimere_moe_layer* w, const float* d_x, const float* d_hidden, float* d_residual, const float* d_norm_weight, float eps, float* d_y, int T,
+                     chimere_moe_workspace* ws, cudaStream_t stream) {
+    const bool ks = kshared(w);
+    const chimere_moe_layer wr = ks ? routed_only(w) : *w;
+    const Layout L = make_layout(&wr, ws->max_T);
+    PairExtras x = pair_extras(w, ws);
+    RouteParams rp = route_params(&wr, d_x, T, ws, ks);
+    rp.logits_only = 1;
+    cudaError_t e;
+    if (d_hidden) {
+        x.hidden = d_hidden; x.residual = d_residual;
+        e = launch_route_norm(rp, d_hidden, d_residual, d_norm_weight, eps, stream);
+    } else e = launch_route(rp, stream);
+    if (e == cudaSuccess) e = launch_pair_gate_up(rp, gate_up_params(&wr, T, ws, L), x, stream);
+    if (e == cudaSuccess) e = launch_pair_down(rp, down_params(&wr, d_y, T, ws, L), x, stream);
+    return e != cudaSuccess || !ks || x.type ? cuda_rc(e) : kshared_chain(w, T, d_y, ws, stream);
+}
+
 int chimere_b200_moe_forward(const chimere_moe_layer* w, const float* d_x, float* d_y, int T, chimere_moe_workspace* ws,
                              cudaStream_t stream) {
     int rc = check_call(w, d_x, d_y, T, ws, true);
@@ -621,7 +664,9 @@ int chimere_b200_moe_forward(const chimere_moe_layer* w, const float* d_x, float
     const chimere_moe_layer* wr = &wr_;
     cudaError_t e;
     const Layout L = make_layout(wr, ws->max_T);
-    if (forward_gemm(wr, T) && ws->prefill_arena && ws->prefill_bytes >= prefill_arena(wr, ws->max_T).total &&
+    if (pairs_forward(w, T, ws)) {
+        return run_pairs(w, d_x, nullptr, nullptr, nullptr, 0.0f, d_y, T, ws, stream);
+    } else if (forward_gemm(wr, T) && ws->prefill_arena && ws->prefill_bytes >= prefill_arena(wr, ws->max_T).total &&
         tiled_bulk_runs(gate_up_params(wr, T, ws, L), down_params(wr, d_y, T, ws, L))) {
         RouteParams rp = route_params(wr, d_x, T, ws, ks);
         rp.list_mode = 2;
@@ -652,10 +697,11 @@ int chimere_b200_moe_forward_host(const chimere_moe_layer* w, const float* h_x, 
     if (e != cudaSuccess) return cuda_rc(e);
     // A pinned result buffer is addressable from the device under a pointer of its own: the last kernel then stores y
     // straight into host memory and the copy back (a second trip through the copy engine, serial behind the kernels) is
-    // not needed.  Pageable memory, or a K-quant shared expert (whose last step reads y back), takes the staged copy.
+    // not needed.  Pageable memory, or a K-quant shared expert as launches of its own (the last of which reads y back), takes the staged copy.
     float* y_dev = d_y;
     cudaPointerAttributes attr{};
-    if (!kshared(w) && cudaPointerGetAttributes(&attr, h_y) == cudaSuccess && attr.type == cudaMemoryTypeHost && attr.devicePointer)
+    const bool last_stores = !kshared(w) || (pairs_forward(w, T, ws) && pair_extras(w, ws).type);
+    if (last_stores && cudaPointerGetAttributes(&attr, h_y) == cudaSuccess && attr.type == cudaMemoryTypeHost && attr.devicePointer)
         y_dev = static_cast<float*>(attr.devicePointer);
     else
         (void)cudaGetLastError();   // (an unregistered pointer leaves an error behind on older runtimes)
@@ -1019,6 +1065,10 @@ int chimere_b200_moe_forward_residual_norm(const chimere_moe_layer* w, const chi
     int rc = check_call(w, d_hidden, d_y, T, ws, true);
     if (rc) return rc;
     if (!d_residual || !d_norm_weight || !ws->pair_out) return -1;
+    if (!pw && pairs_forward(w, T, ws)) {
+        const chimere_moe_layer wr = kshared(w) ? routed_only(w) : *w;
+        if (route_norm_runs(route_params(&wr, nullptr, T, ws))) return run_pairs(w, nullptr, d_hidden, d_residual, d_norm_weight, eps, d_y, T, ws, stream);
+    }
     // the normalised rows live in the first T rows of the per-pair output area until the router and the Q8_1 step have
     // read them; the down stage writes that area only afterwards
     float* normed = ws->pair_out;

@@ -3,6 +3,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "../../include/chimere_b200_moe.h"
+
 namespace chimere {
 
 // layout of the workspace's integer scratch ("counters"); everything returns to zero after a call
@@ -16,6 +18,7 @@ struct RouteParams {
     int idx_stride;             // permute only: distance in int32 between consecutive ids (0 or 1 = dense)
     int list_mode;              // 0: work list for routed + shared entries; 1: shared-expert entries only (expert-parallel home
                                 // rank); 2: an empty list (the prefill path builds its own from offsets and perm)
+    int logits_only;            // no top-k, no dispatch: the kernels behind do both (pairs.cu)
     int group;                  // pairs per routed work entry (0 = kMaxGroupTokens)
     int list_capacity;          // entries the work list has room for (more raise kStatusListFull and are left out)
     float route_scale;
@@ -202,6 +205,23 @@ cudaError_t launch_pack(int type, const void* raw, void* out, int n_mats, int nr
 // fallback adds in another order): what the grouped GEMM needs to form the same sums.
 int tiled_slice_units(int type, int ncols, int wk);
 bool tiled_bulk_runs(const GemvParams& gate_up, const GemvParams& down);
+// What rides along with the pair kernels: a K-quant shared expert (type 0 = none) and the residual update of a half-layer whose router
+// has taken the sum itself (hidden null = none).
+struct PairExtras {
+    int type, type_down, F_s;                     // gate and up have one type
+    const uint8_t* gate; const uint8_t* up; const uint8_t* down;
+    float* rows;                                  // [2][T][F_s] up and gate rows between the two launches
+    const float* logit;                           // [T] or null
+    const float* hidden; float* residual;         // residual += hidden, [T][H]
+};
+// decode batches without a work list (pairs.cu): whether these kernels take a layer, and its two launches behind the router's logits
+bool pairs_run(const GemvParams& gate_up, const GemvParams& down, const PairExtras& x);
+bool pairs_take_kquant(const chimere_moe_layer& w);
+cudaError_t launch_pair_gate_up(const RouteParams& r, const GemvParams& p, const PairExtras& x, cudaStream_t stream);
+cudaError_t launch_pair_down(const RouteParams& r, const GemvParams& p, const PairExtras& x, cudaStream_t stream);
+// the router's logits and the Q8_1 rows of normed = rmsnorm(residual + hidden) * weight; residual is left for launch_pair_gate_up
+bool route_norm_runs(const RouteParams& p);
+cudaError_t launch_route_norm(const RouteParams& p, const float* hidden, const float* residual, const float* weight, float eps, cudaStream_t stream);
 cudaError_t launch_gate_up_tiled(const GemvParams& p, int max_entries, cudaStream_t stream);
 cudaError_t launch_down_tiled(const GemvParams& p, int max_entries, cudaStream_t stream);
 cudaError_t launch_block_sumi_tiled(int type, const void* packed, const void* xq8, int32_t* sumi, int ncols, int nrows,

@@ -10,6 +10,7 @@
 //   ggml_quantize_q8_1   chimere-server/kernels/chimere_kernels.cu:1495-1523
 #include "common.cuh"
 #include "kernels.h"
+#include "routing.cuh"
 
 namespace chimere {
 
@@ -26,294 +27,6 @@ __device__ __forceinline__ void quantize_block_q8_1(float xi, uint8_t* out, int 
     // the same block as planes (what the tiled GEMV kernels stream)
     plane_q[lane] = q;
     if (lane == 0) *plane_d = __half2float(dh);
-}
-
-// One token's scores -> top-k, by one warp.  Lane l owns experts l, l+32, ...
-__device__ void topk_warp(const RouteParams& p, const float* logit_row, int t, int lane, float* tree_scratch, int* ids_out) {
-    const int E = p.E, k = p.top_k;
-    float v[8], pr[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int e = lane + 32 * i;
-        v[i] = (e < E) ? __ldcg(logit_row + e) : -1.0e30f;
-    }
-    if (p.route_mode == CHIMERE_ROUTE_SOFTMAX_RENORM) {
-        float mx = v[0];
-#pragma unroll
-        for (int i = 1; i < 8; ++i) mx = fmaxf(mx, v[i]);
-#pragma unroll
-        for (int m = 16; m > 0; m >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, m));
-        float ev[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const int e = lane + 32 * i;
-            ev[i] = (e < E) ? expf(v[i] - mx) : 0.0f;
-            tree_scratch[e] = ev[i];
-        }
-        __syncwarp();
-        float sum = tree256(tree_scratch, lane);
-        sum = __shfl_sync(0xffffffffu, sum, 0);
-        __syncwarp();
-#pragma unroll
-        for (int i = 0; i < 8; ++i) pr[i] = (sum > 0.0f) ? (ev[i] / sum) : (1.0f / (float)E);
-    } else {
-#pragma unroll
-        for (int i = 0; i < 8; ++i) pr[i] = 1.0f / (1.0f + expf(-v[i]));
-    }
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-        if (lane + 32 * i >= E) pr[i] = -2.0f;  // never selected
-
-    // Selection on integer keys: probabilities are >= 0, so their bit patterns order like the values; key 0 = not
-    // available (beyond E, or already taken).  One warp-wide max and one warp-wide min per slot (redux.sync) instead
-    // of a shuffle butterfly: the largest value wins, equal values go to the lowest index, like a strict-greater
-    // scan from index 0.
-    uint32_t key[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) key[i] = (lane + 32 * i < E) ? __float_as_uint(pr[i]) + 1u : 0u;
-    float wsum = 0.0f;
-    float wsel = 0.0f;  // lane j keeps the weight of slot j
-    int isel = 0;
-    for (int j = 0; j < k; ++j) {
-        uint32_t lm = key[0];
-#pragma unroll
-        for (int i = 1; i < 8; ++i) lm = max(lm, key[i]);
-        const uint32_t m = __reduce_max_sync(0xffffffffu, lm);
-        uint32_t cand = 0xffffffffu;   // lowest index in this lane that holds the maximum
-#pragma unroll
-        for (int i = 7; i >= 0; --i)
-            if (key[i] == m) cand = (uint32_t)(lane + 32 * i);
-        const int bi = (int)__reduce_min_sync(0xffffffffu, cand);
-        const float bv = __uint_as_float(m - 1u);
-        wsum += bv;
-        if (lane == j) { wsel = bv; isel = bi; }
-        if ((bi & 31) == lane) {
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
-                if (i == (bi >> 5)) key[i] = 0u;
-        }
-    }
-    if (lane < k) {
-        float w = wsel;
-        if (wsum > 0.0f) {
-            const float inv = 1.0f / wsum;
-            w = w * inv;
-        }
-        if (p.route_mode != CHIMERE_ROUTE_SOFTMAX_RENORM || p.route_scale != 1.0f) w = w * p.route_scale;
-        p.topk_idx[(size_t)t * k + lane] = isel;
-        p.topk_w[(size_t)t * k + lane] = w;
-        if (ids_out) ids_out[lane] = isel;
-    }
-}
-
-// Stable counting sort of the T*k pairs by expert, plus the GEMV work list.  One CTA of 256.
-// s_ids: the T*k expert ids in shared memory if the caller has them there (else they are read from p.topk_idx).
-// Each warp takes one contiguous eighth of the pairs: it counts its pairs per expert, the counts are turned into
-// every warp's first position within every expert, and the warp places its pairs in order; so the only CTA
-// barriers are between those steps, however many pairs there are.  The work entries are then filled by all
-// threads (entry -> expert by bisection of the entry offsets).
-constexpr int kDispatchSmemInts = 256 + 256 + 2048 + 32 + 288 + 1024;
-// The dispatch step is written for 256 threads; in a larger CTA only the first 256 threads call it, so its meeting
-// point is a named barrier of those threads (in a CTA of 256 it is the same as a CTA-wide barrier).
-__device__ __forceinline__ void dispatch_sync() { asm volatile("bar.sync 2, 256;" ::: "memory"); }
-// ids_room: ints of shared memory behind the kDispatchSmemInts of scratch; if the ids fit there they are fetched
-// once, all loads in flight together, instead of one dependent load per step of the two passes.
-// The same result for at most 32 pairs whose ids are in shared memory (a decode batch of up to four tokens): every thread counts directly --
-// pair q its position (ids below its own, equal ids before it), thread e the offset of expert e -- and the work entries
-// come from the sorted ids by two ballots.  Two barriers instead of six and no scratch to clear: a third of the time.
-constexpr int kSmallDispatchPairs = 32;   // (at 64 pairs the direct counting is no faster than the general form)
-__device__ void build_dispatch_small(const RouteParams& p, int* smem_i, const int* s_ids) {
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int E = p.E, P = p.T * p.top_k;
-    int* s_sid = smem_i;          // [64] expert ids in sorted order (room for two warps of positions)
-    int* s_perm = smem_i + 64;    // [64] the permutation
-    const int gt = p.group > 0 ? p.group : kMaxGroupTokens;
-    int* s_lead = smem_i + 128;   // [2] distinct experts among sorted positions 0..31 / 32..63
-    const int my_e = tid < P ? s_ids[tid] : -1;
-    const bool valid = my_e >= 0 && my_e < E;
-    int below_tid = 0, below_mine = 0, before_me = 0, total = 0;
-    for (int q = 0; q < P; ++q) {
-        const int e = s_ids[q];                      // (the same address in every thread: a broadcast)
-        const bool v = e >= 0 && e < E;
-        total += v;
-        below_tid += v && e < tid;
-        below_mine += v && e < my_e;
-        before_me += q < tid && e == my_e;
-    }
-    if (tid < E) p.offsets[tid] = below_tid;
-    if (tid == 0) p.offsets[E] = total;
-    if (valid) {
-        const int pos = below_mine + before_me;
-        p.perm[pos] = tid;
-        s_perm[pos] = tid;
-        s_sid[pos] = my_e;
-    }
-    // shared-expert entries first (all tokens, identity order), as in the general form
-    const int sgt = shared_group_tokens(p.T);
-    const int nsh = p.has_shared ? (p.T + sgt - 1) / sgt : 0;
-    const int nsh_listed = p.list_mode == 2 ? 0 : nsh;
-    for (int i = tid; i < nsh_listed; i += 256) {
-        int* ent = p.group_list + kListHeader + kListEntry * i;
-        const int t0 = i * sgt, mm = min(sgt, p.T - t0);
-        ent[0] = -1; ent[1] = t0; ent[2] = mm; ent[3] = 0;
-        for (int j = 0; j < kMaxGroupTokens; ++j) ent[4 + j] = j < mm ? p.T * p.top_k + t0 + j : 0;
-    }
-    dispatch_sync();
-    // sorted position tid starts a new expert?  (warps 0 and 1 hold the 64 positions)
-    unsigned lead = 0u;
-    if (warp < 2) {
-        // (entry starts: every gt-th pair of an expert, gt a power of two; an expert has at most T <= 4 pairs here.  One pair per
-        // entry needs no look at the neighbours: this is on the chain of a single token's layer)
-        int rank = 0;
-        if (gt > 1) while (rank < tid && tid < total && s_sid[tid - rank - 1] == s_sid[tid]) ++rank;
-        const bool first = tid < total && (rank & (gt - 1)) == 0;
-        lead = __ballot_sync(0xffffffffu, first);
-        if (lane == 0) s_lead[warp] = __popc(lead);
-    }
-    dispatch_sync();
-    const int total_routed = p.list_mode != 0 ? 0 : s_lead[0] + s_lead[1];
-    if (tid == 0) {
-        p.group_list[0] = total_routed + nsh_listed;
-        p.group_list[1] = total_routed;
-        p.group_list[2] = nsh_listed;
-        p.group_list[3] = 0;
-    }
-    if (warp < 2 && total_routed > 0 && ((lead >> lane) & 1u)) {
-        const int idx = __popc(lead & ((1u << lane) - 1u)) + (warp == 1 ? s_lead[0] : 0);
-        const int e = s_sid[tid];
-        int mm = 1;
-        while (mm < gt && tid + mm < total && s_sid[tid + mm] == e) ++mm;
-        int* ent = p.group_list + kListHeader + kListEntry * (nsh + idx);
-        ent[0] = e; ent[1] = tid; ent[2] = mm; ent[3] = 0;
-        for (int j = 0; j < kMaxGroupTokens; ++j) ent[4 + j] = j < mm ? s_perm[tid + j] : 0;
-    }
-}
-
-__device__ void build_dispatch(const RouteParams& p, int* smem_i, const int* s_ids, int ids_room) {
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int E = p.E, P = p.T * p.top_k;
-    if (s_ids && P <= kSmallDispatchPairs && p.T <= kMaxGroupTokens) { build_dispatch_small(p, smem_i, s_ids); return; }
-    if (!s_ids && P <= ids_room) {
-        int* stage = smem_i + kDispatchSmemInts;
-        const int istr0 = p.idx_stride > 1 ? p.idx_stride : 1;
-        for (int q = tid; q < P; q += 256) stage[q] = __ldcg(p.topk_idx + (size_t)q * istr0);
-        s_ids = stage;   // visible after the barrier below
-    }
-    int* hist = smem_i;               // [256] pairs per expert
-    int* cursor = smem_i + 256;       // [256] first position of each expert
-    int* warp_cnt = smem_i + 512;     // [8][256] per warp: pairs of each expert, then the warp's next position within it
-    int* scan = smem_i + 2560;        // [32]
-    int* ent_base = smem_i + 2592;    // [257] first routed entry of each expert, [256] = their number
-    int* s_perm = smem_i + 2880;      // [1024] copy of the permutation when it is that short
-    const bool perm_in_smem = P <= 1024;
-    for (int i = tid; i < 2048; i += 256) warp_cnt[i] = 0;
-    dispatch_sync();
-    // ids outside [0, E) mark pairs that are not there (padding of a fixed-size exchange): they get no work
-    const int istr = p.idx_stride > 1 ? p.idx_stride : 1;
-    const int chunk = (((P + 7) >> 3) + 31) & ~31;
-    const int q0 = min(P, warp * chunk), q1 = min(P, q0 + chunk);
-    for (int base = q0; base < q1; base += 32) {
-        const int q = base + lane;
-        int e = q < q1 ? (s_ids ? s_ids[q] : __ldcg(p.topk_idx + (size_t)q * istr)) : -1;
-        const bool valid = e >= 0 && e < E;
-        if (!valid) e = 0x40000000 + lane;
-        const unsigned same = __match_any_sync(0xffffffffu, e);
-        if (valid && (same & ((1u << lane) - 1u)) == 0u) warp_cnt[warp * 256 + e] += __popc(same);
-        __syncwarp();
-    }
-    dispatch_sync();
-    // thread = expert: its pair count, and where each warp's pairs start within it
-    int cnt = 0;
-    if (tid < E) {
-#pragma unroll
-        for (int w = 0; w < 8; ++w) {
-            const int t = warp_cnt[w * 256 + tid];
-            warp_cnt[w * 256 + tid] = cnt;
-            cnt += t;
-        }
-    }
-    hist[tid] = cnt;
-    // exclusive scans over the experts: pair offsets and work-entry offsets
-    const int gt = p.group > 0 ? p.group : kMaxGroupTokens;
-    const int nent = (cnt + gt - 1) / gt;
-    int incl_c = cnt, incl_n = nent;
-#pragma unroll
-    for (int s = 1; s < 32; s <<= 1) {
-        const int a = __shfl_up_sync(0xffffffffu, incl_c, s), b = __shfl_up_sync(0xffffffffu, incl_n, s);
-        if (lane >= s) { incl_c += a; incl_n += b; }
-    }
-    if (lane == 31) { scan[warp] = incl_c; scan[8 + warp] = incl_n; }
-    dispatch_sync();
-    int base_c = 0, base_n = 0;
-    for (int w = 0; w < warp; ++w) { base_c += scan[w]; base_n += scan[8 + w]; }
-    const int off = base_c + incl_c - cnt;      // exclusive
-    const int ent0 = base_n + incl_n - nent;
-    cursor[tid] = off;
-    ent_base[tid] = ent0;
-    if (tid < E) p.offsets[tid] = off;
-    if (tid == 255) {
-        p.offsets[E] = base_c + incl_c;  // tid 255 holds the inclusive total (cnt = 0 beyond E)
-        ent_base[256] = base_n + incl_n;
-    }
-    int total_routed = 0;
-    for (int w = 0; w < 8; ++w) total_routed += scan[8 + w];
-    // shared-expert entries first (all tokens, identity order), then the routed ones
-    const int sgt = shared_group_tokens(p.T);
-    const int nsh = p.has_shared ? (p.T + sgt - 1) / sgt : 0;
-    if (p.list_mode != 0) total_routed = 0;
-    if (nsh + total_routed > p.list_capacity) {   // (never, if the workspace was made for this layer and batch)
-        total_routed = max(0, p.list_capacity - nsh);
-        if (tid == 0 && p.status) atomicOr(p.status, kStatusListFull);
-    }
-    for (int i = tid; i < (p.list_mode == 2 ? 0 : nsh); i += 256) {
-        int* ent = p.group_list + kListHeader + kListEntry * i;
-        const int t0 = i * sgt, mm = min(sgt, p.T - t0);
-        ent[0] = -1; ent[1] = t0; ent[2] = mm; ent[3] = 0;
-        for (int j = 0; j < kMaxGroupTokens; ++j) ent[4 + j] = j < mm ? p.T * p.top_k + t0 + j : 0;
-    }
-    if (tid == 0) {
-        const int nsh_listed = p.list_mode == 2 ? 0 : nsh;
-        p.group_list[0] = total_routed + nsh_listed;
-        p.group_list[1] = total_routed;
-        p.group_list[2] = nsh_listed;
-        p.group_list[3] = 0;
-    }
-    dispatch_sync();   // cursor and the warps' first positions are in place
-    // stable placement: each warp walks its pairs in order
-    for (int base = q0; base < q1; base += 32) {
-        const int q = base + lane;
-        int e = q < q1 ? (s_ids ? s_ids[q] : __ldcg(p.topk_idx + (size_t)q * istr)) : -1;
-        const bool valid = e >= 0 && e < E;
-        if (!valid) e = 0x40000000 + lane;
-        const unsigned same = __match_any_sync(0xffffffffu, e);
-        const int rank = __popc(same & ((1u << lane) - 1u));
-        if (valid) {
-            const int pos = cursor[e] + warp_cnt[warp * 256 + e] + rank;
-            p.perm[pos] = q;
-            if (perm_in_smem) s_perm[pos] = q;
-        }
-        __syncwarp();
-        if (valid && rank == 0) warp_cnt[warp * 256 + e] += __popc(same);
-        __syncwarp();
-    }
-    dispatch_sync();
-    // the routed entries with their pair rows (perm was written by this CTA: visible after the barrier above)
-    for (int idx = tid; idx < total_routed; idx += 256) {
-        int lo = 0, hi = 256;   // ent_base[lo] <= idx < ent_base[hi]
-        while (hi - lo > 1) {
-            const int mid = (lo + hi) >> 1;
-            if (ent_base[mid] <= idx) lo = mid; else hi = mid;
-        }
-        const int e = lo, i = idx - ent_base[e], c = hist[e], o = cursor[e];
-        const int mm = min(gt, c - i * gt);
-        int* ent = p.group_list + kListHeader + kListEntry * (nsh + idx);
-        ent[0] = e;
-        ent[1] = o + i * gt;
-        ent[2] = mm;
-        ent[3] = 0;
-        for (int j = 0; j < kMaxGroupTokens; ++j)
-            ent[4 + j] = j < mm ? (perm_in_smem ? s_perm[o + i * gt + j] : p.perm[o + i * gt + j]) : 0;
-    }
 }
 
 // grid = (row tiles, token tiles), 256 threads; TOKENS_X: (token tiles, row tiles), for more than the 65535 token tiles that the
@@ -399,6 +112,8 @@ __global__ void __launch_bounds__(256) route_kernel(const RouteParams p) {
         }
     }
 
+    if (p.logits_only) return;
+
     // ---- last CTA of the token tile: scores and top-k ----
     __shared__ int s_flag;
     __shared__ int s_ids[TT * kMaxTopK];
@@ -409,7 +124,7 @@ __global__ void __launch_bounds__(256) route_kernel(const RouteParams p) {
     if (tid == 0) p.counters[kCtrRouteTile + ttile] = 0;
     for (int a = warp; a < TT; a += 8) {
         const int t = t0 + a;
-        if (t < p.T) topk_warp(p, p.router_logits + (size_t)t * E, t, lane, red + warp * 256, s_ids + a * p.top_k);
+        if (t < p.T) topk_warp(p, p.router_logits + (size_t)t * E, t, lane, s_ids + a * p.top_k);
     }
 
     // ---- last token tile overall: dispatch permutation and work list ----
@@ -425,6 +140,85 @@ __global__ void __launch_bounds__(256) route_kernel(const RouteParams p) {
     if (!s_flag) return;
     if (tid == 0) p.counters[kCtrRouteAll] = 0;
     build_dispatch(p, reinterpret_cast<int*>(smem_f), nullptr, (int)(TT * TE * 256) - kDispatchSmemInts);
+}
+
+// The same for the first step of a half-layer of a few tokens: x = rmsnorm(residual + hidden) * weight is formed here (in every CTA: a
+// thread holds the very elements that it sums squares of and multiplies with its router rows) instead of by a launch in front
+// that stands for 4 us of latency.  In add_residual_rmsnorm_kernel's order (gemv.cu).  The logits alone, and x's Q8_1 form; the
+// residual is updated by the launch behind, when every CTA has read it.  H <= 256 * KS.
+template <int TT, int KS>
+__global__ void __launch_bounds__(256) route_norm_kernel(const RouteParams p, const float* hidden, const float* residual, const float* weight, float eps) {
+    __shared__ float s_red[TT * 2][256];
+    __shared__ float s_sq[TT][256];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, H = p.H, E = p.E, r0 = blockIdx.x * 2;
+    const int nrows = E + (p.shexp_gate_w ? 1 : 0);
+    float wv[KS][2], x[TT][KS], nw[KS];
+#pragma unroll
+    for (int b = 0; b < 2; ++b) {
+        const int r = r0 + b;
+        const float* row = r < E ? p.router_w + (size_t)r * H : r == E && r < nrows ? p.shexp_gate_w : nullptr;
+#pragma unroll
+        for (int i = 0; i < KS; ++i) wv[i][b] = row && i * 256 + tid < H ? __ldg(row + i * 256 + tid) : 0.0f;
+    }
+    griddep_wait();
+    if (tid == 0) griddep_launch();
+    float hv[TT][KS];
+#pragma unroll
+    for (int a = 0; a < TT; ++a)
+#pragma unroll
+        for (int i = 0; i < KS; ++i) {
+            const bool on = a < p.T && i * 256 + tid < H;
+            hv[a][i] = on ? hidden[(size_t)a * H + i * 256 + tid] : 0.0f;
+            x[a][i] = on ? residual[(size_t)a * H + i * 256 + tid] : 0.0f;
+        }
+#pragma unroll
+    for (int i = 0; i < KS; ++i) nw[i] = i * 256 + tid < H ? weight[i * 256 + tid] : 0.0f;
+#pragma unroll
+    for (int a = 0; a < TT; ++a) {
+        float sq = 0.0f;
+#pragma unroll
+        for (int i = 0; i < KS; ++i) {
+            x[a][i] = hv[a][i] + x[a][i];
+            if (i * 256 + tid < H) sq = fmaf(x[a][i], x[a][i], sq);
+        }
+        s_sq[a][tid] = sq;
+    }
+    __syncthreads();
+    float acc[TT][2];
+#pragma unroll
+    for (int a = 0; a < TT; ++a) {
+        const float total = __shfl_sync(0xffffffffu, tree256(s_sq[a], lane), 0);
+        const float rms = sqrtf(total / (float)H + eps);
+        const float inv_rms = 1.0f / rms;
+        acc[a][0] = acc[a][1] = 0.0f;
+#pragma unroll
+        for (int i = 0; i < KS; ++i) {
+            x[a][i] = x[a][i] * inv_rms * nw[i];
+            if (i * 256 + tid < H) { acc[a][0] = fmaf(wv[i][0], x[a][i], acc[a][0]); acc[a][1] = fmaf(wv[i][1], x[a][i], acc[a][1]); }
+        }
+        s_red[2 * a][tid] = acc[a][0];
+        s_red[2 * a + 1][tid] = acc[a][1];
+    }
+    // Q8_1: elements i * 256 + 32 * warp .. of a token are block 8 * i + warp, lane = element; (token, i) pairs are dealt to the CTAs
+    for (int q = blockIdx.x; q < p.T * KS; q += gridDim.x) {
+        const int t = q / KS, b = (q - t * KS) * 8 + warp;
+        float xi = 0.0f;
+#pragma unroll
+        for (int a = 0; a < TT; ++a)
+#pragma unroll
+            for (int i = 0; i < KS; ++i)
+                if (q == a * KS + i) xi = x[a][i];
+        if (b < H >> 5) quantize_block_q8_1(xi, p.x_q8 + ((size_t)t * (H >> 5) + b) * kQ81Bytes, lane, p.x_soa_q + (size_t)t * H + b * 32, p.x_soa_d + (size_t)t * p.x_soa_d_stride + b);
+    }
+    __syncthreads();
+    for (int o = warp; o < TT * 2; o += 8) {
+        const float v = tree256(s_red[o], lane);
+        const int t = o >> 1, r = r0 + (o & 1);
+        if (lane == 0 && t < p.T && r < nrows) {
+            if (r < E) p.router_logits[(size_t)t * E + r] = p.router_bias ? v + p.router_bias[r] : v;
+            else p.sh_gate_logit[t] = v;
+        }
+    }
 }
 
 // Larger batches, as a register-tiled product.  The order of the additions is fixed (256 partial sums per output, partial p over
@@ -626,7 +420,7 @@ __global__ void __launch_bounds__(256) route_topk_kernel(const RouteParams p, in
     __shared__ int s_flag;
     griddep_wait();
     if (tid == 0) griddep_launch();
-    if (t < p.T) topk_warp(p, p.router_logits + (size_t)t * p.E, t, lane, smem_f + warp * 256, nullptr);
+    if (t < p.T) topk_warp(p, p.router_logits + (size_t)t * p.E, t, lane, nullptr);
     if (split_dispatch) return;
     __syncthreads();   // every thread's writes are ordered before thread 0's counter increment, which releases them
     if (tid == 0) s_flag = (atom_add_acq_rel_gpu(&p.counters[kCtrRouteAll], 1) == (int)gridDim.x - 1);   // ... and acquires the other CTAs'
@@ -1153,12 +947,28 @@ static cudaError_t launch_route_tiles(const RouteParams& p, cudaStream_t stream)
     return e == cudaSuccess && split ? launch_dispatch_split(p, stream) : e;
 }
 
+bool route_norm_runs(const RouteParams& p) { return p.T <= 4 && p.H <= 256 * 12; }
+template <int TT>
+static cudaError_t launch_route_norm_t(const RouteParams& p, const float* hidden, const float* residual, const float* weight, float eps, cudaStream_t stream) {
+    const dim3 grid((p.E + (p.shexp_gate_w ? 1 : 0) + 1) / 2);
+    if (p.H <= 256 * 8) return launch_pdl(route_norm_kernel<TT, 8>, grid, 256, 0, stream, p, hidden, residual, weight, eps);
+    return launch_pdl(route_norm_kernel<TT, 12>, grid, 256, 0, stream, p, hidden, residual, weight, eps);
+}
+cudaError_t launch_route_norm(const RouteParams& p, const float* hidden, const float* residual, const float* weight, float eps, cudaStream_t stream) {
+    return p.T == 1 ? launch_route_norm_t<1>(p, hidden, residual, weight, eps, stream)
+                    : p.T == 2 ? launch_route_norm_t<2>(p, hidden, residual, weight, eps, stream) : launch_route_norm_t<4>(p, hidden, residual, weight, eps, stream);
+}
+
 cudaError_t launch_route(const RouteParams& p, cudaStream_t stream) {
     const int nrows = p.E + (p.shexp_gate_w ? 1 : 0);
     const int ttiles8 = (p.T + 7) / 8;
     // few experts: a row per CTA, up to 3072 columns in flight at once, as long as that is one CTA per SM (64 experts of H = 2048, 8 tokens
     // 9.6 -> 9.1 us, but 24 tokens 10.9 -> 11.7); a single row of 2048 is faster in pairs of outputs (6.9 against 7.3)
-    if (p.T <= 32 && nrows * ttiles8 <= sm_count() && (p.T > 1 || p.H > 2048)) {
+    if (p.T <= 2) {
+        constexpr int TE = 2;
+        const dim3 grid((nrows + TE - 1) / TE);
+        return p.T == 1 ? launch_pdl(route_kernel<1, TE>, grid, 256, route_smem(1, TE), stream, p) : launch_pdl(route_kernel<2, TE>, grid, 256, route_smem(2, TE), stream, p);
+    } else if (p.T <= 32 && nrows * ttiles8 <= sm_count() && (p.T > 1 || p.H > 2048)) {
         constexpr int TT = 8, TE = 1;
         return launch_pdl(route_kernel<TT, TE>, dim3(nrows, (p.T + TT - 1) / TT), 256, route_smem(TT, TE), stream, p);
     } else if (p.T <= 32) {

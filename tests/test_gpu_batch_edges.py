@@ -7,7 +7,8 @@ import torch
 
 import oracle
 from chimere_b200 import configs, formats
-from chimere_b200.layer import MoeScratch, MoeWeightsPrefill, MoeWeightsTiled, forward_moe, forward_moe_host, forward_moe_prefill, route_only
+from chimere_b200.layer import (MoeScratch, MoeWeightsPrefill, MoeWeightsTiled, forward_moe, forward_moe_host, forward_moe_prefill, forward_moe_residual_norm,
+                                route_only)
 from parity_util import check_rows, oracle_on_gpu_routing
 
 pytestmark = pytest.mark.gpu
@@ -207,3 +208,71 @@ def test_router_of_many_tokens():
         route_only(tiled, small, x[part].contiguous())
         assert torch.equal(sc.router_logits(T)[part], small.router_logits(n)) and torch.equal(ids[part], small.topk_indices(n).flatten())
     assert torch.equal(sc.perm(T).long(), torch.argsort(ids, stable=True))
+
+
+# pairs as items of their own: rows of one unit to several K slices, slices and groups that are not full, more items than CTAs, warps that
+# carry two slices, layers without a shared expert
+@pytest.mark.parametrize("cfg", [configs.scaled(Q4, E=64, H=128, F=32, F_s=64, top_k=1), configs.scaled(Q4, E=64, H=1152, F=96, F_s=32, top_k=3),
+                                 configs.scaled(IQ3, E=64, H=4096, F=256, F_s=256, top_k=8), configs.scaled(IQ3, E=64, H=256, F=512, F_s=0, type_down=configs.IQ3_S),
+                                 configs.scaled(configs.NEMOTRON_Q4_0, E=64, H=2688, F=1856, F_s=3712, top_k=6),
+                                 configs.scaled(configs.NEMOTRON_Q4_0, E=32, H=640, F=800, F_s=1600, top_k=2),
+                                 configs.scaled(configs.NEMOTRON_Q4_0, E=32, H=384, F=1120, F_s=0, top_k=8)],
+                         ids=lambda c: f"{c.name}-{c.H}-{c.F}-{c.F_s}-{c.top_k}")
+@pytest.mark.parametrize("T", [1, 2, 5, 10, 40])
+def test_pairs_as_items(cfg, T):
+    _check(cfg, T, prefill=False)
+
+
+# a K-quant shared expert beside the pair kernels: one and two rows per step, every type, against the oracle and, bit for bit, against the
+# launches of its own that a larger batch takes
+@pytest.mark.parametrize("types", [(formats.TYPE_Q5_K, formats.TYPE_Q5_K), (formats.TYPE_Q4_K, formats.TYPE_Q6_K), (formats.TYPE_Q6_K, formats.TYPE_Q4_K)], ids=str)
+@pytest.mark.parametrize("H,F_s", [(256, 256), (1024, 512), (2048, 768), (1280, 1024), (2304, 512)])
+def test_kquant_shared_expert_beside_pairs(types, H, F_s):
+    cfg = configs.scaled(IQ3, E=64, top_k=8, H=H, F=256, F_s=F_s, type_sh_gate_up=types[0], type_sh_down=types[1])
+    raw = configs.make_layer(cfg, device="cuda")
+    tiled, T = MoeWeightsTiled(raw), 48
+    x, sc = configs.make_input(cfg, T, device="cuda"), MoeScratch(tiled, 48)
+    y = forward_moe(tiled, sc, x)
+    for n in (1, 4, 5, 10):
+        part = torch.cat([forward_moe(tiled, sc, x[t:t + n].contiguous()) for t in range(0, 20, n)])
+        assert torch.equal(part, y[:20]), n
+    _check(cfg, 3, prefill=False)
+    assert sc.status() == 0
+
+
+# residual + norm inside the router (up to four tokens, rows of up to 3072) and as a launch in front of it: the same bits, also in place
+@pytest.mark.parametrize("H", [256, 2048, 2176, 3072, 3200])
+@pytest.mark.parametrize("cfg", [Q4, configs.scaled(IQ3, type_sh_gate_up=formats.TYPE_Q5_K, type_sh_down=formats.TYPE_Q5_K)], ids=["q4", "q5k"])
+def test_residual_norm_in_the_router(cfg, H):
+    if H % 256 and cfg is not Q4:
+        pytest.skip("IQ3_S rows are multiples of 256")
+    cfg = configs.scaled(cfg, E=64, H=H, F=256, F_s=256)
+    tiled = MoeWeightsTiled(configs.make_layer(cfg, device="cuda"))
+    sc, gen = MoeScratch(tiled, 12), torch.Generator(device="cuda").manual_seed(H)
+    hidden, residual = (torch.randn(12, H, generator=gen, device="cuda") for _ in range(2))
+    norm = 1.0 + 0.1 * torch.randn(H, generator=gen, device="cuda")
+    res = residual.clone()
+    y = forward_moe_residual_norm(tiled, sc, hidden, res, norm, 1e-6)
+    assert torch.equal(res, hidden + residual)
+    for n in (1, 2, 3, 4):
+        part = residual.clone()
+        rows = [forward_moe_residual_norm(tiled, sc, hidden[t:t + n].contiguous(), part[t:t + n], norm, 1e-6) for t in range(0, 12, n)]
+        assert torch.equal(torch.cat(rows), y) and torch.equal(part, res), n
+    assert sc.status() == 0
+
+
+# equal probabilities everywhere: the lowest indices win, in the kernels that select their experts themselves and at the router's end
+@pytest.mark.parametrize("E,k", [(256, 8), (33, 8), (8, 8), (64, 1)])
+@pytest.mark.parametrize("T", [1, 3, 40])
+def test_equal_experts(E, k, T):
+    cfg = configs.scaled(Q4, E=E, top_k=k, H=256, F=64, F_s=64)
+    raw = configs.make_layer(cfg, device="cuda")
+    raw.router_weight[:] = raw.router_weight[0]
+    tiled = MoeWeightsTiled(raw)
+    sc, x = MoeScratch(tiled, T), configs.make_input(cfg, T, device="cuda")
+    forward_moe(tiled, sc, x)
+    want = torch.arange(k, device="cuda", dtype=torch.int32).expand(T, k)
+    assert torch.equal(sc.topk_indices(T), want)
+    forward_moe(tiled, sc, torch.zeros_like(x))
+    route_only(tiled, sc, x)
+    assert torch.equal(sc.topk_indices(T), want) and sc.status() == 0
