@@ -687,24 +687,31 @@ int chimere_b200_moe_forward(const chimere_moe_layer* w, const float* d_x, float
     return kshared_chain(w, T, d_y, ws, stream);
 }
 
+// The device's address of pinned host memory; null for any other.
+static float* pinned_address(const float* h) {
+    cudaPointerAttributes attr{};
+    if (cudaPointerGetAttributes(&attr, h) == cudaSuccess && attr.type == cudaMemoryTypeHost && attr.devicePointer) return static_cast<float*>(attr.devicePointer);
+    (void)cudaGetLastError();   // (an unregistered pointer leaves an error behind on older runtimes)
+    return nullptr;
+}
+constexpr size_t kFetchBytes = 256 * 1024;   // rows of up to so many bytes come in by a kernel
+
 int chimere_b200_moe_forward_host(const chimere_moe_layer* w, const float* h_x, float* h_y, int T, float* d_x, float* d_y,
                                   chimere_moe_workspace* ws, cudaStream_t stream) {
     if (!h_x || !h_y) return -1;
     int rc = check_call(w, d_x, d_y, T, ws, true);
     if (rc) return rc;
     const size_t bytes = (size_t)T * w->H * sizeof(float);
-    cudaError_t e = cudaMemcpyAsync(d_x, h_x, bytes, cudaMemcpyHostToDevice, stream);
+    const float* x_host = pinned_address(h_x);
+    cudaError_t e = x_host && bytes <= kFetchBytes ? launch_fetch_rows(x_host, d_x, (int64_t)T * w->H, stream)
+                                                   : cudaMemcpyAsync(d_x, h_x, bytes, cudaMemcpyHostToDevice, stream);
     if (e != cudaSuccess) return cuda_rc(e);
     // A pinned result buffer is addressable from the device under a pointer of its own: the last kernel then stores y
     // straight into host memory and the copy back (a second trip through the copy engine, serial behind the kernels) is
     // not needed.  Pageable memory, or a K-quant shared expert as launches of its own (the last of which reads y back), takes the staged copy.
     float* y_dev = d_y;
-    cudaPointerAttributes attr{};
-    const bool last_stores = !kshared(w) || (pairs_forward(w, T, ws) && pair_extras(w, ws).type);
-    if (last_stores && cudaPointerGetAttributes(&attr, h_y) == cudaSuccess && attr.type == cudaMemoryTypeHost && attr.devicePointer)
-        y_dev = static_cast<float*>(attr.devicePointer);
-    else
-        (void)cudaGetLastError();   // (an unregistered pointer leaves an error behind on older runtimes)
+    if (!kshared(w) || (pairs_forward(w, T, ws) && pair_extras(w, ws).type))
+        if (float* y_host = pinned_address(h_y)) y_dev = y_host;
     rc = chimere_b200_moe_forward(w, d_x, y_dev, T, ws, stream);
     if (rc) return rc;
     if (y_dev == d_y) {

@@ -466,6 +466,22 @@ cudaError_t launch_add_residual_rmsnorm(const float* hidden, float* residual, co
     return launch_pdl(add_residual_rmsnorm_kernel, dim3(T), 256, 0, stream, hidden, residual, weight, normed, H, eps);
 }
 
+// A batch's rows from pinned host memory (its device address) by ordinary loads: a few lines per SM over the bus, and the layer's kernels follow it
+// like one another, where a copy engine's transfer ends before the first of them is started (five tokens of H = 2048, a call of the host
+// entry: 50 us with the copy, 46 so).
+__global__ void __launch_bounds__(128) fetch_rows_kernel(const float* src, float* dst, int64_t n4, int64_t n) {
+    griddep_wait();   // (dst is the workspace of the call before)
+    if (threadIdx.x == 0) griddep_launch();
+    const int64_t i = (int64_t)blockIdx.x * 128 + threadIdx.x;
+    if (i < n4) reinterpret_cast<float4*>(dst)[i] = __ldcv(reinterpret_cast<const float4*>(src) + i);
+    else if (i - n4 < n - 4 * n4) dst[4 * n4 + i - n4] = __ldcv(src + 4 * n4 + i - n4);
+}
+cudaError_t launch_fetch_rows(const float* src, float* dst, int64_t n, cudaStream_t stream) {
+    const int64_t n4 = (((uintptr_t)src | (uintptr_t)dst) & 15) ? 0 : n / 4, threads = n4 + (n - 4 * n4);
+    if (n <= 0) return cudaSuccess;
+    return launch_pdl(fetch_rows_kernel, dim3((unsigned)((threads + 127) / 128)), 128, 0, stream, src, dst, n4, n);
+}
+
 // ------------------------------------------------------------------ launchers --------------
 constexpr int kSmemCap = 200 * 1024;
 

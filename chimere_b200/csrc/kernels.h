@@ -132,6 +132,8 @@ cudaError_t launch_quantize_q8_1(const float* x, void* out, int64_t ncols, int64
 cudaError_t launch_rmsnorm(const float* x, float* y, int T, int H, float eps, cudaStream_t stream);
 cudaError_t launch_add_residual_rmsnorm(const float* hidden, float* residual, const float* weight, float* normed, int T, int H, float eps,
                                         cudaStream_t stream);
+// dst[n] = src[n] with src in pinned host memory (its device address)
+cudaError_t launch_fetch_rows(const float* src, float* dst, int64_t n, cudaStream_t stream);
 // routing trace: ids as bytes [T][k] for the drafter tooling, and (optional) per-expert pair counts added into load[E]
 cudaError_t launch_routing_trace(const int32_t* topk_idx, uint8_t* trace, int32_t* load, int T, int k, int E, cudaStream_t stream);
 int down_tile_rows(int type_routed, int ncols_routed, int type_shared, int ncols_shared);

@@ -276,3 +276,23 @@ def test_equal_experts(E, k, T):
     forward_moe(tiled, sc, torch.zeros_like(x))
     route_only(tiled, sc, x)
     assert torch.equal(sc.topk_indices(T), want) and sc.status() == 0
+
+
+# rows from pinned memory (on any float boundary), from pageable memory, around the size up to which a kernel fetches them
+@pytest.mark.parametrize("T", [1, 5, 32, 33])
+def test_host_rows(T):
+    cfg = configs.scaled(Q4, E=64, H=2048, F=64, F_s=64)
+    tiled = MoeWeightsTiled(configs.make_layer(cfg, device="cuda"))
+    sc, x = MoeScratch(tiled, T), configs.make_input(cfg, T, device="cuda")
+    want = forward_moe(tiled, sc, x).cpu()
+    for shift in (0, 1, 2, None):
+        room = torch.empty(T * cfg.H + 4, pin_memory=shift is not None)
+        rows = room[shift or 0:(shift or 0) + T * cfg.H].reshape(T, cfg.H)
+        rows.copy_(x)
+        y = torch.empty(T, cfg.H, pin_memory=True)
+        for _ in range(3):   # (new values in the same buffer are seen)
+            rows.neg_()
+            forward_moe_host(tiled, sc, rows, y)
+        assert torch.equal(y, forward_moe(tiled, sc, -x).cpu())
+        rows.neg_()
+        assert torch.equal(forward_moe_host(tiled, sc, rows, y), want)
