@@ -75,14 +75,22 @@ int validate_layer(const chimere_moe_layer* w) {
     return 0;
 }
 
-// Decode batches whose every (token, expert) pair is an item of its own (pairs.cu).  us per layer against the work list's entries of one or
-// two pairs: 256 experts of 512 x 2048, top 8: 8 tokens 31 / 38, 24: 65 / 78, 40 tokens 101 / 115 (skewed 90 / 104); 128 of
-// 1856 x 2688, top 6: 1 token 24 / 28, 8: 88 / 101, 12: 121 / 136, 16: 159 / 172.
+// Packed experts (Q4_0, IQ3_S) in the decode entry: up to pair_batch()'s line every (token, expert) pair is an item of its own (pairs.cu), which
+// reads an expert once per pair, from L2 behind the first; above it 16 pairs of an expert share a tile (mma_tiles.cu), which costs as much
+// with one pair as with eight.  us per layer, pairs / tiles:
+//   256 experts of 512 x 2048, top 8, uniform routing: 32 tokens 81 / 111, 40: 101 / 127; skewed: 20: 49 / 47, 40: 90 / 62
+//   128 of 1856 x 2688, top 6: 8 tokens 88 / 101, 12: 121 / 122, 16: 159 / 142, 24 (on the GEMM) 189 / 180
+// (Before: 40 tokens 115 and 104, 64 tokens 192 and 145, now on the tiles 145 and 70.)  The best line depends on the routing, which the host does
+// not know: this one is where neither is slower than the work list's entries of one or two pairs were.
 bool pair_batch(const chimere_moe_layer* w, int T) {
     const int64_t P = (int64_t)T * w->top_k;
     return T <= 4 || (T <= 40 && ((int64_t)w->F * w->H > (1 << 21) ? 16 * P <= 9 * w->E : 4 * P <= 5 * w->E));
 }
+// ... and in the prefill entry: the tiles up to five pairs per expert, then the tcgen05 GEMM (GEMM / tiles: 256 experts 128 tokens 254 / 175 us,
+// 256: 278 / 219, 777: 378 / 425, skewed 128: 109 / 102, 256: 144 / 156; 128 of 1856 x 2688 128 tokens 331 / 298, 256: 374 / 437).
+bool prefill_mma(const chimere_moe_layer* w, int T) { return (int64_t)T * w->top_k <= 5 * (int64_t)w->E; }
 
+// Layers that neither takes (experts and shared expert of different packed types, rows too long for the tiles' shared memory):
 // From forward_gemm_tokens() tokens on the decode entry sends experts with at least kForwardGemmPairs pairs, and the shared expert,
 // to the grouped GEMM and the others to the GEMV kernels: a GEMM tile costs the same with 1 pair as with 16, a GEMV entry grows
 // with every pair.  Q4_0, us per layer, GEMV kernels alone / with the GEMM, uniform and (skewed) routing:
@@ -307,7 +315,7 @@ int chimere_b200_moe_route(const chimere_moe_layer* w, const float* d_x, int T, 
 
 static int kshared_chain(const chimere_moe_layer* w, int T, float* d_y, chimere_moe_workspace* ws, cudaStream_t stream);
 static int gemm_experts(const chimere_moe_layer* w, const chimere_moe_prefill_weights* pw, int E, int T, chimere_moe_workspace* ws, cudaStream_t stream,
-                        const void* d_packed = nullptr, int row_bytes = 0, bool mixed = false);
+                        const void* d_packed = nullptr, int row_bytes = 0, bool mixed = false, bool mma = false);
 static cudaError_t finish_tokens(const chimere_moe_layer* w, float* d_y, int T, chimere_moe_workspace* ws, cudaStream_t stream);
 static float* gemm_shared_rows(const chimere_moe_layer* w, int T, const chimere_moe_workspace* ws);
 static GemvParams gate_up_params(const chimere_moe_layer* w, int T, chimere_moe_workspace* ws, const Layout& L);
@@ -655,6 +663,19 @@ static int run_pairs(const chimere_moe_layer* w, const float* d_x, const float* 
     return e != cudaSuccess || !ks || x.type ? cuda_rc(e) : kshared_chain(w, T, d_y, ws, stream);
 }
 
+// Products of a batch on the warp-level MMA (mma_tiles.cu), 16 pairs of an expert at a time; w: without a K-quant shared expert.
+static bool mma_runs(const chimere_moe_layer* w, int T, chimere_moe_workspace* ws) {
+    if (w->layout != CHIMERE_LAYOUT_TILED32) return false;
+    const Layout L = make_layout(w, ws->max_T);
+    return mma_tiles_run(gate_up_params(w, T, ws, L), down_params(w, nullptr, T, ws, L));
+}
+static int run_mma(const chimere_moe_layer* w, int T, chimere_moe_workspace* ws, cudaStream_t stream) {
+    const Layout L = make_layout(w, ws->max_T);
+    cudaError_t e = launch_mma_gate_up(gate_up_params(w, T, ws, L), ws->offsets, w->E, stream);
+    if (e == cudaSuccess) e = launch_mma_down(down_params(w, nullptr, T, ws, L), ws->offsets, w->E, stream);
+    return cuda_rc(e);
+}
+
 int chimere_b200_moe_forward(const chimere_moe_layer* w, const float* d_x, float* d_y, int T, chimere_moe_workspace* ws,
                              cudaStream_t stream) {
     int rc = check_call(w, d_x, d_y, T, ws, true);
@@ -666,6 +687,14 @@ int chimere_b200_moe_forward(const chimere_moe_layer* w, const float* d_x, float
     const Layout L = make_layout(wr, ws->max_T);
     if (pairs_forward(w, T, ws)) {
         return run_pairs(w, d_x, nullptr, nullptr, nullptr, 0.0f, d_y, T, ws, stream);
+    } else if (!pair_batch(wr, T) && mma_runs(wr, T, ws)) {
+        RouteParams rp = route_params(wr, d_x, T, ws, ks);
+        rp.list_mode = 2;
+        e = launch_route(rp, stream);
+        if (e != cudaSuccess) return cuda_rc(e);
+        rc = run_mma(wr, T, ws, stream);
+        if (rc) return rc;
+        e = finish_tokens(wr, d_y, T, ws, stream);
     } else if (forward_gemm(wr, T) && ws->prefill_arena && ws->prefill_bytes >= prefill_arena(wr, ws->max_T).total &&
         tiled_bulk_runs(gate_up_params(wr, T, ws, L), down_params(wr, d_y, T, ws, L))) {
         RouteParams rp = route_params(wr, d_x, T, ws, ks);
@@ -912,7 +941,7 @@ static PrefillGemmMats gemm_mats(const chimere_moe_layer* w, const chimere_moe_p
 // of an exchange) are in place: token tiles of every expert with pairs (and of the shared expert; E = 0: of it alone), the
 // gate/up GEMM with the activation and the Q8_1 step, the down GEMM; per-pair rows land in ws->pair_out.
 static int gemm_experts(const chimere_moe_layer* w, const chimere_moe_prefill_weights* pw, int E, int T, chimere_moe_workspace* ws, cudaStream_t stream,
-                        const void* d_packed, int row_bytes, bool mixed) {
+                        const void* d_packed, int row_bytes, bool mixed, bool mma) {
     if (!ws->prefill_arena) return -1;
     if (w->layout != CHIMERE_LAYOUT_TILED32 || !prefill_dims_ok(w)) return -2;
     const PrefillArena A = prefill_arena(w, ws->max_T);
@@ -921,7 +950,8 @@ static int gemm_experts(const chimere_moe_layer* w, const chimere_moe_prefill_we
     int32_t* tiles = (int32_t*)(base + A.tiles);
     const Layout L = make_layout(w, ws->max_T);
     const int widest = mixed ? kForwardTileColumns : kTileColumns;
-    const int n_tiles_max = E > 0 ? n_tiles_max_for(w, T, widest) : (T + 127) / 128;
+    if (mma) E = 0;   // (the routed experts go elsewhere: tiles of the shared expert alone)
+    const int n_tiles_max = E > 0 ? n_tiles_max_for(w, T, widest) : kshared(w) ? (T + 31) / 32 : (T + 127) / 128;
     cudaError_t e = launch_build_tiles(ws->offsets, ws->perm, tiles, mixed ? ws->group_list : nullptr, E, T, w->F_s > 0, mixed ? kForwardGemmPairs : 1, kshared(w), widest, stream);
     if (e != cudaSuccess) return cuda_rc(e);
     // the rows' Q8_1 planes: the workspace's, or (expert-parallel owner) the received packed rows in place
@@ -965,7 +995,12 @@ static int gemm_experts(const chimere_moe_layer* w, const chimere_moe_prefill_we
                                 : tiled_gate_up_geom(w->type_up, w->type_sh_up, w->H, w->F_s > 0).wk;
             for (PrefillGemmMats& m : g.m) m.slice = m.ncols > 0 ? tiled_slice_units(m.type, m.ncols, wk) / 4 : 1;
         }
-        e = launch_prefill_gemm(g, down != 0, n_tiles_max, stream);
+        if (mma) {   // the routed experts' products in front; the tiles with minimums alone behind them
+            const chimere_moe_layer r = routed_only(w);
+            e = down ? launch_mma_down(down_params(&r, nullptr, T, ws, L), ws->offsets, r.E, stream) : launch_mma_gate_up(gate_up_params(&r, T, ws, L), ws->offsets, r.E, stream);
+            if (e != cudaSuccess) break;
+        }
+        e = launch_prefill_gemm(g, down != 0, n_tiles_max, mma, stream);
     }
     return cuda_rc(e);
 }
@@ -998,10 +1033,11 @@ int chimere_b200_moe_forward_prefill(const chimere_moe_layer* w, const chimere_m
     if (ws->prefill_bytes < prefill_arena(wr, ws->max_T).total || ((uintptr_t)ws->prefill_arena & 255)) return -4;
     if (prefill_as_decode(&route_, T)) return chimere_b200_moe_forward(w, d_x, d_y, T, ws, stream);
     RouteParams rp = route_params(&route_, d_x, T, ws, ks);
-    rp.list_mode = 2;   // no work entries: the tile builder makes its own list
+    rp.list_mode = 2;   // no work entries: the kernels make their own tiles
     cudaError_t e = launch_route(rp, stream);
     if (e != cudaSuccess) return cuda_rc(e);
-    rc = gemm_experts(wr, pw, wr->E, T, ws, stream);
+    const bool mma = prefill_mma(&route_, T) && mma_runs(&route_, T, ws);
+    rc = mma && !gemm ? run_mma(&route_, T, ws, stream) : gemm_experts(wr, pw, wr->E, T, ws, stream, nullptr, 0, false, mma);
     if (rc) return rc;
     e = finish_tokens(wr, d_y, T, ws, stream);
     if (e != cudaSuccess || !ks || gemm) return cuda_rc(e);

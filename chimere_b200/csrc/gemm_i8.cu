@@ -1149,12 +1149,13 @@ cudaError_t launch_gemm_i8_f32(const GemmParams& p_in, int n_items, int32_t* til
 }
 
 // The tile list's header words 4 (gate/up) and 5 (down) are the launches' tile counters; build_tiles_kernel zeroes them.
-cudaError_t launch_prefill_gemm(const PrefillGemmParams& p, bool down, int n_tiles_max, cudaStream_t stream) {
+cudaError_t launch_prefill_gemm(const PrefillGemmParams& p, bool down, int n_tiles_max, bool min_only, cudaStream_t stream) {
     const int n_items = n_tiles_max * p.row_tiles_max;
     if (n_items <= 0) return cudaSuccess;
     int32_t* counter = const_cast<int32_t*>(p.tiles) + (down ? 5 : 4);
-    cudaError_t e;
-    if (p.as_gemv) e = down ? launch_gemm<DownPolicy, kOrdered>(p, n_items, counter, stream) : launch_gemm<GateUpPolicy, kOrdered>(p, n_items, counter, stream);
+    cudaError_t e = cudaSuccess;
+    if (min_only) {}
+    else if (p.as_gemv) e = down ? launch_gemm<DownPolicy, kOrdered>(p, n_items, counter, stream) : launch_gemm<GateUpPolicy, kOrdered>(p, n_items, counter, stream);
     else e = down ? launch_gemm<DownPolicy>(p, n_items, counter, stream) : launch_gemm<GateUpPolicy>(p, n_items, counter, stream);
     if (e == cudaSuccess && p.m[1].type == kTypeOperandMin) {   // (words 6 / 7: these launches' counters)
         const int n_min = (p.T + 31) / 32 * p.m[1].row_tiles;

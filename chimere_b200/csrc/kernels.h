@@ -176,7 +176,8 @@ struct PrefillGemmParams {
     int as_gemv;                     // sums bit for bit as the GEMV kernels form them (packed weights, token tiles of up to 64 columns)
     int32_t* status;
 };
-cudaError_t launch_prefill_gemm(const PrefillGemmParams& p, bool down, int n_tiles_max, cudaStream_t stream);
+// min_only: the launch of the tiles with minimums alone, behind a kernel that has waited for what fills their operands
+cudaError_t launch_prefill_gemm(const PrefillGemmParams& p, bool down, int n_tiles_max, bool min_only, cudaStream_t stream);
 cudaError_t launch_build_tiles(const int32_t* offsets, const int32_t* perm, int32_t* tiles, int32_t* list, int E, int T, int has_shared, int gemm_min,
                                int shared_32, int widest, cudaStream_t stream);   // widest: columns of a full token tile, 128 or 64
 cudaError_t launch_gather_tiles(const int32_t* tiles, const int32_t* perm, const int8_t* x_q, int64_t x_q_stride, const float* x_d,
@@ -224,6 +225,10 @@ cudaError_t launch_pair_down(const RouteParams& r, const GemvParams& p, const Pa
 // the router's logits and the Q8_1 rows of normed = rmsnorm(residual + hidden) * weight; residual is left for launch_pair_gate_up
 bool route_norm_runs(const RouteParams& p);
 cudaError_t launch_route_norm(const RouteParams& p, const float* hidden, const float* residual, const float* weight, float eps, cudaStream_t stream);
+// batches whose experts hold a few tokens to a few dozen (mma_tiles.cu): from the dispatch step's offsets and perm, no list; per-pair rows only
+bool mma_tiles_run(const GemvParams& gate_up, const GemvParams& down);
+cudaError_t launch_mma_gate_up(const GemvParams& p, const int32_t* offsets, int E, cudaStream_t stream);
+cudaError_t launch_mma_down(const GemvParams& p, const int32_t* offsets, int E, cudaStream_t stream);
 cudaError_t launch_gate_up_tiled(const GemvParams& p, int max_entries, cudaStream_t stream);
 cudaError_t launch_down_tiled(const GemvParams& p, int max_entries, cudaStream_t stream);
 cudaError_t launch_block_sumi_tiled(int type, const void* packed, const void* xq8, int32_t* sumi, int ncols, int nrows,

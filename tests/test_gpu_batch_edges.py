@@ -223,6 +223,15 @@ def test_pairs_as_items(cfg, T):
     _check(cfg, T, prefill=False)
 
 
+# 16 pairs of an expert per tile: one column to a full tile and one more, eight and nine (the MMA's halves), ragged row tiles and K slices
+@pytest.mark.parametrize("cfg", [configs.scaled(Q4, E=1, top_k=1, H=512, F=256, F_s=256), configs.scaled(IQ3, E=1, top_k=1, H=1280, F=256, F_s=0),
+                                 configs.scaled(configs.NEMOTRON_Q4_0, E=1, top_k=1, H=640, F=1120, F_s=96), configs.scaled(Q4, E=3, top_k=2, H=128, F=64, F_s=64),
+                                 configs.scaled(IQ3, E=5, top_k=4, H=2048, F=512, F_s=512, type_down=configs.IQ3_S)], ids=lambda c: f"{c.name}-{c.H}-{c.F}-{c.F_s}")
+@pytest.mark.parametrize("T", [5, 8, 9, 15, 16, 17, 33, 70])
+def test_tiles_of_sixteen_pairs(cfg, T):
+    _check(cfg, T, prefill=False)
+
+
 # a K-quant shared expert beside the pair kernels: one and two rows per step, every type, against the oracle and, bit for bit, against the
 # launches of its own that a larger batch takes
 @pytest.mark.parametrize("types", [(formats.TYPE_Q5_K, formats.TYPE_Q5_K), (formats.TYPE_Q4_K, formats.TYPE_Q6_K), (formats.TYPE_Q6_K, formats.TYPE_Q4_K)], ids=str)
