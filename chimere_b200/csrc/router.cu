@@ -932,7 +932,7 @@ cudaError_t launch_ep_pack(const int32_t* topk_idx, const int8_t* x_q, const flo
 
 // The tiled product's three launches start to pay where the simple kernel (a CTA per 8 tokens x 8 experts, partials through shared
 // memory) fills the GPU more than once: 19.6 against 29 us at 61 x 257 outputs of H = 2048, 32 against 33 at 130 x 257.
-constexpr int64_t kRouteTileWork = 32768;
+constexpr int kRouteTileWork = 65536;
 template <int NQ>
 static cudaError_t launch_route_tiles(const RouteParams& p, cudaStream_t stream) {
     using R = RouteTile<NQ>;
@@ -975,7 +975,7 @@ cudaError_t launch_route(const RouteParams& p, cudaStream_t stream) {
         constexpr int TT = 8, TE = 2;
         dim3 grid((nrows + TE - 1) / TE, (p.T + TT - 1) / TT);
         return launch_pdl(route_kernel<TT, TE>, grid, 256, route_smem(TT, TE), stream, p);
-    } else if (p.scratch && (int64_t)p.T * p.E > kRouteTileWork && p.H <= 4096 && route_scratch_floats(p.T, p.E, p.H) <= p.scratch_floats) {
+    } else if (p.scratch && (int64_t)p.T * p.E * route_nq(p.H) > kRouteTileWork && p.H <= 4096 && route_scratch_floats(p.T, p.E, p.H) <= p.scratch_floats) {
         switch (route_nq(p.H)) {
             case 1: return launch_route_tiles<1>(p, stream);
             case 2: return launch_route_tiles<2>(p, stream);
