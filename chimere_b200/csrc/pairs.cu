@@ -88,7 +88,10 @@ __device__ __forceinline__ int dot16(const uint4& v, const uint4& q0, const uint
 
 // One group of one or two matrices against the token at shared addresses xq (int8 plane) / xd ({ f32 scale, correction word } per
 // unit), both of the group's first unit; nu units.  The registers are asked for again from group gn of tiles na / nb (nn units there).
-template <int TYPE, bool DUAL>
+// AHEAD: a unit's token values are loaded in front of the products of the unit before (a warp issues in order), where there are registers
+// for that: ungated experts of 1856 columns, 12 tokens, four layers 466 -> 441 us (and 416 with three groups of a down row in flight instead of
+// four, which spilled 108 bytes); gated ones and short down rows gain nothing.
+template <int TYPE, bool DUAL, bool AHEAD>
 __device__ __forceinline__ void pair_group(PairGroup<TYPE>& ra, PairGroup<TYPE>& rb, int g, int nu, uint32_t xq, uint32_t xd, float& acc_a, float& acc_b,
                                            const uint8_t* na, const uint8_t* nb, int gn, int nn, int lane) {
     constexpr bool kLow = Tiled<TYPE>::kCorrLow, kGroupScale = Tiled<TYPE>::kGroupScale;
@@ -97,13 +100,17 @@ __device__ __forceinline__ void pair_group(PairGroup<TYPE>& ra, PairGroup<TYPE>&
     float pa = 0.0f, pb = 0.0f;
     uint32_t sa = 0, sb = 0;
     if constexpr (TYPE == CHIMERE_TYPE_IQ3_S) { sa = ra.sc >> (16 * (g & 1)); if (DUAL) sb = rb.sc >> (16 * (g & 1)); }
+    uint4 q0[2], q1[2];
+    uint2 dc[2];
+    auto token = [&](int u) { q0[u & 1] = lds128(xq + u * 32); q1[u & 1] = lds128(xq + u * 32 + 16); dc[u & 1] = lds64(xd + u * 8); };
+    if (AHEAD) token(0);
 #pragma unroll
     for (int u = 0; u < kGroupUnits; ++u) {
+        if (AHEAD ? u + 1 < kGroupUnits : u < nu) token(AHEAD ? u + 1 : u);
         if (u < nu) {
-            const uint4 q0 = lds128(xq + u * 32), q1 = lds128(xq + u * 32 + 16);
-            const uint2 dc = lds64(xd + u * 8);
-            const float dx = __uint_as_float(dc.x);
-            int ta = dot16(ra.v[u], q0, q1, (int)dc.y, kLow), tb = DUAL ? dot16(rb.v[u], q0, q1, (int)dc.y, kLow) : 0;
+            const float dx = __uint_as_float(dc[u & 1].x);
+            const int corr = (int)dc[u & 1].y;
+            int ta = dot16(ra.v[u], q0[u & 1], q1[u & 1], corr, kLow), tb = DUAL ? dot16(rb.v[u], q0[u & 1], q1[u & 1], corr, kLow) : 0;
             if constexpr (TYPE == CHIMERE_TYPE_IQ3_S) {
                 ta *= (int)(1u + 2u * ((sa >> (4 * u)) & 15u));
                 pa = fmaf((float)ta, dx, pa);
@@ -253,7 +260,7 @@ __global__ void __launch_bounds__(256, CTAS) pair_gate_up_kernel(const __grid_co
                 const int g = gg + d;
                 if (g < ng) {
                     const bool same = g + D < ng;
-                    pair_group<TYPE, DUAL>(ra[d], rb[d], g0 + g, 4, xq + (uint32_t)g * 128, xd + (uint32_t)g * 32, acc_u, acc_g, same ? ta : na, same ? tg : ngt,
+                    pair_group<TYPE, DUAL, true>(ra[d], rb[d], g0 + g, 4, xq + (uint32_t)g * 128, xd + (uint32_t)g * 32, acc_u, acc_g, same ? ta : na, same ? tg : ngt,
                                            g0 + (same ? g + D : d), same || more ? 4 : 0, lane);
                 }
             }
@@ -423,7 +430,7 @@ __global__ void __launch_bounds__(THREADS, CTAS) pair_down_kernel(const __grid_c
                 const int g = gg + d;
                 if (g < ng) {
                     const bool same = g + D < ng;
-                    pair_group<TYPE, false>(ra[d], rb, g0 + g, units(g), xq + (uint32_t)g * 128, xd + (uint32_t)g * 32, acc, none, same ? ta : na, nullptr,
+                    pair_group<TYPE, false, (D > 1)>(ra[d], rb, g0 + g, units(g), xq + (uint32_t)g * 128, xd + (uint32_t)g * 32, acc, none, same ? ta : na, nullptr,
                                             g0 + (same ? g + D : d), same ? units(g + D) : more ? units(d) : 0, lane);
                     if (--left == 0 || g + 1 == ng) { mine[s * 32 + lane] = acc; acc = 0.0f; left = gpw; ++s; }
                 }
@@ -539,8 +546,8 @@ cudaError_t launch_pair_gate_up(const RouteParams& r, const GemvParams& p, const
 
 template <int TYPE>
 static cudaError_t launch_pair_dn_t(const RouteParams& r, const GemvParams& p, const PairExtras& x, const PairDown& c, int threads, cudaStream_t stream) {
-    if (x.type) return launch_pair_dn<TYPE, true, 4, 512, 1>(r, p, x, c, threads, stream);
-    if (threads > 288) return launch_pair_dn<TYPE, false, 4, 512, 1>(r, p, x, c, threads, stream);
+    if (x.type) return launch_pair_dn<TYPE, true, 3, 512, 1>(r, p, x, c, threads, stream);
+    if (threads > 288) return launch_pair_dn<TYPE, false, 3, 512, 1>(r, p, x, c, threads, stream);
     // Up to one item per SM the whole tile is in flight at once.  Else two CTAs per SM with two groups in flight each, or three with one where
     // that saves a round of items (256 experts of 512 columns, H = 2048, us per layer: 5 tokens 26.8 / 23.1, 8: 30.9 / 31.9, 16: 49.6 / 47.7).
     const int n = p.T * (p.H / 32), sms = sm_count();
