@@ -287,7 +287,7 @@ static RouteParams route_params(const chimere_moe_layer* w, const float* d_x, in
     const Layout L = make_layout(w, ws->max_T);
     p.list_capacity = L.max_entries;
     const size_t combine_ints = (size_t)L.n_counters - kCtrRouteTile - (ws->max_T + 7) / 8;
-    const size_t need = (size_t)((T * w->top_k + 127) / 128) * 256 + 260;
+    const size_t need = dispatch_scratch_ints(T, w->top_k);
     // the router of a large batch rewrites its rows into the per-pair output area, which the down stage fills only later; its
     // first T rows may hold the input (the residual + norm entry)
     p.scratch = ws->pair_out + (size_t)T * w->H;

@@ -43,9 +43,14 @@ struct RouteParams {
     int wait_n, wait_expect;    // ... `wait_n` of them, each has to reach `wait_expect`; they are taken down again (null = none)
     float* scratch;             // room for the rewritten rows of a large batch's router (16-byte aligned; may be null)
     size_t scratch_floats;
-    int32_t* dispatch_scratch;  // zeroed scratch for the dispatch of large batches: ceil(T*top_k / 128) * 256 + 260 ints, left
-                                // zeroed again; null = always sort in one CTA
+    int32_t* dispatch_scratch;  // zeroed scratch for the dispatch of large batches: dispatch_scratch_ints, left zeroed again; null = always
+                                // sort in one CTA
 };
+// the dispatch of a large batch goes by chunks of whole tokens, at most 128 pairs
+constexpr int kDispatchChunk = 128;
+inline int dispatch_tokens(int top_k) { return kDispatchChunk / top_k; }
+inline int dispatch_chunks(int T, int top_k) { return (T + dispatch_tokens(top_k) - 1) / dispatch_tokens(top_k); }
+inline size_t dispatch_scratch_ints(int T, int top_k) { return (size_t)dispatch_chunks(T, top_k) * 256 + 260; }
 
 // Grouped GEMV over work entries (see common.cuh for the list layout).
 struct GemvParams {

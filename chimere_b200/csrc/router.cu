@@ -29,6 +29,60 @@ __device__ __forceinline__ void quantize_block_q8_1(float xi, uint8_t* out, int 
     if (lane == 0) *plane_d = __half2float(dh);
 }
 
+// Q8_1 of a whole row by a CTA of 256, four elements per lane and four blocks per warp step: a third of the instructions of a block per
+// warp (quantize_block_q8_1), same bits -- the sum's butterfly has its strides 16, 8 and 4 across lanes and 2 and 1 within one.
+__device__ __forceinline__ void quantize_row_q8_1(const float* src, int H, uint8_t* out, int8_t* plane_q, float* plane_d, int tid, int lane, int warp) {
+    const bool aligned = ((uintptr_t)src & 15) == 0;
+    for (int f0 = warp * 32; f0 < H >> 2; f0 += 256) {
+        const int f = f0 + lane;
+        const bool on = f < H >> 2;
+        float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        if (on) {
+            if (aligned) { const float4 x = *reinterpret_cast<const float4*>(src + 4 * f); v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w; }
+            else
+#pragma unroll
+                for (int c = 0; c < 4; ++c) v[c] = src[4 * f + c];
+        }
+        float t[4];
+        uint32_t m = 0u;   // largest magnitude: bit patterns of non-negative floats order like the values, with the NaNs above infinity
+#pragma unroll
+        for (int c = 0; c < 4; ++c) { t[c] = v[c]; m = max(m, __float_as_uint(fabsf(v[c]))); }
+#pragma unroll
+        for (int s = 4; s > 0; s >>= 1) {
+            m = max(m, __shfl_xor_sync(0xffffffffu, m, s));
+#pragma unroll
+            for (int c = 0; c < 4; ++c) t[c] += __shfl_xor_sync(0xffffffffu, t[c], s);
+        }
+        const float sum = (t[0] + t[2]) + (t[1] + t[3]);
+        float amax = __uint_as_float(m), d;
+        int q[4];
+        if (__all_sync(0xffffffffu, !on || (amax > 1e-25f && amax < 1e25f))) {
+            d = div_by_recip(amax, 127.0f, 1.0f / 127.0f);
+            const float r = __frcp_rn(d);
+#pragma unroll
+            for (int c = 0; c < 4; ++c) q[c] = round_int(div_by_recip(v[c], d, r));
+        } else {   // (see q8_1_warp)
+            amax = fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fmaxf(fabsf(v[2]), fabsf(v[3])));
+#pragma unroll
+            for (int s = 4; s > 0; s >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, s));
+            d = amax / 127.0f;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) q[c] = amax == 0.0f ? 0 : (int)(int8_t)roundf(v[c] / d);
+        }
+        if (on) {
+            const uint32_t w = (uint32_t)(q[0] & 255) | ((uint32_t)(q[1] & 255) << 8) | ((uint32_t)(q[2] & 255) << 16) | ((uint32_t)(q[3] & 255) << 24);
+            uint8_t* blk = out + (size_t)(f >> 3) * kQ81Bytes;
+            *reinterpret_cast<uint32_t*>(blk + 4 + 4 * (f & 7)) = w;
+            *reinterpret_cast<uint32_t*>(plane_q + 4 * f) = w;
+            if ((f & 7) == 0) {
+                const __half dh = __float2half(d);
+                *reinterpret_cast<__half2*>(blk) = __halves2half2(dh, __float2half(sum));
+                plane_d[f >> 3] = __half2float(dh);
+            }
+        }
+    }
+}
+
 // grid = (row tiles, token tiles), 256 threads; TOKENS_X: (token tiles, row tiles), for more than the 65535 token tiles that the
 // second dimension holds.  Thread p owns partial sum p of every output of the tile: elements p, p+256, ... in ascending order, one
 // fused multiply-add each.
@@ -268,13 +322,7 @@ __global__ void __launch_bounds__(256) route_prep_kernel(const RouteParams p) {
             if (i * 256 + tid < H) acc = fmaf(p.shexp_gate_w[i * 256 + tid], v[i], acc);
         red[tid] = acc;
     }
-    const int nbH = H >> 5;
-#pragma unroll
-    for (int i = 0; i < 4 * NQ; ++i) {
-        const int b = i * 8 + warp;
-        if (b < nbH) quantize_block_q8_1(v[i], p.x_q8 + ((size_t)row * nbH + b) * kQ81Bytes, lane, p.x_soa_q + (size_t)row * H + b * 32,
-                                         p.x_soa_d + (size_t)row * p.x_soa_d_stride + b);
-    }
+    quantize_row_q8_1(src, H, p.x_q8 + (size_t)row * (H >> 5) * kQ81Bytes, p.x_soa_q + (size_t)row * H, p.x_soa_d + (size_t)row * p.x_soa_d_stride, tid, lane, warp);
     if (p.shexp_gate_w) {
         __syncthreads();
         if (warp == 0) {
@@ -412,16 +460,30 @@ __global__ void __launch_bounds__(256, 2) route_tile_kernel(const RouteParams p)
     }
 }
 
-// Scores and top-k, one warp per token; unless the dispatch follows as launches of its own, the last CTA does it.
+// Scores and top-k, one warp per token; unless the dispatch follows as launches of its own (hist: its counts, a chunk of `tokens` per CTA), the
+// last CTA does it (tokens = 0: nobody here).
 constexpr int kTopkIdsRoom = 4096;
-__global__ void __launch_bounds__(256) route_topk_kernel(const RouteParams p, int split_dispatch) {
+__global__ void __launch_bounds__(256) route_topk_kernel(const RouteParams p, int32_t* hist, int tokens) {
     extern __shared__ __align__(16) float smem_f[];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, t = blockIdx.x * 8 + warp;
     __shared__ int s_flag;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     griddep_wait();
     if (tid == 0) griddep_launch();
+    if (hist) {
+        int* cnt = reinterpret_cast<int*>(smem_f);
+        int* ids = cnt + 256;
+        cnt[tid] = 0;
+        const int t0 = blockIdx.x * tokens, n = min(tokens, p.T - t0);
+        for (int a = warp; a < n; a += 8) topk_warp(p, p.router_logits + (size_t)(t0 + a) * p.E, t0 + a, lane, ids + a * p.top_k);
+        __syncthreads();
+        if (tid < n * p.top_k) atomicAdd(cnt + ids[tid], 1);
+        __syncthreads();
+        hist[(size_t)blockIdx.x * 256 + tid] = cnt[tid];
+        return;
+    }
+    const int t = blockIdx.x * 8 + warp;
     if (t < p.T) topk_warp(p, p.router_logits + (size_t)t * p.E, t, lane, nullptr);
-    if (split_dispatch) return;
+    if (tokens == 0) return;
     __syncthreads();   // every thread's writes are ordered before thread 0's counter increment, which releases them
     if (tid == 0) s_flag = (atom_add_acq_rel_gpu(&p.counters[kCtrRouteAll], 1) == (int)gridDim.x - 1);   // ... and acquires the other CTAs'
     __syncthreads();
@@ -432,20 +494,19 @@ __global__ void __launch_bounds__(256) route_topk_kernel(const RouteParams p, in
 
 // ---- dispatch of a large batch in three small launches --------------------------------------
 // One CTA sorting tens of thousands of pairs is a serial tail of hundreds of microseconds, so large batches split
-// the same stable counting sort over the GPU: chunks of 128 consecutive pairs are counted per expert (hist),
-// one CTA turns the counts into every chunk's first position within every expert and into the experts' offsets
-// (scan), and the chunks place their own pairs (place); whoever finishes last writes the GEMV work list.
-// Scratch: hist[chunks][256] + 260 ints behind it, zero before and after (it shares memory with the combine
+// the same stable counting sort over the GPU: chunks of up to 128 consecutive pairs are counted per expert -- by the top-k
+// kernel, where a chunk is few tokens, else by a launch --, a warp per expert turns the counts into every chunk's first position within
+// it and the last CTA the totals into offsets (scan), and the chunks place their own pairs (place); whoever finishes last writes the GEMV
+// work list.  Scratch: hist[chunks][256] + 260 ints behind it, zero before and after (it shares memory with the combine
 // counters of the down stage, which need zeros).
-constexpr int kDispatchChunk = 128;
-__host__ __device__ inline int dispatch_chunks(int P) { return (P + kDispatchChunk - 1) / kDispatchChunk; }
-__host__ __device__ inline size_t dispatch_scratch_ints(int P) { return (size_t)dispatch_chunks(P) * 256 + 260; }
 
-__global__ void __launch_bounds__(kDispatchChunk) dispatch_hist_kernel(const RouteParams p, int32_t* hist) {
+__global__ void __launch_bounds__(kDispatchChunk) dispatch_hist_kernel(const RouteParams p, int32_t* hist, int chunk) {
     __shared__ int s_ids[kDispatchChunk];
-    const int tid = threadIdx.x, P = p.T * p.top_k, q = blockIdx.x * kDispatchChunk + tid;
+    const int tid = threadIdx.x, P = p.T * p.top_k, q = blockIdx.x * chunk + tid;
     const int istr = p.idx_stride > 1 ? p.idx_stride : 1;
-    int e = q < P ? __ldcg(p.topk_idx + (size_t)q * istr) : -1;
+    griddep_wait();
+    if (tid == 0) griddep_launch();
+    int e = tid < chunk && q < P ? __ldcg(p.topk_idx + (size_t)q * istr) : -1;
     s_ids[tid] = (e >= 0 && e < p.E) ? e : -1;
     __syncthreads();
     for (int x = tid; x < 256; x += kDispatchChunk) {
@@ -456,39 +517,50 @@ __global__ void __launch_bounds__(kDispatchChunk) dispatch_hist_kernel(const Rou
     }
 }
 
-// One CTA of 1024: thread = (quarter of the chunks, expert).  hist[chunk][e] becomes the number of pairs of expert e in earlier
-// chunks.  Two passes over the counts (sums of the quarters, then the running counts), sixteen independent loads in flight: the
-// latency of a serial walk over the chunks was the kernel (26 us at 512 chunks by 256 threads with eight loads in flight).
-__global__ void __launch_bounds__(1024) dispatch_scan_kernel(const RouteParams p, int32_t* hist, int nchunks) {
+// A warp per expert, a run of consecutive chunks per lane: hist[chunk][e] becomes the number of pairs of expert e in earlier chunks.  (One CTA
+// for all experts: 24 us at 512 chunks, of latency and one SM's loads; now 5.)
+constexpr int kScanBatch = 16;
+__global__ void __launch_bounds__(256) dispatch_scan_kernel(const RouteParams p, int32_t* hist, int nchunks) {
     __shared__ int scan[16];
-    __shared__ int part[4][256];
-    const int tid = threadIdx.x & 255, quarter = threadIdx.x >> 8, lane = tid & 31, warp = tid >> 5;
-    const int per = (nchunks + 3) / 4, c0 = min(nchunks, quarter * per), c1 = min(nchunks, c0 + per);
-    int32_t* col = hist + tid;
-    constexpr int kBatch = 16;
-    int sum = 0;
-    for (int c = c0; c < c1; c += kBatch) {
-        int v[kBatch];
+    __shared__ int s_flag;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, e = blockIdx.x * 8 + warp;
+    griddep_wait();
+    if (tid == 0) griddep_launch();
+    int32_t* ent_base = hist + (size_t)nchunks * 256;   // [257] first routed entry of each expert, then their number; [259] CTAs done here
+    {
+        const int per = (nchunks + 31) / 32, c0 = min(nchunks, lane * per), c1 = min(nchunks, c0 + per);
+        int32_t* col = hist + e;
+        int sum = 0;
+        for (int c = c0; c < c1; c += kScanBatch) {
+            int v[kScanBatch];
 #pragma unroll
-        for (int i = 0; i < kBatch; ++i) v[i] = c + i < c1 ? col[(size_t)(c + i) * 256] : 0;
+            for (int i = 0; i < kScanBatch; ++i) v[i] = c + i < c1 ? __ldcg(col + (size_t)(c + i) * 256) : 0;
 #pragma unroll
-        for (int i = 0; i < kBatch; ++i) sum += v[i];
+            for (int i = 0; i < kScanBatch; ++i) sum += v[i];
+        }
+        int run = sum;
+#pragma unroll
+        for (int s = 1; s < 32; s <<= 1) {
+            const int a = __shfl_up_sync(0xffffffffu, run, s);
+            if (lane >= s) run += a;
+        }
+        if (lane == 31) ent_base[e] = run;   // (the expert's pairs, until the last CTA has them)
+        run -= sum;
+        for (int c = c0; c < c1; c += kScanBatch) {
+            int v[kScanBatch];
+#pragma unroll
+            for (int i = 0; i < kScanBatch; ++i) v[i] = c + i < c1 ? __ldcg(col + (size_t)(c + i) * 256) : 0;
+#pragma unroll
+            for (int i = 0; i < kScanBatch; ++i)
+                if (c + i < c1) { col[(size_t)(c + i) * 256] = run; run += v[i]; }
+        }
     }
-    part[quarter][tid] = sum;
+    __syncthreads();   // every thread's writes are ordered before thread 0's counter increment, which releases them
+    if (tid == 0) s_flag = (atom_add_acq_rel_gpu(ent_base + 259, 1) == (int)gridDim.x - 1);   // ... and acquires the other CTAs'
     __syncthreads();
-    int run = 0;
-    for (int q = 0; q < quarter; ++q) run += part[q][tid];
-    for (int c = c0; c < c1; c += kBatch) {
-        int v[kBatch];
-#pragma unroll
-        for (int i = 0; i < kBatch; ++i) v[i] = c + i < c1 ? col[(size_t)(c + i) * 256] : 0;
-#pragma unroll
-        for (int i = 0; i < kBatch; ++i)
-            if (c + i < c1) { col[(size_t)(c + i) * 256] = run; run += v[i]; }
-    }
-    if (quarter > 0) return;
-    run = part[0][tid] + part[1][tid] + part[2][tid] + part[3][tid];
-    const int cnt = tid < p.E ? run : 0;
+    if (!s_flag) return;
+    if (tid == 0) ent_base[259] = 0;
+    const int cnt = tid < p.E ? __ldcg(ent_base + tid) : 0;
     const int nent = (cnt + kMaxGroupTokens - 1) / kMaxGroupTokens;
     int incl_c = cnt, incl_n = nent;
 #pragma unroll
@@ -497,21 +569,22 @@ __global__ void __launch_bounds__(1024) dispatch_scan_kernel(const RouteParams p
         if (lane >= sft) { incl_c += a; incl_n += b; }
     }
     if (lane == 31) { scan[warp] = incl_c; scan[8 + warp] = incl_n; }
-    dispatch_sync();   // (the first quarter's 256 threads)
+    __syncthreads();
     int base_c = 0, base_n = 0;
     for (int w = 0; w < warp; ++w) { base_c += scan[w]; base_n += scan[8 + w]; }
-    int32_t* ent_base = hist + (size_t)nchunks * 256;   // [257] first routed entry of each expert, then their number
     if (tid < p.E) p.offsets[tid] = base_c + incl_c - cnt;
     ent_base[tid] = base_n + incl_n - nent;
     if (tid == 255) { p.offsets[p.E] = base_c + incl_c; ent_base[256] = base_n + incl_n; }
 }
 
-__global__ void __launch_bounds__(kDispatchChunk) dispatch_place_kernel(const RouteParams p, int32_t* hist, int nchunks) {
+__global__ void __launch_bounds__(kDispatchChunk) dispatch_place_kernel(const RouteParams p, int32_t* hist, int nchunks, int chunk) {
     __shared__ int s_ids[kDispatchChunk];
     __shared__ int s_last;
-    const int tid = threadIdx.x, P = p.T * p.top_k, q = blockIdx.x * kDispatchChunk + tid;
+    const int tid = threadIdx.x, P = p.T * p.top_k, q = blockIdx.x * chunk + tid;
     const int istr = p.idx_stride > 1 ? p.idx_stride : 1;
-    int e = q < P ? __ldcg(p.topk_idx + (size_t)q * istr) : -1;
+    griddep_wait();
+    if (tid == 0) griddep_launch();
+    int e = tid < chunk && q < P ? __ldcg(p.topk_idx + (size_t)q * istr) : -1;
     if (e < 0 || e >= p.E) e = -1;
     s_ids[tid] = e;
     __syncthreads();
@@ -565,12 +638,14 @@ __global__ void __launch_bounds__(kDispatchChunk) dispatch_place_kernel(const Ro
     for (int x = tid; x < 258; x += kDispatchChunk) ent_base[x] = 0;
 }
 
-static cudaError_t launch_dispatch_split(const RouteParams& p, cudaStream_t stream) {
-    const int nchunks = dispatch_chunks(p.T * p.top_k);
-    dispatch_hist_kernel<<<nchunks, kDispatchChunk, 0, stream>>>(p, p.dispatch_scratch);
-    dispatch_scan_kernel<<<1, 1024, 0, stream>>>(p, p.dispatch_scratch, nchunks);
-    dispatch_place_kernel<<<nchunks, kDispatchChunk, 0, stream>>>(p, p.dispatch_scratch, nchunks);
-    return cudaGetLastError();
+// counted: the top-k kernel has left the counts
+static cudaError_t launch_dispatch_split(const RouteParams& p, bool counted, cudaStream_t stream) {
+    const int nchunks = dispatch_chunks(p.T, p.top_k), chunk = dispatch_tokens(p.top_k) * p.top_k;
+    cudaError_t e = cudaSuccess;
+    if (!counted) e = launch_pdl(dispatch_hist_kernel, dim3(nchunks), kDispatchChunk, 0, stream, p, p.dispatch_scratch, chunk);
+    if (e == cudaSuccess) e = launch_pdl(dispatch_scan_kernel, dim3(32), 256, 0, stream, p, p.dispatch_scratch, nchunks);
+    if (e == cudaSuccess) e = launch_pdl(dispatch_place_kernel, dim3(nchunks), kDispatchChunk, 0, stream, p, p.dispatch_scratch, nchunks, chunk);
+    return e;
 }
 // Batches from this many pairs on take the three-launch dispatch (below, the single CTA at the router's end is faster).
 constexpr int kSplitDispatchPairs = 4096;
@@ -866,7 +941,7 @@ static size_t route_smem(int TT, int TE) {
 }
 
 cudaError_t launch_permute(const RouteParams& p, cudaStream_t stream) {
-    if (use_split_dispatch(p) && !p.wait_flags) return launch_dispatch_split(p, stream);
+    if (use_split_dispatch(p) && !p.wait_flags) return launch_dispatch_split(p, false, stream);
     permute_kernel<<<1, 256, (kDispatchSmemInts + kPermuteIdsRoom) * sizeof(int), stream>>>(p);
     return cudaGetLastError();
 }
@@ -942,9 +1017,12 @@ static cudaError_t launch_route_tiles(const RouteParams& p, cudaStream_t stream)
     if (e == cudaSuccess) e = launch_pdl(route_tile_kernel<NQ>, dim3((p.E + R::kExp - 1) / R::kExp, (p.T + R::kTok - 1) / R::kTok), 256, R::kSmem, stream, p);
     if (e != cudaSuccess) return e;
     const bool split = use_split_dispatch(p);
-    const size_t smem = (split ? 2048 : kDispatchSmemInts + kTopkIdsRoom) * 4;
-    e = launch_pdl(route_topk_kernel, dim3((p.T + 7) / 8), 256, smem, stream, p, split ? 1 : 0);
-    return e == cudaSuccess && split ? launch_dispatch_split(p, stream) : e;
+    // (four tokens per warp at most: with fewer experts per token the counts are a launch of their own)
+    const bool counted = split && p.top_k >= 4;
+    const int tokens = counted ? dispatch_tokens(p.top_k) : 8;
+    e = counted ? launch_pdl(route_topk_kernel, dim3(dispatch_chunks(p.T, p.top_k)), 256, (256 + kDispatchChunk) * 4, stream, p, p.dispatch_scratch, tokens)
+                : launch_pdl(route_topk_kernel, dim3((p.T + 7) / 8), 256, (kDispatchSmemInts + kTopkIdsRoom) * 4, stream, p, (int32_t*)nullptr, split ? 0 : tokens);
+    return e == cudaSuccess && split ? launch_dispatch_split(p, counted, stream) : e;
 }
 
 bool route_norm_runs(const RouteParams& p) { return p.T <= 4 && p.H <= 256 * 12; }

@@ -305,3 +305,38 @@ def test_host_rows(T):
         assert torch.equal(y, forward_moe(tiled, sc, -x).cpu())
         rows.neg_()
         assert torch.equal(forward_moe_host(tiled, sc, rows, y), want)
+
+
+# the dispatch of a large batch: counts by the top-k kernel (four experts per token and more) and by a launch, chunks that 128 is no multiple
+# of, a last chunk of one token, more chunks than a lane of the scan takes at a time
+@pytest.mark.parametrize("k,T", [(1, 4096), (1, 4225), (3, 1366), (4, 1024), (6, 683), (7, 10009), (8, 512), (8, 513), (8, 8209)])
+def test_dispatch_of_large_batches(k, T):
+    cfg = configs.scaled(Q4, E=40, top_k=k, H=2048, F=32, F_s=0)
+    tiled, x = MoeWeightsTiled(configs.make_layer(cfg, device="cuda")), configs.make_input(cfg, T, device="cuda")
+    sc = MoeScratch(tiled, T)
+    for _ in range(2):   # (the scratch is left as it was found)
+        route_only(tiled, sc, x)
+        ids = sc.topk_indices(T).flatten()
+        assert torch.equal(sc.perm(T).long(), torch.argsort(ids, stable=True))
+        assert torch.equal(sc.offsets().long(), torch.cat([ids.new_zeros(1), torch.bincount(ids, minlength=cfg.E).cumsum(0)]).long())
+    assert sc.status() == 0
+
+
+# Q8_1 of whole rows: rows of any float alignment, blocks of zeros, of tiny and huge values, of NaN and infinities, against the one-warp form
+def test_rows_quantised_four_elements_per_lane():
+    cfg = configs.scaled(Q4, E=128, top_k=1, H=1152, F=32, F_s=0)
+    tiled, T = MoeWeightsTiled(configs.make_layer(cfg, device="cuda")), 600
+    sc, small = MoeScratch(tiled, T), MoeScratch(tiled, 8)
+    room = torch.empty(T * cfg.H + 1, device="cuda")
+    for shift in (0, 1):
+        x = room[shift:shift + T * cfg.H].reshape(T, cfg.H)
+        x.copy_(configs.make_input(cfg, T, device="cuda"))
+        x[0] = 0.0
+        x[1] *= 1e-30
+        x[2] *= 1e30
+        x[3, 40], x[3, 70], x[3, 200] = float("nan"), float("inf"), -float("inf")
+        x[4, ::3] = 0.0
+        x[5, 32:64] *= 1e-38
+        route_only(tiled, sc, x)
+        route_only(tiled, small, x[:8].contiguous())
+        assert torch.equal(sc.x_q8(T)[:8], small.x_q8(8))
