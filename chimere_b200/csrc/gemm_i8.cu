@@ -30,6 +30,8 @@
 // three-operand f32x2 multiply-adds themselves take 3.2 cycles per warp (two operand pairs of the three fresh: register ports),
 // i.e. 410 of those cycles.  Narrow tiles: the weight bytes, and what a stage costs its warps however few columns it has
 // (an MMA takes 46 cycles at least, a commit another hundred; the read-back's shares are dealt stage by stage).
+// The same tiles on the warp-level MMA, sums in registers, two CTAs of eight warps: 8192 tokens 1888 -> 2080 us, 256 wide 371 -> 437: too few
+// warps to cover the way from an MMA to its multiply-adds.
 // All waits are bounded; a wait that runs out raises a status bit, nothing blocks for good, and the CTA still
 // frees its TMEM.
 #include "common.cuh"
@@ -1342,9 +1344,10 @@ __global__ void __launch_bounds__(256) build_tiles_kernel(const int32_t* offsets
 }
 
 // Token tiles of the gate/up GEMM: the Q8_1 planes of each tile's tokens in the MMA's operand order.
-// grid = (max tiles, 16 groups of 8 token slots), 256 threads = 8 slots x 32 chunk lanes: the eight slots of a group
-// are the 8 x 16 bytes of one core-matrix row group, so every 128-byte segment of the tile is written whole, and a
-// token's 16-byte chunks are read four in a row.  Columns without a token are left as they are (nobody reads their sums).
+// grid = (max tiles, 16 groups of 8 token slots), a warp takes 8 chunks of 16 bytes of the group's eight tokens at a time: read row by row
+// (128 bytes in a row), turned in shared memory, written as the 8 x 16 bytes of one core-matrix row group.  Columns without a token are
+// left as they are (nobody reads their sums).  Bound by L1 wavefronts: lanes that read the eight tokens side by side, as their stores want them,
+// took 32 a load where a row takes 4 (8192 tokens x 8 of 2048 columns: 74 -> 55 us; 512 x 8: 14.9 -> 14.0, where the chain tile, pair, row is the time).
 __global__ void __launch_bounds__(256) gather_tiles_kernel(const int32_t* tiles, const int32_t* perm, const int8_t* x_q, int64_t x_q_stride,
                                                            const float* x_d, int x_d_stride, const uint8_t* x_q8, uint8_t* b_tiles,
                                                            int64_t b_col16_bytes, int H, int top_k, int shared_sums, int T) {
@@ -1359,19 +1362,42 @@ __global__ void __launch_bounds__(256) gather_tiles_kernel(const int32_t* tiles,
         if (!shared_sums || i * 32 >= T) return;
         t = make_int4(-1, i * 32, min(32, T - i * 32), __ldcg(tiles + 1) + 2 * i);
     }
-    const int sl = threadIdx.x & 7, lane_ch = threadIdx.x >> 3;
+    __shared__ uint4 s_turn[8][2][8 * 9];   // (a row of nine: no two lanes of a quarter warp on the same banks, either way)
+    const int sl = threadIdx.x & 7, lane_ch = threadIdx.x >> 3, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const bool sums = t.x < 0 && shared_sums;   // a shared expert with minimums
     const int c = grp * 8 + sl, npad = sums ? 32 : tile_width(t.z);   // token slot of the tile
-    if (c >= t.z) return;
-    const int tok = t.x < 0 ? t.y + c : __ldcg(perm + t.y + c) / top_k;
+    if (grp * 8 >= t.z) return;
+    auto token = [&](int c) { return c >= t.z ? -1 : t.x < 0 ? t.y + c : __ldcg(perm + t.y + c) / top_k; };
+    const int rows[2] = {token(grp * 8 + (lane >> 3)), token(grp * 8 + 4 + (lane >> 3))};
+    const int tok = token(c), nch = H / 16;
     uint8_t* base = b_tiles + (size_t)t.w * b_col16_bytes;
     // a shared expert with minimums: blocks in tree order, stages of four, each with the blocks' sums (the Q8_1 rows' second half) behind it
     auto place = [&](int b) { return sums ? operand_min_block(b, H / 32) : b; };
     auto block = [&](int b) { return base + (sums ? (size_t)(b >> 2) * (npad * 160) + (b & 3) * (npad * 36) : (size_t)b * (npad * 36)); };
-    for (int ch = lane_ch; ch < H / 16; ch += 32) {
-        const uint4 v = __ldcg(reinterpret_cast<const uint4*>(x_q + (size_t)tok * x_q_stride) + ch);
-        *reinterpret_cast<uint4*>(block(place(ch >> 1)) + (ch & 1) * (npad * 16) + grp * 128 + sl * 16) = v;
+    for (int g = warp * 8; g < nch; g += 128) {
+        uint4 v[2][2];
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int ch = g + 64 * u + (lane & 7);
+                v[u][h] = ch < nch && rows[h] >= 0 ? __ldcg(reinterpret_cast<const uint4*>(x_q + (size_t)rows[h] * x_q_stride) + ch) : make_uint4(0u, 0u, 0u, 0u);
+            }
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) s_turn[warp][u][((lane >> 3) + 4 * h) * 9 + (lane & 7)] = v[u][h];
+        __syncwarp();
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int i = 4 * h + (lane >> 3), ch = g + 64 * u + i;
+                if (ch < nch && tok >= 0) *reinterpret_cast<uint4*>(block(place(ch >> 1)) + (ch & 1) * (npad * 16) + grp * 128 + sl * 16) = s_turn[warp][u][sl * 9 + i];
+            }
+        __syncwarp();
     }
+    if (tok < 0) return;
     for (int b = lane_ch; b < H / 32; b += 32) {
         const int at = place(b);
         *reinterpret_cast<float*>(block(at) + npad * 32 + c * 4) = __ldcg(x_d + (size_t)tok * x_d_stride + b);
