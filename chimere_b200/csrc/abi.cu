@@ -3,7 +3,7 @@
 // The layer-level entries are the C++ counterpart of the reference's Rust orchestration
 // (forward_moe_cudarc_with_cache, chimere-server/src/qwen35_model/moe_ffn.rs:1081-1768, and its
 // scratch owner GgmlGpuBuffers, src/kernels/ggml_gpu.rs:292-407): they validate, lay the
-// caller's arena out, and enqueue three kernels per decode call (eight where the grouped GEMM takes
+// caller's arena out, and enqueue three kernels per decode call (up to nine where the grouped GEMM takes
 // part, up to eleven in prefill).  Nothing here allocates device memory or synchronises, except chimere_b200_moe_forward_host which waits for its stream.
 #include <cstdio>
 #include <cstring>
@@ -148,7 +148,7 @@ bool forward_gemm(const chimere_moe_layer* w, int T) {
     return T >= forward_gemm_tokens(w) && w->layout == CHIMERE_LAYOUT_TILED32 && prefill_dims_ok(w) && packed_types(w);
 }
 // Whether a batch is too small for the prefill entry's GEMM: tiles of mostly one pair.  256 IQ3_S experts of 512 x 2048, 16 tokens: uniform
-// routing 115 us on the GEMM, 57 as decode (103 when the prefill entry left experts of fewer than eight pairs to the GEMV kernels), skewed
+// routing 115 us on the GEMM, 57 as decode, 48 on the pair kernels (103 when the prefill entry left experts of fewer than eight pairs to the GEMV kernels), skewed
 // routing 47 and 53; eight experts, one token 43 and 26.  Q8_0 weights, whose GEMV entries fill an SM each, are the faster on the GEMM at one token.
 bool prefill_as_decode(const chimere_moe_layer* w, int T) { return 2 * (int64_t)T * w->top_k <= w->E && packed_types(w); }
 
@@ -630,9 +630,13 @@ int chimere_b200_moe_down_combine(const chimere_moe_layer* w, float* d_y, int T,
 
 // Decode batches up to pair_batch()'s line run without a work list where the pair kernels take the layer: the router's logits, then
 // two launches that select their experts themselves.  A K-quant shared expert rides along or follows as kshared_chain.
-static PairExtras pair_extras(const chimere_moe_layer* w, chimere_moe_workspace* ws) {
+// Up to five tokens it rides along: a row of it decodes its blocks for every token, and kshared_chain for eight at a time.  us per layer (256 IQ3_S /
+// Q4_0 experts, Q5_K shared, in the pair launches / behind them): 1 token 18.3 / 20.3, 4: 28.2 / 29.4, 5: 33.9 / 34.3, 6: 37.1 / 35.9, 12: 59.9 / 54.1,
+// 33: 143.8 / 107.7 (123.9 on the work list).
+constexpr int kPairKquantTokens = 5;
+static PairExtras pair_extras(const chimere_moe_layer* w, int T, chimere_moe_workspace* ws) {
     PairExtras x{};
-    if (!kshared(w) || !pairs_take_kquant(*w)) return x;
+    if (!kshared(w) || T > kPairKquantTokens || !pairs_take_kquant(*w)) return x;
     x.type = w->type_sh_up; x.type_down = w->type_sh_down; x.F_s = w->F_s;
     x.gate = (const uint8_t*)w->sh_gate; x.up = (const uint8_t*)w->sh_up; x.down = (const uint8_t*)w->sh_down;
     x.rows = ws->pair_out;
@@ -643,14 +647,14 @@ static bool pairs_forward(const chimere_moe_layer* w, int T, chimere_moe_workspa
     if (!pair_batch(w, T) || w->layout != CHIMERE_LAYOUT_TILED32) return false;
     const chimere_moe_layer wr = kshared(w) ? routed_only(w) : *w;
     const Layout L = make_layout(&wr, ws->max_T);
-    return pairs_run(gate_up_params(&wr, T, ws, L), down_params(&wr, nullptr, T, ws, L), pair_extras(w, ws));
+    return pairs_run(gate_up_params(&wr, T, ws, L), down_params(&wr, nullptr, T, ws, L), pair_extras(w, T, ws));
 }
 static int run_pairs(const chimere_moe_layer* w, const float* d_x, const float* d_hidden, float* d_residual, const float* d_norm_weight, float eps, float* d_y, int T,
                      chimere_moe_workspace* ws, cudaStream_t stream) {
     const bool ks = kshared(w);
     const chimere_moe_layer wr = ks ? routed_only(w) : *w;
     const Layout L = make_layout(&wr, ws->max_T);
-    PairExtras x = pair_extras(w, ws);
+    PairExtras x = pair_extras(w, T, ws);
     RouteParams rp = route_params(&wr, d_x, T, ws, ks);
     rp.logits_only = 1;
     cudaError_t e;
@@ -739,7 +743,7 @@ int chimere_b200_moe_forward_host(const chimere_moe_layer* w, const float* h_x, 
     // straight into host memory and the copy back (a second trip through the copy engine, serial behind the kernels) is
     // not needed.  Pageable memory, or a K-quant shared expert as launches of its own (the last of which reads y back), takes the staged copy.
     float* y_dev = d_y;
-    if (!kshared(w) || (pairs_forward(w, T, ws) && pair_extras(w, ws).type))
+    if (!kshared(w) || (pairs_forward(w, T, ws) && pair_extras(w, T, ws).type))
         if (float* y_host = pinned_address(h_y)) y_dev = y_host;
     rc = chimere_b200_moe_forward(w, d_x, y_dev, T, ws, stream);
     if (rc) return rc;
