@@ -282,7 +282,7 @@ __global__ void __launch_bounds__(256) route_norm_kernel(const RouteParams p, co
 // are split over WP warps of the CTA and meet in shared memory once at the end.
 //   route_prep_kernel : one CTA per token or router row: the row rewritten in that order (below), and for a token the Q8_1 form
 //                       and the shared expert's gate logit
-//   route_tile_kernel : CTA tile of 32 tokens x 16 experts, its eight warps with an eighth of the partials each; chunks of two
+//   route_tile_kernel : CTA tile of 32 tokens x 16 experts (16 x 16 in small batches), its eight warps with an eighth of the partials each; chunks of two
 //                       partials come through a ring of bulk copies of every warp's own (no CTA barrier until the end)
 //   route_topk_kernel : scores and top-k, one warp per token; the last CTA does the dispatch
 // Bound by the FMA pipe and its operands: 8 LDS.128 per 64 multiply-adds and thread.  (The form before it kept one partial of 32
@@ -332,10 +332,11 @@ __global__ void __launch_bounds__(256) route_prep_kernel(const RouteParams p) {
     }
 }
 
-template <int NQ> struct RouteTile {
-    static constexpr int kTok = 32, kExp = 16, kWarps = 8, kPitch = route_pitch(NQ), kSteps = kRouteChunks / kWarps;
-    static constexpr int kStage = (kTok + kExp) * kPitch, kRing = 2;   // floats of a warp's stage; two CTAs per SM up to NQ = 2
-    static constexpr int kLevels = 4, kPending = (kLevels - 1) * 16 * 256;   // pending sums of the levels above the first
+// TA: tokens of a thread (tokens of a tile / 8)
+template <int NQ, int TA> struct RouteTile {
+    static constexpr int kTok = 8 * TA, kExp = 16, kOut = 4 * TA, kWarps = 8, kPitch = route_pitch(NQ), kSteps = kRouteChunks / kWarps;
+    static constexpr int kStage = (kTok + kExp) * kPitch, kRing = TA == 2 && NQ > 2 ? 4 : 2;   // floats of a warp's stage; two CTAs per SM up to NQ = 2
+    static constexpr int kLevels = 4, kPending = (kLevels - 1) * kOut * 256;   // pending sums of the levels above the first
     static constexpr size_t kSmem = ((size_t)kWarps * kRing * kStage + kPending) * 4;
     static_assert(kSteps == 1 << kLevels, "a warp's chunks are the leaves of its part of the tree");
     static_assert(kTok * kExp <= kRing * kStage, "the shares of the outputs meet in the ring's memory");
@@ -348,9 +349,9 @@ __device__ __forceinline__ float4 lds_f4(uint32_t a) {
 }
 
 // grid = (expert tiles, token tiles)
-template <int NQ>
+template <int NQ, int TA>
 __global__ void __launch_bounds__(256, 2) route_tile_kernel(const RouteParams p) {
-    using R = RouteTile<NQ>;
+    using R = RouteTile<NQ, TA>;
     extern __shared__ __align__(128) float smem_f[];
     __shared__ __align__(8) uint64_t s_full[R::kWarps][R::kRing];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -382,7 +383,7 @@ __global__ void __launch_bounds__(256, 2) route_tile_kernel(const RouteParams p)
     // pending sums: the first level's in registers, the others in shared memory, thread beside thread (a register file of them
     // would leave one CTA per SM, local memory costs a small batch 10 us of first touches)
     float* st = smem_f + R::kWarps * R::kRing * R::kStage + tid;
-    float pend[16], v[16];
+    float pend[R::kOut], v[R::kOut];
     bool ok = true;
     uint32_t phase = 0;
     int slot = 0;
@@ -391,16 +392,16 @@ __global__ void __launch_bounds__(256, 2) route_tile_kernel(const RouteParams p)
         const uint32_t xs = xs0 + 4u * (slot * R::kStage), ws = ws0 + 4u * (slot * R::kStage);
 #pragma unroll
         for (int j = 0; j < kRoutePartials; ++j) {
-            float acc[16];
+            float acc[R::kOut];
 #pragma unroll
-            for (int i = 0; i < 16; ++i) acc[i] = 0.0f;
+            for (int i = 0; i < R::kOut; ++i) acc[i] = 0.0f;
 #pragma unroll
             for (int q = 0; q < NQ; ++q) {
                 float4 w[4];
 #pragma unroll
                 for (int b = 0; b < 4; ++b) w[b] = lds_f4(ws + 4u * (4 * b * R::kPitch + (j * NQ + q) * 4));
 #pragma unroll
-                for (int a = 0; a < 4; ++a) {
+                for (int a = 0; a < TA; ++a) {
                     const float4 x = lds_f4(xs + 4u * (8 * a * R::kPitch + (j * NQ + q) * 4));
 #pragma unroll
                     for (int b = 0; b < 4; ++b) acc[4 * a + b] = fmaf(w[b].x, x.x, acc[4 * a + b]);   // ascending elements, one fused multiply-add each
@@ -413,7 +414,7 @@ __global__ void __launch_bounds__(256, 2) route_tile_kernel(const RouteParams p)
                 }
             }
 #pragma unroll
-            for (int i = 0; i < 16; ++i) v[i] = j == 0 ? acc[i] : v[i] + acc[i];
+            for (int i = 0; i < R::kOut; ++i) v[i] = j == 0 ? acc[i] : v[i] + acc[i];
         }
         __syncwarp();   // every lane has read the slot
         if (lane == 0 && k + R::kRing < R::kSteps) ask(slot);
@@ -421,20 +422,20 @@ __global__ void __launch_bounds__(256, 2) route_tile_kernel(const RouteParams p)
         // the binary counter: v completes level after level as long as that level has a pending left half
         if (!(k & 1)) {
 #pragma unroll
-            for (int i = 0; i < 16; ++i) pend[i] = v[i];
+            for (int i = 0; i < R::kOut; ++i) pend[i] = v[i];
             continue;
         }
 #pragma unroll
-        for (int i = 0; i < 16; ++i) v[i] += pend[i];
+        for (int i = 0; i < R::kOut; ++i) v[i] += pend[i];
 #pragma unroll
         for (int l = 1; l < R::kLevels; ++l) {
-            float* sl = st + (l - 1) * 16 * 256;
+            float* sl = st + (l - 1) * R::kOut * 256;
             if ((k >> l) & 1) {
 #pragma unroll
-                for (int i = 0; i < 16; ++i) v[i] += sl[i * 256];
+                for (int i = 0; i < R::kOut; ++i) v[i] += sl[i * 256];
             } else {
 #pragma unroll
-                for (int i = 0; i < 16; ++i) sl[i * 256] = v[i];
+                for (int i = 0; i < R::kOut; ++i) sl[i * 256] = v[i];
                 break;
             }
         }
@@ -446,7 +447,7 @@ __global__ void __launch_bounds__(256, 2) route_tile_kernel(const RouteParams p)
     __syncwarp();
     // the warps' shares of every output, each in its own ring's memory (row pitch 17: the lanes of a store on different banks)
 #pragma unroll
-    for (int a = 0; a < 4; ++a)
+    for (int a = 0; a < TA; ++a)
 #pragma unroll
         for (int b = 0; b < 4; ++b) ring[(tg + 8 * a) * 17 + eg + 4 * b] = v[4 * a + b];
     __syncthreads();
@@ -1008,13 +1009,27 @@ cudaError_t launch_ep_pack(const int32_t* topk_idx, const int8_t* x_q, const flo
 // The tiled product's three launches start to pay where the simple kernel (a CTA per 8 tokens x 8 experts, partials through shared
 // memory) fills the GPU more than once: 19.6 against 29 us at 61 x 257 outputs of H = 2048, 32 against 33 at 130 x 257.
 constexpr int kRouteTileWork = 65536;
+// Tiles of 16 tokens instead of 32 while all of them run at once, two per SM (one where a row has more than 2048 columns, whose rings are then four
+// deep: a warp alone on its SM quarter waits for its copies).  Prefill call, us, 32 / 16: 256 experts of H = 2048, 160 tokens 120.6 / 112.8, 256: 137.0 /
+// 130.6, 288: 147.0 / 144.0, 384 and 512 (over the line) 166.4 / 168.1, 189.5 / 194.0; 128 of H = 2688, 180 tokens 352.6 / 347.5, 256: 371.9 / 367.4 (372.9 /
+// 373.4 with a ring of two), 512 (over the line) 505.8 / 510.3.
+template <int NQ, int TA> static int64_t route_tiles(const RouteParams& p) {
+    using R = RouteTile<NQ, TA>;
+    return (int64_t)((p.E + R::kExp - 1) / R::kExp) * ((p.T + R::kTok - 1) / R::kTok);
+}
+template <int NQ, int TA>
+static cudaError_t launch_route_tile(const RouteParams& p, cudaStream_t stream) {
+    using R = RouteTile<NQ, TA>;
+    static bool attr_done[64] = {};
+    const cudaError_t e = max_smem_once(route_tile_kernel<NQ, TA>, (int)R::kSmem, attr_done);
+    if (e != cudaSuccess) return e;
+    return launch_pdl(route_tile_kernel<NQ, TA>, dim3((p.E + R::kExp - 1) / R::kExp, (p.T + R::kTok - 1) / R::kTok), 256, R::kSmem, stream, p);
+}
 template <int NQ>
 static cudaError_t launch_route_tiles(const RouteParams& p, cudaStream_t stream) {
-    using R = RouteTile<NQ>;
-    static bool attr_done[64] = {};
-    cudaError_t e = max_smem_once(route_tile_kernel<NQ>, (int)R::kSmem, attr_done);
-    if (e == cudaSuccess) e = launch_pdl(route_prep_kernel<NQ>, dim3(p.T + p.E), 256, 0, stream, p);
-    if (e == cudaSuccess) e = launch_pdl(route_tile_kernel<NQ>, dim3((p.E + R::kExp - 1) / R::kExp, (p.T + R::kTok - 1) / R::kTok), 256, R::kSmem, stream, p);
+    const bool half = route_tiles<NQ, 2>(p) <= (NQ > 2 ? 1 : 2) * sm_count();
+    cudaError_t e = launch_pdl(route_prep_kernel<NQ>, dim3(p.T + p.E), 256, 0, stream, p);
+    if (e == cudaSuccess) e = half ? launch_route_tile<NQ, 2>(p, stream) : launch_route_tile<NQ, 4>(p, stream);
     if (e != cudaSuccess) return e;
     const bool split = use_split_dispatch(p);
     // (four tokens per warp at most: with fewer experts per token the counts are a launch of their own)

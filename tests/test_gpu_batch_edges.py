@@ -86,6 +86,12 @@ def test_tiled_router(H, T):
     _check(configs.scaled(Q4, E=256, H=H, F=64, F_s=64), T, prefill=False)
 
 
+# ... and around a tile of 16 and the line between the two, with a last tile of a few experts
+@pytest.mark.parametrize("E,H,T", [(70, 4096, 239), (70, 3200, 465), (70, 1152, 471), (72, 2048, 944), (72, 2048, 945), (200, 1024, 335)])
+def test_tiled_router_of_small_tiles(E, H, T):
+    _check(configs.scaled(Q4, E=E, H=H, F=64, F_s=64), T, prefill=False)
+
+
 # The decode entry sends popular experts to the GEMM and the others to the GEMV kernels; a token's row is the same bits either way,
 # whatever the batch: odd numbers of K slices and units, IQ3_S in both places, a shared expert narrower than the routed ones.
 @pytest.mark.parametrize("cfg", [configs.scaled(Q4, E=16, F=256, F_s=512, H=2048, name="q4"),
