@@ -1344,16 +1344,17 @@ __global__ void __launch_bounds__(256) build_tiles_kernel(const int32_t* offsets
 }
 
 // Token tiles of the gate/up GEMM: the Q8_1 planes of each tile's tokens in the MMA's operand order.
-// grid = (max tiles, 16 groups of 8 token slots), a warp takes 8 chunks of 16 bytes of the group's eight tokens at a time: read row by row
+// grid = (max tiles, kCtas), a CTA takes every kCtas-th group of 8 token slots of its tile, a warp 8 chunks of 16 bytes of the group's eight tokens at a time: read row by row
 // (128 bytes in a row), turned in shared memory, written as the 8 x 16 bytes of one core-matrix row group.  Columns without a token are
 // left as they are (nobody reads their sums).  Bound by L1 wavefronts: lanes that read the eight tokens side by side, as their stores want them,
 // took 32 a load where a row takes 4 (8192 tokens x 8 of 2048 columns: 74 -> 55 us; 512 x 8: 14.9 -> 14.0, where the chain tile, pair, row is the time).
+template <int kCtas>
 __global__ void __launch_bounds__(256) gather_tiles_kernel(const int32_t* tiles, const int32_t* perm, const int8_t* x_q, int64_t x_q_stride,
                                                            const float* x_d, int x_d_stride, const uint8_t* x_q8, uint8_t* b_tiles,
                                                            int64_t b_col16_bytes, int H, int top_k, int shared_sums, int T) {
     griddep_wait();
     if (threadIdx.x == 0) griddep_launch();
-    const int j = blockIdx.x, grp = blockIdx.y;
+    const int j = blockIdx.x;
     const int listed = __ldcg(tiles);
     int4 t;
     if (j < listed) t = __ldcg(reinterpret_cast<const int4*>(tiles + kTileHeader) + j);
@@ -1365,46 +1366,56 @@ __global__ void __launch_bounds__(256) gather_tiles_kernel(const int32_t* tiles,
     __shared__ uint4 s_turn[8][2][8 * 9];   // (a row of nine: no two lanes of a quarter warp on the same banks, either way)
     const int sl = threadIdx.x & 7, lane_ch = threadIdx.x >> 3, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const bool sums = t.x < 0 && shared_sums;   // a shared expert with minimums
-    const int c = grp * 8 + sl, npad = sums ? 32 : tile_width(t.z);   // token slot of the tile
-    if (grp * 8 >= t.z) return;
+    const int npad = sums ? 32 : tile_width(t.z), nch = H / 16;
+    if ((int)blockIdx.y * 8 >= t.z) return;
+    // the tokens of the CTA's groups: those whose rows this lane reads, and the one of the slot that it writes
     auto token = [&](int c) { return c >= t.z ? -1 : t.x < 0 ? t.y + c : __ldcg(perm + t.y + c) / top_k; };
-    const int rows[2] = {token(grp * 8 + (lane >> 3)), token(grp * 8 + 4 + (lane >> 3))};
-    const int tok = token(c), nch = H / 16;
+    int rows[16 / kCtas][2], toks[16 / kCtas];
+#pragma unroll
+    for (int n = 0; n < 16 / kCtas; ++n) {
+        const int c0 = (blockIdx.y + n * kCtas) * 8;
+        rows[n][0] = token(c0 + (lane >> 3)); rows[n][1] = token(c0 + 4 + (lane >> 3)); toks[n] = token(c0 + sl);
+    }
     uint8_t* base = b_tiles + (size_t)t.w * b_col16_bytes;
     // a shared expert with minimums: blocks in tree order, stages of four, each with the blocks' sums (the Q8_1 rows' second half) behind it
     auto place = [&](int b) { return sums ? operand_min_block(b, H / 32) : b; };
     auto block = [&](int b) { return base + (sums ? (size_t)(b >> 2) * (npad * 160) + (b & 3) * (npad * 36) : (size_t)b * (npad * 36)); };
-    for (int g = warp * 8; g < nch; g += 128) {
-        uint4 v[2][2];
 #pragma unroll
-        for (int u = 0; u < 2; ++u)
+    for (int n = 0; n < 16 / kCtas; ++n) {
+        const int grp = blockIdx.y + n * kCtas, c = grp * 8 + sl, tok = toks[n];
+        if (grp * 8 >= t.z) return;
+        for (int g = warp * 8; g < nch; g += 128) {
+            uint4 v[2][2];
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const int ch = g + 64 * u + (lane & 7);
-                v[u][h] = ch < nch && rows[h] >= 0 ? __ldcg(reinterpret_cast<const uint4*>(x_q + (size_t)rows[h] * x_q_stride) + ch) : make_uint4(0u, 0u, 0u, 0u);
-            }
+            for (int u = 0; u < 2; ++u)
 #pragma unroll
-        for (int u = 0; u < 2; ++u)
+                for (int h = 0; h < 2; ++h) {
+                    const int ch = g + 64 * u + (lane & 7);
+                    v[u][h] = ch < nch && rows[n][h] >= 0 ? __ldcg(reinterpret_cast<const uint4*>(x_q + (size_t)rows[n][h] * x_q_stride) + ch) : make_uint4(0u, 0u, 0u, 0u);
+                }
 #pragma unroll
-            for (int h = 0; h < 2; ++h) s_turn[warp][u][((lane >> 3) + 4 * h) * 9 + (lane & 7)] = v[u][h];
-        __syncwarp();
+            for (int u = 0; u < 2; ++u)
 #pragma unroll
-        for (int u = 0; u < 2; ++u)
+                for (int h = 0; h < 2; ++h) s_turn[warp][u][((lane >> 3) + 4 * h) * 9 + (lane & 7)] = v[u][h];
+            __syncwarp();
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const int i = 4 * h + (lane >> 3), ch = g + 64 * u + i;
-                if (ch < nch && tok >= 0) *reinterpret_cast<uint4*>(block(place(ch >> 1)) + (ch & 1) * (npad * 16) + grp * 128 + sl * 16) = s_turn[warp][u][sl * 9 + i];
-            }
-        __syncwarp();
-    }
-    if (tok < 0) return;
-    for (int b = lane_ch; b < H / 32; b += 32) {
-        const int at = place(b);
-        *reinterpret_cast<float*>(block(at) + npad * 32 + c * 4) = __ldcg(x_d + (size_t)tok * x_d_stride + b);
-        if (sums) {
-            const uint32_t ds = __ldcg(reinterpret_cast<const uint32_t*>(x_q8 + ((size_t)tok * (H / 32) + b) * kQ81Bytes));
-            *reinterpret_cast<float*>(base + (size_t)(at >> 2) * (npad * 160) + npad * 144 + (at & 3) * (npad * 4) + c * 4) = h2f(ds >> 16);
+            for (int u = 0; u < 2; ++u)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int i = 4 * h + (lane >> 3), ch = g + 64 * u + i;
+                    if (ch < nch && tok >= 0) *reinterpret_cast<uint4*>(block(place(ch >> 1)) + (ch & 1) * (npad * 16) + grp * 128 + sl * 16) = s_turn[warp][u][sl * 9 + i];
+                }
+            __syncwarp();
         }
+        if (tok >= 0)
+            for (int b = lane_ch; b < H / 32; b += 32) {
+                const int at = place(b);
+                *reinterpret_cast<float*>(block(at) + npad * 32 + c * 4) = __ldcg(x_d + (size_t)tok * x_d_stride + b);
+                if (sums) {
+                    const uint32_t ds = __ldcg(reinterpret_cast<const uint32_t*>(x_q8 + ((size_t)tok * (H / 32) + b) * kQ81Bytes));
+                    *reinterpret_cast<float*>(base + (size_t)(at >> 2) * (npad * 160) + npad * 144 + (at & 3) * (npad * 4) + c * 4) = h2f(ds >> 16);
+                }
+            }
     }
 }
 
@@ -1417,7 +1428,10 @@ cudaError_t launch_gather_tiles(const int32_t* tiles, const int32_t* perm, const
                                 int x_d_stride, const uint8_t* x_q8, uint8_t* b_tiles, int64_t b_col16_bytes, int H, int top_k, int n_tiles_max,
                                 bool shared_sums, int T, cudaStream_t stream) {
     if (n_tiles_max <= 0) return cudaSuccess;
-    return launch_pdl(gather_tiles_kernel, dim3(n_tiles_max, 16), 256, 0, stream, tiles, perm, x_q, x_q_stride, x_d, x_d_stride, x_q8, b_tiles, b_col16_bytes,
+    // eight CTAs per tile rather than sixteen, most of which have nothing to do, up to four tiles per SM.  Prefill call, us, 16 / 8: 256 Q8_0 experts, skewed, 512
+    // tokens 188.1 / 185.9, 1024: 305.0 / 302.0, 2048: 526.7 / 523.3, 8192 (over the line) 1876 / 1886; with four 189.9, 304.6, 523.9, 1892
+    auto* kernel = n_tiles_max <= 4 * sm_count() ? gather_tiles_kernel<8> : gather_tiles_kernel<16>;
+    return launch_pdl(kernel, dim3(n_tiles_max, n_tiles_max <= 4 * sm_count() ? 8 : 16), 256, 0, stream, tiles, perm, x_q, x_q_stride, x_d, x_d_stride, x_q8, b_tiles, b_col16_bytes,
                       H, top_k, shared_sums ? 1 : 0, T);
 }
 
