@@ -620,6 +620,7 @@ def main():
             # table (None when this kernel and shape have not been captured)
             "traffic": traffic, "traffic_source": traffic_src,
             "us_per_launch": gu_secs * 1e6, "algorithmic_bytes_per_launch": gu_bytes,
+            "note": "the stage entries' kernels, over the work list; the layer call runs pair_gate_up_kernel and pair_down_kernel, timed under 'layer'",
             "down_kernel": {"achieved": dn_bytes / dn_secs / 1e9, "frac": dn_bytes / dn_secs / 1e9 / hbm_peak,
                             "us_per_launch": dn_secs * 1e6, "algorithmic_bytes_per_launch": dn_bytes},
             "route_kernel": {"us_per_launch": rt_secs * 1e6},

@@ -1,4 +1,5 @@
-// gemv_tiled.cu -- the decode-path GEMV kernels on tiled32 weights (see tiled.cuh).
+// gemv_tiled.cu -- the GEMV kernels of a work list on tiled32 weights (see tiled.cuh): Q8_0 and mixed-type layers, batches beside the grouped
+// GEMM, the step-wise and expert-parallel entries.  Packed layers in decode calls run on pairs.cu and mma_tiles.cu.
 //
 // One warp = 32 consecutive rows of one expert matrix, lane = row: a warp-wide 128-bit load is one
 // contiguous 512-byte read of the tiled layout and hands every lane whole 32-weight units of its own
