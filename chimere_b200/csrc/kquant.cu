@@ -46,7 +46,7 @@ __global__ void __launch_bounds__(32 * kRowsPerCta) kquant_mmvq_kernel(const uin
         decode_sub<TYPE>(rowp + (size_t)(sb >> 3) * KBlock<TYPE>::kBytes, sb & 7, s);
 #pragma unroll
         for (int i = 0; i < kTokensPerCta; ++i)
-            if (i < nt) acc[i] += dot_sub<TYPE>(s, xr + (size_t)i * x_stride + (size_t)sb * kQ81Bytes);
+            if (i < nt) acc[i] = add_dot<TYPE>(acc[i], s, xr + (size_t)i * x_stride + (size_t)sb * kQ81Bytes);
     }
 #pragma unroll
     for (int i = 0; i < kTokensPerCta; ++i) {

@@ -55,21 +55,22 @@ __device__ __forceinline__ void decode_sub(const uint8_t* blk, int j, SubBlock& 
     }
 }
 
-// ... against one Q8_1 block `xb` (36 bytes: f16 d, f16 s, 32 int8).
+// acc + its product with one Q8_1 block `xb` (36 bytes: f16 d, f16 s, 32 int8).  The rounding is written out, addition included: a row has the
+// same bits in every kernel, whatever the compiler would make of a product and a sum there.
 template <int TYPE>
-__device__ __forceinline__ float dot_sub(const SubBlock& s, const uint8_t* xb) {
+__device__ __forceinline__ float add_dot(float acc, const SubBlock& s, const uint8_t* xb) {
     const __half2 ds = *reinterpret_cast<const __half2*>(xb);
     const float d8 = __low2float(ds), s8 = __high2float(ds);
     if (TYPE == CHIMERE_TYPE_Q6_K) {
         int da = 0, db = 0;
 #pragma unroll
         for (int g = 0; g < 4; ++g) { da = __dp4a(s.w[g], (int)ld32(xb + 4 + 4 * g), da); db = __dp4a(s.w[4 + g], (int)ld32(xb + 20 + 4 * g), db); }
-        return s.d * d8 * (float)(s.sc * da + s.mn * db);
+        return fmaf(__fmul_rn(s.d, d8), (float)(s.sc * da + s.mn * db), acc);
     } else {
         int dot = 0;
 #pragma unroll
         for (int g = 0; g < 8; ++g) dot = __dp4a(s.w[g], (int)ld32(xb + 4 + 4 * g), dot);
-        return fmaf(-(s.dmin * (float)s.mn), s8, s.d * d8 * (float)(s.sc * dot));
+        return __fadd_rn(acc, fmaf(-__fmul_rn(s.dmin, (float)s.mn), s8, __fmul_rn(__fmul_rn(s.d, d8), (float)(s.sc * dot))));
     }
 }
 
@@ -83,8 +84,8 @@ __device__ __forceinline__ void decode_sub(int type, const uint8_t* row, int sb,
     else if (type == CHIMERE_TYPE_Q4_K) decode_sub<CHIMERE_TYPE_Q4_K>(blk, sb & 7, s);
     else decode_sub<CHIMERE_TYPE_Q6_K>(blk, sb & 7, s);
 }
-__device__ __forceinline__ float dot_sub(int type, const SubBlock& s, const uint8_t* xb) {
-    return type == CHIMERE_TYPE_Q6_K ? dot_sub<CHIMERE_TYPE_Q6_K>(s, xb) : dot_sub<CHIMERE_TYPE_Q5_K>(s, xb);   // (Q4_K: as Q5_K)
+__device__ __forceinline__ float add_dot(int type, float acc, const SubBlock& s, const uint8_t* xb) {
+    return type == CHIMERE_TYPE_Q6_K ? add_dot<CHIMERE_TYPE_Q6_K>(acc, s, xb) : add_dot<CHIMERE_TYPE_Q5_K>(acc, s, xb);   // (Q4_K: as Q5_K)
 }
 
 }  // namespace chimere

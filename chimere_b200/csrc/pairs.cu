@@ -216,7 +216,7 @@ __global__ void __launch_bounds__(256, CTAS) pair_gate_up_kernel(const __grid_co
                     const uint8_t* xb = p.in_q8 + (size_t)min(t0 + j, T - 1) * p.in_stride + (size_t)lane * kQ81Bytes;
 #pragma unroll
                     for (int i = 0; i < kKqSub; ++i)
-                        if (lane + 32 * i < nb) v[j] += dot_sub(x.type, ks[i], xb + i * 32 * kQ81Bytes);
+                        if (lane + 32 * i < nb) v[j] = add_dot(x.type, v[j], ks[i], xb + i * 32 * kQ81Bytes);
                 }
 #pragma unroll
                 for (int s = 16; s > 0; s >>= 1)
@@ -390,7 +390,7 @@ __global__ void __launch_bounds__(THREADS, CTAS) pair_down_kernel(const __grid_c
                 asm volatile("bar.sync 3, %0;" ::"r"(c.warps_k * 32) : "memory");
 #pragma unroll
                 for (int q = 0; q < kKqSteps; ++q) {
-                    float v = ksb < ksub ? 0.0f + dot_sub(x.type_down, ks[q], kx + ksb * kQ81Bytes) : 0.0f;
+                    float v = ksb < ksub ? add_dot(x.type_down, 0.0f, ks[q], kx + ksb * kQ81Bytes) : 0.0f;
                     if (!two) v += __shfl_xor_sync(0xffffffffu, v, 16);
 #pragma unroll
                     for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);

@@ -255,6 +255,19 @@ def test_kquant_shared_expert_beside_pairs(types, H, F_s):
     assert sc.status() == 0
 
 
+# ... rows of two sub-blocks per lane, whose sums meet in a lane before they meet across the warp: enough tokens that a sum which is rounded
+# differently shows in some intermediate's 8 bits
+@pytest.mark.parametrize("type_gate_up", [formats.TYPE_Q4_K, formats.TYPE_Q5_K, formats.TYPE_Q6_K])
+def test_kquant_rows_do_not_depend_on_the_batch(type_gate_up):
+    cfg = configs.scaled(IQ3, E=32, top_k=2, H=2048, F=512, F_s=512, type_sh_gate_up=type_gate_up, type_sh_down=formats.TYPE_Q4_K)
+    tiled, T = MoeWeightsTiled(configs.make_layer(cfg, device="cuda")), 400
+    x, sc = configs.make_input(cfg, T, device="cuda"), MoeScratch(tiled, T)
+    y = forward_moe(tiled, sc, x)
+    for n in (5, 2):
+        assert torch.equal(torch.cat([forward_moe(tiled, sc, x[t:t + n].contiguous()) for t in range(0, T, n)]), y), n
+    assert sc.status() == 0
+
+
 # residual + norm inside the router (up to four tokens, rows of up to 3072) and as a launch in front of it: the same bits, also in place
 @pytest.mark.parametrize("H", [256, 2048, 2176, 3072, 3200])
 @pytest.mark.parametrize("cfg", [Q4, configs.scaled(IQ3, type_sh_gate_up=formats.TYPE_Q5_K, type_sh_down=formats.TYPE_Q5_K)], ids=["q4", "q5k"])
