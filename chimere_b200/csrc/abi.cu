@@ -720,12 +720,19 @@ int chimere_b200_moe_forward(const chimere_moe_layer* w, const float* d_x, float
     return kshared_chain(w, T, d_y, ws, stream);
 }
 
-// The device's address of pinned host memory; null for any other.
-static float* pinned_address(const float* h) {
-    cudaPointerAttributes attr{};
-    if (cudaPointerGetAttributes(&attr, h) == cudaSuccess && attr.type == cudaMemoryTypeHost && attr.devicePointer) return static_cast<float*>(attr.devicePointer);
+// The device's address of `bytes` of pinned host memory; null for pageable memory and for ranges that the device does not see in one piece.  The
+// kernels read and write such a range by themselves, so its end is looked at as well: memory that is pinned only up to somewhere inside the
+// rows is refused, as a copy of it is.
+static cudaError_t pinned_address(const float* h, size_t bytes, float** device) {
+    const char* last = (const char*)h + bytes - 1;
+    cudaPointerAttributes a{}, z{};
+    *device = nullptr;
+    const bool first_pinned = cudaPointerGetAttributes(&a, h) == cudaSuccess && a.type == cudaMemoryTypeHost && a.devicePointer;
+    const bool last_pinned = first_pinned && cudaPointerGetAttributes(&z, last) == cudaSuccess && z.type == cudaMemoryTypeHost && z.devicePointer;
     (void)cudaGetLastError();   // (an unregistered pointer leaves an error behind on older runtimes)
-    return nullptr;
+    if (first_pinned && !last_pinned) return cudaErrorInvalidValue;
+    if (first_pinned && (const char*)z.devicePointer - (const char*)a.devicePointer == last - (const char*)h) *device = static_cast<float*>(a.devicePointer);
+    return cudaSuccess;
 }
 constexpr size_t kFetchBytes = 256 * 1024;   // rows of up to so many bytes come in by a kernel
 
@@ -735,16 +742,16 @@ int chimere_b200_moe_forward_host(const chimere_moe_layer* w, const float* h_x, 
     int rc = check_call(w, d_x, d_y, T, ws, true);
     if (rc) return rc;
     const size_t bytes = (size_t)T * w->H * sizeof(float);
-    const float* x_host = pinned_address(h_x);
-    cudaError_t e = x_host && bytes <= kFetchBytes ? launch_fetch_rows(x_host, d_x, (int64_t)T * w->H, stream)
-                                                   : cudaMemcpyAsync(d_x, h_x, bytes, cudaMemcpyHostToDevice, stream);
-    if (e != cudaSuccess) return cuda_rc(e);
+    float *x_host = nullptr, *y_host = nullptr;
+    cudaError_t e = bytes <= kFetchBytes ? pinned_address(h_x, bytes, &x_host) : cudaSuccess;
     // A pinned result buffer is addressable from the device under a pointer of its own: the last kernel then stores y
     // straight into host memory and the copy back (a second trip through the copy engine, serial behind the kernels) is
     // not needed.  Pageable memory, or a K-quant shared expert as launches of its own (the last of which reads y back), takes the staged copy.
-    float* y_dev = d_y;
-    if (!kshared(w) || (pairs_forward(w, T, ws) && pair_extras(w, T, ws).type))
-        if (float* y_host = pinned_address(h_y)) y_dev = y_host;
+    if (e == cudaSuccess && (!kshared(w) || (pairs_forward(w, T, ws) && pair_extras(w, T, ws).type))) e = pinned_address(h_y, bytes, &y_host);
+    if (e != cudaSuccess) return cuda_rc(e);
+    float* y_dev = y_host ? y_host : d_y;
+    e = x_host ? launch_fetch_rows(x_host, d_x, (int64_t)T * w->H, stream) : cudaMemcpyAsync(d_x, h_x, bytes, cudaMemcpyHostToDevice, stream);
+    if (e != cudaSuccess) return cuda_rc(e);
     rc = chimere_b200_moe_forward(w, d_x, y_dev, T, ws, stream);
     if (rc) return rc;
     if (y_dev == d_y) {

@@ -326,6 +326,30 @@ def test_host_rows(T):
         assert torch.equal(forward_moe_host(tiled, sc, rows, y), want)
 
 
+# rows that begin in pinned memory and end outside it are refused before anything is launched, on either side of the call
+@pytest.mark.parametrize("T", [1, 4])
+def test_host_rows_pinned_in_part(T):
+    cfg = configs.scaled(Q4, E=16, H=2048, F=64, F_s=64)
+    tiled = MoeWeightsTiled(configs.make_layer(cfg, device="cuda"))
+    sc, x = MoeScratch(tiled, T), configs.make_input(cfg, T, device="cuda")
+    want, cudart, page = forward_moe(tiled, sc, x).cpu(), torch.cuda.cudart(), 4096
+    room = np.zeros(T * cfg.H + 3 * page // 4, np.float32)
+    skip = -room.ctypes.data % page // 4
+    rows = torch.from_numpy(room[skip:skip + T * cfg.H].reshape(T, cfg.H))   # (from a page's start)
+    rows.copy_(x)
+    for pages in (1, T * cfg.H * 4 // page):
+        assert int(cudart.cudaHostRegister(rows.data_ptr(), pages * page, 0)) == 0
+        y, x_pinned = torch.empty(T, cfg.H).pin_memory(), x.cpu().pin_memory()
+        if pages == 1:
+            for a, b in ((rows, y), (x_pinned, rows)):
+                with pytest.raises(RuntimeError, match="-101"):
+                    forward_moe_host(tiled, sc, a, b)
+        else:
+            assert torch.equal(forward_moe_host(tiled, sc, rows, y), want) and torch.equal(forward_moe_host(tiled, sc, x_pinned, rows), want)
+        assert int(cudart.cudaHostUnregister(rows.data_ptr())) == 0
+    assert sc.status() == 0
+
+
 # the dispatch of a large batch: counts by the top-k kernel (four experts per token and more) and by a launch, chunks that 128 is no multiple
 # of, a last chunk of one token, more chunks than a lane of the scan takes at a time
 @pytest.mark.parametrize("k,T", [(1, 4096), (1, 4225), (3, 1366), (4, 1024), (6, 683), (7, 10009), (8, 512), (8, 513), (8, 8209)])
