@@ -5,6 +5,7 @@
 // scratch owner GgmlGpuBuffers, src/kernels/ggml_gpu.rs:292-407): they validate, lay the
 // caller's arena out, and enqueue three kernels per decode call (up to nine where the grouped GEMM takes
 // part, up to eleven in prefill).  Nothing here allocates device memory or synchronises, except chimere_b200_moe_forward_host which waits for its stream.
+#include <cmath>
 #include <cstdio>
 #include <cstring>
 #include <vector>
@@ -75,17 +76,35 @@ int validate_layer(const chimere_moe_layer* w) {
     return 0;
 }
 
-// Packed experts (Q4_0, IQ3_S) in the decode entry: up to pair_batch()'s line every (token, expert) pair is an item of its own (pairs.cu), which
-// reads an expert once per pair, from L2 behind the first; above it 16 pairs of an expert share a tile (mma_tiles.cu), which costs as much
-// with one pair as with eight.  us per layer, pairs / tiles:
+// Packed experts (Q4_0, IQ3_S) in the decode entry: up to pair_batch()'s line every (token, expert) pair is an item of its own (pairs.cu; the work
+// list where those kernels do not take the layer), which reads an expert once per pair, from L2 behind the first; above it 16 pairs of an
+// expert share a tile (mma_tiles.cu), which costs as much with one pair as with eight.  us per layer, pairs / tiles:
 //   256 experts of 512 x 2048, top 8, uniform routing: 32 tokens 81 / 111, 40: 101 / 127; skewed: 20: 49 / 47, 40: 90 / 62
 //   128 of 1856 x 2688, top 6: 8 tokens 88 / 101, 12: 121 / 122, 16: 159 / 142, 24 (on the GEMM) 189 / 180
 // (Before: 40 tokens 115 and 104, 64 tokens 192 and 145, now on the tiles 145 and 70.)  The best line depends on the routing, which the host does
 // not know: this one is where neither is slower than the work list's entries of one or two pairs were.
-bool pair_batch(const chimere_moe_layer* w, int T) {
+// A call of the tiles has some 14 us that one of the pairs has not (dispatch, combine, longer chains), and small layers or few experts have nothing
+// to set against it: what the pairs read again comes from L2 in less.  So whatever the pairs per expert, pairs while they read no more
+// weights again than this (uniform routing taken for it).  us, list / tiles / pairs:
+//   8 experts of 512 x 2048 top 2: 8 tokens (50M) 22.5 / 31.7 / 19.7, 24 (198M) 37 / 38 / 32, 32 (274M) 41 / 38 / 39, 40 (349M) 65 / 54 / 60
+//   64 of 512 x 2048 top 8: 12 tokens (176M) 45 / 55 / 35, 16 (272M) 54 / 58 / 43;   of 256 x 1024: 40 (232M) 50 / 42 / 41, 64 (402M) 72 / 48 / 60
+//   128 of 512 x 2048 top 1 (a CTA of the down launch has one routed expert): 41 tokens (144M) 66 / 55 / 52, 64 (241M) 83 / 60 / 73
+// and on layers that pairs.cu does not take, list / tiles: 8 of 2880 x 1024 top 2: 8 tokens (79M) 42 / 52, 12 (145M) 51 / 55, 16 (215M) 59 / 56
+constexpr int kPairTokens = 64;
+constexpr double kPairAgain = 170e6, kPairAgainFew = 275e6;   // ... and with at least four experts per token, up to 40 tokens
+double weights_again(const chimere_moe_layer* w, int T) {
+    const double distinct = w->E * (1.0 - std::pow(1.0 - (double)w->top_k / w->E, T));
+    return (w->act == CHIMERE_ACT_SWIGLU ? 3.0 : 2.0) * w->H * (((double)T * w->top_k - distinct) * w->F + (T - 1.0) * w->F_s);
+}
+// (w here and below: without a K-quant shared expert)
+bool few_per_expert(const chimere_moe_layer* w, int T) {
     const int64_t P = (int64_t)T * w->top_k;
     return T <= 4 || (T <= 40 && ((int64_t)w->F * w->H > (1 << 21) ? 16 * P <= 9 * w->E : 4 * P <= 5 * w->E));
 }
+bool pair_batch(const chimere_moe_layer* w, int T) {
+    return few_per_expert(w, T) || (T <= kPairTokens && weights_again(w, T) <= (w->top_k >= 4 && T <= kFewTokens ? kPairAgainFew : kPairAgain));
+}
+bool list_batch(const chimere_moe_layer* w, int T) { return T <= kFewTokens && (few_per_expert(w, T) || weights_again(w, T) <= kPairAgain); }
 // ... and in the prefill entry: the tiles up to five pairs per expert, then the tcgen05 GEMM (GEMM / tiles: 256 experts 128 tokens 254 / 175 us,
 // 256: 278 / 219, 777: 378 / 425, skewed 128: 109 / 102, 256: 144 / 156; 128 of 1856 x 2688 128 tokens 331 / 298, 256: 374 / 437).
 bool prefill_mma(const chimere_moe_layer* w, int T) { return (int64_t)T * w->top_k <= 5 * (int64_t)w->E; }
@@ -644,8 +663,8 @@ static PairExtras pair_extras(const chimere_moe_layer* w, int T, chimere_moe_wor
     return x;
 }
 static bool pairs_forward(const chimere_moe_layer* w, int T, chimere_moe_workspace* ws) {
-    if (!pair_batch(w, T) || w->layout != CHIMERE_LAYOUT_TILED32) return false;
     const chimere_moe_layer wr = kshared(w) ? routed_only(w) : *w;
+    if (!pair_batch(&wr, T) || w->layout != CHIMERE_LAYOUT_TILED32) return false;
     const Layout L = make_layout(&wr, ws->max_T);
     return pairs_run(gate_up_params(&wr, T, ws, L), down_params(&wr, nullptr, T, ws, L), pair_extras(w, T, ws));
 }
@@ -691,7 +710,7 @@ int chimere_b200_moe_forward(const chimere_moe_layer* w, const float* d_x, float
     const Layout L = make_layout(wr, ws->max_T);
     if (pairs_forward(w, T, ws)) {
         return run_pairs(w, d_x, nullptr, nullptr, nullptr, 0.0f, d_y, T, ws, stream);
-    } else if (!pair_batch(wr, T) && mma_runs(wr, T, ws)) {
+    } else if (!list_batch(wr, T) && mma_runs(wr, T, ws)) {
         RouteParams rp = route_params(wr, d_x, T, ws, ks);
         rp.list_mode = 2;
         e = launch_route(rp, stream);

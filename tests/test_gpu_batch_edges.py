@@ -238,6 +238,39 @@ def test_tiles_of_sixteen_pairs(cfg, T):
     _check(cfg, T, prefill=False)
 
 
+# ... and in the prefill entry, which takes them for small layers too: every token on the same experts, the batch the column count
+@pytest.mark.parametrize("cfg", [configs.scaled(Q4, top_k=1, H=512, F=256, F_s=256), configs.scaled(IQ3, top_k=1, H=1280, F=256, F_s=0),
+                                 configs.scaled(configs.NEMOTRON_Q4_0, top_k=1, H=640, F=1120, F_s=96), configs.scaled(Q4, top_k=2, H=128, F=64, F_s=64),
+                                 configs.scaled(IQ3, top_k=4, H=2048, F=512, F_s=512, type_down=configs.IQ3_S)], ids=lambda c: f"{c.name}-{c.H}-{c.F}-{c.F_s}")
+@pytest.mark.parametrize("T", [5, 8, 9, 15, 16, 17, 33, 70])
+def test_tiles_of_sixteen_pairs_in_prefill(cfg, T):
+    cfg = configs.scaled(cfg, E=max(cfg.top_k + 1, -(-T * cfg.top_k // 5)))   # (the fewest experts with which the batch is one for these tiles)
+    raw = configs.make_layer(cfg, device="cuda")
+    raw.router_bias = torch.zeros(cfg.E, device="cuda")
+    raw.router_bias[:cfg.top_k] = 40.0
+    tiled, x = MoeWeightsTiled(raw), configs.make_input(cfg, T, device="cuda")
+    sc = MoeScratch(tiled, T)
+    y = forward_moe_prefill(tiled, MoeWeightsPrefill(raw), sc, x)
+    idx = sc.topk_indices(T).cpu().numpy()
+    assert sc.status() == 0 and sc.offsets().cpu().tolist() == [min(i, cfg.top_k) * T for i in range(cfg.E + 1)]
+    check_rows(y.cpu().numpy(), oracle_on_gpu_routing(raw.to("cpu"), x.cpu().numpy(), idx)["y"])
+    assert torch.equal(y, forward_moe(tiled, sc, x))      # (the pairs' bits)
+
+
+# small layers run pair by pair up to 64 tokens, on the work list up to 40 where a shared expert of one row tile makes the rows of a slice too
+# long for the pair kernels
+@pytest.mark.parametrize("cfg", [configs.scaled(Q4, E=8, top_k=2, H=256, F=64, F_s=64), configs.scaled(IQ3, E=64, H=512, F=256, F_s=0),
+                                 configs.scaled(configs.NEMOTRON_Q4_0, E=1, top_k=1, H=384, F=96, F_s=96), configs.scaled(Q4, E=8, top_k=2, H=512, F=2880, F_s=32)],
+                         ids=lambda c: f"{c.name}-{c.H}-{c.F}-{c.F_s}")
+@pytest.mark.parametrize("T", [6, 33, 40, 41, 64, 65])
+def test_small_layers_pair_by_pair(cfg, T):
+    _check(cfg, T, prefill=False)
+    tiled, x = MoeWeightsTiled(configs.make_layer(cfg, device="cuda")), configs.make_input(cfg, T, device="cuda")
+    sc = MoeScratch(tiled, T)
+    y = forward_moe(tiled, sc, x)
+    assert torch.equal(torch.cat([forward_moe(tiled, sc, x[t:t + 1].contiguous()) for t in range(T)]), y) and sc.status() == 0
+
+
 # a K-quant shared expert beside the pair kernels: one and two rows per step, every type, against the oracle and, bit for bit, against the
 # launches of its own that a larger batch takes
 @pytest.mark.parametrize("types", [(formats.TYPE_Q5_K, formats.TYPE_Q5_K), (formats.TYPE_Q4_K, formats.TYPE_Q6_K), (formats.TYPE_Q6_K, formats.TYPE_Q4_K)], ids=str)
