@@ -105,11 +105,24 @@ bool pair_batch(const chimere_moe_layer* w, int T) {
     return few_per_expert(w, T) || (T <= kPairTokens && weights_again(w, T) <= (w->top_k >= 4 && T <= kFewTokens ? kPairAgainFew : kPairAgain));
 }
 bool list_batch(const chimere_moe_layer* w, int T) { return T <= kFewTokens && (few_per_expert(w, T) || weights_again(w, T) <= kPairAgain); }
+// Upwards the tiles, which fetch and decode an expert's weights again for every 16 pairs, end where the grouped GEMM (64 pairs at a time) is the faster:
+// a number of weights times pairs, less of them for wide rows, whose experts do not stay in L2 from one tile to the next, and for IQ3_S, whose sub-block
+// factors are unpacked along.  us per layer, tiles / GEMM:
+//   256 Q4_0 experts of 512 x 2048, top 8, 6144 tokens (52G) 2462 / 2514, 8192 (69G) 3704 / 3291; IQ3_S, 1024 tokens (9G) 521 / 598, 3072 (26G) 1367 / 1381,
+//   4096 (34G) 1776 / 1730, and 64 of them, 1024 (9G) 1.03 times faster, 2048 (17G) 0.99
+//   128 of 1024 x 2048, 768 tokens (13G) 1.01, 1024 (17G) 0.99; 64 of 1408 x 2048, top 6, 1024 (18G) 748 / 770; 128 of 1856 x 2688, 512 (15G) 703 / 731, 1024 (31G) 1240 / 1206, skewed 632 / 624 and 1194 / 1121
+//   64 of 1536 x 4096, 256 tokens (13G) 683 / 687, 512 (26G) 1192 / 971; 8 of them, 512 (6G) 1.07, 768 (10G) 0.93; IQ3_S, 32 of them, 256 (6G) 1.03, 384 (10G) 0.93
+//   (of 1024 x 1024 and smaller the tiles are the faster at any size that was tried, IQ3_S 256 x 1024 up to 4096 tokens, 9G: 1.00)
+bool tile_batch(const chimere_moe_layer* w, int T) {
+    const bool iq3 = w->type_up == CHIMERE_TYPE_IQ3_S;
+    const double most = w->H <= 1024 ? (iq3 ? 8e9 : 64e9) : w->H <= 2048 && w->F <= 768 ? (iq3 ? 12e9 : 54e9) : w->H <= 2816 ? (iq3 ? 8e9 : 18e9) : iq3 ? 5e9 : 10e9;
+    return (double)T * w->top_k * w->F * w->H <= most;
+}
 // ... and in the prefill entry: the tiles up to five pairs per expert, then the tcgen05 GEMM (GEMM / tiles: 256 experts 128 tokens 254 / 175 us,
 // 256: 278 / 219, 777: 378 / 425, skewed 128: 109 / 102, 256: 144 / 156; 128 of 1856 x 2688 128 tokens 331 / 298, 256: 374 / 437).
 bool prefill_mma(const chimere_moe_layer* w, int T) { return (int64_t)T * w->top_k <= 5 * (int64_t)w->E; }
 
-// Layers that neither takes (experts and shared expert of different packed types, rows too long for the tiles' shared memory):
+// Layers that neither takes (experts and shared expert of different packed types, rows too long for the tiles' shared memory), and batches above tile_batch():
 // From forward_gemm_tokens() tokens on the decode entry sends experts with at least kForwardGemmPairs pairs, and the shared expert,
 // to the grouped GEMM and the others to the GEMV kernels: a GEMM tile costs the same with 1 pair as with 16, a GEMV entry grows
 // with every pair.  Q4_0, us per layer, GEMV kernels alone / with the GEMM, uniform and (skewed) routing:
@@ -708,9 +721,11 @@ int chimere_b200_moe_forward(const chimere_moe_layer* w, const float* d_x, float
     const chimere_moe_layer* wr = &wr_;
     cudaError_t e;
     const Layout L = make_layout(wr, ws->max_T);
+    const bool gemm = forward_gemm(wr, T) && ws->prefill_arena && ws->prefill_bytes >= prefill_arena(wr, ws->max_T).total &&
+                      tiled_bulk_runs(gate_up_params(wr, T, ws, L), down_params(wr, d_y, T, ws, L));
     if (pairs_forward(w, T, ws)) {
         return run_pairs(w, d_x, nullptr, nullptr, nullptr, 0.0f, d_y, T, ws, stream);
-    } else if (!list_batch(wr, T) && mma_runs(wr, T, ws)) {
+    } else if (!list_batch(wr, T) && (tile_batch(wr, T) || !gemm) && mma_runs(wr, T, ws)) {
         RouteParams rp = route_params(wr, d_x, T, ws, ks);
         rp.list_mode = 2;
         e = launch_route(rp, stream);
@@ -718,8 +733,7 @@ int chimere_b200_moe_forward(const chimere_moe_layer* w, const float* d_x, float
         rc = run_mma(wr, T, ws, stream);
         if (rc) return rc;
         e = finish_tokens(wr, d_y, T, ws, stream);
-    } else if (forward_gemm(wr, T) && ws->prefill_arena && ws->prefill_bytes >= prefill_arena(wr, ws->max_T).total &&
-        tiled_bulk_runs(gate_up_params(wr, T, ws, L), down_params(wr, d_y, T, ws, L))) {
+    } else if (gemm) {
         RouteParams rp = route_params(wr, d_x, T, ws, ks);
         rp.list_mode = 2;
         e = launch_route(rp, stream);

@@ -111,6 +111,25 @@ def test_decode_rows_do_not_depend_on_the_batch(cfg, T):
     assert torch.equal(y, single)
 
 
+# ... on the GEMM itself and the GEMV kernels behind it: experts and shared expert of different packed types, rows that the tiles' shared memory does
+# not hold, and batches above the tiles' last one
+@pytest.mark.parametrize("cfg,T", [(c, t) for c in (configs.scaled(IQ3, E=32, top_k=4, H=1024, F=256, F_s=256, type_sh_gate_up=configs.Q4_0, name="iq3, q4 shared"),
+                                                    configs.scaled(Q4, E=32, top_k=4, H=1024, F=256, F_s=512, type_sh_gate_up=configs.IQ3_S, type_sh_down=configs.IQ3_S, name="q4, iq3 shared"),
+                                                    configs.scaled(Q4, E=16, top_k=4, H=5120, F=128, F_s=128, name="rows of 5120"),
+                                                    configs.scaled(configs.NEMOTRON_Q4_0, E=32, top_k=3, H=5120, F=800, F_s=96, name="relu, rows of 5120")) for t in (17, 41, 64, 150)] +
+                                  [(configs.scaled(IQ3, E=16, H=4096, F=512, F_s=256, type_down=d, name="above the tiles"), 330) for d in (configs.Q4_0, configs.IQ3_S)],
+                         ids=lambda v: getattr(v, "name", str(v)))
+def test_decode_rows_on_the_gemm_do_not_depend_on_the_batch(cfg, T):
+    raw = configs.make_layer(cfg, device="cuda")
+    tiled, x = MoeWeightsTiled(raw), configs.make_input(cfg, T, device="cuda")
+    sc, one = MoeScratch(tiled, T), MoeScratch(tiled, 1)
+    y = forward_moe(tiled, sc, x)
+    assert torch.equal(y, torch.cat([forward_moe(tiled, one, x[t:t + 1].contiguous()) for t in range(T)]))
+    assert sc.status() == 0 and one.status() == 0
+    if T <= 64:
+        check_rows(y.cpu().numpy(), oracle_on_gpu_routing(raw.to("cpu"), x.cpu().numpy(), sc.topk_indices(T).cpu().numpy())["y"])
+
+
 # a workspace for more tokens than the call has: the smaller batch may cut its pairs into more entries than the full one
 @pytest.mark.parametrize("kw", [dict(E=8), dict(E=16), dict(E=64), dict(E=4, top_k=2, F_s=0)], ids=str)
 @pytest.mark.parametrize("max_T", [25, 32, 40, 64])
