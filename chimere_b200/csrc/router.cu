@@ -1007,8 +1007,15 @@ cudaError_t launch_ep_pack(const int32_t* topk_idx, const int8_t* x_q, const flo
 }
 
 // The tiled product's three launches start to pay where the simple kernel (a CTA per 8 tokens x 8 experts, partials through shared
-// memory) fills the GPU more than once: 19.6 against 29 us at 61 x 257 outputs of H = 2048, 32 against 33 at 130 x 257.
-constexpr int kRouteTileWork = 65536;
+// memory) fills the GPU more than once: 19.6 against 29 us at 61 x 257 outputs of H = 2048, 32 against 33 at 130 x 257.  From 513 columns on,
+// though the row is one kilo-element, 256 experts of H = 1024: 128 tokens 1.15 times the simple kernel's time, 160 0.94, 256 35 us against 41; H = 640: 1.16,
+// 0.97, 0.83.  Shorter rows: H = 512, 65536 outputs 0.91 (256 experts) to 1.12 (64), H = 256 0.99 to 1.12.
+constexpr int kRouteTileWork = 65536, kRouteTileOutputs = 36864;
+static bool route_tiled(const RouteParams& p) {
+    const int64_t outputs = (int64_t)p.T * p.E;
+    return (outputs * route_nq(p.H) > kRouteTileWork || (p.H > 512 && outputs > kRouteTileOutputs)) && p.scratch && p.H <= 4096 &&
+           route_scratch_floats(p.T, p.E, p.H) <= p.scratch_floats;
+}
 // Tiles of 16 tokens instead of 32 while all of them run at once, two per SM (one where a row has more than 2048 columns, whose rings are then four
 // deep: a warp alone on its SM quarter waits for its copies).  Prefill call, us, 32 / 16: 256 experts of H = 2048, 160 tokens 120.6 / 112.8, 256: 137.0 /
 // 130.6, 288: 147.0 / 144.0, 384 and 512 (over the line) 166.4 / 168.1, 189.5 / 194.0; 128 of H = 2688, 180 tokens 352.6 / 347.5, 256: 371.9 / 367.4 (372.9 /
@@ -1068,7 +1075,7 @@ cudaError_t launch_route(const RouteParams& p, cudaStream_t stream) {
         constexpr int TT = 8, TE = 2;
         dim3 grid((nrows + TE - 1) / TE, (p.T + TT - 1) / TT);
         return launch_pdl(route_kernel<TT, TE>, grid, 256, route_smem(TT, TE), stream, p);
-    } else if (p.scratch && (int64_t)p.T * p.E * route_nq(p.H) > kRouteTileWork && p.H <= 4096 && route_scratch_floats(p.T, p.E, p.H) <= p.scratch_floats) {
+    } else if (route_tiled(p)) {
         switch (route_nq(p.H)) {
             case 1: return launch_route_tiles<1>(p, stream);
             case 2: return launch_route_tiles<2>(p, stream);

@@ -92,6 +92,12 @@ def test_tiled_router_of_small_tiles(E, H, T):
     _check(configs.scaled(Q4, E=E, H=H, F=64, F_s=64), T, prefill=False)
 
 
+# rows of up to one kilo-element on both sides of the tiled product's line, which counts the outputs for those of more than 512 columns
+@pytest.mark.parametrize("E,H,T", [(128, 512, 289), (128, 512, 513), (128, 640, 288), (128, 640, 289), (36, 1024, 1024), (36, 1024, 1025)])
+def test_tiled_router_of_short_rows(E, H, T):
+    _check(configs.scaled(Q4, E=E, H=H, F=64, F_s=64), T, prefill=False)
+
+
 # The decode entry sends popular experts to the GEMM and the others to the GEMV kernels; a token's row is the same bits either way,
 # whatever the batch: odd numbers of K slices and units, IQ3_S in both places, a shared expert narrower than the routed ones.
 @pytest.mark.parametrize("cfg", [configs.scaled(Q4, E=16, F=256, F_s=512, H=2048, name="q4"),
