@@ -518,8 +518,27 @@ __global__ void __launch_bounds__(kDispatchChunk) dispatch_hist_kernel(const Rou
     }
 }
 
-// A warp per expert, a run of consecutive chunks per lane: hist[chunk][e] becomes the number of pairs of expert e in earlier chunks.  (One CTA
-// for all experts: 24 us at 512 chunks, of latency and one SM's loads; now 5.)
+// The last step of both scans, by 256 threads, thread = expert: pair counts to offsets and to the first work entries.
+__device__ __forceinline__ void scan_totals(const RouteParams& p, int32_t* ent_base, int cnt, int* scan) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int nent = (cnt + kMaxGroupTokens - 1) / kMaxGroupTokens;
+    int incl_c = cnt, incl_n = nent;
+#pragma unroll
+    for (int sft = 1; sft < 32; sft <<= 1) {
+        const int a = __shfl_up_sync(0xffffffffu, incl_c, sft), b = __shfl_up_sync(0xffffffffu, incl_n, sft);
+        if (lane >= sft) { incl_c += a; incl_n += b; }
+    }
+    if (lane == 31) { scan[warp] = incl_c; scan[8 + warp] = incl_n; }
+    dispatch_sync();
+    int base_c = 0, base_n = 0;
+    for (int w = 0; w < warp; ++w) { base_c += scan[w]; base_n += scan[8 + w]; }
+    if (tid < p.E) p.offsets[tid] = base_c + incl_c - cnt;
+    ent_base[tid] = base_n + incl_n - nent;
+    if (tid == 255) { p.offsets[p.E] = base_c + incl_c; ent_base[256] = base_n + incl_n; }
+}
+
+// hist[chunk][e] becomes the number of pairs of expert e in earlier chunks.  Many chunks: a warp per expert, a run of consecutive chunks per
+// lane, the CTA that finishes last does the totals (512 chunks: 5 us, where one CTA for all experts takes 24, of one SM's loads).
 constexpr int kScanBatch = 16;
 __global__ void __launch_bounds__(256) dispatch_scan_kernel(const RouteParams p, int32_t* hist, int nchunks) {
     __shared__ int scan[16];
@@ -561,21 +580,33 @@ __global__ void __launch_bounds__(256) dispatch_scan_kernel(const RouteParams p,
     __syncthreads();
     if (!s_flag) return;
     if (tid == 0) ent_base[259] = 0;
-    const int cnt = tid < p.E ? __ldcg(ent_base + tid) : 0;
-    const int nent = (cnt + kMaxGroupTokens - 1) / kMaxGroupTokens;
-    int incl_c = cnt, incl_n = nent;
+    scan_totals(p, ent_base, tid < p.E ? __ldcg(ent_base + tid) : 0, scan);
+}
+// Few chunks: one CTA, thread = (quarter of the chunks, expert), a quarter of up to 16 chunks in registers between the two passes; no counter and
+// no second look at the totals.  Route entry, us, 32 CTAs / one: 256 experts of H = 2048, 512 tokens (32 chunks) 59.4 / 55.0, 1024 (64) 93.0 / 88.2; 200 of
+// H = 1152, 1024: 92.6 / 87.2 (88.9 when this was a launch behind one that counted).
+constexpr int kScanFewChunks = 4 * kScanBatch;
+__global__ void __launch_bounds__(1024) dispatch_scan_few_kernel(const RouteParams p, int32_t* hist, int nchunks) {
+    __shared__ int scan[16];
+    __shared__ int part[4][256];
+    const int e = threadIdx.x & 255, quarter = threadIdx.x >> 8, per = (nchunks + 3) / 4, c0 = quarter * per;
+    int32_t* col = hist + (size_t)c0 * 256 + e;
+    griddep_wait();
+    if (threadIdx.x == 0) griddep_launch();
+    int v[kScanBatch], sum = 0;
 #pragma unroll
-    for (int sft = 1; sft < 32; sft <<= 1) {
-        const int a = __shfl_up_sync(0xffffffffu, incl_c, sft), b = __shfl_up_sync(0xffffffffu, incl_n, sft);
-        if (lane >= sft) { incl_c += a; incl_n += b; }
-    }
-    if (lane == 31) { scan[warp] = incl_c; scan[8 + warp] = incl_n; }
+    for (int i = 0; i < kScanBatch; ++i) v[i] = i < per && c0 + i < nchunks ? __ldcg(col + (size_t)i * 256) : 0;
+#pragma unroll
+    for (int i = 0; i < kScanBatch; ++i) sum += v[i];
+    part[quarter][e] = sum;
     __syncthreads();
-    int base_c = 0, base_n = 0;
-    for (int w = 0; w < warp; ++w) { base_c += scan[w]; base_n += scan[8 + w]; }
-    if (tid < p.E) p.offsets[tid] = base_c + incl_c - cnt;
-    ent_base[tid] = base_n + incl_n - nent;
-    if (tid == 255) { p.offsets[p.E] = base_c + incl_c; ent_base[256] = base_n + incl_n; }
+    int run = 0;
+    for (int q = 0; q < quarter; ++q) run += part[q][e];
+#pragma unroll
+    for (int i = 0; i < kScanBatch; ++i)
+        if (i < per && c0 + i < nchunks) { col[(size_t)i * 256] = run; run += v[i]; }
+    if (quarter > 0) return;
+    scan_totals(p, hist + (size_t)nchunks * 256, e < p.E ? part[0][e] + part[1][e] + part[2][e] + part[3][e] : 0, scan);
 }
 
 __global__ void __launch_bounds__(kDispatchChunk) dispatch_place_kernel(const RouteParams p, int32_t* hist, int nchunks, int chunk) {
@@ -644,7 +675,9 @@ static cudaError_t launch_dispatch_split(const RouteParams& p, bool counted, cud
     const int nchunks = dispatch_chunks(p.T, p.top_k), chunk = dispatch_tokens(p.top_k) * p.top_k;
     cudaError_t e = cudaSuccess;
     if (!counted) e = launch_pdl(dispatch_hist_kernel, dim3(nchunks), kDispatchChunk, 0, stream, p, p.dispatch_scratch, chunk);
-    if (e == cudaSuccess) e = launch_pdl(dispatch_scan_kernel, dim3(32), 256, 0, stream, p, p.dispatch_scratch, nchunks);
+    if (e == cudaSuccess)
+        e = nchunks <= kScanFewChunks ? launch_pdl(dispatch_scan_few_kernel, dim3(1), 1024, 0, stream, p, p.dispatch_scratch, nchunks)
+                                      : launch_pdl(dispatch_scan_kernel, dim3(32), 256, 0, stream, p, p.dispatch_scratch, nchunks);
     if (e == cudaSuccess) e = launch_pdl(dispatch_place_kernel, dim3(nchunks), kDispatchChunk, 0, stream, p, p.dispatch_scratch, nchunks, chunk);
     return e;
 }

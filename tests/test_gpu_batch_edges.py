@@ -423,6 +423,12 @@ def test_dispatch_of_large_batches(k, T):
     assert sc.status() == 0
 
 
+# ... numbers of chunks around a multiple of four, the most that one CTA scans and one more
+@pytest.mark.parametrize("k,T", [(8, 528), (8, 529), (8, 545), (8, 576), (8, 1024), (8, 1025), (1, 4097), (6, 1324)])
+def test_dispatch_of_few_chunks(k, T):
+    test_dispatch_of_large_batches(k, T)
+
+
 # Q8_1 of whole rows: rows of any float alignment, blocks of zeros, of tiny and huge values, of NaN and infinities, against the one-warp form
 def test_rows_quantised_four_elements_per_lane():
     cfg = configs.scaled(Q4, E=128, top_k=1, H=1152, F=32, F_s=0)
