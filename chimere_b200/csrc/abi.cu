@@ -721,11 +721,10 @@ int chimere_b200_moe_forward(const chimere_moe_layer* w, const float* d_x, float
     const chimere_moe_layer* wr = &wr_;
     cudaError_t e;
     const Layout L = make_layout(wr, ws->max_T);
+    if (pairs_forward(w, T, ws)) return run_pairs(w, d_x, nullptr, nullptr, nullptr, 0.0f, d_y, T, ws, stream);
     const bool gemm = forward_gemm(wr, T) && ws->prefill_arena && ws->prefill_bytes >= prefill_arena(wr, ws->max_T).total &&
                       tiled_bulk_runs(gate_up_params(wr, T, ws, L), down_params(wr, d_y, T, ws, L));
-    if (pairs_forward(w, T, ws)) {
-        return run_pairs(w, d_x, nullptr, nullptr, nullptr, 0.0f, d_y, T, ws, stream);
-    } else if (!list_batch(wr, T) && (tile_batch(wr, T) || !gemm) && mma_runs(wr, T, ws)) {
+    if (!list_batch(wr, T) && (tile_batch(wr, T) || !gemm) && mma_runs(wr, T, ws)) {
         RouteParams rp = route_params(wr, d_x, T, ws, ks);
         rp.list_mode = 2;
         e = launch_route(rp, stream);
@@ -762,9 +761,11 @@ static cudaError_t pinned_address(const float* h, size_t bytes, float** device) 
     *device = nullptr;
     const bool first_pinned = cudaPointerGetAttributes(&a, h) == cudaSuccess && a.type == cudaMemoryTypeHost && a.devicePointer;
     const bool last_pinned = first_pinned && cudaPointerGetAttributes(&z, last) == cudaSuccess && z.type == cudaMemoryTypeHost && z.devicePointer;
-    (void)cudaGetLastError();   // (an unregistered pointer leaves an error behind on older runtimes)
-    if (first_pinned && !last_pinned) return cudaErrorInvalidValue;
-    if (first_pinned && (const char*)z.devicePointer - (const char*)a.devicePointer == last - (const char*)h) *device = static_cast<float*>(a.devicePointer);
+    if (!last_pinned) {
+        (void)cudaGetLastError();   // (an unregistered pointer leaves an error behind on older runtimes)
+        return first_pinned ? cudaErrorInvalidValue : cudaSuccess;
+    }
+    if ((const char*)z.devicePointer - (const char*)a.devicePointer == last - (const char*)h) *device = static_cast<float*>(a.devicePointer);
     return cudaSuccess;
 }
 constexpr size_t kFetchBytes = 256 * 1024;   // rows of up to so many bytes come in by a kernel
@@ -777,14 +778,18 @@ int chimere_b200_moe_forward_host(const chimere_moe_layer* w, const float* h_x, 
     const size_t bytes = (size_t)T * w->H * sizeof(float);
     float *x_host = nullptr, *y_host = nullptr;
     cudaError_t e = bytes <= kFetchBytes ? pinned_address(h_x, bytes, &x_host) : cudaSuccess;
+    if (e == cudaSuccess) e = x_host ? launch_fetch_rows(x_host, d_x, (int64_t)T * w->H, stream) : cudaMemcpyAsync(d_x, h_x, bytes, cudaMemcpyHostToDevice, stream);
+    if (e != cudaSuccess) return cuda_rc(e);
     // A pinned result buffer is addressable from the device under a pointer of its own: the last kernel then stores y
     // straight into host memory and the copy back (a second trip through the copy engine, serial behind the kernels) is
     // not needed.  Pageable memory, or a K-quant shared expert as launches of its own (the last of which reads y back), takes the staged copy.
-    if (e == cudaSuccess && (!kshared(w) || (pairs_forward(w, T, ws) && pair_extras(w, T, ws).type))) e = pinned_address(h_y, bytes, &y_host);
-    if (e != cudaSuccess) return cuda_rc(e);
+    // (Looked at while the rows are on their way.)
+    if (!kshared(w) || (pairs_forward(w, T, ws) && pair_extras(w, T, ws).type)) e = pinned_address(h_y, bytes, &y_host);
+    if (e != cudaSuccess) {
+        (void)cudaStreamSynchronize(stream);   // (h_x is the caller's again)
+        return cuda_rc(e);
+    }
     float* y_dev = y_host ? y_host : d_y;
-    e = x_host ? launch_fetch_rows(x_host, d_x, (int64_t)T * w->H, stream) : cudaMemcpyAsync(d_x, h_x, bytes, cudaMemcpyHostToDevice, stream);
-    if (e != cudaSuccess) return cuda_rc(e);
     rc = chimere_b200_moe_forward(w, d_x, y_dev, T, ws, stream);
     if (rc) return rc;
     if (y_dev == d_y) {

@@ -384,7 +384,7 @@ def test_host_rows(T):
         assert torch.equal(forward_moe_host(tiled, sc, rows, y), want)
 
 
-# rows that begin in pinned memory and end outside it are refused before anything is launched, on either side of the call
+# rows that begin in pinned memory and end outside it are refused before a kernel touches them, on either side of the call
 @pytest.mark.parametrize("T", [1, 4])
 def test_host_rows_pinned_in_part(T):
     cfg = configs.scaled(Q4, E=16, H=2048, F=64, F_s=64)
