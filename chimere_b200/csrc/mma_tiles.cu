@@ -53,12 +53,6 @@ __device__ __forceinline__ void cp_async4(uint32_t dst, const void* src) { asm v
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 __device__ __forceinline__ void ldg32(uint32_t& v, const uint8_t* a) { asm volatile("ld.global.nc.L1::no_allocate.u32 %0, [%1];" : "=r"(v) : "l"(a)); }
 __device__ __forceinline__ void ldg16(uint16_t& v, const uint8_t* a) { asm volatile("ld.global.nc.L1::no_allocate.u16 %0, [%1];" : "=h"(v) : "l"(a)); }
-__device__ __forceinline__ void ldg32_if(uint32_t& v, const uint8_t* a, int on) {
-    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\t@p ld.global.nc.L1::no_allocate.u32 %0, [%1];\n\t}" : "+r"(v) : "l"(a), "r"(on));
-}
-__device__ __forceinline__ void ldg16_if(uint16_t& v, const uint8_t* a, int on) {
-    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\t@p ld.global.nc.L1::no_allocate.u16 %0, [%1];\n\t}" : "+h"(v) : "l"(a), "r"(on));
-}
 
 // Four units of a 32-row tile: word [u][i] = bytes 4 * (lane & 3) .. of row (lane >> 2) + 8 i, i.e. what the MMA's A fragments hold
 // of the low and of the high nibbles; scales of row `lane`.

@@ -29,16 +29,10 @@ namespace chimere {
 
 constexpr int kPairItems = 64;      // items of a CTA (their experts are looked up together)
 
-// ---- predicated weight loads: the registers keep their value where there is nothing to ask for ----
+// (a predicated weight load, as those of tiled.cuh)
 __device__ __forceinline__ void ldg128_if(uint4& v, const uint8_t* a, int on) {
     asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %5, 0;\n\t@p ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];\n\t}"
                  : "+r"(v.x), "+r"(v.y), "+r"(v.z), "+r"(v.w) : "l"(a), "r"(on));
-}
-__device__ __forceinline__ void ldg32_if(uint32_t& v, const uint8_t* a, int on) {
-    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\t@p ld.global.nc.L1::no_allocate.u32 %0, [%1];\n\t}" : "+r"(v) : "l"(a), "r"(on));
-}
-__device__ __forceinline__ void ldg16_if(uint16_t& v, const uint8_t* a, int on) {
-    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\t@p ld.global.nc.L1::no_allocate.u16 %0, [%1];\n\t}" : "+h"(v) : "l"(a), "r"(on));
 }
 __device__ __forceinline__ void sts_v4(uint32_t a, const uint4& v) { asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory"); }
 __device__ __forceinline__ void sts_v2(uint32_t a, uint32_t x, uint32_t y) { asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(a), "r"(x), "r"(y) : "memory"); }

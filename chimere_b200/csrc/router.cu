@@ -1095,13 +1095,14 @@ cudaError_t launch_route_norm(const RouteParams& p, const float* hidden, const f
 cudaError_t launch_route(const RouteParams& p, cudaStream_t stream) {
     const int nrows = p.E + (p.shexp_gate_w ? 1 : 0);
     const int ttiles8 = (p.T + 7) / 8;
-    // few experts: a row per CTA, up to 3072 columns in flight at once, as long as that is one CTA per SM (64 experts of H = 2048, 8 tokens
-    // 9.6 -> 9.1 us, but 24 tokens 10.9 -> 11.7); a single row of 2048 is faster in pairs of outputs (6.9 against 7.3)
+    // One and two tokens: pairs of router rows per CTA, sized for so many tokens (route entry of 128 experts, one token of 2048 columns 7.3 -> 5.3 us,
+    // of 2688 7.9 -> 5.7, against the forms for eight).  Up to 32, few experts: a row per CTA, up to 3072 columns in flight at once, as long as that is one
+    // CTA per SM (64 experts of H = 2048, 8 tokens 9.6 -> 9.1 us, but 24 tokens 10.9 -> 11.7).
     if (p.T <= 2) {
         constexpr int TE = 2;
         const dim3 grid((nrows + TE - 1) / TE);
         return p.T == 1 ? launch_pdl(route_kernel<1, TE>, grid, 256, route_smem(1, TE), stream, p) : launch_pdl(route_kernel<2, TE>, grid, 256, route_smem(2, TE), stream, p);
-    } else if (p.T <= 32 && nrows * ttiles8 <= sm_count() && (p.T > 1 || p.H > 2048)) {
+    } else if (p.T <= 32 && nrows * ttiles8 <= sm_count()) {
         constexpr int TT = 8, TE = 1;
         return launch_pdl(route_kernel<TT, TE>, dim3(nrows, (p.T + TT - 1) / TT), 256, route_smem(TT, TE), stream, p);
     } else if (p.T <= 32) {

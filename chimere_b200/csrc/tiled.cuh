@@ -79,6 +79,14 @@ __device__ __forceinline__ uint2 lds64(uint32_t a) {
 // streamed in slabs (an IQ3_S super-block keeps its scales behind its eight units).
 constexpr int kGroupUnits = 4;
 
+// predicated weight loads: the register keeps its value where there is nothing to ask for
+__device__ __forceinline__ void ldg32_if(uint32_t& v, const uint8_t* a, int on) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\t@p ld.global.nc.L1::no_allocate.u32 %0, [%1];\n\t}" : "+r"(v) : "l"(a), "r"(on));
+}
+__device__ __forceinline__ void ldg16_if(uint16_t& v, const uint8_t* a, int on) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\t@p ld.global.nc.L1::no_allocate.u16 %0, [%1];\n\t}" : "+h"(v) : "l"(a), "r"(on));
+}
+
 template <int TYPE> struct Tiled;
 
 template <> struct Tiled<CHIMERE_TYPE_Q4_0> {
