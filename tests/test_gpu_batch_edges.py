@@ -53,6 +53,32 @@ def test_kquant_shared_expert_beside_packed_experts(types, H, T):
     _check(configs.scaled(IQ3, E=4, top_k=2, H=H, F=256, F_s=512, type_sh_gate_up=types[0], type_sh_down=types[1]), T, prefill=True)
 
 
+# ... with the routed experts on the 16-pair tiles (up to five pairs per expert) and the K-quant tiles behind them, several of 32 tokens: the launches
+# overlap, so the bits are looked at again and again
+@pytest.mark.parametrize("types", [(formats.TYPE_Q5_K, formats.TYPE_Q5_K), (formats.TYPE_Q4_K, formats.TYPE_Q5_K)], ids=str)
+@pytest.mark.parametrize("E,k,H", [(256, 8, 1024), (64, 2, 2048), (100, 3, 1024)])
+@pytest.mark.parametrize("T", [33, 65, 129, 160])
+def test_kquant_tiles_behind_tiles_of_sixteen_pairs(types, E, k, H, T):
+    cfg = configs.scaled(IQ3, E=E, top_k=k, H=H, F=256, F_s=512, type_sh_gate_up=types[0], type_sh_down=types[1])
+    _check(cfg, T, prefill=True)
+    raw = configs.make_layer(cfg, device="cuda")
+    tiled, pw, x = MoeWeightsTiled(raw), MoeWeightsPrefill(raw), configs.make_input(cfg, T, device="cuda")
+    sc = MoeScratch(tiled, T)
+    sc.enable_prefill()
+    first = forward_moe_prefill(tiled, pw, sc, x)
+    outs = [torch.empty_like(x) for _ in range(20)]
+    for y in outs:
+        forward_moe_prefill(tiled, pw, sc, x, y)
+    assert all(torch.equal(y, first) for y in outs) and sc.status() == 0
+    # Against the decode entry (K-quant GEMVs behind the routed part), also behind the residual and the norm: the same intermediates, the down rows' 16 sub-blocks
+    # and the k + 1 rows of a token added in another order, i.e. at most 25 roundings of 2^-24 of sums up to twice the row's largest value: 3e-6
+    # of that (3.3e-7 seen; one 8-bit step of an intermediate is 1e-4 and more).
+    norm = torch.ones(H, device="cuda")
+    half = [forward_moe_residual_norm(tiled, sc, x, torch.zeros_like(x), norm, 1e-6, None, p) for p in (pw, None)]
+    for a, b in ((first, forward_moe(tiled, sc, x)), half):
+        assert ((a - b).abs().amax(1) <= 3e-6 * b.abs().amax(1)).all()
+
+
 # weights read packed and weights in operand order in one launch
 @pytest.mark.parametrize("T", [20, 90])
 def test_mixed_operand_forms(T):
@@ -98,8 +124,8 @@ def test_tiled_router_of_short_rows(E, H, T):
     _check(configs.scaled(Q4, E=E, H=H, F=64, F_s=64), T, prefill=False)
 
 
-# The decode entry sends popular experts to the GEMM and the others to the GEMV kernels; a token's row is the same bits either way,
-# whatever the batch: odd numbers of K slices and units, IQ3_S in both places, a shared expert narrower than the routed ones.
+# The decode entry runs pair by pair, on the 16-pair tiles or on the GEMM; a token's row is the same bits on each of them (the first two here,
+# the GEMM in the next test), whatever the batch: odd numbers of K slices and units, IQ3_S in both places, a shared expert narrower than the routed ones.
 @pytest.mark.parametrize("cfg", [configs.scaled(Q4, E=16, F=256, F_s=512, H=2048, name="q4"),
                                  configs.scaled(IQ3, E=16, F=512, F_s=256, H=1024, type_down=configs.IQ3_S, name="iq3"),
                                  configs.scaled(IQ3, E=8, top_k=4, F=320, F_s=0, H=2560, name="iq3 gate, q4 down"),
@@ -219,7 +245,7 @@ def test_prefill_entry_of_a_few_tokens(cfg, T):
     _check(cfg, T, prefill=True)
 
 
-# one or two router rows per CTA: around one CTA per SM, around the row width that takes one row of inputs in pairs
+# one or two router rows per CTA: around one CTA per SM; a single row of inputs is always on pairs of router rows
 @pytest.mark.parametrize("E,T", [(73, 9), (74, 9), (147, 8), (148, 8), (36, 32), (37, 32), (8, 1)])
 @pytest.mark.parametrize("H", [2048, 2176])
 def test_small_router(E, T, H):
@@ -382,6 +408,24 @@ def test_host_rows(T):
         assert torch.equal(y, forward_moe(tiled, sc, -x).cpu())
         rows.neg_()
         assert torch.equal(forward_moe_host(tiled, sc, rows, y), want)
+
+
+# ... with a K-quant shared expert: inside the pair launches (up to five tokens) the result goes straight to pinned memory on any float boundary
+@pytest.mark.parametrize("T", [1, 4, 5, 6])
+def test_host_rows_kquant(T):
+    cfg = configs.scaled(IQ3, E=64, H=1024, F=256, F_s=512, type_sh_gate_up=formats.TYPE_Q5_K, type_sh_down=formats.TYPE_Q5_K)
+    tiled = MoeWeightsTiled(configs.make_layer(cfg, device="cuda"))
+    sc, x = MoeScratch(tiled, T), configs.make_input(cfg, T, device="cuda")
+    want = forward_moe(tiled, sc, x).cpu()
+    for shift in (0, 1, 2, 3, None):
+        room = torch.zeros(T * cfg.H + 4, pin_memory=shift is not None)
+        at = shift or 0
+        y = room[at:at + T * cfg.H].reshape(T, cfg.H)
+        for rows in (x.cpu().pin_memory(), x.cpu()):
+            y.zero_()
+            assert torch.equal(forward_moe_host(tiled, sc, rows, y), want)
+        assert room[:at].abs().sum() == 0 and room[at + T * cfg.H:].abs().sum() == 0
+    assert sc.status() == 0
 
 
 # rows that begin in pinned memory and end outside it are refused before a kernel touches them, on either side of the call
