@@ -16,8 +16,9 @@
 // Sums are bit for bit those of bulk_kernel (gemv_tiled.cu): same K slices, same order.
 //
 // What bounds it.  One to two tokens: three chains per layer (256 IQ3_S / Q4_0 experts, H 2048, F 512, one token, us: router 0.7 behind the wait, logits to
-// experts 1.6 - 2.5, weights and products 2.0, a grid's end to the next one's start 0.8 each time, down stage 3.1).  From eight tokens on: DRAM
-// under the same chains.  Layer, us, against the list and bulk_kernel with its one item per CTA and 7 400 warp instructions per item (here 4 000):
+// experts 1.6 - 2.5, weights and products 2.0, a grid's end to the next one's start 0.8 each time, down stage 3.1).  From eight tokens on the weights'
+// latency under the same chains: with 15 warps per SM (registers) gate/up asks for enough to keep DRAM 41 % busy, down 23 %, and 47 and 37 % of
+// the issue slots are used (captured alone, cold).  Layer, us, against the list and bulk_kernel with its one item per CTA and 7 400 warp instructions per item (here 4 000):
 // 1 token 18.1 -> 13.4, 2: 21.6 -> 15.4, 5: 29.8 -> 23.0, 8: 38.3 -> 30.7, 16: 57.3 -> 47.6, 24: 77.8 -> 65.1.
 #include "common.cuh"
 #include "kernels.h"

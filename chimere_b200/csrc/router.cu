@@ -538,7 +538,7 @@ __device__ __forceinline__ void scan_totals(const RouteParams& p, int32_t* ent_b
 }
 
 // hist[chunk][e] becomes the number of pairs of expert e in earlier chunks.  Many chunks: a warp per expert, a run of consecutive chunks per
-// lane, the CTA that finishes last does the totals (512 chunks: 5 us, where one CTA for all experts takes 24, of one SM's loads).
+// lane, the CTA that finishes last does the totals (512 chunks, the launch alone: 13.6 us, where one CTA for all experts takes 22.5, of one SM's loads).
 constexpr int kScanBatch = 16;
 __global__ void __launch_bounds__(256) dispatch_scan_kernel(const RouteParams p, int32_t* hist, int nchunks) {
     __shared__ int scan[16];
@@ -583,7 +583,7 @@ __global__ void __launch_bounds__(256) dispatch_scan_kernel(const RouteParams p,
     scan_totals(p, ent_base, tid < p.E ? __ldcg(ent_base + tid) : 0, scan);
 }
 // Few chunks: one CTA, thread = (quarter of the chunks, expert), a quarter of up to 16 chunks in registers between the two passes; no counter and
-// no second look at the totals.  Route entry, us, 32 CTAs / one: 256 experts of H = 2048, 512 tokens (32 chunks) 59.4 / 55.0, 1024 (64) 93.0 / 88.2; 200 of
+// no second look at the totals (32 chunks, the launch alone: 9.0 -> 4.2).  Route entry, us, 32 CTAs / one: 256 experts of H = 2048, 512 tokens (32 chunks) 59.4 / 55.0, 1024 (64) 93.0 / 88.2; 200 of
 // H = 1152, 1024: 92.6 / 87.2 (88.9 when this was a launch behind one that counted).
 constexpr int kScanFewChunks = 4 * kScanBatch;
 __global__ void __launch_bounds__(1024) dispatch_scan_few_kernel(const RouteParams p, int32_t* hist, int nchunks) {

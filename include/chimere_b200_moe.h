@@ -115,7 +115,8 @@ typedef struct chimere_moe_workspace {
 /* Bytes of device memory a workspace for up to max_T tokens needs.  A 4-bit layer in the TILED32 layout gets, from the batch size on at
  * which chimere_b200_moe_forward may use the grouped GEMM (41 tokens, 17 where a matrix has more than 2M weights), the GEMM's
  * scratch as well (prefill_arena / prefill_bytes below): for 256 experts of 512 x 2048 21 MB instead of 6 at 64 tokens, 1.2 GB
- * instead of 0.7 at 8192.  It serves the prefill entry too where chimere_b200_moe_prefill_bytes is not larger. */
+ * instead of 0.7 at 8192.  (Layers of one packed type per stage use it there only in large batches, hundreds
+ * of tokens for the widest experts and thousands for these, others from that size on.)  It serves the prefill entry too where chimere_b200_moe_prefill_bytes is not larger. */
 size_t chimere_b200_moe_workspace_bytes(const chimere_moe_layer* w, int max_T);
 
 /* Carve `ws` out of the caller's device arena (`bytes` >= workspace_bytes, 256-byte aligned)
@@ -312,8 +313,8 @@ int chimere_b200_moe_pack_prefill(const chimere_moe_layer* raw, void* d_arena, s
                                   chimere_moe_prefill_weights* out, cudaStream_t stream);
 /* Extra scratch the prefill path needs for up to max_T tokens; pass it with ws->prefill_arena / prefill_bytes. */
 size_t chimere_b200_moe_prefill_bytes(const chimere_moe_layer* w, int max_T);
-/* y = MoE(x) like chimere_b200_moe_forward; `w` TILED32, `pw` what chimere_b200_moe_pack_prefill made of the same layer.  A 4-bit layer
- * of at most five pairs per expert runs on the kernels of chimere_b200_moe_forward. */
+/* y = MoE(x) like chimere_b200_moe_forward; `w` TILED32, `pw` what chimere_b200_moe_pack_prefill made of the same layer.  4-bit routed
+ * experts with at most five pairs each (on average) run on the kernels of chimere_b200_moe_forward. */
 int chimere_b200_moe_forward_prefill(const chimere_moe_layer* w, const chimere_moe_prefill_weights* pw,
                                      const float* d_x, float* d_y, int T, chimere_moe_workspace* ws,
                                      cudaStream_t stream);
