@@ -123,8 +123,8 @@ bool tile_batch(const chimere_moe_layer* w, int T) {
 // Of wide experts the two sides part below that line already, by the routing, which the host does not know: 128 of 1856 x 2688, 66 tokens 308 / 254 uniform and
 // 138 / 133 skewed, 106: 326 / 285 and 160 / 185; 128 of 1536 x 4096, 80: 506 / 431 and 242 / 277; 128 of 2048 x 2048 top 4, 64: 306 / 240 and 103 / 98,
 // 160: 378 / 312 and 157 / 185; 64 of 4096 x 1024, 24: 205 / 169 and 92 / 109.  The line stands for the even routing that such layers are trained to.  (Both launched,
-// and a count of the tiles beyond an expert's first in each one's prologue to say which has work: skewed batches within 5 % of the better side, even ones 10 to
-// 24 us slower for the launches that find nothing to do.)
+// and a count of the tiles beyond an expert's first in each one's prologue to say which has work: skewed batches within 5 % of the better side, even ones 9 to
+// 14 us slower for the launches that find nothing to do.)
 bool prefill_mma(const chimere_moe_layer* w, int T) { return (int64_t)T * w->top_k <= 5 * (int64_t)w->E; }
 
 // Layers that neither takes (experts and shared expert of different packed types, rows too long for the tiles' shared memory), and batches above tile_batch():
